@@ -82,4 +82,37 @@ __device__ __forceinline__ float expf_libm(float x) {
     return k == 0 ? y : scalbnf_dev(y, k);
 }
 
+// expf_libm for x <= 0 (or NaN) without branches, the same bits: the three
+// reduction ranges differ only in k (k = 0 makes hi = x, lo = 0 and scales by
+// 1), the truncation of the negative quotient is a round-up onto the integers
+// at 1.5 * 2^23, and the scaling below 2^-126 takes its extra exact factor by a
+// select.  The lanes of a warp hold values of every range, so expf_libm runs
+// its branches one after another there.
+__device__ __forceinline__ float expf_libm_nonpos(float x) {
+    const float ln2_hi = __uint_as_float(0x3f317200u);
+    const float ln2_lo = __uint_as_float(0x35bfbe8eu);
+    const float inv_ln2 = __uint_as_float(0x3fb8aa3bu);
+    const float p1 = __uint_as_float(0x3e2aaa8fu);
+    const float p2 = __uint_as_float(0xbb355215u);
+    const uint32_t mag = __float_as_uint(x) & 0x7fffffffu;
+    const float on_int = __fadd_ru(__fadd_rn(__fmul_rn(inv_ln2, x), -0.5f), 12582912.0f);
+    const float kf = mag > 0x3f851592u ? __fsub_rn(on_int, 12582912.0f) : (mag > 0x3eb17218u ? -1.0f : 0.0f);
+    int k = mag > 0x3f851592u ? __float_as_int(on_int) - 0x4b400000 : (mag > 0x3eb17218u ? -1 : 0);
+    const float hi = __fsub_rn(x, __fmul_rn(kf, ln2_hi));
+    const float lo = __fmul_rn(kf, ln2_lo);
+    const float r = __fsub_rn(hi, lo);
+    const float rr = __fmul_rn(r, r);
+    const float poly = __fmul_rn(rr, __fadd_rn(p1, __fmul_rn(rr, p2)));
+    const float c = __fsub_rn(r, poly);
+    float q = __fdiv_rn(__fmul_rn(r, c), __fsub_rn(2.0f, c));
+    q = __fadd_rn(__fsub_rn(q, lo), hi);
+    const float y = __fadd_rn(1.0f, q);
+    const float pre = k < -126 ? __uint_as_float(0x0c800000u) : 1.0f;  // 2^-102
+    k += k < -126 ? 102 : 0;
+    float e = __fmul_rn(__fmul_rn(y, pre), __uint_as_float((uint32_t)(0x7f + k) << 23));
+    if (mag <= 0x39000000u) e = __fadd_rn(1.0f, x);
+    if (mag >= 0x42cff1b5u) e = mag > 0x7f800000u ? x : 0.0f;
+    return e;
+}
+
 }  // namespace hm

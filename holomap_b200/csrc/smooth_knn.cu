@@ -4,22 +4,23 @@
 // MIN_K_DIST_SCALE floors), mean at :82-84, and libm::expf reached through
 // src/fmath.rs:119-122.
 //
-// Rows of jobs with k <= 32 take four lanes each (smooth_knn_quad_kernel: the
-// row in registers, exp terms in parallel, the adds in the reference's order),
-// or one thread each when the rows alone fill the device
-// (smooth_knn_row_kernel).  Larger k: one warp per
-// row (of any job).  Lanes evaluate the row's exp terms in parallel; the
-// binary32 partial sum is then formed in the reference's order (j = 1, 2, ...,
-// k-1, each add rounded) by broadcasting the terms, so every lane holds the
-// same psum and all control flow is warp-uniform.  All arithmetic uses
-// explicitly rounded intrinsics and the file is compiled without FMA
-// contraction or flush-to-zero.
+// smooth_rows_kernel (k <= 256): G lanes per row (1 to 16), the row in
+// registers.  sigma is defined by the bisection's steps, and a step only asks
+// on which side of the target the row's sum lies, so most steps are settled
+// without the sum itself: a bracket [A, B] around the root with proven margins
+// answers every step outside it, and the few steps inside evaluate the sum
+// exactly as the reference does.  smooth_knn_kernel: k above 256, one warp per
+// row, every step evaluated.  Every evaluated sum is formed in the reference's
+// order (j = 1, 2, ..., k-1, each binary32 add rounded) with explicitly rounded
+// intrinsics; the file is compiled without FMA contraction or flush-to-zero.
 #include <cuda_runtime.h>
 
 #include "hm_internal.cuh"
 #include "libm_expf.cuh"
 
 namespace hm {
+
+constexpr uint32_t SK_MAX_K = 256;  // widest row of smooth_rows_kernel
 
 // One warp per row of the all-rows space; the row's values are read per
 // 32-element chunk from global memory (L1 resident after the first pass).
@@ -30,7 +31,7 @@ __global__ void __launch_bounds__(256) smooth_knn_kernel(const JobDev *__restric
     const uint32_t ar = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (ar >= rows) return;
     const JobDev &J = jobs[row_starts ? find_job(row_starts, njobs, ar) : 0];
-    if (!J.sigma || !J.rho || J.k <= 32) return;  // k <= 32: the row kernels
+    if (!J.sigma || !J.rho || J.k <= SK_MAX_K) return;  // smooth_rows_kernel's rows
     const uint32_t row = ar - J.arow0, k = J.k;
     const double target = J.target;
     const float *v = J.dist + (size_t)row * k;
@@ -104,154 +105,212 @@ __global__ void __launch_bounds__(256) smooth_knn_kernel(const JobDev *__restric
     }
 }
 
-// One thread per row for k <= KC: the row stays in registers and the whole
-// calibration is the reference's sequential loop, with no shuffles.  Rows of
-// jobs with k > KC are left to smooth_knn_kernel.
-// k <= KC (16 or 32), many rows: one thread per row, the row in registers and
-// the reference's loop as written.
-template <int KC>
-__global__ void __launch_bounds__(128) smooth_knn_row_kernel(const JobDev *__restrict__ jobs, uint32_t njobs,
-                                                             const uint32_t *__restrict__ row_starts,
-                                                             uint32_t rows) {
-    const uint32_t ar = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ar >= rows) return;
-    const JobDev &J = jobs[row_starts ? find_job(row_starts, njobs, ar) : 0];
-    if (!J.sigma || !J.rho || J.k > KC) return;
-    const uint32_t row = ar - J.arow0, k = J.k;
-    const double target = J.target;
-    const float *src = J.dist + (size_t)row * k;
-    float v[KC];
+__device__ __forceinline__ float ex2_approx(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// sum / maximum over the G lanes of a row (every lane of the warp takes part)
+template <int G>
+__device__ __forceinline__ float row_sum(float v) {
 #pragma unroll
-    for (int j = 0; j < KC; ++j) v[j] = (j < (int)k) ? src[j] : 0.0f;
-
-    // rho: first positive distance in row order, else 0 (src/smooth_knn.rs:35)
-    float rh = 0.0f;
-    bool found = false;
+    for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+template <int G>
+__device__ __forceinline__ float row_max(float v) {
 #pragma unroll
-    for (int j = 0; j < KC; ++j) {
-        if (!found && j < (int)k && v[j] > 0.0f) {
-            rh = v[j];
-            found = true;
-        }
-    }
-    // bisection, binary32 state, hi seeded at f32::MAX (src/smooth_knn.rs:39-65)
-    const float f32max = __uint_as_float(0x7f7fffffu);
-    float lo = 0.0f, hi = f32max, mid = 1.0f;
-    for (int it = 0; it < 64; ++it) {
-        float psum = 0.0f;
-#pragma unroll
-        for (int j = 1; j < KC; ++j) {
-            if (j < (int)k) {
-                const float dd = __fsub_rn(v[j], rh);
-                psum = __fadd_rn(psum, (dd > 0.0f) ? expf_libm(-__fdiv_rn(dd, mid)) : 1.0f);
-            }
-        }
-        const double ps = (double)psum;
-        if (fabs(__dsub_rn(ps, target)) < 1e-5) break;
-        if (ps > target) {
-            hi = mid;
-            mid = __fdiv_rn(__fadd_rn(lo, hi), 2.0f);
-        } else {
-            lo = mid;
-            if (hi >= f32max)
-                mid = __fmul_rn(mid, 2.0f);
-            else
-                mid = __fdiv_rn(__fadd_rn(lo, hi), 2.0f);
-        }
-    }
-    float sg = mid;
-    if (rh > 0.0f) {
-        // floor = 1e-3 * mean(row), mean = f32(sequential f64 sum / k)
-        double s = 0.0;
-#pragma unroll
-        for (int j = 0; j < KC; ++j)
-            if (j < (int)k) s = __dadd_rn(s, (double)v[j]);
-        const float floor_v = __fmul_rn(1e-3f, __double2float_rn(__ddiv_rn(s, (double)k)));
-        if (sg < floor_v) sg = floor_v;
-    } else {
-        // floored later with the job's global mean (mean_all_floor_kernel)
-        const uint32_t slot = atomicAdd(&J.cnt->zero_count, 1u);
-        J.zero_rows[slot] = row;
-    }
-    J.sigma[row] = sg;
-    J.rho[row] = rh;
+    for (int o = G / 2; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
 }
 
-// k <= KC (16 or 32): four lanes per row.  Lane q of a row holds the row's
-// values j = 4 i + q and evaluates their exp terms; every lane then forms the
-// binary32 partial sum in the reference's order (j = 1, ..., k - 1, each add
-// rounded) from the four lanes' terms, so the four lanes hold the same psum
-// and take the same branches (shuffles stay within the row's lanes).
-template <int KC>
-__global__ void __launch_bounds__(128) smooth_knn_quad_kernel(const JobDev *__restrict__ jobs, uint32_t njobs,
-                                                              const uint32_t *__restrict__ row_starts,
-                                                              uint32_t rows) {
-    constexpr int NV = KC / 4;
-    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t ar = tid >> 2, q = tid & 3;
-    if (ar >= rows) return;  // the row's four lanes leave together
+// Rows with k_lo < k <= G * NV: lane q of a row holds its values j = G i + q.
+//
+// With gaps g_j = max(d_j - rho, 0) the row's sum S(mid) = sum_j exp(-g_j / mid)
+// is nondecreasing in mid.  Near the target T the reference's binary32 sum psum
+// and the quick sum S~ (ex2.approx, any order) lie within
+//   |psum - S| <= (k + 2) 2^-24 (T + 1)  (k - 1 rounded adds)
+//               + k 2^-23                (the rounded quotient and expf)
+//   |S~ - S|   <= 1.3 k 2^-22            (ex2.approx and its rounded argument)
+//               + 32 2^-24 (T + 1)       (at most 32 adds a lane and the tree)
+// and M is the break tolerance 1e-5 plus 1.1 times their sum.  So S~(B) >= T + M
+// proves psum > T + 1e-5 at every mid >= B, S~(A) <= T - M proves psum < T - 1e-5
+// at every mid <= A, and the bisection's steps outside (A, B) need no evaluation.
+// A and B come from Newton's iteration on c = 1 / mid, where S is convex and
+// decreasing: from c = 0 it approaches the root from one side, in 5 to 8 cheap
+// evaluations (one ex2 and two multiply-adds a value, no order to keep).  About
+// 3 of the bisection's 19 to 40 steps then remain to be evaluated.  Rows outside
+// the premises (an infinite gap, gaps beyond 1e+-20) keep A = 0, B = inf: every
+// step is evaluated.
+//
+// What bounds it: instruction issue of the evaluated expf terms and the latency
+// of their ordered sum.  Whole calibration, every step evaluated before -> now:
+// 1,000 x 15 43 -> 14 us, 50,000 x 30 162 -> 41 us, 150,001 x 15 149 -> 45 us,
+// 10,000 x 100 285 -> 45 us.
+template <int G, int NV>
+__global__ void __launch_bounds__(128, G == 1 ? 4 : 6) smooth_rows_kernel(const JobDev *__restrict__ jobs, uint32_t njobs,
+                                                          const uint32_t *__restrict__ row_starts, uint32_t rows,
+                                                          uint32_t k_lo) {
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr float PAD = 1e30f;  // gap of the positions that are not summed: exp(-PAD c) = 0
+    const int lane = threadIdx.x & 31;
+    const uint32_t q = threadIdx.x & (G - 1);
+    const uint32_t at = (blockIdx.x * blockDim.x + threadIdx.x) / G;
+    const uint32_t ar = min(at, rows - 1);  // lanes past the last row idle along
     const JobDev &J = jobs[row_starts ? find_job(row_starts, njobs, ar) : 0];
-    if (!J.sigma || !J.rho || J.k > KC) return;
-    const unsigned gmask = 0xfu << (threadIdx.x & 28u);
-    const uint32_t row = ar - J.arow0, k = J.k;
-    const double target = J.target;
+    const uint32_t k = J.k;
+    const bool mine = at < rows && J.sigma && J.rho && k > k_lo && k <= (uint32_t)(G * NV);
+    if (!__any_sync(FULL, mine)) return;
+    const uint32_t row = ar - J.arow0;
     const float *src = J.dist + (size_t)row * k;
-    float v[NV];
+    float g[NV];  // the values, then the gaps
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-        const uint32_t j = 4 * i + q;
-        v[i] = j < k ? src[j] : 0.0f;
+        const uint32_t j = i * G + q;
+        g[i] = mine && j < k ? src[j] : 0.0f;
     }
-    // value j of the row, from the lane that holds it
-    auto at = [&](int j) { return __shfl_sync(gmask, v[j >> 2], j & 3, 4); };
-
     // rho: first positive distance in row order, else 0 (src/smooth_knn.rs:35)
-    float rh = 0.0f;
+    float rh = 0.0f, abs_sum = 0.0f;
+    bool found = false;
 #pragma unroll
-    for (int j = 0; j < KC; ++j) {
-        const float x = at(j);
-        if (rh == 0.0f && j < (int)k && x > 0.0f) rh = x;
+    for (int i = 0; i < NV; ++i) {
+        abs_sum += fabsf(g[i]);
+        if (G == 1) {
+            if (!found && g[i] > 0.0f) {
+                rh = g[i];
+                found = true;
+            }
+        } else {
+            const unsigned m = (__ballot_sync(FULL, g[i] > 0.0f) >> (lane & ~(G - 1))) & ((1u << G) - 1u);
+            const float x = __shfl_sync(FULL, g[i], m ? __ffs(m) - 1 : 0, G);
+            if (!found && m) {
+                rh = x;
+                found = true;
+            }
+        }
     }
+    abs_sum = row_sum<G>(abs_sum);
+    float zeros = 0.0f, slope = 0.0f, gmax = 0.0f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const uint32_t j = i * G + q;
+        const float dd = __fsub_rn(g[i], rh);
+        const bool summed = mine && j >= 1 && j < k;
+        g[i] = !summed ? PAD : (dd > 0.0f ? dd : 0.0f);
+        if (summed) {
+            zeros += g[i] == 0.0f ? 1.0f : 0.0f;
+            slope += g[i];
+            gmax = fmaxf(gmax, g[i]);
+        }
+    }
+    zeros = row_sum<G>(zeros);
+    slope = row_sum<G>(slope);
+    gmax = row_max<G>(gmax);
+
+    // the bracket
+    const double target = J.target;
+    const float T = (float)target, kf = (float)k;
+    const float M = 1e-5f + 1.1f * 0x1p-22f * ((0.25f * kf + 8.0f) * (T + 1.0f) + 1.8f * kf);
+    const float L2E = 1.44269504f;
+    float A = 0.0f, B = __uint_as_float(0x7f800000u);
+    const bool newton = mine && k >= 3 && gmax <= 1e20f && gmax >= 1e-20f && zeros < T - M;
+    if (zeros >= T + M) B = 0.0f;  // the zero gaps alone exceed the target at every mid
+    if (__any_sync(FULL, newton)) {
+        float f = kf - 1.0f - T, c = newton ? __fdividef(f, slope) : 1.0f;
+        auto eval = [&](float cc, float &S, float &D) {
+            const float l = cc * L2E;
+            S = 0.0f;
+            D = 0.0f;
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {
+                const float e = ex2_approx(-g[i] * l);
+                S += e;
+                D += g[i] * e;
+            }
+            S = row_sum<G>(S);
+            D = row_sum<G>(D);
+        };
+        float S, D;
+        for (int it = 0; it < 16; ++it) {
+            eval(c, S, D);
+            f = S - T;
+            const bool more = newton && f > M;
+            if (!__any_sync(FULL, more)) break;
+            if (more) c += __fdividef(f, D);
+        }
+        const float cb = c - __fdividef(1.1f * M - f, D), ca = c + __fdividef(1.1f * M + f, D);
+        eval(cb, S, D);
+        if (newton && cb > 0.0f && S >= T + M) B = __fdiv_rn(1.0f, cb);
+        eval(ca, S, D);
+        if (newton && ca < 1e30f && S <= T - M) A = __fdiv_rn(1.0f, ca);
+    }
+
     // bisection, binary32 state, hi seeded at f32::MAX (src/smooth_knn.rs:39-65)
     const float f32max = __uint_as_float(0x7f7fffffu);
     float lo = 0.0f, hi = f32max, mid = 1.0f;
-    for (int it = 0; it < 64; ++it) {
-        float term[NV];
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            const float dd = __fsub_rn(v[i], rh);
-            term[i] = (dd > 0.0f) ? expf_libm(-__fdiv_rn(dd, mid)) : 1.0f;
-        }
-        float psum = 0.0f;
-#pragma unroll
-        for (int j = 1; j < KC; ++j) {
-            const float t = __shfl_sync(gmask, term[j >> 2], j & 3, 4);
-            if (j < (int)k) psum = __fadd_rn(psum, t);
-        }
-        const double ps = (double)psum;
-        if (fabs(__dsub_rn(ps, target)) < 1e-5) break;
-        if (ps > target) {
+    auto advance = [&](bool over) {
+        if (over) {
             hi = mid;
-            mid = __fdiv_rn(__fadd_rn(lo, hi), 2.0f);
+            mid = __fmul_rn(__fadd_rn(lo, hi), 0.5f);  // halving rounds as dividing by 2 does
         } else {
             lo = mid;
-            if (hi >= f32max)
-                mid = __fmul_rn(mid, 2.0f);
-            else
-                mid = __fdiv_rn(__fadd_rn(lo, hi), 2.0f);
+            mid = hi >= f32max ? __fmul_rn(mid, 2.0f) : __fmul_rn(__fadd_rn(lo, hi), 0.5f);
+        }
+    };
+    int it = mine ? 0 : 64;
+    for (;;) {
+        while (it < 64 && (mid <= A || mid >= B)) {
+            advance(mid >= B);
+            ++it;
+        }
+        __syncwarp();
+        if (!__any_sync(FULL, it < 64)) break;
+        float psum = 0.0f;
+        // gap / mid rounded to binary32: a quotient of two 24-bit numbers lies at
+        // least 2^-49 (relative) from every rounding boundary, and the product
+        // with the binary64 reciprocal is within 2^-52 of it (below 2^-126, where
+        // that fails, exp of either rounding is 1)
+        const double inv = __ddiv_rn(1.0, (double)mid);
+        auto term_of = [&](float gap) {
+            const float e = expf_libm_nonpos(-__double2float_rn(__dmul_rn((double)gap, inv)));
+            return gap > 0.0f ? e : 1.0f;
+        };
+        if (G == 1) {
+#pragma unroll
+            for (int j = 1; j < NV; ++j) {
+                const float t = term_of(g[j]);
+                psum = __fadd_rn(psum, j < (int)k ? t : 0.0f);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {
+                // positions that are not summed add +0, which changes nothing
+                const float t_i = term_of(g[i]), term = i * G + q < k ? t_i : 0.0f;
+#pragma unroll
+                for (int s = i == 0 ? 1 : 0; s < G; ++s) psum = __fadd_rn(psum, __shfl_sync(FULL, term, s, G));
+            }
+        }
+        if (it < 64) {
+            const double ps = (double)psum;
+            if (fabs(__dsub_rn(ps, target)) < 1e-5) {
+                it = 64;
+            } else {
+                advance(ps > target);
+                ++it;
+            }
         }
     }
+    if (!mine) return;
     float sg = mid;
     if (rh > 0.0f) {
-        // floor = 1e-3 * mean(row), mean = f32(sequential f64 sum / k)
-        double s = 0.0;
-#pragma unroll
-        for (int j = 0; j < KC; ++j) {
-            const float x = at(j);
-            if (j < (int)k) s = __dadd_rn(s, (double)x);
+        // floor = 1e-3 * mean(row), mean = f32(sequential f64 sum / k); formed
+        // only where the row's mean magnitude allows it to matter
+        if (q == 0 && !(sg >= 1.001e-3f * __fdividef(abs_sum, kf))) {
+            double s = 0.0;
+            for (uint32_t j = 0; j < k; ++j) s = __dadd_rn(s, (double)src[j]);
+            const float floor_v = __fmul_rn(1e-3f, __double2float_rn(__ddiv_rn(s, (double)k)));
+            if (sg < floor_v) sg = floor_v;
         }
-        const float floor_v = __fmul_rn(1e-3f, __double2float_rn(__ddiv_rn(s, (double)k)));
-        if (sg < floor_v) sg = floor_v;
     } else if (q == 0) {
         // floored later with the job's global mean (mean_all_floor_kernel)
         const uint32_t slot = atomicAdd(&J.cnt->zero_count, 1u);
@@ -263,27 +322,38 @@ __global__ void __launch_bounds__(128) smooth_knn_quad_kernel(const JobDev *__re
     }
 }
 
+template <int G, int NV>
+static int launch_rows(const JobDev *jobs, uint32_t njobs, const uint32_t *row_starts, uint32_t rows, uint32_t k_lo,
+                       cudaStream_t s) {
+    constexpr uint32_t per_block = 128 / G;
+    smooth_rows_kernel<G, NV><<<(rows + per_block - 1) / per_block, 128, 0, s>>>(jobs, njobs, row_starts, rows, k_lo);
+    HM_CUDA_TRY(cudaGetLastError());
+    count_launch();
+    return HM_OK;
+}
+
 int launch_smooth(const JobDev *jobs, uint32_t njobs, const uint32_t *row_starts, uint32_t rows,
                   uint32_t kmax, cudaStream_t s) {
     ScopedKernelTimer timer(HM_KCLASS_SMOOTH, s);
-    // every job with k <= 32 (the kernel returns for rows of larger k)
-    // four lanes per row unless the rows alone fill the device (then the
-    // extra lanes' shuffles cost more than the shorter exp chains save)
-    const bool quad = rows < (1u << 17);
+    // Lanes per row: more shorten a row's chain, fewer waste less on shuffles
+    // and on waiting for the warp's slowest row.  Measured (whole calibration):
+    // k = 15: 5,003 rows 8 lanes 16.4 us, 4 lanes 18.5, 1 lane 22.6; 20,000 rows
+    // 20.5 / 18.5 / 20.6; 50,000 rows 34.7 / 28.7 / 24.6.  k = 30: 50,000 rows
+    // 45.1 / 41.0 / 66.2.  k = 100, 10,000 rows: 16 lanes 45.0, 32 lanes 49.4.
     if (kmax <= 16) {
-        if (quad)
-            smooth_knn_quad_kernel<16><<<(rows + 31) / 32, 128, 0, s>>>(jobs, njobs, row_starts, rows);
-        else
-            smooth_knn_row_kernel<16><<<(rows + 127) / 128, 128, 0, s>>>(jobs, njobs, row_starts, rows);
-    } else {
-        if (quad)
-            smooth_knn_quad_kernel<32><<<(rows + 31) / 32, 128, 0, s>>>(jobs, njobs, row_starts, rows);
-        else
-            smooth_knn_row_kernel<32><<<(rows + 127) / 128, 128, 0, s>>>(jobs, njobs, row_starts, rows);
+        if (rows < 16384) HM_TRY((launch_rows<8, 2>(jobs, njobs, row_starts, rows, 0, s)));
+        else if (rows < 32768) HM_TRY((launch_rows<4, 4>(jobs, njobs, row_starts, rows, 0, s)));
+        else HM_TRY((launch_rows<1, 16>(jobs, njobs, row_starts, rows, 0, s)));
+    } else if (kmax <= 32 || njobs > 1) {
+        if (rows < 16384) HM_TRY((launch_rows<8, 4>(jobs, njobs, row_starts, rows, 0, s)));
+        else HM_TRY((launch_rows<4, 8>(jobs, njobs, row_starts, rows, 0, s)));
     }
-    HM_CUDA_TRY(cudaGetLastError());
-    count_launch();
-    if (kmax > 32) {  // rows of jobs with k > 32, one warp per row
+    if (kmax > 32 && !(njobs == 1 && kmax > SK_MAX_K)) {
+        if (kmax <= 64) HM_TRY((launch_rows<16, 4>(jobs, njobs, row_starts, rows, 32, s)));
+        else if (kmax <= 128) HM_TRY((launch_rows<16, 8>(jobs, njobs, row_starts, rows, 32, s)));
+        else HM_TRY((launch_rows<16, 16>(jobs, njobs, row_starts, rows, 32, s)));
+    }
+    if (kmax > SK_MAX_K) {
         smooth_knn_kernel<<<(int)((rows + 7) / 8), 256, 0, s>>>(jobs, njobs, row_starts, rows);
         HM_CUDA_TRY(cudaGetLastError());
         count_launch();
