@@ -201,3 +201,41 @@ def test_device_entry_points_on_a_stream(oracle):
     ref = hm.smallest_eigenpairs(graph_of(r, c, v, n), 3)
     assert_same_bytes(vals.view(np.uint64), ref.values.view(np.uint64), "values")
     assert_same_bytes(vecs.view(np.uint64), ref.vectors.reshape(-1).view(np.uint64), "vectors")
+
+
+def expander(n, degree, hub, seed):
+    """A symmetric graph with a spectral gap: every node joined to `degree`
+    random others (node 0, if `hub`, to a quarter of all), hashed weights."""
+    g = np.random.default_rng(seed)
+    a = np.repeat(np.arange(n), degree)
+    b = g.integers(0, n, a.size)
+    if hub:
+        b = np.concatenate([b, np.arange(1, n, 4)])
+        a = np.concatenate([a, np.zeros(b.size - a.size, dtype=a.dtype)])
+    keep = a != b
+    lo, hi = np.minimum(a[keep], b[keep]), np.maximum(a[keep], b[keep])
+    key = np.unique(lo.astype(np.int64) * n + hi)
+    lo, hi = key // n, key % n
+    w = (0.5 + (key % 101) / 101.0).astype(np.float32)
+    r, c, v = np.concatenate([lo, hi]), np.concatenate([hi, lo]), np.concatenate([w, w])
+    o = np.lexsort((c, r))
+    return r[o].astype(np.uint32), c[o].astype(np.uint32), v[o]
+
+
+@pytest.mark.parametrize("n,degree,hub,k", [
+    (65, 4, False, 2),       # a second block of one row
+    (1000, 6, True, 3),      # a hub row of one segment per warp
+    (9473, 5, True, 3),      # hub segments; chunks of 64 and a remainder
+    (3000, 6, False, 40),    # basis partly in global memory, several Ritz launches
+    (80000, 4, True, 2),     # chunks of more rows than one list holds
+])
+def test_eigenpairs_of_expanders(oracle, n, degree, hub, k):
+    """Residuals within ten times the lock tolerance 1e-10 and orthonormal
+    vectors, at the edges of the cooperative Lanczos kernel's work split."""
+    r, c, v = expander(n, degree, hub, seed=n)
+    pairs = hm.smallest_eigenpairs(graph_of(r, c, v, n), k)
+    assert pairs.values.size == k
+    assert abs(pairs.values[0]) < 1e-9  # connected: L has one zero eigenvalue
+    ip, sv, _ = oracle.laplacian(r, c, v, n)
+    eigen_close(oracle, ip, c, sv, pairs, 1e-9)
+    assert np.abs(pairs.vectors @ pairs.vectors.T - np.eye(k)).max() < 1e-9
