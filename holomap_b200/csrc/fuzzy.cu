@@ -7,34 +7,39 @@
 // the rows s whose lists hold r with A[s][r] nonzero.  Each is a set (the
 // indices of a row are distinct), so
 //
-//   1. fuzzy_rows_kernel (one warp per row) computes the strengths (self
-//      skipped; 1 when d - rho <= 0 or sigma == 0, else libm expf(-(d /
-//      sigma)); zeros dropped), orders F_r by rank (the count of smaller
-//      columns), and writes each entry's reverse copy as (key col, value e)
-//      with e its position in the kNN arrays; dropped entries get the key n.
-//   2. A stable radix sort of the reverse copies over the bits of n groups
-//      them by column with ascending e, so each R_r comes out sorted by
-//      source row (CUB onesweep).
-//   3. fuzzy_merge_kernel (one warp per row) binary-searches every element
-//      of F_r in R_r: it finds the partner strength A[c][r], forms the
-//      binary32 t-conorm (v + vt) - v * vt in the reference's order
-//      (src/fuzzy.rs:67-75), and places the element at j + lb - dups_below
-//      (F elements below it, R elements below it, minus those counted in
-//      both).  The row's entry count |F_r| + |R_r| - |F_r and R_r| goes
-//      through an exclusive scan (CUB) to row offsets.
-//   4. fuzzy_write_kernel writes the F elements at their places and every R
-//      element without an F partner at u + lb_F - dups_below (the same rule
-//      seen from the other list), with strength (0 + vt) - 0 * vt.
+//   1. fuzzy_entries_kernel (one thread per kNN entry) computes the strengths
+//      (self skipped; 1 when d - rho <= 0 or sigma == 0, else libm
+//      expf(-(d / sigma)); zeros dropped) and counts each column's arrivals:
+//      the count returned is the entry's slot in R_col.
+//   2. fuzzy_segments_kernel gives every row a segment of k + |R_r| slots (in
+//      any order: one atomic per block).
+//   3. fuzzy_scatter_kernel drops (source, strength) into R_r's slots.
+//   4. fuzzy_union_kernel (one warp per row of at most 128 slots) sorts the
+//      row's F and R entries in registers, forms the binary32 t-conorm
+//      (v + vt) - v * vt of equal columns in the reference's order
+//      (src/fuzzy.rs:67-75) and leaves the sorted row at the front of its
+//      segment; fuzzy_long_kernel does the rows above 128 slots: a warp each up
+//      to 512, a block each beyond.
+//   5. fuzzy_write_kernel (one block per tile of rows) sums the tiles before
+//      it, scans its rows' counts and writes the COO.
 //
 // Strengths lie in [0, 1] (or are NaN) when every sigma is non-negative, and
 // then no fused value of a union coordinate is zero: fl(v * vt) <= min(v,
 // vt) <= max(v, vt) <= fl(v + vt) with one of the inequalities strict, so
 // the difference is positive.  The reference's zero filter after the fusion
-// therefore drops nothing and the union size is the entry count.  Every
-// step is a function of the inputs alone: the output is the reference's,
-// entry for entry.
-#include <cub/cub.cuh>
+// therefore drops nothing and the union size is the entry count.  The slots
+// depend on the order of the atomics, the sorted rows do not: the output is
+// the reference's, entry for entry.
+//
+// What bounds it: latency of the L2-resident arrays and the sorts' issue.  With a
+// radix sort of the reverse copies and binary-search merges -> now: kNN graph of
+// 50,000 x 384 embeddings, k = 30 (2.7 M entries) 180 -> 117 us; random graphs of
+// 50,000 x 15 140 -> 76, 2,000 x 15 62 -> 42, 1,000,000 x 15 2133 -> 1274.  A graph
+// whose rows all share the same 29 neighbours (29 rows of 50,000 entries, one
+// block each) is slower, 151 -> 194 us.
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "hm_internal.cuh"
 #include "libm_expf.cuh"
@@ -42,220 +47,455 @@
 namespace hm {
 
 constexpr unsigned FZ_FULL = 0xffffffffu;
-// bits of the status word the rows kernel sets for inputs outside the
-// precondition (each row's indices distinct and below n)
+// bits of the status word for inputs outside the precondition (each row's
+// indices distinct and below n)
 constexpr uint32_t FZ_BAD_INDEX = 1u, FZ_BAD_DUPLICATE = 2u;
+constexpr uint32_t FZ_SLOT_BITS = 9;                     // slots of a warp-sorted row: 512
+constexpr uint32_t FZ_WARP_SLOTS = 1u << FZ_SLOT_BITS;
+constexpr uint32_t FZ_SHORT_SLOTS = 128;                 // and of the short-row kernel
+constexpr uint32_t FZ_TILES = 1024;                      // write tiles at most
+constexpr uint32_t FZ_TILE_ROWS = 32;                    // and rows per tile at least
+constexpr uint32_t FZ_WINDOW = 1u << 19;                 // columns per pass of the hub kernel
+enum { FZ_ALLOCATED = 0, FZ_HUBS = 1, FZ_BAD = 2, FZ_MIDS = 3, FZ_NEXT = 4, FZ_WORDS = 8 };
+
+struct FuzzyDev {
+    const uint32_t *idx;
+    const float *dist, *sigma, *rho;
+    uint32_t n, k, entries, tile_rows;
+    float *w;           // directed strengths (0: dropped)
+    uint32_t *slot;     // slot of the entry in its column's R list
+    uint32_t *indeg;    // |R_r|
+    uint32_t *seg;      // first slot of row r's segment
+    uint2 *stage;       // segments: (source or column, strength bits)
+    uint32_t *count;    // entries of output row r
+    uint32_t *tile_sum;
+    uint32_t *hub_off;  // output offset of a hub row
+    uint32_t *hubs, *mids;  // rows of more than 512 and of 129 to 512 slots
+    uint32_t *words;    // FZ_*
+};
 
 __device__ __forceinline__ float tconorm(float v, float vt) {
     return __fsub_rn(__fadd_rn(v, vt), __fmul_rn(v, vt));
 }
 
-__global__ void __launch_bounds__(256) fuzzy_rows_kernel(
-    const uint32_t *__restrict__ idx, const float *__restrict__ dist, const float *__restrict__ sigma,
-    const float *__restrict__ rho, uint32_t n, uint32_t k, float *__restrict__ wdir, uint32_t *__restrict__ rkey,
-    uint32_t *__restrict__ rval, uint32_t *__restrict__ fcol, float *__restrict__ fw,
-    uint32_t *__restrict__ fcount, uint32_t *__restrict__ bad) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t r = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (r >= n) return;  // whole warps
-    const uint64_t base = r * k;
-    const float rh = rho[r], sg = sigma[r];
-    uint32_t cnt = 0;
-    for (uint32_t j0 = 0; j0 < k; j0 += 32) {
-        const uint32_t j = j0 + lane;
-        bool valid = false;
-        if (j < k) {
-            const uint32_t col = idx[base + j];
-            float w = 0.0f;
-            if (col >= n) {
-                // outside the precondition: dropped (so every later index
-                // stays in bounds) and reported through the status word
-                atomicOr(bad, FZ_BAD_INDEX);
-            } else if ((uint64_t)col != r) {
-                const float d = __fsub_rn(dist[base + j], rh);
-                w = (d <= 0.0f || sg == 0.0f) ? 1.0f : expf_libm(-__fdiv_rn(d, sg));
-                valid = w != 0.0f;
-            }
-            wdir[base + j] = w;
-            rkey[base + j] = valid ? col : n;
-            rval[base + j] = (uint32_t)(base + j);
-        }
-        cnt += __popc(__ballot_sync(FZ_FULL, valid));
-    }
-    __syncwarp();
-    // rank of each valid column among the row's valid columns (dropped
-    // entries carry the key n, above every column).  Equal columns (outside
-    // the precondition: exact_knn's indices are distinct) rank by position,
-    // so every slot of the row's F list is still written, and are reported.
-    for (uint32_t j0 = 0; j0 < k; j0 += 32) {
-        const uint32_t j = j0 + lane;
-        const uint32_t mine = j < k ? rkey[base + j] : n;
-        uint32_t rank = 0;
-        bool dup = false;
-        for (uint32_t c0 = 0; c0 < k; c0 += 32) {
-            const uint32_t other = c0 + lane < k ? rkey[base + c0 + lane] : n;
+constexpr uint32_t FZ_PER_THREAD = 4;  // entries in flight per thread of the entry kernels
+__global__ void __launch_bounds__(256) fuzzy_entries_kernel(const FuzzyDev D) {
+    const uint32_t e0 = blockIdx.x * 256 * FZ_PER_THREAD + threadIdx.x;
+    uint32_t col[FZ_PER_THREAD], row[FZ_PER_THREAD], slot[FZ_PER_THREAD];
+    float d[FZ_PER_THREAD], sg[FZ_PER_THREAD], w[FZ_PER_THREAD];
 #pragma unroll
-            for (int s = 0; s < 32; ++s) {
-                const uint32_t o = __shfl_sync(FZ_FULL, other, s);
-                const uint32_t pos = c0 + (uint32_t)s;
-                rank += (o < mine || (o == mine && pos < j)) ? 1u : 0u;
-                dup |= o == mine && pos != j;
+    for (uint32_t q = 0; q < FZ_PER_THREAD; ++q) {
+        const uint32_t e = min(e0 + 256 * q, D.entries - 1);
+        row[q] = e / D.k;
+        col[q] = D.idx[e];
+        d[q] = __fsub_rn(D.dist[e], D.rho[row[q]]);
+        sg[q] = D.sigma[row[q]];
+    }
+#pragma unroll
+    for (uint32_t q = 0; q < FZ_PER_THREAD; ++q) {
+        w[q] = 0.0f;
+        slot[q] = 0;
+        if (e0 + 256 * q >= D.entries) continue;
+        if (col[q] >= D.n) {
+            // outside the precondition: dropped (so every later index stays in
+            // bounds) and reported through the status word
+            atomicOr(&D.words[FZ_BAD], FZ_BAD_INDEX);
+        } else if (col[q] != row[q]) {
+            if (!(d[q] <= 0.0f || sg[q] == 0.0f)) {
+                const float x = -__fdiv_rn(d[q], sg[q]);
+                w[q] = x <= 0.0f ? expf_libm_nonpos(x) : expf_libm(x);
+            } else {
+                w[q] = 1.0f;
             }
-        }
-        if (dup && mine < n) atomicOr(bad, FZ_BAD_DUPLICATE);
-        if (mine < n) {
-            fcol[base + rank] = mine;
-            fw[base + rank] = wdir[base + j];
+            if (w[q] != 0.0f) slot[q] = atomicAdd(&D.indeg[col[q]], 1u);
         }
     }
-    if (lane == 0) fcount[r] = cnt;
-}
-
-// first position in [lo, hi) of the sorted array a whose value is >= x
-__device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t *__restrict__ a, uint32_t lo, uint32_t hi,
-                                                    uint32_t x) {
-    while (lo < hi) {
-        const uint32_t mid = lo + ((hi - lo) >> 1);
-        if (a[mid] < x) lo = mid + 1;
-        else hi = mid;
+#pragma unroll
+    for (uint32_t q = 0; q < FZ_PER_THREAD; ++q) {
+        if (e0 + 256 * q >= D.entries) continue;
+        D.w[e0 + 256 * q] = w[q];
+        D.slot[e0 + 256 * q] = slot[q];
     }
-    return lo;
 }
 
-__global__ void __launch_bounds__(256) fuzzy_merge_kernel(
-    const uint32_t *__restrict__ skey, const uint32_t *__restrict__ sval, const float *__restrict__ wdir,
-    uint32_t entries, uint32_t n, uint32_t k, const uint32_t *__restrict__ fcol, float *__restrict__ fw,
-    const uint32_t *__restrict__ fcount, uint32_t *__restrict__ fpos, uint32_t *__restrict__ dpre,
-    uint32_t *__restrict__ rstart, uint32_t *__restrict__ rdups, uint32_t *__restrict__ count) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t r = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (r >= n) return;  // whole warps
-    const uint64_t base = r * k;
-    uint32_t b = 0;
-    if (lane < 2) b = lower_bound_u32(skey, 0, entries, (uint32_t)r + lane);
-    const uint32_t start = __shfl_sync(FZ_FULL, b, 0), end = __shfl_sync(FZ_FULL, b, 1);
-    const uint32_t fc = fcount[r];
-    uint32_t dups = 0;
-    for (uint32_t j0 = 0; j0 < fc; j0 += 32) {
-        const uint32_t j = j0 + lane;
-        bool found = false;
-        uint32_t lb = 0;
-        float v = 0.0f, vt = 0.0f;
-        if (j < fc) {
-            const uint32_t f = fcol[base + j];
-            // R_r is sorted by source row sval / k
-            uint32_t lo = start, hi = end;
-            while (lo < hi) {
-                const uint32_t mid = lo + ((hi - lo) >> 1);
-                if (sval[mid] / k < f) lo = mid + 1;
-                else hi = mid;
+// inclusive scan of v over the warp
+__device__ __forceinline__ uint32_t warp_scan(uint32_t v, uint32_t lane) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(FZ_FULL, v, o);
+        if (lane >= (uint32_t)o) v += y;
+    }
+    return v;
+}
+// exclusive scan of v over a block of 256 threads, its total in `sum`
+__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t *warp_sums, uint32_t &sum) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t incl = warp_scan(v, lane);
+    __syncthreads();
+    if (lane == 31) warp_sums[warp] = incl;
+    __syncthreads();
+    uint32_t before = 0;
+    sum = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < 8; ++q) {
+        before += q < warp ? warp_sums[q] : 0u;
+        sum += warp_sums[q];
+    }
+    return before + incl - v;
+}
+
+__global__ void __launch_bounds__(256) fuzzy_segments_kernel(const FuzzyDev D) {
+    __shared__ uint32_t warp_sums[8], base;
+    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t mine = r < D.n ? D.k + D.indeg[r] : 0u;
+    uint32_t sum;
+    const uint32_t at = block_scan(mine, warp_sums, sum);
+    if (threadIdx.x == 0) base = atomicAdd(&D.words[FZ_ALLOCATED], sum);
+    __syncthreads();
+    if (r < D.n) D.seg[r] = base + at;
+}
+
+__global__ void __launch_bounds__(256) fuzzy_scatter_kernel(const FuzzyDev D) {
+    const uint32_t e0 = blockIdx.x * 256 * FZ_PER_THREAD + threadIdx.x;
+    float w[FZ_PER_THREAD];
+    uint32_t at[FZ_PER_THREAD];
+#pragma unroll
+    for (uint32_t q = 0; q < FZ_PER_THREAD; ++q) {
+        const uint32_t e = min(e0 + 256 * q, D.entries - 1);
+        w[q] = e0 + 256 * q < D.entries ? D.w[e] : 0.0f;
+        at[q] = (w[q] != 0.0f ? D.seg[D.idx[e]] : 0u) + D.k + D.slot[e];
+    }
+#pragma unroll
+    for (uint32_t q = 0; q < FZ_PER_THREAD; ++q)
+        if (w[q] != 0.0f) D.stage[at[q]] = make_uint2((e0 + 256 * q) / D.k, __float_as_uint(w[q]));
+}
+
+// Bitonic sort, ascending, of 32 * NQ keys, element lane * NQ + q in v[q]: strides
+// below NQ stay in the lane.
+template <typename K, int NQ>
+__device__ __forceinline__ void warp_sort(K (&v)[NQ], uint32_t lane) {
+#pragma unroll
+    for (uint32_t size = 2; size <= 32 * NQ; size <<= 1) {
+#pragma unroll
+        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+            if (stride >= NQ) {
+                const uint32_t ls = stride / NQ;
+                const bool keep_min = ((lane & ls) == 0) == ((lane & (size / NQ)) == 0);
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) {
+                    const K o = __shfl_xor_sync(FZ_FULL, v[q], ls);
+                    v[q] = keep_min ? min(v[q], o) : max(v[q], o);
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) {
+                    if (q & stride) continue;
+                    const K a = min(v[q], v[q | stride]), b = max(v[q], v[q | stride]);
+                    const bool up = size < NQ ? (q & size) == 0 : (lane & (size / NQ)) == 0;
+                    v[q] = up ? a : b;
+                    v[q | stride] = up ? b : a;
+                }
             }
-            found = lo < end && sval[lo] / k == f;
-            lb = lo - start;
-            v = fw[base + j];
-            if (found) vt = wdir[sval[lo]];
         }
-        const unsigned ball = __ballot_sync(FZ_FULL, found);
-        const uint32_t before = dups + __popc(ball & ((1u << lane) - 1u));
-        if (j < fc) {
-            fpos[base + j] = j + lb - before;
-            dpre[base + j] = before;
-            fw[base + j] = tconorm(v, vt);
+    }
+}
+
+// A row of at most 32 * NQ slots: keys column << 9 | slot (F slots below k, so an
+// F entry precedes its R partner), strengths in shared memory by slot.
+template <typename K, int NQ>
+__device__ __forceinline__ uint32_t union_row(const FuzzyDev &D, uint32_t r, uint32_t slots, float *w, uint32_t lane) {
+    const uint32_t k = D.k;
+    const uint64_t base = (uint64_t)r * k;
+    uint2 *seg = D.stage + D.seg[r];
+    K v[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const uint32_t e = q * 32 + lane;
+        v[q] = ~(K)0;
+        if (e < k) {
+            const float f = D.w[base + e];
+            if (f != 0.0f) v[q] = (K)D.idx[base + e] << FZ_SLOT_BITS | e;
+            w[e] = f;
+        } else if (e < slots) {
+            const uint2 s = seg[e];
+            v[q] = (K)s.x << FZ_SLOT_BITS | e;
+            w[e] = __uint_as_float(s.y);
         }
-        dups += __popc(ball);
+    }
+    warp_sort<K, NQ>(v, lane);
+    __syncwarp();  // w, and every read of the segment before its first write
+    const K before = __shfl_up_sync(FZ_FULL, v[NQ - 1], 1), after = __shfl_down_sync(FZ_FULL, v[0], 1);
+    auto col = [](K key) { return key >> FZ_SLOT_BITS; };
+    uint32_t keep = 0;
+    bool dup = false;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const bool first = q == 0 && lane == 0;
+        const K prev = q == 0 ? before : v[q - 1];
+        const bool same = !first && col(prev) == col(v[q]);
+        if (v[q] != ~(K)0) {
+            if (!same) keep |= 1u << q;
+            else dup |= ((uint32_t)v[q] & (FZ_WARP_SLOTS - 1)) < k;  // an F entry after another
+        }
+    }
+    if (dup) atomicOr(&D.words[FZ_BAD], FZ_BAD_DUPLICATE);
+    const uint32_t mine = __popc(keep), incl = warp_scan(mine, lane);
+    uint32_t at = incl - mine;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        if (!(keep >> q & 1u)) continue;
+        const K next = q == NQ - 1 ? after : v[q + 1];
+        const bool last = q == NQ - 1 && lane == 31;
+        const uint32_t slot = (uint32_t)v[q] & (FZ_WARP_SLOTS - 1);
+        const float own = w[slot];
+        const bool pair = !last && next != ~(K)0 && col(next) == col(v[q]);
+        const float other = pair ? w[(uint32_t)next & (FZ_WARP_SLOTS - 1)] : 0.0f;
+        const float f = slot < k ? tconorm(own, other) : tconorm(0.0f, own);
+        seg[at++] = make_uint2((uint32_t)col(v[q]), __float_as_uint(f));
+    }
+    return __shfl_sync(FZ_FULL, incl, 31);
+}
+
+// Rows of at most 128 slots (nine in ten at k = 30), one warp each; the others go
+// to the lists of the next kernel, which keeps this one at 32 registers and its
+// blocks even.
+constexpr int FZ_WARPS = 4;
+template <typename K>
+__global__ void __launch_bounds__(FZ_WARPS * 32, sizeof(K) == 4 ? 16 : 8) fuzzy_union_kernel(const FuzzyDev D) {
+    __shared__ float w_all[FZ_WARPS][FZ_SHORT_SLOTS];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t r = blockIdx.x * FZ_WARPS + warp;
+    if (r >= D.n) return;  // whole warps
+    const uint32_t slots = D.k + D.indeg[r];
+    uint32_t count;
+    if (slots <= 64) count = union_row<K, 2>(D, r, slots, w_all[warp], lane);
+    else if (slots <= FZ_SHORT_SLOTS) count = union_row<K, 4>(D, r, slots, w_all[warp], lane);
+    else {
+        if (lane == 0) {
+            if (slots <= FZ_WARP_SLOTS) D.mids[atomicAdd(&D.words[FZ_MIDS], 1u)] = r;
+            else D.hubs[atomicAdd(&D.words[FZ_HUBS], 1u)] = r;
+        }
+        return;
     }
     if (lane == 0) {
-        rstart[r] = start;
-        rdups[r] = dups;
-        count[r] = fc + (end - start) - dups;
+        D.count[r] = count;
+        atomicAdd(&D.tile_sum[r / D.tile_rows], count);
     }
 }
 
-__global__ void __launch_bounds__(256) fuzzy_write_kernel(
-    const uint32_t *__restrict__ skey, const uint32_t *__restrict__ sval, const float *__restrict__ wdir,
-    uint32_t n, uint32_t k, const uint32_t *__restrict__ fcol, const float *__restrict__ fval,
-    const uint32_t *__restrict__ fcount, const uint32_t *__restrict__ fpos, const uint32_t *__restrict__ dpre,
-    const uint32_t *__restrict__ rstart, const uint32_t *__restrict__ rdups, const uint32_t *__restrict__ count,
-    const uint32_t *__restrict__ off, uint32_t *__restrict__ rows, uint32_t *__restrict__ cols,
-    float *__restrict__ vals, unsigned long long *__restrict__ nnz) {
-    const uint64_t entries = (uint64_t)n * k;
-    const uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p == 0) *nnz = (unsigned long long)off[n - 1] + count[n - 1];
-    if (p < entries) {  // F element j of row r
-        const uint32_t r = (uint32_t)(p / k), j = (uint32_t)(p - (uint64_t)r * k);
-        if (j < fcount[r]) {
-            const uint32_t q = off[r] + fpos[p];
-            rows[q] = r;
-            cols[q] = fcol[p];
-            vals[q] = fval[p];
-        }
-    } else if (p < 2 * entries) {  // reverse copy t, an element of R_r
-        const uint32_t t = (uint32_t)(p - entries);
-        const uint32_t r = skey[t];
-        if (r >= n) return;  // dropped entry
-        const uint32_t e = sval[t];
-        const uint32_t s = e / k;
+// Rows of more than 512 slots, one block each (taken in turn): R_r and F_r as
+// bitmaps over the columns (windows of 2^19), whose prefix counts give every
+// entry's place with no sort.  Zero vectors under cosine are at distance 0 from
+// every point, so rows with n entries do occur.  The row is built beside the
+// segments (`out_all`) and copied back, since every window reads the segment.
+// The blocks' warps then take the rows of 129 to 512 slots, one each.
+template <typename K>
+__global__ void __launch_bounds__(1024) fuzzy_long_kernel(const FuzzyDev D, uint2 *out_all) {
+    extern __shared__ uint32_t hub_smem[];
+    __shared__ uint32_t warp_sums[32];
+    const uint32_t words_n = (min(D.n, FZ_WINDOW) + 31) / 32;
+    uint32_t *rbits = hub_smem, *fbits = rbits + words_n, *pre = fbits + words_n;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t hubs = D.words[FZ_HUBS], k = D.k;
+    for (uint32_t h = blockIdx.x; h < hubs; h += gridDim.x) {
+        const uint32_t r = D.hubs[h], rc = D.indeg[r];
         const uint64_t base = (uint64_t)r * k;
-        const uint32_t fc = fcount[r];
-        const uint32_t lbf = lower_bound_u32(fcol + base, 0, fc, s);
-        if (lbf < fc && fcol[base + lbf] == s) return;  // written with its F partner
-        // F elements below s that also lie in R_r
-        const uint32_t dup_below = lbf < fc ? dpre[base + lbf] : rdups[r];
-        const uint32_t q = off[r] + (t - rstart[r]) + lbf - dup_below;
-        rows[q] = r;
-        cols[q] = s;
-        vals[q] = tconorm(0.0f, wdir[e]);
+        uint2 *seg = D.stage + D.seg[r], *out = out_all + D.seg[r];
+        uint32_t total = 0;
+        for (uint32_t c0 = 0; c0 < D.n; c0 += FZ_WINDOW) {
+            const uint32_t c1 = min(D.n - c0, FZ_WINDOW), nw = (c1 + 31) / 32;  // the window's columns, words
+            __syncthreads();
+            for (uint32_t q = tid; q < nw; q += 1024) rbits[q] = fbits[q] = 0u;
+            __syncthreads();
+            for (uint32_t e = tid; e < rc; e += 8 * 1024) {  // eight loads in flight: n arrivals, one block
+                uint32_t c[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) c[q] = e + 1024 * q < rc ? seg[k + e + 1024 * q].x - c0 : ~0u;
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    if (c[q] < c1) atomicOr(&rbits[c[q] >> 5], 1u << (c[q] & 31));
+            }
+            for (uint32_t e = tid; e < k; e += 1024) {
+                const uint32_t c = D.idx[base + e] - c0, bit = 1u << (c & 31);
+                if (D.w[base + e] != 0.0f && c < c1 && (atomicOr(&fbits[c >> 5], bit) & bit))
+                    atomicOr(&D.words[FZ_BAD], FZ_BAD_DUPLICATE);
+            }
+            __syncthreads();
+            uint32_t carry = total;
+            for (uint32_t q0 = 0; q0 < nw; q0 += 1024) {
+                const uint32_t q = q0 + tid, v = q < nw ? __popc(rbits[q] | fbits[q]) : 0u;
+                const uint32_t incl = warp_scan(v, lane);
+                if (lane == 31) warp_sums[warp] = incl;
+                __syncthreads();
+                const uint32_t ws = warp_scan(warp_sums[lane], lane);
+                const uint32_t before = __shfl_sync(FZ_FULL, ws, warp ? warp - 1 : 0);
+                if (q < nw) pre[q] = carry + (warp ? before : 0u) + incl - v;
+                carry += __shfl_sync(FZ_FULL, ws, 31);
+                __syncthreads();
+            }
+            auto place = [&](uint32_t c) {
+                const uint32_t q = c >> 5;
+                return pre[q] + __popc((rbits[q] | fbits[q]) & ((1u << (c & 31)) - 1u));
+            };
+            // R entries; one with an F partner leaves its strength for it
+            for (uint32_t e = tid; e < rc; e += 4 * 1024) {
+                uint2 s[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) s[q] = e + 1024 * q < rc ? seg[k + e + 1024 * q] : make_uint2(~0u, 0u);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const uint32_t c = s[q].x - c0;
+                    if (e + 1024 * q >= rc || c >= c1) continue;
+                    const bool partner = fbits[c >> 5] >> (c & 31) & 1u;
+                    out[place(c)] = make_uint2(
+                        s[q].x, partner ? s[q].y : __float_as_uint(tconorm(0.0f, __uint_as_float(s[q].y))));
+                }
+            }
+            __syncthreads();
+            for (uint32_t e = tid; e < k; e += 1024) {
+                const uint32_t col = D.idx[base + e], c = col - c0;
+                const float v = D.w[base + e];
+                if (v == 0.0f || c >= c1) continue;
+                const uint32_t at = place(c);
+                const float vt = rbits[c >> 5] >> (c & 31) & 1u ? __uint_as_float(out[at].y) : 0.0f;
+                out[at] = make_uint2(col, __float_as_uint(tconorm(v, vt)));
+            }
+            total = carry;
+        }
+        __syncthreads();
+        for (uint32_t e = tid; e < total; e += 4 * 1024) {
+            uint2 s[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (e + 1024 * q < total) s[q] = out[e + 1024 * q];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (e + 1024 * q < total) seg[e + 1024 * q] = s[q];
+        }
+        if (tid == 0) {
+            D.count[r] = total;
+            atomicAdd(&D.tile_sum[r / D.tile_rows], total);
+        }
+    }
+    __syncthreads();
+    float *w = reinterpret_cast<float *>(hub_smem) + warp * FZ_WARP_SLOTS;
+    const uint32_t mids = D.words[FZ_MIDS];
+    for (;;) {  // taken as warps come free: blocks without hubs take most
+        uint32_t i = lane == 0 ? atomicAdd(&D.words[FZ_NEXT], 1u) : 0u;
+        i = __shfl_sync(FZ_FULL, i, 0);
+        if (i >= mids) break;
+        const uint32_t r = D.mids[i], slots = k + D.indeg[r];
+        const uint32_t count = slots <= 256 ? union_row<K, 8>(D, r, slots, w, lane) : union_row<K, 16>(D, r, slots, w, lane);
+        __syncwarp();
+        if (lane == 0) {
+            D.count[r] = count;
+            atomicAdd(&D.tile_sum[r / D.tile_rows], count);
+        }
     }
 }
 
-// bits that hold every value 0..n (the key n marks a dropped entry)
-static int key_bits(uint64_t n) {
-    int b = 1;
-    while (b < 32 && (1ull << b) <= n) ++b;
-    return b;
+// One block per tile of tile_rows rows.
+__global__ void __launch_bounds__(256) fuzzy_write_kernel(const FuzzyDev D, uint32_t tiles, uint32_t *__restrict__ rows,
+                                                          uint32_t *__restrict__ cols, float *__restrict__ vals,
+                                                          unsigned long long *__restrict__ nnz) {
+    __shared__ uint32_t warp_sums[8], off[256], cnt[256], first[256];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tile = blockIdx.x;
+    uint32_t sum = 0;
+    for (uint32_t t = threadIdx.x; t < tile; t += 256) sum += D.tile_sum[t];
+    uint32_t at;
+    block_scan(sum, warp_sums, at);  // at: entries of the tiles before
+    const uint32_t r0 = tile * D.tile_rows, r1 = min(D.n, r0 + D.tile_rows);
+    for (uint32_t b = r0; b < r1; b += 256) {
+        const uint32_t r = b + threadIdx.x, c = r < r1 ? D.count[r] : 0u;
+        first[threadIdx.x] = r < r1 ? D.seg[r] : 0u;
+        uint32_t chunk;
+        const uint32_t before = block_scan(c, warp_sums, chunk);
+        const bool hub = c > FZ_WARP_SLOTS;  // fuzzy_hub_write_kernel's
+        if (hub) D.hub_off[r] = at + before;
+        off[threadIdx.x] = at + before;
+        cnt[threadIdx.x] = hub ? 0u : c;
+        __syncthreads();
+        // two rows a warp, 64 entries of each, loaded before any is stored
+        for (uint32_t q = warp; q < min(256u, r1 - b); q += 16) {
+            const uint32_t q2 = q + 8;
+            const uint32_t c0 = cnt[q], c1 = q2 < 256u ? cnt[q2] : 0u;
+            const uint2 *g0 = D.stage + first[q], *g1 = D.stage + first[q2 < 256u ? q2 : q];
+            for (uint32_t e = lane; e < max(c0, c1); e += 64) {
+                uint2 v[4];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    if (e + 32 * h < c0) v[h] = g0[e + 32 * h];
+                    if (e + 32 * h < c1) v[2 + h] = g1[e + 32 * h];
+                }
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    const uint32_t x = e + 32 * (h & 1), row = h < 2 ? q : q2;
+                    if (x < (h < 2 ? c0 : c1)) {
+                        const uint32_t o = off[row] + x;
+                        rows[o] = b + row;
+                        cols[o] = v[h].x;
+                        vals[o] = __uint_as_float(v[h].y);
+                    }
+                }
+            }
+        }
+        at += chunk;
+        __syncthreads();
+    }
+    if (tile == tiles - 1 && threadIdx.x == 0) *nnz = at;
 }
 
-// Workspace: the directed strengths, the reverse copies (double-buffered
-// for the sort), the ordered F lists and their merge results, per-row
-// counters, and CUB's temporary storage.
+// Rows of more than 512 entries (all of them hubs), each spread over the grid.
+__global__ void __launch_bounds__(256) fuzzy_hub_write_kernel(const FuzzyDev D, uint32_t *__restrict__ rows,
+                                                              uint32_t *__restrict__ cols, float *__restrict__ vals) {
+    const uint32_t hubs = D.words[FZ_HUBS];
+    const uint32_t parts = max(1u, gridDim.x / max(hubs, 1u)), at_once = gridDim.x / parts;  // blocks a row, rows
+    if (blockIdx.x >= parts * at_once) return;
+    for (uint32_t h = blockIdx.x / parts; h < hubs; h += at_once) {
+        const uint32_t r = D.hubs[h], c = D.count[r];
+        if (c <= FZ_WARP_SLOTS) continue;  // many partners: written with the others
+        const uint2 *seg = D.stage + D.seg[r];
+        const uint32_t o = D.hub_off[r];
+        for (uint32_t e = blockIdx.x % parts * 256 + threadIdx.x; e < c; e += parts * 256) {
+            const uint2 s = seg[e];
+            rows[o + e] = r;
+            cols[o + e] = s.x;
+            vals[o + e] = __uint_as_float(s.y);
+        }
+    }
+}
+
+// Workspace.  The hub kernel's output buffer doubles the segments; it is only
+// touched when there are rows of more than 512 slots.
 struct FuzzyLayout {
-    size_t wdir, rk0, rk1, rv0, rv1, fcol, fw, fpos, dpre, fcount, rstart, rdups, count, off, bad, temp,
-        temp_bytes, total;
+    size_t w, slot, stage, hub_out, seg, count, hubs, mids, zeroed, zeroed_bytes, bad, total;
+    uint32_t tiles, tile_rows;
 };
 
 static int fuzzy_layout(uint64_t n, uint32_t k, FuzzyLayout *L) {
     const uint64_t entries = n * k;
     if (n >= 0x7fffffffull || entries > 0x7fffffffull)
         return set_error(HM_ERR_UNSUPPORTED, "n k above 2^31 - 1 entries");
-    size_t sort_bytes = 0, scan_bytes = 0;
-    cub::DoubleBuffer<uint32_t> kb(nullptr, nullptr), vb(nullptr, nullptr);
-    HM_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, kb, vb, (int)entries));
-    HM_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, (uint32_t *)nullptr, (uint32_t *)nullptr,
-                                              (int)n));
     size_t at = 0;
     auto take = [&](size_t bytes) {
         const size_t here = at;
         at = round_up(at + std::max<size_t>(bytes, 1), 256);
         return here;
     };
-    const size_t e4 = entries * 4, n4 = n * 4;
-    L->wdir = take(e4);
-    L->rk0 = take(e4);
-    L->rk1 = take(e4);
-    L->rv0 = take(e4);
-    L->rv1 = take(e4);
-    L->fcol = take(e4);
-    L->fw = take(e4);
-    L->fpos = take(e4);
-    L->dpre = take(e4);
-    L->fcount = take(n4);
-    L->rstart = take(n4);
-    L->rdups = take(n4);
-    L->count = take(n4);
-    L->off = take(n4);
-    L->bad = take(4);
-    L->temp_bytes = std::max(sort_bytes, scan_bytes);
-    L->temp = take(L->temp_bytes);
+    L->tile_rows = (uint32_t)std::max<uint64_t>(FZ_TILE_ROWS, (n + FZ_TILES - 1) / FZ_TILES);
+    L->tiles = (uint32_t)((n + L->tile_rows - 1) / L->tile_rows);
+    L->w = take(entries * 4);
+    L->slot = take(entries * 4);
+    L->stage = take(2 * entries * sizeof(uint2));
+    L->hub_out = take(2 * entries * sizeof(uint2));
+    L->seg = take(n * 4);
+    L->count = take(n * 4);
+    L->hubs = take(n * 4);
+    L->mids = take(n * 4);
+    // cleared at the start of every run: in-degrees, tile sums, words
+    L->zeroed_bytes = (n + FZ_TILES + FZ_WORDS) * 4;
+    L->zeroed = take(L->zeroed_bytes);
+    L->bad = L->zeroed + (n + FZ_TILES + FZ_BAD) * 4;
     L->total = at;
     return HM_OK;
 }
@@ -292,34 +532,59 @@ int hm_fuzzy_graph_device(const uint32_t *d_idx, const float *d_dist, const floa
         return set_error(HM_ERR_INVALID, "workspace must be 256-byte aligned");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     char *ws = static_cast<char *>(d_workspace);
-    auto u32 = [&](size_t o) { return reinterpret_cast<uint32_t *>(ws + o); };
-    auto f32 = [&](size_t o) { return reinterpret_cast<float *>(ws + o); };
-    const uint32_t nn = (uint32_t)n, entries = (uint32_t)(n * k);
-    const unsigned warp_blocks = (unsigned)((n * 32 + 255) / 256);
-    HM_CUDA_TRY(cudaMemsetAsync(ws + L.bad, 0, 4, s));
-    fuzzy_rows_kernel<<<warp_blocks, 256, 0, s>>>(d_idx, d_dist, d_sigma, d_rho, nn, k, f32(L.wdir), u32(L.rk0),
-                                                  u32(L.rv0), u32(L.fcol), f32(L.fw), u32(L.fcount),
-                                                  u32(L.bad));
+    FuzzyDev D{};
+    D.idx = d_idx;
+    D.dist = d_dist;
+    D.sigma = d_sigma;
+    D.rho = d_rho;
+    D.n = (uint32_t)n;
+    D.k = k;
+    D.entries = (uint32_t)(n * k);
+    D.tile_rows = L.tile_rows;
+    D.w = reinterpret_cast<float *>(ws + L.w);
+    D.slot = reinterpret_cast<uint32_t *>(ws + L.slot);
+    D.stage = reinterpret_cast<uint2 *>(ws + L.stage);
+    D.seg = reinterpret_cast<uint32_t *>(ws + L.seg);
+    D.count = reinterpret_cast<uint32_t *>(ws + L.count);
+    D.hubs = reinterpret_cast<uint32_t *>(ws + L.hubs);
+    D.mids = reinterpret_cast<uint32_t *>(ws + L.mids);
+    D.indeg = reinterpret_cast<uint32_t *>(ws + L.zeroed);
+    D.hub_off = D.slot;  // the entries' slots are used up by then
+    D.tile_sum = D.indeg + n;
+    D.words = D.tile_sum + FZ_TILES;
+    const unsigned entry_blocks = (D.entries + 256 * FZ_PER_THREAD - 1) / (256 * FZ_PER_THREAD);
+    HM_CUDA_TRY(cudaMemsetAsync(ws + L.zeroed, 0, L.zeroed_bytes, s));
+    fuzzy_entries_kernel<<<entry_blocks, 256, 0, s>>>(D);
     HM_CUDA_TRY(cudaGetLastError());
-    count_launch();
-    cub::DoubleBuffer<uint32_t> kb(u32(L.rk0), u32(L.rk1)), vb(u32(L.rv0), u32(L.rv1));
-    size_t temp_bytes = L.temp_bytes;
-    HM_CUDA_TRY(cub::DeviceRadixSort::SortPairs(ws + L.temp, temp_bytes, kb, vb, (int)entries, 0, key_bits(n), s));
-    count_launch();
-    fuzzy_merge_kernel<<<warp_blocks, 256, 0, s>>>(kb.Current(), vb.Current(), f32(L.wdir), entries, nn, k,
-                                                   u32(L.fcol), f32(L.fw), u32(L.fcount), u32(L.fpos), u32(L.dpre),
-                                                   u32(L.rstart), u32(L.rdups), u32(L.count));
+    fuzzy_segments_kernel<<<(D.n + 255u) / 256u, 256, 0, s>>>(D);
     HM_CUDA_TRY(cudaGetLastError());
-    count_launch();
-    temp_bytes = L.temp_bytes;
-    HM_CUDA_TRY(cub::DeviceScan::ExclusiveSum(ws + L.temp, temp_bytes, u32(L.count), u32(L.off), (int)n, s));
-    count_launch();
-    fuzzy_write_kernel<<<(unsigned)((2ull * entries + 255) / 256), 256, 0, s>>>(
-        kb.Current(), vb.Current(), f32(L.wdir), nn, k, u32(L.fcol), f32(L.fw), u32(L.fcount), u32(L.fpos),
-        u32(L.dpre), u32(L.rstart), u32(L.rdups), u32(L.count), u32(L.off), d_rows, d_cols, d_vals,
-        reinterpret_cast<unsigned long long *>(d_nnz));
+    fuzzy_scatter_kernel<<<entry_blocks, 256, 0, s>>>(D);
     HM_CUDA_TRY(cudaGetLastError());
-    count_launch();
+    // column and slot share a 32-bit sort key while both fit
+    const bool narrow = n < 1ull << (32 - FZ_SLOT_BITS);
+    const unsigned union_blocks = (D.n + FZ_WARPS - 1) / FZ_WARPS;
+    if (narrow) fuzzy_union_kernel<uint32_t><<<union_blocks, FZ_WARPS * 32, 0, s>>>(D);
+    else fuzzy_union_kernel<unsigned long long><<<union_blocks, FZ_WARPS * 32, 0, s>>>(D);
+    HM_CUDA_TRY(cudaGetLastError());
+    if (n + k > FZ_SHORT_SLOTS) {  // a row's slots: k and at most n - 1 sources
+        const void *kernel = narrow ? (const void *)fuzzy_long_kernel<uint32_t> : (const void *)fuzzy_long_kernel<unsigned long long>;
+        const size_t bitmaps = (size_t)3 * ((std::min(D.n, FZ_WINDOW) + 31) / 32) * 4, rows_w = 32 * FZ_WARP_SLOTS * 4;
+        const size_t smem = std::max(bitmaps, rows_w);
+        HM_TRY(ensure_dynamic_smem(kernel, (int)(3 * FZ_WINDOW / 8)));
+        uint2 *out = reinterpret_cast<uint2 *>(ws + L.hub_out);
+        void *args[] = {&D, &out};
+        HM_CUDA_TRY(cudaLaunchKernel(kernel, dim3(device_sm_count()), dim3(1024), args, smem, s));
+        count_launch();
+    }
+    fuzzy_write_kernel<<<L.tiles, 256, 0, s>>>(D, L.tiles, d_rows, d_cols, d_vals,
+                                               reinterpret_cast<unsigned long long *>(d_nnz));
+    HM_CUDA_TRY(cudaGetLastError());
+    count_launch(5);
+    if (n + k > FZ_WARP_SLOTS) {
+        fuzzy_hub_write_kernel<<<4 * device_sm_count(), 256, 0, s>>>(D, d_rows, d_cols, d_vals);
+        HM_CUDA_TRY(cudaGetLastError());
+        count_launch();
+    }
     return HM_OK;
 }
 

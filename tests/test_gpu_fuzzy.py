@@ -218,3 +218,46 @@ def test_device_entry_point_reports_an_index_not_below_n(oracle):
                                        stream))
     assert lib.hm_fuzzy_graph_status(ws.data_ptr(), n, k, stream) == hm.HM_OK
     assert int(nnz.item()) == r.size
+
+
+def test_rows_at_the_sort_widths(oracle):
+    """Hubs whose k + in-degree sits on and just past 64, 128, 256 and 512
+    slots, the widths of the row kernels (the last one is the hub kernel's)."""
+    n, k = 3000, 9
+    indeg = [64 - k, 65 - k, 128 - k, 129 - k, 256 - k, 257 - k, 512 - k, 513 - k]
+    idx = np.empty((n, k), dtype=np.uint32)
+    for i in range(n):
+        row = [i] + [j for j, m in enumerate(indeg) if 100 <= i < 100 + m and j != i]
+        t = 1
+        while len(row) < k:
+            c = 100 + (i * 7 + t * 13) % (n - 100)
+            if c not in row:
+                row.append(c)
+            t += 1
+        idx[i] = row
+    g = np.random.default_rng(3)
+    dist = np.sort(g.gamma(2.0, 1.0, (n, k)).astype(np.float32), axis=1)
+    dist[:, 0] = 0.0
+    rho = dist[:, 1].copy()
+    out = check(oracle, idx.reshape(-1), dist.reshape(-1), f32(np.full(n, 0.7)), rho, k)
+    # node j < 8 lists no hub, so its row is its own k - 1 entries and its arrivals
+    assert np.bincount(out.rows, minlength=n)[:8].max() >= 513 - k
+
+
+@pytest.mark.parametrize("n,k,hubs", [
+    (600000, 3, 2),          # hub rows of n entries, wider than one bitmap window
+    ((1 << 23) + 3, 2, 0),   # column and slot no longer share a 32-bit sort key
+])
+def test_wide_columns(oracle, n, k, hubs):
+    g = np.random.default_rng(n)
+    i = np.arange(n)
+    idx = np.empty((n, k), dtype=np.uint32)
+    idx[:, 0] = i
+    for j in range(1, k):
+        # (the last columns by name, so that the widest keys occur)
+        idx[:, j] = (n - j) if j <= hubs else (i + 1 + (j - 1) * (n // k) + g.integers(0, n // k - 1, n)) % n
+    dist = np.sort(g.gamma(2.0, 1.0, (n, k)).astype(np.float32), axis=1)
+    dist[:, 0] = 0.0
+    for j in range(1, hubs + 1):  # a hub's own entry for itself would repeat its first
+        idx[n - j, j] = j
+    check(oracle, idx.reshape(-1), dist.reshape(-1), f32(np.ones(n)), dist[:, 1].copy(), k)
