@@ -7,8 +7,8 @@
 // at least k screened values are <= tau1 and the row's k-th smallest screened
 // value tau^ <= tau1.
 //
-// rerank: one warp per 8 consecutive group rows (always of one job: each job's
-// rows start 32-aligned in the group), in three phases.
+// rerank: one warp per 2 or 4 consecutive group rows (always of one job: each
+// job's rows start 32-aligned in the group) in the second of three phases.
 //   1. select, per row: tau^ is recomputed as the k-th smallest screened
 //      value among the emitted candidates (the emission pass wrote every
 //      column with c^ <= tau1 + band, which includes the k smallest), rounded
@@ -38,15 +38,26 @@
 namespace hm {
 
 // One dimension of the reference's accumulation: euclidean (x - y)^2,
-// cosine x * y, each operation rounded to nearest in binary64.
+// cosine x * y, each operation rounded to nearest in binary64.  The product of
+// two widened binary32 values has at most 48 bits, so the cosine's multiply is
+// exact and a fused multiply-add rounds exactly as the reference's add does.
 template <int METRIC>
 __device__ __forceinline__ double step(double acc, double x, double y) {
     if (METRIC == HM_METRIC_EUCLIDEAN) {
         const double diff = __dsub_rn(x, y);
         return __dadd_rn(acc, __dmul_rn(diff, diff));
     }
-    return __dadd_rn(acc, __dmul_rn(x, y));
+    return __fma_rn(x, y, acc);
 }
+
+// x 2^-896, exactly, without the conversion unit: binary32's exponent field is
+// read as binary64's (a zero or subnormal x stays one).  RR_UNSCALE undoes it on
+// the other factor, also exactly (2^128 2^896 is within range).
+__device__ __forceinline__ double widen_scaled(float x) {
+    const uint32_t u = __float_as_uint(x);
+    return __hiloint2double((int)((uint32_t)((int)u >> 3) & 0x8fffffffu), (int)(u << 29));
+}
+constexpr double RR_UNSCALE = 0x1p896;
 
 // Upper bound of the k-th smallest of a warp's `total` keys (at most 32 * NQ;
 // lane l holds keys l, l + 32, ...; absent keys are ~0) that is exact but for
@@ -104,7 +115,6 @@ __device__ __forceinline__ uint32_t kth_of(KeyFn key, uint32_t total, uint32_t k
     return kth_load<16>(key, total, k, lo, lane);
 }
 
-constexpr int RR_ROWS = 8;        // group rows per warp of the exact phase
 constexpr int RR_WARPS = 4;       // warps per block of the exact phase
 constexpr int RR_CBUF = 512;      // emitted candidates a warp stages in shared memory
 constexpr int RS_WARPS = 8;       // rows (warps) per block of the select and top-k phases
@@ -407,13 +417,13 @@ __device__ __forceinline__ unsigned long long pair_key(const JobDev &J, uint32_t
 }
 
 // Phase 2: exact distances of the flat survivor sequence of the warp's rows
-// (group rows gr0 .. gr0 + 7; lane r < 8 holds row r's count in `cnt_l`).
-template <int METRIC>
+// (group rows gr0 .. gr0 + RR_ROWS - 1; lane r < RR_ROWS holds row r's count).
+template <int METRIC, int RR_ROWS>
 __device__ __forceinline__ void exact_pairs(const JobDev &J, const GroupDev &G, uint32_t gr0, uint32_t cnt_l,
                                             RrWarpSmem &sm, int lane) {
     const uint32_t d = J.d;
     const float *__restrict__ x = J.x;
-    // inclusive / exclusive scans of the eight counts (lanes 0-7)
+    // inclusive / exclusive scans of the rows' counts
     uint32_t incl = lane < RR_ROWS ? cnt_l : 0u;
 #pragma unroll
     for (int o = 1; o < RR_ROWS; o <<= 1) {
@@ -498,7 +508,9 @@ __device__ __forceinline__ void exact_pairs(const JobDev &J, const GroupDev &G, 
             cp_async_wait<RR_STAGES - 1>();
             __syncwarp();
             const uint32_t st = c % RR_STAGES;
-            for (uint32_t a = 0; a < nr; ++a) sm.ex.xid[a][lane] = (double)sm.ex.xi[st][a][lane];
+            // cosine: odd dimensions carry the factor of widen_scaled
+            const double unscale = METRIC == HM_METRIC_COSINE && (lane & 1) ? RR_UNSCALE : 1.0;
+            for (uint32_t a = 0; a < nr; ++a) sm.ex.xid[a][lane] = __dmul_rn((double)sm.ex.xi[st][a][lane], unscale);
             __syncwarp();
             const double *xiv = sm.ex.xid[ri];
             const float *xjv = sm.ex.xj[st][lane];
@@ -510,12 +522,14 @@ __device__ __forceinline__ void exact_pairs(const JobDev &J, const GroupDev &G, 
                     const double2 a0 = *reinterpret_cast<const double2 *>(xiv + 4 * q);
                     const double2 a1 = *reinterpret_cast<const double2 *>(xiv + 4 * q + 2);
                     acc = step<METRIC>(acc, a0.x, (double)y.x);
-                    acc = step<METRIC>(acc, a0.y, (double)y.y);
+                    acc = step<METRIC>(acc, a0.y, METRIC == HM_METRIC_COSINE ? widen_scaled(y.y) : (double)y.y);
                     acc = step<METRIC>(acc, a1.x, (double)y.z);
-                    acc = step<METRIC>(acc, a1.y, (double)y.w);
+                    acc = step<METRIC>(acc, a1.y, METRIC == HM_METRIC_COSINE ? widen_scaled(y.w) : (double)y.w);
                 }
             } else {
-                for (uint32_t t = 0; t < tmax; ++t) acc = step<METRIC>(acc, xiv[t], (double)xjv[t]);
+                for (uint32_t t = 0; t < tmax; ++t)
+                    acc = step<METRIC>(acc, xiv[t],
+                                       METRIC == HM_METRIC_COSINE && (t & 1) ? widen_scaled(xjv[t]) : (double)xjv[t]);
             }
             __syncwarp();
         }
@@ -525,23 +539,24 @@ __device__ __forceinline__ void exact_pairs(const JobDev &J, const GroupDev &G, 
     }
 }
 
-// Exact phase: one warp per 8 consecutive group rows (always of one job:
-// each job's rows start 32-aligned in the group).
+// Exact phase: one warp per ROWS consecutive group rows (always of one job: each
+// job's rows start 32-aligned in the group).
+template <int ROWS>
 __global__ void __launch_bounds__(RR_WARPS * 32) rr_exact_kernel(const JobDev *__restrict__ jobs,
                                                                  const GroupDev *__restrict__ Gp) {
     extern __shared__ __align__(16) unsigned char rr_smem_raw[];
     const GroupDev &G = *Gp;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     RrWarpSmem &sm = reinterpret_cast<RrWarpSmem *>(rr_smem_raw)[warp];
-    const uint32_t gr0 = (blockIdx.x * RR_WARPS + warp) * RR_ROWS;
+    const uint32_t gr0 = (blockIdx.x * RR_WARPS + warp) * ROWS;
     if (gr0 >= G.rows) return;
     const JobDev &J = jobs[G.job_ids[find_job(G.row_starts, G.njobs, gr0)]];
-    const uint32_t cnt_l = lane < RR_ROWS ? G.row_cnt[gr0 + lane] : 0u;
+    const uint32_t cnt_l = lane < ROWS && gr0 + lane < G.rows ? G.row_cnt[gr0 + lane] : 0u;
     if (!__any_sync(0xffffffffu, cnt_l != 0)) return;
     if (J.metric == HM_METRIC_EUCLIDEAN)
-        exact_pairs<HM_METRIC_EUCLIDEAN>(J, G, gr0, cnt_l, sm, lane);
+        exact_pairs<HM_METRIC_EUCLIDEAN, ROWS>(J, G, gr0, cnt_l, sm, lane);
     else
-        exact_pairs<HM_METRIC_COSINE>(J, G, gr0, cnt_l, sm, lane);
+        exact_pairs<HM_METRIC_COSINE, ROWS>(J, G, gr0, cnt_l, sm, lane);
 }
 
 // Bitonic sort of 64 keys held two per lane (element lane and 32 + lane),
@@ -801,10 +816,17 @@ int launch_rerank(const JobDev *jobs, const GroupDev &G, const GroupDev *Gd, uin
     }
     HM_CUDA_TRY(cudaGetLastError());
     const size_t ex_smem = (size_t)RR_WARPS * sizeof(RrWarpSmem);
-    const uint32_t warps = (G.rows + RR_ROWS - 1) / RR_ROWS;
-    HM_TRY(ensure_dynamic_smem((const void *)rr_exact_kernel, (int)ex_smem));
-    rr_exact_kernel<<<(int)((warps + RR_WARPS - 1) / RR_WARPS), RR_WARPS * 32, ex_smem, s>>>(jobs, Gd);
-    HM_CUDA_TRY(cudaGetLastError());
+    // Rows per warp: more fill the 32-pair slices better, fewer give more warps
+    // (16 fit an SM).  Measured (this phase, us; 8 / 4 / 2 rows): 3,000 x 64 14 / 9
+    // / 8, 5,003 x 300 with 139 survivors a row 476 / 345 / 245, 8,000 x 128 32 /
+    // 22 / 25, 20,000 x 128 56 / 45 / 50, 50,000 x 384 492 / 453 / 465.
+    const bool few = G.rows < 8000;
+    const uint32_t rpw = few ? 2u : 4u;
+    const void *exact = few ? (const void *)rr_exact_kernel<2> : (const void *)rr_exact_kernel<4>;
+    HM_TRY(ensure_dynamic_smem(exact, (int)ex_smem));
+    void *args[] = {(void *)&jobs, (void *)&Gd};
+    HM_CUDA_TRY(cudaLaunchKernel(exact, dim3((G.rows + rpw * RR_WARPS - 1) / (rpw * RR_WARPS)), dim3(RR_WARPS * 32), args,
+                                 ex_smem, s));
     if (kpl == 1)
         rr_topk_kernel<1><<<rs_blocks, RS_WARPS * 32, 0, s>>>(jobs, Gd);
     else

@@ -258,3 +258,25 @@ def test_batch_escalates_only_the_job_that_needs_it():
     paths = [batch.stats(j).path_used for j in range(2)]
     assert paths[0] == int(hm.KnnPath.SCREEN_BF16X3), paths
     assert paths[1] != int(hm.KnnPath.SCREEN_BF16X3), paths
+
+
+@pytest.mark.parametrize("n", [7999, 8001])
+@pytest.mark.parametrize("metric", ["euclidean", "cosine"])
+@pytest.mark.parametrize("d", [37, 64])
+def test_rerank_of_mixed_magnitudes(oracle, n, metric, d):
+    """The exact rerank on both sides of its change of rows per warp (8,000
+    rows), on rows that mix signed zeros, subnormals, tiny and large values in
+    odd and even dimensions (the cosine's odd dimensions take another exact
+    conversion)."""
+    g = np.random.default_rng(n + d)
+    x = g.normal(size=(n, d)).astype(np.float32)
+    x[::3, ::5] = -0.0
+    x[1::3, 1::4] = np.float32(1e-40) * g.integers(-9, 9, x[1::3, 1::4].shape).astype(np.float32)
+    x[2::5, 3::7] *= np.float32(1e-30)
+    x[::7, 2::9] *= np.float32(64.0)
+    k = 12
+    knn = hm.exact_knn(x, d, k, metric, "screen_bf16x3")
+    for r0 in (0, 4000, n - 96):
+        oi, od = oracle.exact_knn(x, k, metric, rows=(r0, r0 + 96), threads=8)
+        assert_same_bytes(knn.indices.reshape(n, k)[r0:r0 + 96], oi, f"indices {r0}")
+        assert_same_bytes(knn.dists.reshape(n, k)[r0:r0 + 96], od, f"dists {r0}")
