@@ -104,6 +104,7 @@ struct JobPlan {
     uint64_t eslot0 = 0;
     // escalation: the job's split-BF16 copy (clone), or the job a copy is of
     int clone = -1, clone_of = -1;
+    bool shares_cand = false;  // the copy's candidate lists lie in the original's room
 };
 
 struct GroupPlan {
@@ -375,12 +376,19 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
             const double per_list = (double)P.spec.n / ((double)per_part * eparts);
             const double expect = 1.5 * P.spec.k * (2.0 + std::log(std::fmax(1.0, per_list / P.spec.k)));
             P.cap = std::min<uint32_t>(std::max<uint32_t>(pow2ceil((uint32_t)expect), 128), 4096);
-            // an escalation copy runs only where the coarse screen kept most of
-            // the dataset, and its band is about 2^-16 of the norms: the
-            // smallest lists suffice (an overflowing row takes the exact path)
-            if (P.clone_of >= 0) P.cap = 128;
             P.eslot0 = Gp.elists;
             Gp.elists += P.spec.n * (uint64_t)P.elists;
+            if (P.clone_of >= 0) {
+                // an escalation copy takes its original's candidate room (only one
+                // of the two emits; the offset is set with the layout), or, where
+                // its lists would not fit there, the smallest lists of its own (an
+                // overflowing row takes the exact path)
+                const JobPlan &O = B.jobs[P.clone_of];
+                const uint32_t room = O.elists * O.cap / P.elists;
+                P.shares_cand = room >= P.cap;
+                P.cap = P.shares_cand ? std::min<uint32_t>(room, 4096) : 128;
+                if (P.shares_cand) continue;
+            }
             P.cand0 = Gp.cand;
             Gp.cand += P.spec.n * (uint64_t)P.elists * P.cap;
         }
@@ -543,6 +551,12 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
             Gp.off_stage_cnt = take(slots * sizeof(uint32_t));
         }
     }
+    for (JobPlan &P : B.jobs)
+        if (P.shares_cand) {
+            const JobPlan &O = B.jobs[P.clone_of];
+            const int64_t apart = (int64_t)B.groups[O.group].off_cand - (int64_t)B.groups[P.group].off_cand;
+            P.cand0 = (uint64_t)((int64_t)O.cand0 + apart / (int64_t)sizeof(unsigned long long));
+        }
     B.total = off;
     return HM_OK;
 }

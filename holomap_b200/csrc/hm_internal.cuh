@@ -167,6 +167,8 @@ struct JobCounters {
     uint32_t escalate;       // 1: the job's screen was too coarse for its data; its
                              // split-BF16 copy produced the rows (see JobDev::gate)
     uint32_t escalate_rows;  // rows whose band exceeded the escalation share of tau1
+    uint32_t swamped_rows;   // rows with half of their k sampled minima within the band of tau1
+    uint32_t pad0;
     // screen prep maxima (non-negative doubles as bits): |u|, |e|, |r|,
     // |A row|, |B row|, |u|^2, largest centred |x - mu|^2; then zero rows
     unsigned long long maxb[8];

@@ -280,3 +280,31 @@ def test_rerank_of_mixed_magnitudes(oracle, n, metric, d):
         oi, od = oracle.exact_knn(x, k, metric, rows=(r0, r0 + 96), threads=8)
         assert_same_bytes(knn.indices.reshape(n, k)[r0:r0 + 96], oi, f"indices {r0}")
         assert_same_bytes(knn.dists.reshape(n, k)[r0:r0 + 96], od, f"dists {r0}")
+
+
+@pytest.mark.parametrize("sizes", [(5003,), (9000, 4100, 6000)])
+def test_auto_escalates_where_the_band_spans_the_nearest_neighbours(sizes):
+    """Gaussian mixtures under cosine at d = 300: the BF16 band is well below
+    half of the thresholds but spans most of a row's nearest neighbours, so the
+    split-BF16 copies take over, alone and in a batch (whose copies lie in their
+    originals' candidate room); the bytes are the plain path's, no row overflows."""
+    import torch
+    from holomap_b200.device import DeviceBatch
+    from holomap_b200.synth import gaussian_mixture
+    d, k = 300, 15
+    g = np.random.default_rng(11)
+    data = [gaussian_mixture(g, n, d, 12, 4.0, 0.3, 3.0).astype(np.float32) for n in sizes]
+    batch = DeviceBatch([(torch.from_numpy(x).cuda(), k, "cosine") for x in data])
+    batch.run()
+    torch.cuda.synchronize()
+    for j, x in enumerate(data):
+        plain, psm = hm.knn_smooth(x, d, k, "cosine", "plain")
+        idx, dist, sig, rho = batch.result(j)
+        assert_same_bytes(idx.reshape(-1), plain.indices, f"job {j} indices")
+        assert_same_bytes(dist.reshape(-1), plain.dists, f"job {j} dists")
+        assert_same_bytes(sig, psm.sigmas, f"job {j} sigma")
+        assert_same_bytes(rho, psm.rhos, f"job {j} rho")
+        st = batch.stats(j)
+        if hm.autotune_path(x.shape[0], d, k, "cosine", batched=len(sizes) > 1) == hm.KnnPath.SCREEN_BF16:
+            assert st.path_used == int(hm.KnnPath.SCREEN_BF16X3)
+        assert st.overflow_rows == 0
