@@ -7,9 +7,9 @@
 // operand format groups the jobs), lays out every buffer in one workspace
 // and writes the job tables; the run enqueues, on one stream:
 //   init counters + input check + cosine norms        (all jobs)
-//   binary64 copies + exact plain kernel              (exact-path jobs)
+//   exact plain kernel                                (exact-path jobs)
 //   screen prep -> band -> screen -> rerank           (per screen group)
-//   binary64 copies + plain kernel on fallback rows   (screened jobs)
+//   plain kernel on fallback rows                     (screened jobs)
 //   split merge                                       (exact jobs with splits)
 //   smooth-kNN + global-mean floors                   (all jobs with outputs)
 // Validation mirrors src/api.rs:114-145 on exact_knn's own domain.
@@ -89,9 +89,9 @@ static bool screen_capable(uint32_t d, uint32_t k, int metric) {
 struct JobPlan {
     hm_job spec{};
     int path = HM_PATH_PLAIN;
-    uint32_t ldd = 0, n_pad = 0, splits = 1, split_cols = 0, arow0 = 0;
+    uint32_t splits = 1, split_cols = 0, arow0 = 0;
     uint32_t q0 = 0, q1 = 0, rb0 = 0;  // query rows [q0, q1) (a row shard)
-    size_t off_x64 = 0, off_rnorm = 0, off_partial = 0, off_zero_rows = 0, off_ovf = 0;
+    size_t off_rnorm = 0, off_partial = 0, off_zero_rows = 0, off_ovf = 0;
     size_t off_mu = 0, off_csum = 0;
     int group = -1;
     uint32_t row0 = 0, unit0 = 0, kp1 = 0, k_stages = 0, row_blocks = 0, col_tiles = 0;
@@ -142,9 +142,8 @@ struct hm_batch {
     std::vector<uint2> items[3];       // exact-path work per metric
     std::vector<uint32_t> fb_jobs[3];  // screened jobs per metric (fallback rows)
     uint32_t fb_per_job[3] = {1, 1, 1};
-    std::vector<uint32_t> job_blocks;  // prep block offsets
     bool any_plain = false, any_screen = false, any_smooth = false, any_split = false;
-    size_t off_tables = 0, off_jobs = 0, off_counters = 0, off_row_starts = 0, off_job_blocks = 0;
+    size_t off_tables = 0, off_jobs = 0, off_counters = 0, off_row_starts = 0;
     size_t off_items[3] = {}, off_fb[3] = {};
     size_t tables_bytes = 0, tables_used = 0, total = 0;
     // bound state
@@ -167,6 +166,33 @@ static int group_of_path(int path) {
     case HM_PATH_SCREEN_BF16X3: return 2;
     default: return -1;
     }
+}
+
+// Column splits of one exact-path job: the waves of resident CTAs times a split's
+// instructions per warp (8 rows: the tiles' arithmetic and the filling of the
+// rows' lists, k (1 + ln(columns / k)) keys in merges of 32), least over the
+// splits.  More splits even out the last wave, fewer fill fewer lists: 12,007 x 64
+// manhattan, k = 15 (376 row groups, 444 CTAs resident) 1,565 us with the 7 it
+// chooses, 1,602 with 4; 1,000 points take one per 128-column tile.
+static uint32_t plain_splits(const JobPlan &P, uint64_t groups, uint32_t sms) {
+    const hm_job &s = P.spec;
+    const uint32_t tiles = (uint32_t)((s.n + PL_BN - 1) / PL_BN);
+    const int kpl = kpl_for_k(s.k);
+    const double resident = (double)sms * (kpl <= 2 ? 3 : kpl == 4 ? 2 : 1);
+    const double ops = s.metric == HM_METRIC_EUCLIDEAN ? 3 : s.metric == HM_METRIC_MANHATTAN ? 2 : 1;
+    const double tile = s.d * (32 * ops + 12) + 400, merge = 150 + 70 * kpl;
+    double best = 1e300;
+    uint32_t splits = 1;
+    for (uint32_t c = 1; c <= std::min<uint32_t>(32, tiles); ++c) {
+        const double per = std::ceil((double)tiles / c), cols = per * PL_BN;
+        const double fill = 8 * merge * (1 + s.k / 32.0 * (1 + std::log(std::max(1.0, cols / s.k))));
+        const double cost = std::ceil(groups * (double)c / resident) * (per * tile + fill) + 40.0 * c;
+        if (cost < best * 0.999) {
+            best = cost;
+            splits = c;
+        }
+    }
+    return splits;
 }
 
 // `ranges` (optional): 2 per job, the job's query rows [begin, end); every
@@ -244,8 +270,6 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
             return set_error(HM_ERR_INVALID, "a row shard has no smooth-kNN outputs");
         P.q0 = (uint32_t)q0;
         P.q1 = (uint32_t)q1;
-        P.ldd = (uint32_t)round_up(s.d, PL_BK);
-        P.n_pad = (uint32_t)(round_up(s.n, PL_ROW_PAD) + PL_ROW_PAD);
         P.arow0 = B.all_rows;
         B.all_rows += (uint32_t)s.n;
         B.kpl_all = std::max<uint32_t>(B.kpl_all, (uint32_t)kpl_for_k(s.k));
@@ -253,11 +277,10 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
         if (s.sigma_out && s.rho_out) B.any_smooth = true;
         if (path == HM_PATH_PLAIN) plain_groups += (P.q1 + PL_BM - 1) / PL_BM - P.q0 / PL_BM;
     }
-    // column splits of the exact path: about 8 CTAs per SM over the batch, down
-    // to one 128-column tile per split (C1, 1,000 points: 0.147 -> 0.128 ms
-    // against splits of at least two tiles)
+    // column splits of the exact path: a batch takes about 8 CTAs per SM
     uint32_t S = plain_groups ? (uint32_t)((1184 + plain_groups - 1) / plain_groups) : 1;
     S = std::min<uint32_t>(std::max<uint32_t>(S, 1), 32);
+    if (njobs == 1 && plain_groups) S = plain_splits(B.jobs[0], plain_groups, G);
     for (uint32_t j = 0; j < njobs; ++j) {
         JobPlan &P = B.jobs[j];
         const uint64_t n = P.spec.n;
@@ -455,15 +478,6 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
         if (!B.fb_jobs[m].empty())
             B.fb_per_job[m] = std::max<uint32_t>(
                 1, std::min<uint32_t>(64, (uint32_t)((2 * G + B.fb_jobs[m].size() - 1) / B.fb_jobs[m].size())));
-    // prep blocks: about one block per 2048 elements of a job, at most 2048
-    B.job_blocks.assign(njobs + 1, 0);
-    for (uint32_t j = 0; j < njobs; ++j) {
-        const JobPlan &P = B.jobs[j];
-        const uint64_t work = std::max<uint64_t>(P.spec.n * P.spec.d, (uint64_t)P.n_pad * P.ldd);
-        const uint32_t b = (uint32_t)std::min<uint64_t>(2048, std::max<uint64_t>(1, (work + 2047) / 2048));
-        B.job_blocks[j + 1] = B.job_blocks[j] + b;
-    }
-
     // ---------------------------------------------------------- layout
     size_t off = 0;
     auto take = [&](size_t bytes) {
@@ -481,7 +495,6 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
     };
     B.off_jobs = pack(sizeof(JobDev) * njobs);
     B.off_row_starts = pack(sizeof(uint32_t) * (njobs + 1));
-    B.off_job_blocks = pack(sizeof(uint32_t) * (njobs + 1));
     for (int m = 0; m < 3; ++m) {
         B.off_items[m] = pack(sizeof(uint2) * B.items[m].size());
         B.off_fb[m] = pack(sizeof(uint32_t) * B.fb_jobs[m].size());
@@ -504,10 +517,9 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
         JobPlan &P = B.jobs[j];
         const uint64_t n = P.spec.n;
         if (P.clone_of >= 0) {
-            // an escalation copy shares its original's norms, binary64 rows
-            // and overflow list (only one of the two reaches them)
+            // an escalation copy shares its original's norms and overflow list
+            // (only one of the two reaches them)
             const JobPlan &O = B.jobs[P.clone_of];
-            P.off_x64 = O.off_x64;
             P.off_rnorm = O.off_rnorm;
             P.off_zero_rows = O.off_zero_rows;
             P.off_ovf = O.off_ovf;
@@ -515,8 +527,12 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
             P.off_csum = take((size_t)64 * P.spec.d * sizeof(double));
             continue;
         }
-        P.off_x64 = take((size_t)P.n_pad * P.ldd * sizeof(double));  // exact path or fallback rows
-        P.off_rnorm = take((size_t)P.n_pad * sizeof(double));
+        // The plain path's scratch keeps the room of the binary64 copy it once held
+        // (rows padded to 128 and one block more, dimensions to 16): which problems
+        // fit a caller's fixed scratch, the allocation-free entry point's above all,
+        // is part of its contract.
+        if (P.path == HM_PATH_PLAIN) take((round_up(n, 128) + 128) * round_up(P.spec.d, 16) * sizeof(double));
+        P.off_rnorm = take(n * sizeof(double));
         P.off_zero_rows = take(n * sizeof(uint32_t));
         if (P.splits > 1) P.off_partial = take((size_t)P.splits * n * P.spec.k * sizeof(uint64_t));
         if (P.group >= 0) {
@@ -617,10 +633,7 @@ static int bind_batch(hm_batch &B, void *d_ws, size_t bytes, cudaStream_t s) {
                                            (uintptr_t)P.q0 * s.k * sizeof(float));
         J.sigma = (s.sigma_out && s.rho_out) ? s.sigma_out : nullptr;
         J.rho = (s.sigma_out && s.rho_out) ? s.rho_out : nullptr;
-        J.x64 = at<double>(ws, P.off_x64);
         J.rnorm = at<double>(ws, P.off_rnorm);
-        J.ldd = P.ldd;
-        J.n_pad = P.n_pad;
         J.splits = P.splits;
         J.split_cols = P.split_cols;
         J.partial = P.splits > 1 ? at<uint64_t>(ws, P.off_partial) : nullptr;
@@ -663,7 +676,6 @@ static int bind_batch(hm_batch &B, void *d_ws, size_t bytes, cudaStream_t s) {
         row_starts[j + 1] = row_starts[j] + J.n;
     }
     memcpy(host + B.off_row_starts, row_starts.data(), sizeof(uint32_t) * (njobs + 1));
-    memcpy(host + B.off_job_blocks, B.job_blocks.data(), sizeof(uint32_t) * (njobs + 1));
     for (int m = 0; m < 3; ++m) {
         if (!B.items[m].empty())
             memcpy(host + B.off_items[m], B.items[m].data(), sizeof(uint2) * B.items[m].size());
@@ -757,11 +769,8 @@ static int run_batch(hm_batch &B, cudaStream_t s) {
     const uint32_t njobs = (uint32_t)B.jobs.size();
     const JobDev *jobs = at<JobDev>(ws, B.off_jobs);
     const uint32_t *row_starts = at<uint32_t>(ws, B.off_row_starts);
-    const uint32_t *job_blocks = at<uint32_t>(ws, B.off_job_blocks);
-    const uint32_t blocks = B.job_blocks.back();
 
-    HM_TRY(launch_prep_jobs(jobs, njobs, job_blocks, blocks, PREP_CHECK_AND_NORMS, s, row_starts, B.all_rows));
-    if (B.any_plain) HM_TRY(launch_prep_jobs(jobs, njobs, job_blocks, blocks, PREP_X64_EXACT, s));
+    HM_TRY(launch_check(jobs, njobs, row_starts, B.all_rows, s));
     for (int m = 0; m < 3; ++m) {
         if (B.items[m].empty()) continue;
         PlainWork w{};
@@ -794,9 +803,7 @@ static int run_batch(hm_batch &B, cudaStream_t s) {
         HM_TRY(launch_rerank(jobs, Gp.host, Gd, Gp.kpl, Gp.dmax, Gp.metric_mask, s));
     }
     if (B.any_screen) {
-        // exact plain path for the rows the screen could not settle (binary64
-        // copies are built only for jobs that have such rows)
-        HM_TRY(launch_prep_jobs(jobs, njobs, job_blocks, blocks, PREP_X64_FALLBACK, s));
+        // exact plain path for the rows the screen could not settle
         for (int m = 0; m < 3; ++m) {
             if (B.fb_jobs[m].empty()) continue;
             PlainWork w{};

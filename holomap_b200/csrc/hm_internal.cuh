@@ -135,6 +135,41 @@ struct WarpTopK {
         refresh_tau(k, lane);
     }
 
+    // Merge 32 keys, one per lane (absent ones KEY_NONE), into the list: the batch
+    // is sorted (unless it comes so), laid reversed over the list's last 32
+    // places, and the smaller of each pair kept, which leaves the list's KPL * 32
+    // smallest as one bitonic sequence.
+    template <bool SORTED = false>
+    __device__ __forceinline__ void merge32(uint64_t b, uint32_t k, int lane) {
+        if (!SORTED) {
+#pragma unroll
+            for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll
+                for (int stride = size >> 1; stride > 0; stride >>= 1) b = exchange(b, stride, (lane & size) == 0, lane);
+        }
+        const uint64_t rb = shfl_u64(b, 31 - lane);
+        v[KPL - 1] = v[KPL - 1] < rb ? v[KPL - 1] : rb;
+#pragma unroll
+        for (int stride = KPL / 2; stride > 0; stride >>= 1)
+#pragma unroll
+            for (int q = 0; q < KPL; ++q)
+                if (!(q & stride)) {
+                    const uint64_t lo = v[q], hi = v[q | stride];
+                    v[q] = lo < hi ? lo : hi;
+                    v[q | stride] = lo < hi ? hi : lo;
+                }
+#pragma unroll
+        for (int q = 0; q < KPL; ++q)
+#pragma unroll
+            for (int stride = 16; stride > 0; stride >>= 1) v[q] = exchange(v[q], stride, true, lane);
+        refresh_tau(k, lane);
+    }
+    // compare-exchange with lane ^ stride, ascending where `up`
+    static __device__ __forceinline__ uint64_t exchange(uint64_t x, int stride, bool up, int lane) {
+        const uint64_t o = shfl_xor_u64(x, stride);
+        return (((lane & stride) == 0) == up) == (x < o) ? x : o;
+    }
+
     // Offer one key per lane; all lanes' keys below tau are inserted.
     __device__ __forceinline__ void offer(uint64_t key, uint32_t k, int lane) {
         unsigned m = __ballot_sync(0xffffffffu, key < tau);
@@ -184,9 +219,8 @@ struct JobDev {
     uint32_t *idx;              // addressed as idx[row * k] for rows in [q0, q1)
     float *dist, *sigma, *rho;  // sigma / rho null: no smooth-kNN
     // exact path (and the screened path's fallback)
-    double *x64;                 // n_pad x ldd binary64 copy
     double *rnorm;               // sqrt of the sequential sum of squares (cosine)
-    uint32_t ldd, n_pad, splits, split_cols;
+    uint32_t splits, split_cols;
     uint64_t *partial;           // splits x n x k keys (splits > 1)
     // smooth-kNN
     double target;               // log2(k), host platform log2
@@ -254,11 +288,10 @@ int autotune_choice(uint64_t n, uint32_t d, uint32_t k, int metric, uint32_t *se
 bool tuning_escalation();
 
 // ------------------------------------------------------------- plain path
-constexpr int PL_BM = 32;     // rows per CTA (8 warps x 4 rows)
+constexpr int PL_BM = 32;     // rows per CTA (4 warps x 8 rows)
 constexpr int PL_BN = 128;    // columns per tile (32 lanes x 4)
 constexpr int PL_BK = 16;     // dimensions per shared-memory stage
-constexpr int PL_THREADS = 256;
-constexpr int PL_ROW_PAD = 128;  // binary64 copy is padded to this many rows
+constexpr int PL_THREADS = 128;
 
 // Work table of the exact path: item i = (job, group of PL_BM rows, column
 // split); or, in fallback mode, each job's overflow list strided over
@@ -275,15 +308,10 @@ struct PlainWork {
     uint32_t fb_njobs;
 };
 
-// PREP_CHECK_AND_NORMS: zeroes the job counters, checks every input for
-// finiteness and forms the cosine row norms (all rows of every job;
-// row_starts / all_rows: the all-rows space).  PREP_X64_*: the binary64 copy
-// of the points, only for exact-path jobs, or (fallback mode) only for
-// screened jobs whose overflow count is nonzero.
-int launch_prep_jobs(const JobDev *jobs, uint32_t njobs, const uint32_t *job_blocks,
-                     uint32_t total_blocks, int mode, cudaStream_t s, const uint32_t *row_starts = nullptr,
-                     uint32_t all_rows = 0);
-enum { PREP_CHECK_AND_NORMS = 0, PREP_X64_EXACT = 1, PREP_X64_FALLBACK = 2 };
+// Zeroes the job counters, checks every input for finiteness and forms the
+// cosine row norms (all rows of every job; row_starts / all_rows: the all-rows
+// space).
+int launch_check(const JobDev *jobs, uint32_t njobs, const uint32_t *row_starts, uint32_t all_rows, cudaStream_t s);
 
 int launch_plain(const PlainWork &w, int metric, cudaStream_t s);
 // merges split lists of every exact-path job with splits > 1

@@ -13,12 +13,23 @@
 // zero in the padded copy and add an exact +0.0, which leaves a sum that is
 // never -0.0 unchanged.
 //
-// Layout: a CTA owns 32 query rows of one job (8 warps x 4 rows) and walks the
-// columns of its split 128 at a time; every lane computes a 4x4 block of pairs (rows of
-// its warp x columns lane + 32c).  A warp therefore holds all 128 candidate
-// keys of its 4 rows for the tile and feeds them to a warp-distributed sorted
-// top-k list (WarpTopK).  Column splits (grid.y) write partial lists that
-// merge_splits combines.
+// Layout: a CTA owns 32 query rows of one job (4 warps x 8 rows) and walks the
+// columns of its split 128 at a time; every lane computes an 8x4 block of pairs
+// (rows of its warp x columns lane + 32c) from binary64 stages in shared memory,
+// widened once per CTA from the binary32 points.  A pair whose accumulator cannot
+// reach the row's k-th distance is dropped before its square root or quotient;
+// the others are collected 32 at a time and merged into the row's sorted list
+// (WarpTopK::merge32), which lives in shared memory.  Column splits write partial
+// lists that merge_splits combines.
+//
+// What bounds it: the binary64 pipe (3 operations per pair and dimension for
+// euclidean, 2 manhattan, 1 cosine: the product of two widened binary32 values is
+// exact, so the reference's multiply and add are one fused operation).
+// Whole calls, with every key inserted one at a time and a separate binary64 copy
+// of the points -> now: 1,000 x 50, k = 15 89 -> 65 us; 12,007 x 64 manhattan 1,744
+// -> 1,631 us (0.64 of the binary64 rate); 10,000 x 32, k = 100 4,080 -> 1,766 us.
+// Registers limit it to 12 warps an SM; 16 (128 registers, spills) measured 2,489
+// us on the manhattan call, an unroll of 8 or 16 dimensions 1,668 and 1,875.
 #include <cuda_runtime.h>
 
 #include "hm_internal.cuh"
@@ -33,36 +44,13 @@ int kpl_for_k(uint32_t k) {
     return 0;
 }
 
-// ------------------------------------------------------------------ prep
+// ----------------------------------------------------------------- check
 __global__ void init_counters_kernel(JobDev *jobs, uint32_t njobs) {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= njobs) return;
     JobCounters c{};
     c.nonfinite_min = 0xffffffffu;
     *jobs[j].cnt = c;
-}
-
-// Binary64 copies of the points (exact-path jobs, or screened jobs with rows
-// for the exact fallback).  Blocks are dealt to jobs by `job_blocks` (prefix
-// offsets); each job's blocks stride over that job's elements.
-__global__ void __launch_bounds__(256) prep_jobs_kernel(const JobDev *__restrict__ jobs, uint32_t njobs,
-                                                        const uint32_t *__restrict__ job_blocks,
-                                                        int mode) {
-    const uint32_t jb = find_job(job_blocks, njobs, blockIdx.x);
-    const JobDev &J = jobs[jb];
-    const uint32_t lb = blockIdx.x - job_blocks[jb];
-    const uint32_t nb = job_blocks[jb + 1] - job_blocks[jb];
-    const size_t stride = (size_t)nb * blockDim.x;
-    const size_t t0 = (size_t)lb * blockDim.x + threadIdx.x;
-    if (mode == PREP_X64_EXACT && J.path != HM_PATH_PLAIN) return;
-    // (an escalated job's fallback rows come from its copy's rerank: the
-    // original's row list and count, so no activity check here)
-    if (mode == PREP_X64_FALLBACK && (J.path == HM_PATH_PLAIN || J.cnt->ovf_count == 0)) return;
-    const size_t total = (size_t)J.n_pad * J.ldd;
-    for (size_t t = t0; t < total; t += stride) {
-        const size_t r = t / J.ldd, c = t % J.ldd;
-        J.x64[t] = (r < J.n && c < J.d) ? (double)J.x[r * J.d + c] : 0.0;
-    }
 }
 
 // Input check and cosine row norms, one warp per 32 consecutive rows of the
@@ -129,34 +117,22 @@ __global__ void __launch_bounds__(NRM_WARPS * 32) check_norms_kernel(const JobDe
             const uint32_t tmax = min(32u, d - min(d, c0));
             for (uint32_t t = 0; t < tmax; ++t) {
                 const double e = (double)tile[warp][lane][t];
-                acc = __dadd_rn(acc, __dmul_rn(e, e));
+                acc = __fma_rn(e, e, acc);  // e * e is exact
             }
         }
         __syncwarp();
     }
     if (cos) J.rnorm[row] = __dsqrt_rn(acc);
-    // the plain path reads the norms of its padding rows [n, n_pad): zeros
-    if (cos && row == J.n - 1)
-        for (uint32_t r = J.n; r < J.n_pad; ++r) J.rnorm[r] = 0.0;
 }
 
-int launch_prep_jobs(const JobDev *jobs, uint32_t njobs, const uint32_t *job_blocks,
-                     uint32_t total_blocks, int mode, cudaStream_t s, const uint32_t *row_starts,
-                     uint32_t all_rows) {
+int launch_check(const JobDev *jobs, uint32_t njobs, const uint32_t *row_starts, uint32_t all_rows, cudaStream_t s) {
     ScopedKernelTimer timer(HM_KCLASS_PREP, s);
-    if (mode == PREP_CHECK_AND_NORMS) {
-        init_counters_kernel<<<(njobs + 127) / 128, 128, 0, s>>>(const_cast<JobDev *>(jobs), njobs);
-        HM_CUDA_TRY(cudaGetLastError());
-        const uint32_t warps = (all_rows + 31) / 32;
-        check_norms_kernel<<<(warps + NRM_WARPS - 1) / NRM_WARPS, NRM_WARPS * 32, 0, s>>>(jobs, njobs, row_starts,
-                                                                                        all_rows);
-        HM_CUDA_TRY(cudaGetLastError());
-        count_launch(2);
-        return HM_OK;
-    }
-    prep_jobs_kernel<<<total_blocks, 256, 0, s>>>(jobs, njobs, job_blocks, mode);
+    init_counters_kernel<<<(njobs + 127) / 128, 128, 0, s>>>(const_cast<JobDev *>(jobs), njobs);
     HM_CUDA_TRY(cudaGetLastError());
-    count_launch();
+    const uint32_t warps = (all_rows + 31) / 32;
+    check_norms_kernel<<<(warps + NRM_WARPS - 1) / NRM_WARPS, NRM_WARPS * 32, 0, s>>>(jobs, njobs, row_starts, all_rows);
+    HM_CUDA_TRY(cudaGetLastError());
+    count_launch(2);
     return HM_OK;
 }
 
@@ -167,7 +143,7 @@ __device__ __forceinline__ double pair_step(double acc, double a, double b) {
         const double t = __dsub_rn(a, b);
         return __dadd_rn(acc, __dmul_rn(t, t));
     } else if (METRIC == HM_METRIC_COSINE) {
-        return __dadd_rn(acc, __dmul_rn(a, b));
+        return __fma_rn(a, b, acc);  // a * b is exact
     } else {
         return __dadd_rn(acc, fabs(__dsub_rn(a, b)));
     }
@@ -190,12 +166,51 @@ __device__ __forceinline__ float pair_finish(double acc, double rn_a, double rn_
     }
 }
 
-template <int METRIC, int KPL>
-__global__ void __launch_bounds__(PL_THREADS, (KPL <= 2 ? 2 : 1)) plain_knn_kernel(const PlainWork w) {
-    __shared__ double As[2][PL_BM][PL_BK + 1];
-    __shared__ double Bs[2][PL_BN][PL_BK + 1];
-    __shared__ uint32_t s_rows[PL_BM];
+// What a pair's accumulator has to reach for its distance to be at most the row's
+// k-th distance tau, with room for every rounding on the way: a returned distance
+// of at most tau comes from a value of at most up = tau (1 + 2^-21) + 1.5 * 2^-149.
+// Euclidean: acc <= up^2 (1 + 2^-50); manhattan: acc <= up; cosine: acc >=
+// (1 - up - 2^-44) |a| |b|, returned with |a| multiplied in (test it times |b|).
+template <int METRIC>
+__device__ __forceinline__ double pair_limit(uint64_t tau_key, double rn_a) {
+    const float tau = tau_key == KEY_NONE ? __int_as_float(0x7f800000) : key_dist(tau_key);
+    const double up = (double)tau * (1.0 + 0x1p-21) + 1.5 * 0x1p-149;
+    if (METRIC == HM_METRIC_EUCLIDEAN) return up * up * (1.0 + 0x1p-50);
+    if (METRIC == HM_METRIC_COSINE) return fmax(1.0 - up - 0x1p-44, -1e30) * rn_a;
+    return up;
+}
 
+// Shared memory of one CTA.
+template <int KPL>
+struct PlainSmem {
+    double As[2][PL_BM][PL_BK + 1];
+    double Bs[2][PL_BN][PL_BK + 1];
+    uint64_t list[PL_BM][32 * KPL];  // each row's sorted keys
+    uint64_t fresh[PL_BM][64];       // keys waiting to be merged
+    double rn_a[PL_BM];
+    uint32_t rows[PL_BM];            // the query rows (0xffffffff: none)
+};
+
+// Merges the first `have` (at most 32) waiting keys into the row's list; returns
+// its k-th key.
+template <int KPL>
+__device__ __noinline__ uint64_t plain_merge(uint64_t *list, const uint64_t *fresh, uint32_t have, uint32_t k) {
+    const int lane = threadIdx.x & 31;
+    WarpTopK<KPL> top;
+#pragma unroll
+    for (int q = 0; q < KPL; ++q) top.v[q] = list[q * 32 + lane];
+    const uint64_t b = (uint32_t)lane < have ? fresh[lane] : KEY_NONE;
+    top.merge32(b, k, lane);
+#pragma unroll
+    for (int q = 0; q < KPL; ++q) list[q * 32 + lane] = top.v[q];
+    __syncwarp();
+    return top.tau;
+}
+
+template <int METRIC, int KPL>
+__global__ void __launch_bounds__(PL_THREADS, KPL <= 2 ? 3 : 2) plain_knn_kernel(const PlainWork w) {
+    extern __shared__ __align__(16) unsigned char pl_smem_raw[];
+    PlainSmem<KPL> &sm = *reinterpret_cast<PlainSmem<KPL> *>(pl_smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint32_t jb, first_grp, grp_stride, n_groups, split = 0;
     if (!w.fallback) {
@@ -212,12 +227,13 @@ __global__ void __launch_bounds__(PL_THREADS, (KPL <= 2 ? 2 : 1)) plain_knn_kern
         n_groups = (w.jobs[jb].cnt->ovf_count + PL_BM - 1) / PL_BM;
     }
     const JobDev &J = w.jobs[jb];
-    const uint32_t c_begin = split * J.split_cols;
-    const uint32_t c_end = min(J.n, c_begin + J.split_cols);
-    const uint32_t ldd = J.ldd;
+    const uint32_t c_begin = split * J.split_cols, c_end = min(J.n, c_begin + J.split_cols);
+    const uint32_t n = J.n, d = J.d, k = J.k;
+    const float *__restrict__ x = J.x;
+    const bool vec = (d & 3u) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+    const uint32_t nk = (d + PL_BK - 1) / PL_BK, tiles = (c_end - c_begin + PL_BN - 1) / PL_BN, stages = tiles * nk;
 
     for (uint32_t grp = first_grp; grp < n_groups; grp += grp_stride) {
-        // the 32 query rows of this group (0xffffffff: none)
         if (tid < PL_BM) {
             uint32_t r;
             if (w.fallback) {
@@ -227,129 +243,199 @@ __global__ void __launch_bounds__(PL_THREADS, (KPL <= 2 ? 2 : 1)) plain_knn_kern
                 r = grp * PL_BM + tid;
                 if (r < J.q0 || r >= J.q1) r = 0xffffffffu;
             }
-            s_rows[tid] = r;
+            sm.rows[tid] = r;
+            sm.rn_a[tid] = METRIC == HM_METRIC_COSINE && r != 0xffffffffu ? J.rnorm[r] : 0.0;
         }
+        for (uint32_t e = tid; e < PL_BM * 32 * KPL; e += PL_THREADS) sm.list[e / (32 * KPL)][e % (32 * KPL)] = KEY_NONE;
         __syncthreads();
 
-        WarpTopK<KPL> top[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) top[r].reset();
-        uint32_t my_rows[4];
-        double rn_a[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            my_rows[r] = s_rows[warp * 4 + r];
-            rn_a[r] = (METRIC == HM_METRIC_COSINE && my_rows[r] != 0xffffffffu) ? J.rnorm[my_rows[r]] : 0.0;
-        }
-
-        // loads of one stage: A 32x16 (2 per thread), B 128x16 (8 per thread)
-        auto load_stage = [&](int buf, uint32_t col0, uint32_t k0) {
-#pragma unroll
-            for (int p = 0; p < 2; ++p) {
-                const int lin = tid + p * PL_THREADS;
-                const int r = lin >> 4, c = lin & 15;
-                const uint32_t ar = s_rows[r] == 0xffffffffu ? 0u : s_rows[r];
-                const double *src = J.x64 + (size_t)ar * ldd + k0 + c;
-                const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&As[buf][r][c]);
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src));
+        // A stage: 16 dimensions of the 32 rows and of 128 columns, four values a
+        // thread and row: thread t takes row t / 4 (of each 32), dimensions 4 (t % 4)
+        const uint32_t lr = tid >> 2, lc = 4 * (tid & 3);
+        const uint32_t a_row = min(sm.rows[lr], n - 1);  // no row: any valid one
+        float4 nxt[5];
+        auto load = [&](uint32_t row, uint32_t dim) {
+            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (row < n) {
+                const float *src = x + (size_t)row * d + dim;
+                if (vec && dim < d) {
+                    v = *reinterpret_cast<const float4 *>(src);
+                } else {
+                    if (dim < d) v.x = src[0];
+                    if (dim + 1 < d) v.y = src[1];
+                    if (dim + 2 < d) v.z = src[2];
+                    if (dim + 3 < d) v.w = src[3];
+                }
             }
+            return v;
+        };
+        auto fetch = [&](uint32_t col0, uint32_t kt) {
+            nxt[0] = load(a_row, kt * PL_BK + lc);
 #pragma unroll
-            for (int p = 0; p < 8; ++p) {
-                const int lin = tid + p * PL_THREADS;
-                const int r = lin >> 4, c = lin & 15;
-                const double *src = J.x64 + (size_t)(col0 + r) * ldd + k0 + c;
-                const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&Bs[buf][r][c]);
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src));
-            }
-            asm volatile("cp.async.commit_group;\n" ::);
+            for (int p = 0; p < 4; ++p) nxt[1 + p] = load(col0 + lr + 32 * p, kt * PL_BK + lc);
+        };
+        auto put = [&](double *dst, const float4 &v) {
+            dst[0] = (double)v.x;
+            dst[1] = (double)v.y;
+            dst[2] = (double)v.z;
+            dst[3] = (double)v.w;
+        };
+        auto store = [&](int buf) {
+            put(&sm.As[buf][lr][lc], nxt[0]);
+#pragma unroll
+            for (int p = 0; p < 4; ++p) put(&sm.Bs[buf][lr + 32 * p][lc], nxt[1 + p]);
         };
 
-        const uint32_t nk = ldd / PL_BK;
-        for (uint32_t col0 = c_begin; col0 < c_end; col0 += PL_BN) {
-            double acc[4][4];
+        double limit[8];
+        uint32_t have[8];  // waiting keys
 #pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) acc[r][c] = 0.0;
+        for (int r = 0; r < 8; ++r) {
+            limit[r] = pair_limit<METRIC>(KEY_NONE, sm.rn_a[warp * 8 + r]);
+            have[r] = 0;
+        }
+        fetch(c_begin, 0);
+        store(0);
+        __syncthreads();
 
-            load_stage(0, col0, 0);
-            for (uint32_t kt = 0; kt < nk; ++kt) {
-                const int buf = kt & 1;
-                if (kt + 1 < nk) {
-                    load_stage(buf ^ 1, col0, (kt + 1) * PL_BK);
-                    asm volatile("cp.async.wait_group 1;\n" ::);
-                } else {
-                    asm volatile("cp.async.wait_group 0;\n" ::);
+        double acc[8][4];
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[r][c] = 0.0;
+        uint32_t col0 = c_begin, kt = 0;
+        for (uint32_t s = 0; s < stages; ++s) {
+            // the next stage's loads fly while this one is computed
+            const bool last_k = kt + 1 == nk;
+            const uint32_t ncol = last_k ? col0 + PL_BN : col0, nkt = last_k ? 0u : kt + 1;
+            if (s + 1 < stages) fetch(ncol, nkt);
+            const int buf = s & 1;
+            const double(*A)[PL_BK + 1] = &sm.As[buf][warp * 8];
+            const double(*Bm)[PL_BK + 1] = &sm.Bs[buf][lane];
+            const int kmax = (int)min((uint32_t)PL_BK, d - kt * PL_BK);
+#pragma unroll 4
+            for (int kk = 0; kk < kmax; ++kk) {
+                double bv[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) bv[c] = Bm[32 * c][kk];
+#pragma unroll
+                for (int r = 0; r < 8; ++r) {
+                    const double av = A[r][kk];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) acc[r][c] = pair_step<METRIC>(acc[r][c], av, bv[c]);
                 }
-                __syncthreads();
+            }
+            if (last_k) {
+                // The first tile of a short list: the k-th smallest of the lanes' own
+                // minima bounds the row's k-th distance, so the tile is cut to little
+                // more than k pairs before any is merged (cosine's limit is not on
+                // the accumulator alone; its first tile is merged as it comes).
+                if (KPL == 1 && METRIC != HM_METRIC_COSINE && col0 == c_begin) {
 #pragma unroll
-                for (int kk = 0; kk < PL_BK; ++kk) {
-                    double av[4], bv[4];
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) av[r] = As[buf][warp * 4 + r][kk];
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) bv[c] = Bs[buf][lane + 32 * c][kk];
-#pragma unroll
-                    for (int r = 0; r < 4; ++r)
+                    for (int r = 0; r < 8; ++r) {
+                        double mine = __longlong_as_double(0x7ff0000000000000ll);
 #pragma unroll
                         for (int c = 0; c < 4; ++c)
-                            acc[r][c] = pair_step<METRIC>(acc[r][c], av[r], bv[c]);
+                            if (col0 + lane + 32 * c < c_end) mine = fmin(mine, acc[r][c]);
+                        float f = __double2float_ru(mine);
+#pragma unroll
+                        for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll
+                            for (int stride = size >> 1; stride > 0; stride >>= 1) {
+                                const float o = __shfl_xor_sync(0xffffffffu, f, stride);
+                                f = ((lane & stride) == 0) == ((lane & size) == 0) ? fminf(f, o) : fmaxf(f, o);
+                            }
+                        const double t = (double)__shfl_sync(0xffffffffu, f, (int)k - 1);
+                        const float dist = pair_finish<METRIC>(t, 0.0, 0.0);
+                        limit[r] = pair_limit<METRIC>(make_key(dist, 0), 0.0);
+                    }
                 }
-                __syncthreads();
-            }
-
-            // finish the 16 pairs and feed the keys to the rows' lists
-            double rn_b[4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-                rn_b[c] = (METRIC == HM_METRIC_COSINE) ? J.rnorm[col0 + lane + 32 * c] : 0.0;
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
+                // pairs that may enter a row's list wait in `fresh`
+                double rn_b[4];
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     const uint32_t col = col0 + lane + 32 * c;
-                    float dist = pair_finish<METRIC>(acc[r][c], rn_a[r], rn_b[c]);
-                    if (col == my_rows[r]) dist = 0.0f;  // src/knn.rs:38-39
-                    const uint64_t key = (col < c_end) ? make_key(dist, col) : KEY_NONE;
-                    top[r].offer(key, J.k, lane);
+                    rn_b[c] = METRIC == HM_METRIC_COSINE && col < c_end ? J.rnorm[col] : 0.0;
+                }
+#pragma unroll
+                for (int r = 0; r < 8; ++r) {
+                    const uint32_t row = sm.rows[warp * 8 + r];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const uint32_t col = col0 + lane + 32 * c;
+                        const double a = acc[r][c];
+                        acc[r][c] = 0.0;
+                        const bool near = METRIC == HM_METRIC_COSINE ? a >= __dmul_rn(limit[r], rn_b[c]) : a <= limit[r];
+                        const bool pass = col < c_end && (near || col == row);
+                        const unsigned m = __ballot_sync(0xffffffffu, pass);
+                        if (!m) continue;
+                        uint64_t *fresh = sm.fresh[warp * 8 + r];
+                        if (pass) {
+                            float dist = pair_finish<METRIC>(a, sm.rn_a[warp * 8 + r], rn_b[c]);
+                            if (col == row) dist = 0.0f;  // src/knn.rs:38-39
+                            fresh[have[r] + __popc(m & ((1u << lane) - 1u))] = make_key(dist, col);
+                        }
+                        have[r] += __popc(m);
+                        __syncwarp();
+                        if (have[r] >= 32) {
+                            const uint64_t tau = plain_merge<KPL>(sm.list[warp * 8 + r], fresh, 32, k);
+                            limit[r] = pair_limit<METRIC>(tau, sm.rn_a[warp * 8 + r]);
+                            have[r] -= 32;
+                            const uint64_t rest = fresh[32 + lane];
+                            __syncwarp();
+                            if ((uint32_t)lane < have[r]) fresh[lane] = rest;
+                            __syncwarp();
+                        }
+                    }
                 }
             }
+            if (s + 1 < stages) store(buf ^ 1);
+            col0 = ncol;
+            kt = nkt;
+            __syncthreads();
         }
 
-        // write the first k elements of each valid row
+        // the first k keys of each row
+#pragma unroll 1
+        for (int r = 0; r < 8; ++r) {
+            uint32_t left = 0;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const uint32_t row = my_rows[r];
+            for (int q = 0; q < 8; ++q) left = q == r ? have[q] : left;
+            const uint32_t row = sm.rows[warp * 8 + r];
             if (row == 0xffffffffu) continue;
-#pragma unroll
-            for (int q = 0; q < KPL; ++q) {
-                const uint32_t e = q * 32 + lane;
-                if (e >= J.k) continue;
-                const uint64_t key = top[r].v[q];
+            uint64_t *list = sm.list[warp * 8 + r];
+            if (left) plain_merge<KPL>(list, sm.fresh[warp * 8 + r], left, k);
+            for (uint32_t e = lane; e < k; e += 32) {
+                const uint64_t key = list[e];
                 if (J.splits > 1 && !w.fallback) {
-                    J.partial[((size_t)split * J.n + row) * J.k + e] = key;
+                    J.partial[((size_t)split * n + row) * k + e] = key;
                 } else {
-                    J.idx[(size_t)row * J.k + e] = key_idx(key);
-                    J.dist[(size_t)row * J.k + e] = key_dist(key);
+                    J.idx[(size_t)row * k + e] = key_idx(key);
+                    J.dist[(size_t)row * k + e] = key_dist(key);
                 }
             }
         }
-        __syncthreads();  // s_rows is rewritten by the next group
+        __syncthreads();  // the rows and lists are rewritten by the next group
     }
 }
 
-template <int METRIC>
-static int launch_plain_metric(const PlainWork &w, uint32_t grid, cudaStream_t s) {
-    switch (w.kpl) {
-    case 1: plain_knn_kernel<METRIC, 1><<<grid, PL_THREADS, 0, s>>>(w); break;
-    case 2: plain_knn_kernel<METRIC, 2><<<grid, PL_THREADS, 0, s>>>(w); break;
-    case 4: plain_knn_kernel<METRIC, 4><<<grid, PL_THREADS, 0, s>>>(w); break;
-    case 8: plain_knn_kernel<METRIC, 8><<<grid, PL_THREADS, 0, s>>>(w); break;
-    default: return set_error(HM_ERR_UNSUPPORTED, "select width %u", w.kpl);
-    }
+template <int METRIC, int KPL>
+static int launch_plain_kernel(const PlainWork &w, uint32_t grid, cudaStream_t s) {
+    const int smem = (int)sizeof(PlainSmem<KPL>);
+    HM_TRY(ensure_dynamic_smem((const void *)plain_knn_kernel<METRIC, KPL>, smem));
+    plain_knn_kernel<METRIC, KPL><<<grid, PL_THREADS, smem, s>>>(w);
     HM_CUDA_TRY(cudaGetLastError());
     count_launch();
     return HM_OK;
+}
+template <int METRIC>
+static int launch_plain_metric(const PlainWork &w, uint32_t grid, cudaStream_t s) {
+    switch (w.kpl) {
+    case 1: return launch_plain_kernel<METRIC, 1>(w, grid, s);
+    case 2: return launch_plain_kernel<METRIC, 2>(w, grid, s);
+    case 4: return launch_plain_kernel<METRIC, 4>(w, grid, s);
+    case 8: return launch_plain_kernel<METRIC, 8>(w, grid, s);
+    default: return set_error(HM_ERR_UNSUPPORTED, "select width %u", w.kpl);
+    }
 }
 
 // One launch per metric present (the arithmetic is a template parameter);
@@ -392,7 +478,7 @@ __global__ void __launch_bounds__(256) merge_splits_kernel(const JobDev *__restr
         for (uint32_t e0 = 0; e0 < k; e0 += 32) {
             const uint64_t key = (e0 + lane < k) ? list[e0 + lane] : KEY_NONE;
             if (!__any_sync(0xffffffffu, key < top.tau)) break;  // lists are sorted
-            top.offer(key, k, lane);
+            top.template merge32<true>(key, k, lane);
         }
     }
 #pragma unroll

@@ -854,10 +854,12 @@ int launch_rerank(const JobDev *jobs, const GroupDev &G, const GroupDev *Gd, uin
     // Rows per warp: more fill the 32-pair slices better, fewer give more warps
     // (16 fit an SM).  Measured (this phase, us; 8 / 4 / 2 rows): 3,000 x 64 14 / 9
     // / 8, 5,003 x 300 with 139 survivors a row 476 / 345 / 245, 8,000 x 128 32 /
-    // 22 / 25, 20,000 x 128 56 / 45 / 50, 50,000 x 384 492 / 453 / 465.
-    const bool few = G.rows < 8000;
-    const uint32_t rpw = few ? 2u : 4u;
-    const void *exact = few ? (const void *)rr_exact_kernel<2> : (const void *)rr_exact_kernel<4>;
+    // 22 / 25, 20,000 x 128 56 / 45 / 50, 50,000 x 384 492 / 453 / 465; a batch of
+    // 540,000 rows with 19 survivors each 789 / 864 / -.
+    const uint32_t rpw = G.rows < 8000 ? 2u : (G.rows < 200000 ? 4u : 8u);
+    const void *exact = rpw == 2   ? (const void *)rr_exact_kernel<2>
+                        : rpw == 4 ? (const void *)rr_exact_kernel<4>
+                                   : (const void *)rr_exact_kernel<8>;
     HM_TRY(ensure_dynamic_smem(exact, (int)ex_smem));
     void *args[] = {(void *)&jobs, (void *)&Gd};
     HM_CUDA_TRY(cudaLaunchKernel(exact, dim3((G.rows + rpw * RR_WARPS - 1) / (rpw * RR_WARPS)), dim3(RR_WARPS * 32), args,
