@@ -100,7 +100,7 @@ struct JobPlan {
     // emission pass: symmetric (tiles on and above the diagonal), its column
     // parts per row block of ept tiles, candidate lists per row
     bool sym = false;
-    uint32_t ept = 0, elists = 0;
+    uint32_t ept = 0, elists = 0, erb0 = 0, eparts = 1;
     uint64_t eslot0 = 0;
     // escalation: the job's split-BF16 copy (clone), or the job a copy is of
     int clone = -1, clone_of = -1;
@@ -115,7 +115,8 @@ struct GroupPlan {
     int metric_mask = 0;
     std::vector<uint32_t> jobs;
     uint64_t lists = 0, cand = 0, topk = 0, elists = 0;
-    std::vector<uint4> eunits;  // emission units, largest first
+    uint32_t neunits = 0;       // emission units
+    std::vector<uint4> eunits;  // their table, largest first (none for one job without symmetric units)
     bool any_sym = false;
     bool pair = false;  // emission pass in the 2-SM form (units of 256 rows)
     bool pair_vetoed = false;  // the autotuner table prefers one CTA per row block for a job
@@ -139,7 +140,8 @@ struct hm_batch {
     uint32_t user_jobs = 0;
     hm::GroupPlan groups[3];  // bf16, tf32, split bf16
     uint32_t all_rows = 0, kmax = 0, kpl_all = 1, kpl_plain[3] = {1, 1, 1}, kpl_fb[3] = {1, 1, 1};
-    std::vector<uint2> items[3];       // exact-path work per metric
+    std::vector<uint2> items[3];       // exact-path jobs per metric: (job, first item)
+    uint32_t nitems[3] = {0, 0, 0};    // and their items
     std::vector<uint32_t> fb_jobs[3];  // screened jobs per metric (fallback rows)
     uint32_t fb_per_job[3] = {1, 1, 1};
     bool any_plain = false, any_screen = false, any_smooth = false, any_split = false;
@@ -422,11 +424,16 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
         Gp.pair = !Gp.pair_vetoed && Gp.kpmax / Gp.kslice <= SC_ARES_STAGES;
         // emission units of the group: (job slot | sym, row block (2-SM form:
         // block of 256 rows), first tile, end tile | part); a symmetric unit
-        // starts at the tile holding its diagonal block
+        // starts at the tile holding its diagonal block.  One job without symmetric
+        // units needs no table of them.
         const uint32_t ubm = Gp.pair ? 2 * SC_BM : SC_BM;
         for (uint32_t gj = 0; gj < Gp.jobs.size(); ++gj) {
-            const JobPlan &P = B.jobs[Gp.jobs[gj]];
+            JobPlan &P = B.jobs[Gp.jobs[gj]];
             const uint32_t ub0 = P.q0 / ubm, ub1 = (P.q1 + ubm - 1) / ubm;
+            P.erb0 = ub0;
+            P.eparts = (P.col_tiles + P.ept - 1) / P.ept;
+            Gp.neunits = (ub1 - ub0) * P.eparts;
+            if (Gp.jobs.size() == 1 && !P.sym) break;
             for (uint32_t rb = ub0; rb < ub1; ++rb) {
                 const uint32_t first = P.sym ? rb * ubm / SC_BN : 0u;
                 for (uint32_t part = 0, t0 = first; t0 < P.col_tiles; ++part, t0 += P.ept) {
@@ -435,6 +442,7 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
                 }
             }
         }
+        if (!Gp.eunits.empty()) Gp.neunits = (uint32_t)Gp.eunits.size();
         // symmetric units differ in size: the largest first, so the
         // persistent CTAs' static round-robin finishes together
         if (Gp.any_sym)
@@ -443,8 +451,7 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
             });
         // CTAs of the emission pass (the 2-SM form runs two per unit, at most
         // one per SM): the column-side stages are per CTA
-        const uint64_t eunits_n = Gp.eunits.size();
-        Gp.egrid = (uint32_t)std::min<uint64_t>(Gp.pair ? 2 * eunits_n : eunits_n, G);
+        Gp.egrid = (uint32_t)std::min<uint64_t>(Gp.pair ? 2ull * Gp.neunits : Gp.neunits, G);
         if (Gp.any_sym) {
             // column-side candidates staged per epilogue warp of every CTA
             // (SC_STAGE_SLOTS stages per CTA): room for half of every sym
@@ -463,9 +470,9 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
         const JobPlan &P = B.jobs[j];
         const int m = P.spec.metric;
         if (P.path == HM_PATH_PLAIN) {
-            const uint32_t g_end = (P.q1 + PL_BM - 1) / PL_BM;
-            for (uint32_t gi = P.q0 / PL_BM; gi < g_end; ++gi)
-                for (uint32_t sp = 0; sp < P.splits; ++sp) B.items[m].push_back(make_uint2(j, gi << 6 | sp));
+            const uint32_t groups = (P.q1 + PL_BM - 1) / PL_BM - P.q0 / PL_BM;
+            B.items[m].push_back(make_uint2(j, B.nitems[m]));
+            B.nitems[m] += groups * P.splits;
             B.kpl_plain[m] = std::max<uint32_t>(B.kpl_plain[m], (uint32_t)kpl_for_k(P.spec.k));
         } else if (P.clone_of < 0) {
             // (an escalation copy's fallback rows are the original's: same
@@ -582,12 +589,14 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
 // referenced).
 constexpr uint32_t kParamTable = 3968;  // + the destination pointer: within 4 KB
 struct ParamTable {
+    alignas(16) unsigned char data[kParamTable];
     uint32_t bytes;
-    unsigned char data[kParamTable];
 };
 
-__global__ void write_table_kernel(char *dst, const ParamTable t) {
-    for (uint32_t i = threadIdx.x; i < t.bytes; i += blockDim.x) dst[i] = (char)t.data[i];
+// (a 16-byte piece per thread: the table's parts start and end 16-byte aligned)
+__global__ void write_table_kernel(char *dst, const __grid_constant__ ParamTable t) {
+    const uint32_t i = 16 * (blockIdx.x * blockDim.x + threadIdx.x);
+    if (i < t.bytes) *reinterpret_cast<uint4 *>(dst + i) = *reinterpret_cast<const uint4 *>(t.data + i);
 }
 
 template <typename T>
@@ -656,6 +665,9 @@ static int bind_batch(hm_batch &B, void *d_ws, size_t bytes, cudaStream_t s) {
         J.topk0 = P.topk0;
         J.elists = P.elists;
         J.sym = P.sym ? 1u : 0u;
+        J.erb0 = P.erb0;
+        J.eparts = P.eparts;
+        J.ept = P.ept;
         J.eslot0 = P.eslot0;
         J.scale = s.metric == HM_METRIC_EUCLIDEAN ? 2.0f : 1.0f;
         J.mu = P.group >= 0 ? at<double>(ws, P.off_mu) : nullptr;
@@ -723,8 +735,9 @@ static int bind_batch(hm_batch &B, void *d_ws, size_t bytes, cudaStream_t s) {
         D.cand_cnt = at<uint32_t>(ws, Gp.off_cnt);
         D.topk = at<float>(ws, Gp.off_topk);
         D.row_cnt = at<uint32_t>(ws, Gp.off_rowcnt);
-        D.eunits = at<uint4>(ws, Gp.off_eunits);
-        D.neunits = (uint32_t)Gp.eunits.size();
+        D.eunits = Gp.eunits.empty() ? nullptr : at<uint4>(ws, Gp.off_eunits);
+        D.neunits = Gp.neunits;
+        D.any_euclidean = (Gp.metric_mask >> HM_METRIC_EUCLIDEAN) & 1;
         D.pair = Gp.pair ? 1u : 0u;
         for (uint32_t j : Gp.jobs) {
             const bool short_rows = B.jobs[j].kp1 <= operand_short_k1();
@@ -755,7 +768,7 @@ static int bind_batch(hm_batch &B, void *d_ws, size_t bytes, cudaStream_t s) {
         ParamTable t;
         t.bytes = (uint32_t)std::min<size_t>(kParamTable, used - o);
         memcpy(t.data, B.table.data() + o, t.bytes);
-        write_table_kernel<<<1, 256, 0, s>>>(dst + o, t);
+        write_table_kernel<<<(t.bytes + 511) / 512, 32, 0, s>>>(dst + o, t);
         HM_CUDA_TRY(cudaGetLastError());
         count_launch();
     }
@@ -777,7 +790,8 @@ static int run_batch(hm_batch &B, cudaStream_t s) {
         w.jobs = jobs;
         w.njobs = njobs;
         w.items = at<uint2>(ws, B.off_items[m]);
-        w.nitems = (uint32_t)B.items[m].size();
+        w.nitems = B.nitems[m];
+        w.njobs_m = (uint32_t)B.items[m].size();
         w.kpl = B.kpl_plain[m];
         HM_TRY(launch_plain(w, m, s));
     }
@@ -1165,7 +1179,7 @@ int hm_smooth_knn_device(const float *d_dists, uint64_t n, uint32_t k, float *d_
     write_smooth_job_kernel<<<1, 32, 0, s>>>(jd, J);
     HM_CUDA_TRY(cudaGetLastError());
     count_launch();
-    HM_TRY(launch_smooth(jd, 1, nullptr, (uint32_t)n, k, s));
+    HM_TRY(launch_smooth(jd, 1, nullptr, (uint32_t)n, k, s, false));
     HM_TRY(launch_mean_all_floor(jd, 1, s));
     return HM_OK;
 }
@@ -1202,7 +1216,7 @@ int hm_smooth_knn_rows_device(const float *d_dists, uint64_t n, uint32_t k, uint
     write_smooth_job_kernel<<<1, 32, 0, s>>>(jd, J);
     HM_CUDA_TRY(cudaGetLastError());
     count_launch();
-    HM_TRY(launch_smooth(jd, 1, nullptr, (uint32_t)(row_end - row_begin), k, s));
+    HM_TRY(launch_smooth(jd, 1, nullptr, (uint32_t)(row_end - row_begin), k, s, false));
     HM_TRY(launch_mean_all_floor(jd, 1, s));
     return HM_OK;
 }

@@ -80,6 +80,7 @@ __device__ __forceinline__ float tconorm(float v, float vt) {
 
 constexpr uint32_t FZ_PER_THREAD = 4;  // entries in flight per thread of the entry kernels
 __global__ void __launch_bounds__(256) fuzzy_entries_kernel(const FuzzyDev D) {
+    grid_ready();
     const uint32_t e0 = blockIdx.x * 256 * FZ_PER_THREAD + threadIdx.x;
     uint32_t col[FZ_PER_THREAD], row[FZ_PER_THREAD], slot[FZ_PER_THREAD];
     float d[FZ_PER_THREAD], sg[FZ_PER_THREAD], w[FZ_PER_THREAD];
@@ -145,6 +146,7 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t *warp_sums, 
 }
 
 __global__ void __launch_bounds__(256) fuzzy_segments_kernel(const FuzzyDev D) {
+    grid_ready();
     __shared__ uint32_t warp_sums[8], base;
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t mine = r < D.n ? D.k + D.indeg[r] : 0u;
@@ -156,6 +158,7 @@ __global__ void __launch_bounds__(256) fuzzy_segments_kernel(const FuzzyDev D) {
 }
 
 __global__ void __launch_bounds__(256) fuzzy_scatter_kernel(const FuzzyDev D) {
+    grid_ready();
     const uint32_t e0 = blockIdx.x * 256 * FZ_PER_THREAD + threadIdx.x;
     float w[FZ_PER_THREAD];
     uint32_t at[FZ_PER_THREAD];
@@ -262,6 +265,7 @@ __device__ __forceinline__ uint32_t union_row(const FuzzyDev &D, uint32_t r, uin
 constexpr int FZ_WARPS = 4;
 template <typename K>
 __global__ void __launch_bounds__(FZ_WARPS * 32, sizeof(K) == 4 ? 16 : 8) fuzzy_union_kernel(const FuzzyDev D) {
+    grid_ready();
     __shared__ float w_all[FZ_WARPS][FZ_SHORT_SLOTS];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t r = blockIdx.x * FZ_WARPS + warp;
@@ -291,6 +295,7 @@ __global__ void __launch_bounds__(FZ_WARPS * 32, sizeof(K) == 4 ? 16 : 8) fuzzy_
 // The blocks' warps then take the rows of 129 to 512 slots, one each.
 template <typename K>
 __global__ void __launch_bounds__(1024) fuzzy_long_kernel(const FuzzyDev D, uint2 *out_all) {
+    grid_ready();
     extern __shared__ uint32_t hub_smem[];
     __shared__ uint32_t warp_sums[32];
     const uint32_t words_n = (min(D.n, FZ_WINDOW) + 31) / 32;
@@ -398,6 +403,7 @@ __global__ void __launch_bounds__(1024) fuzzy_long_kernel(const FuzzyDev D, uint
 __global__ void __launch_bounds__(256) fuzzy_write_kernel(const FuzzyDev D, uint32_t tiles, uint32_t *__restrict__ rows,
                                                           uint32_t *__restrict__ cols, float *__restrict__ vals,
                                                           unsigned long long *__restrict__ nnz) {
+    grid_ready();
     __shared__ uint32_t warp_sums[8], off[256], cnt[256], first[256];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tile = blockIdx.x;
     uint32_t sum = 0;
@@ -448,6 +454,7 @@ __global__ void __launch_bounds__(256) fuzzy_write_kernel(const FuzzyDev D, uint
 // Rows of more than 512 entries (all of them hubs), each spread over the grid.
 __global__ void __launch_bounds__(256) fuzzy_hub_write_kernel(const FuzzyDev D, uint32_t *__restrict__ rows,
                                                               uint32_t *__restrict__ cols, float *__restrict__ vals) {
+    grid_ready();
     const uint32_t hubs = D.words[FZ_HUBS];
     const uint32_t parts = max(1u, gridDim.x / max(hubs, 1u)), at_once = gridDim.x / parts;  // blocks a row, rows
     if (blockIdx.x >= parts * at_once) return;
@@ -554,35 +561,27 @@ int hm_fuzzy_graph_device(const uint32_t *d_idx, const float *d_dist, const floa
     D.words = D.tile_sum + FZ_TILES;
     const unsigned entry_blocks = (D.entries + 256 * FZ_PER_THREAD - 1) / (256 * FZ_PER_THREAD);
     HM_CUDA_TRY(cudaMemsetAsync(ws + L.zeroed, 0, L.zeroed_bytes, s));
-    fuzzy_entries_kernel<<<entry_blocks, 256, 0, s>>>(D);
-    HM_CUDA_TRY(cudaGetLastError());
-    fuzzy_segments_kernel<<<(D.n + 255u) / 256u, 256, 0, s>>>(D);
-    HM_CUDA_TRY(cudaGetLastError());
-    fuzzy_scatter_kernel<<<entry_blocks, 256, 0, s>>>(D);
-    HM_CUDA_TRY(cudaGetLastError());
+    HM_CUDA_TRY(launch(false, fuzzy_entries_kernel, entry_blocks, 256, 0, s, D));
+    HM_CUDA_TRY(launch(true, fuzzy_segments_kernel, (D.n + 255u) / 256u, 256, 0, s, D));
+    HM_CUDA_TRY(launch(true, fuzzy_scatter_kernel, entry_blocks, 256, 0, s, D));
     // column and slot share a 32-bit sort key while both fit
     const bool narrow = n < 1ull << (32 - FZ_SLOT_BITS);
     const unsigned union_blocks = (D.n + FZ_WARPS - 1) / FZ_WARPS;
-    if (narrow) fuzzy_union_kernel<uint32_t><<<union_blocks, FZ_WARPS * 32, 0, s>>>(D);
-    else fuzzy_union_kernel<unsigned long long><<<union_blocks, FZ_WARPS * 32, 0, s>>>(D);
-    HM_CUDA_TRY(cudaGetLastError());
+    HM_CUDA_TRY(launch(true, narrow ? fuzzy_union_kernel<uint32_t> : fuzzy_union_kernel<unsigned long long>, union_blocks,
+                       FZ_WARPS * 32, 0, s, D));
     if (n + k > FZ_SHORT_SLOTS) {  // a row's slots: k and at most n - 1 sources
-        const void *kernel = narrow ? (const void *)fuzzy_long_kernel<uint32_t> : (const void *)fuzzy_long_kernel<unsigned long long>;
+        auto *kernel = narrow ? fuzzy_long_kernel<uint32_t> : fuzzy_long_kernel<unsigned long long>;
         const size_t bitmaps = (size_t)3 * ((std::min(D.n, FZ_WINDOW) + 31) / 32) * 4, rows_w = 32 * FZ_WARP_SLOTS * 4;
-        const size_t smem = std::max(bitmaps, rows_w);
-        HM_TRY(ensure_dynamic_smem(kernel, (int)(3 * FZ_WINDOW / 8)));
-        uint2 *out = reinterpret_cast<uint2 *>(ws + L.hub_out);
-        void *args[] = {&D, &out};
-        HM_CUDA_TRY(cudaLaunchKernel(kernel, dim3(device_sm_count()), dim3(1024), args, smem, s));
+        HM_TRY(ensure_dynamic_smem((const void *)kernel, (int)(3 * FZ_WINDOW / 8)));
+        HM_CUDA_TRY(launch(true, kernel, device_sm_count(), 1024, std::max(bitmaps, rows_w), s, D,
+                           reinterpret_cast<uint2 *>(ws + L.hub_out)));
         count_launch();
     }
-    fuzzy_write_kernel<<<L.tiles, 256, 0, s>>>(D, L.tiles, d_rows, d_cols, d_vals,
-                                               reinterpret_cast<unsigned long long *>(d_nnz));
-    HM_CUDA_TRY(cudaGetLastError());
+    HM_CUDA_TRY(launch(true, fuzzy_write_kernel, L.tiles, 256, 0, s, D, L.tiles, d_rows, d_cols, d_vals,
+                       reinterpret_cast<unsigned long long *>(d_nnz)));
     count_launch(5);
     if (n + k > FZ_WARP_SLOTS) {
-        fuzzy_hub_write_kernel<<<4 * device_sm_count(), 256, 0, s>>>(D, d_rows, d_cols, d_vals);
-        HM_CUDA_TRY(cudaGetLastError());
+        HM_CUDA_TRY(launch(true, fuzzy_hub_write_kernel, 4 * device_sm_count(), 256, 0, s, D, d_rows, d_cols, d_vals));
         count_launch();
     }
     return HM_OK;

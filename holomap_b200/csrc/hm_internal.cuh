@@ -38,6 +38,41 @@ void clear_error();
 
 inline size_t round_up(size_t x, size_t m) { return (x + m - 1) / m * m; }
 
+// Kernel launch that may overlap the end of the stream's previous kernel
+// (programmatic dependent launch): the blocks become resident while the previous
+// kernel's last blocks run and wait in grid_ready(), which every kernel launched
+// so calls before anything else.  A kernel starts only when all blocks of the
+// previous one have passed their own grid_ready(), so everything but that one
+// kernel's output is complete by then: its output must not be read through
+// const __restrict__ kernel arguments or __ldg (loads that may move above the
+// wait), which here are the job tables, written two or more kernels earlier, and
+// the caller's points.  `overlap` false: an ordinary launch.  20,000 x 128 call (17
+// launches) 684 -> 656 us, 50,000 x 384 2,717 -> 2,663.  Grids of more than a wave
+// of small blocks launch ordinarily: waiting blocks took the slots of the running
+// kernel's in the big batch (256 datasets, 540,000 rows: 6,760 us with all grids
+// overlapped, 6,648 up to 40,000 blocks, 6,494 up to 2,400).
+constexpr uint64_t OVERLAP_BLOCKS = 16 * 148;
+template <typename... P, typename... A>
+inline cudaError_t launch(bool overlap, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                          A &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    overlap = overlap && (uint64_t)grid.x * grid.y <= OVERLAP_BLOCKS;
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+__device__ __forceinline__ void grid_ready() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Sets a kernel's dynamic shared-memory limit once per device (the attribute
 // call is kept off the per-launch path).
 int ensure_dynamic_smem(const void *func, int bytes);
@@ -203,7 +238,7 @@ struct JobCounters {
                              // split-BF16 copy produced the rows (see JobDev::gate)
     uint32_t escalate_rows;  // rows whose band exceeded the escalation share of tau1
     uint32_t swamped_rows;   // rows with half of their k sampled minima within the band of tau1
-    uint32_t pad0;
+    uint32_t csum_done;      // column-sum blocks that have finished
     // screen prep maxima (non-negative doubles as bits): |u|, |e|, |r|,
     // |A row|, |B row|, |u|^2, largest centred |x - mu|^2; then zero rows
     unsigned long long maxb[8];
@@ -234,6 +269,7 @@ struct JobDev {
     // candidate lists of the emission pass: elists per row (two per column
     // part; with the symmetric emission one more, the row's column list, last)
     uint32_t elists, sym;        // sym: the emission pass covers the tiles on and above the diagonal
+    uint32_t erb0, eparts, ept;  // emission units: first row block, column parts per row block, tiles per part
     unsigned long long eslot0;   // first candidate list of the job
     unsigned long long cand0;    // first candidate slot: list l holds [cand0 + (l - eslot0) * cap, +cap)
     float scale;                 // 1 (cosine) or 2 (euclidean)
@@ -293,14 +329,15 @@ constexpr int PL_BN = 128;    // columns per tile (32 lanes x 4)
 constexpr int PL_BK = 16;     // dimensions per shared-memory stage
 constexpr int PL_THREADS = 128;
 
-// Work table of the exact path: item i = (job, group of PL_BM rows, column
-// split); or, in fallback mode, each job's overflow list strided over
+// Work of the exact path: items (job, group of PL_BM rows, column split); or,
+// in fallback mode, each job's overflow list strided over
 // `per_job` CTAs.
 struct PlainWork {
     const JobDev *jobs;
     uint32_t njobs;
-    const uint2 *items;     // x = job, y = group << 6 | split
-    uint32_t nitems;
+    const uint2 *items;     // per job of the metric: x = job, y = its first item; item i of a job is
+                            // row group q0 / PL_BM + i / splits, split i % splits
+    uint32_t nitems, njobs_m;
     uint32_t kpl;           // WarpTopK width for the largest k
     uint32_t fallback;      // 1: rows come from the jobs' overflow lists
     uint32_t per_job;       // fallback: CTAs per job
@@ -322,8 +359,9 @@ int launch_merge(const JobDev *jobs, uint32_t njobs, const uint32_t *row_starts,
 // Per row of every job with smooth-kNN outputs (row_starts: all-rows space);
 // rows whose rho is 0 get their unfloored sigma and are listed for the
 // job's global-mean floor.
+// (overlap false where the job table was written by the kernel just before)
 int launch_smooth(const JobDev *jobs, uint32_t njobs, const uint32_t *row_starts, uint32_t rows,
-                  uint32_t kmax, cudaStream_t s);
+                  uint32_t kmax, cudaStream_t s, bool overlap = true);
 // Sequential binary64 mean of each job's n*k distances, applied as the floor
 // of its listed rows; one block per job, idle when its list is empty.
 int launch_mean_all_floor(const JobDev *jobs, uint32_t njobs, cudaStream_t s);

@@ -68,6 +68,7 @@ __global__ void __launch_bounds__(NRM_WARPS * 32) check_norms_kernel(const JobDe
                                                                     const uint32_t *__restrict__ row_starts,
                                                                     uint32_t rows) {
     __shared__ float tile[NRM_WARPS][32][33];
+    grid_ready();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t ar0 = (blockIdx.x * NRM_WARPS + warp) * 32;
     if (ar0 >= rows) return;
@@ -130,8 +131,8 @@ int launch_check(const JobDev *jobs, uint32_t njobs, const uint32_t *row_starts,
     init_counters_kernel<<<(njobs + 127) / 128, 128, 0, s>>>(const_cast<JobDev *>(jobs), njobs);
     HM_CUDA_TRY(cudaGetLastError());
     const uint32_t warps = (all_rows + 31) / 32;
-    check_norms_kernel<<<(warps + NRM_WARPS - 1) / NRM_WARPS, NRM_WARPS * 32, 0, s>>>(jobs, njobs, row_starts, all_rows);
-    HM_CUDA_TRY(cudaGetLastError());
+    HM_CUDA_TRY(launch(true, check_norms_kernel, (warps + NRM_WARPS - 1) / NRM_WARPS, NRM_WARPS * 32, 0, s, jobs, njobs,
+                       row_starts, all_rows));
     count_launch(2);
     return HM_OK;
 }
@@ -211,13 +212,19 @@ template <int METRIC, int KPL>
 __global__ void __launch_bounds__(PL_THREADS, KPL <= 2 ? 3 : 2) plain_knn_kernel(const PlainWork w) {
     extern __shared__ __align__(16) unsigned char pl_smem_raw[];
     PlainSmem<KPL> &sm = *reinterpret_cast<PlainSmem<KPL> *>(pl_smem_raw);
+    grid_ready();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint32_t jb, first_grp, grp_stride, n_groups, split = 0;
     if (!w.fallback) {
-        const uint2 it = w.items[blockIdx.x];
-        jb = it.x;
-        first_grp = it.y >> 6;
-        split = it.y & 63u;
+        uint32_t lo = 0, hi = w.njobs_m;  // the job whose items hold this block's
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (w.items[mid].y <= blockIdx.x) lo = mid; else hi = mid;
+        }
+        jb = w.items[lo].x;
+        const uint32_t it = blockIdx.x - w.items[lo].y;
+        first_grp = w.jobs[jb].q0 / PL_BM + it / w.jobs[jb].splits;
+        split = it % w.jobs[jb].splits;
         grp_stride = 1;
         n_groups = first_grp + 1;
     } else {
@@ -422,8 +429,7 @@ template <int METRIC, int KPL>
 static int launch_plain_kernel(const PlainWork &w, uint32_t grid, cudaStream_t s) {
     const int smem = (int)sizeof(PlainSmem<KPL>);
     HM_TRY(ensure_dynamic_smem((const void *)plain_knn_kernel<METRIC, KPL>, smem));
-    plain_knn_kernel<METRIC, KPL><<<grid, PL_THREADS, smem, s>>>(w);
-    HM_CUDA_TRY(cudaGetLastError());
+    HM_CUDA_TRY(launch(true, plain_knn_kernel<METRIC, KPL>, grid, PL_THREADS, smem, s, w));
     count_launch();
     return HM_OK;
 }
@@ -458,6 +464,7 @@ template <int KPL>
 __global__ void __launch_bounds__(256) merge_splits_kernel(const JobDev *__restrict__ jobs, uint32_t njobs,
                                                            const uint32_t *__restrict__ row_starts,
                                                            uint32_t rows) {
+    grid_ready();
     const int lane = threadIdx.x & 31;
     const uint32_t ar = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (ar >= rows) return;
@@ -495,14 +502,13 @@ int launch_merge(const JobDev *jobs, uint32_t njobs, const uint32_t *row_starts,
                  uint32_t kpl, cudaStream_t s) {
     const int blocks = (int)((rows + 7) / 8);
     ScopedKernelTimer timer(HM_KCLASS_SELECT, s);
-    switch (kpl) {
-    case 1: merge_splits_kernel<1><<<blocks, 256, 0, s>>>(jobs, njobs, row_starts, rows); break;
-    case 2: merge_splits_kernel<2><<<blocks, 256, 0, s>>>(jobs, njobs, row_starts, rows); break;
-    case 4: merge_splits_kernel<4><<<blocks, 256, 0, s>>>(jobs, njobs, row_starts, rows); break;
-    case 8: merge_splits_kernel<8><<<blocks, 256, 0, s>>>(jobs, njobs, row_starts, rows); break;
-    default: return set_error(HM_ERR_UNSUPPORTED, "select width %u", kpl);
-    }
-    HM_CUDA_TRY(cudaGetLastError());
+    auto *merge = kpl == 1   ? merge_splits_kernel<1>
+                  : kpl == 2 ? merge_splits_kernel<2>
+                  : kpl == 4 ? merge_splits_kernel<4>
+                  : kpl == 8 ? merge_splits_kernel<8>
+                             : nullptr;
+    if (!merge) return set_error(HM_ERR_UNSUPPORTED, "select width %u", kpl);
+    HM_CUDA_TRY(launch(true, merge, blocks, 256, 0, s, jobs, njobs, row_starts, rows));
     count_launch();
     return HM_OK;
 }

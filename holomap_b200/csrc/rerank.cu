@@ -383,6 +383,8 @@ __global__ void __launch_bounds__(RS_WARPS * 32, 4) rr_select_kernel(const JobDe
     extern __shared__ __align__(16) unsigned char rs_smem_raw[];
     __shared__ uint32_t s_kept[RS_WARPS];
     const GroupDev &G = *Gp;
+    grid_ready();
+    if (group_idle(jobs, G)) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     RsWarpSmem &sm = reinterpret_cast<RsWarpSmem *>(rs_smem_raw)[warp];
     const uint32_t gr = blockIdx.x * RS_WARPS + warp;
@@ -557,6 +559,8 @@ __global__ void __launch_bounds__(RR_WARPS * 32) rr_exact_kernel(const JobDev *_
                                                                  const GroupDev *__restrict__ Gp) {
     extern __shared__ __align__(16) unsigned char rr_smem_raw[];
     const GroupDev &G = *Gp;
+    grid_ready();
+    if (group_idle(jobs, G)) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     RrWarpSmem &sm = reinterpret_cast<RrWarpSmem *>(rr_smem_raw)[warp];
     const uint32_t gr0 = (blockIdx.x * RR_WARPS + warp) * ROWS;
@@ -598,6 +602,8 @@ template <int KPL>
 __global__ void __launch_bounds__(RS_WARPS * 32) rr_topk_kernel(const JobDev *__restrict__ jobs,
                                                                 const GroupDev *__restrict__ Gp) {
     const GroupDev &G = *Gp;
+    grid_ready();
+    if (group_idle(jobs, G)) return;
     const int lane = threadIdx.x & 31;
     const uint32_t gr = blockIdx.x * RS_WARPS + (threadIdx.x >> 5);
     if (gr >= G.rows) return;
@@ -711,6 +717,8 @@ template <int KPL>
 __global__ void __launch_bounds__(256) threshold_kernel(const JobDev *__restrict__ jobs,
                                                        const GroupDev *__restrict__ Gp) {
     const GroupDev &G = *Gp;
+    grid_ready();
+    if (group_idle(jobs, G)) return;
     const int lane = threadIdx.x & 31;
     const uint32_t gr = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (gr >= G.rows) return;
@@ -777,6 +785,7 @@ constexpr uint32_t ESC_ROWS_DIV = 10;
 __global__ void __launch_bounds__(256) escalate_count_kernel(const JobDev *__restrict__ jobs,
                                                              const GroupDev *__restrict__ Gp) {
     const GroupDev &G = *Gp;
+    grid_ready();
     const uint32_t gr = blockIdx.x * blockDim.x + threadIdx.x;
     if (gr - (threadIdx.x & 31) >= G.rows) return;  // whole warps: 32 rows of one job
     const JobDev &J = jobs[G.job_ids[find_job(G.row_starts, G.njobs, gr - (threadIdx.x & 31))]];
@@ -795,6 +804,7 @@ __global__ void __launch_bounds__(256) escalate_count_kernel(const JobDev *__res
 
 __global__ void escalate_decide_kernel(const JobDev *__restrict__ jobs, const GroupDev *__restrict__ Gp) {
     const GroupDev &G = *Gp;
+    grid_ready();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= G.njobs) return;
     const JobDev &J = jobs[G.job_ids[t]];
@@ -809,11 +819,9 @@ __global__ void escalate_decide_kernel(const JobDev *__restrict__ jobs, const Gr
 int launch_escalation(const JobDev *jobs, const GroupDev &G, const GroupDev *Gd, cudaStream_t s) {
     if (G.rows == 0) return HM_OK;
     ScopedKernelTimer timer(HM_KCLASS_SELECT, s);
-    escalate_count_kernel<<<(G.rows + 255) / 256, 256, 0, s>>>(jobs, Gd);
-    HM_CUDA_TRY(cudaGetLastError());
+    HM_CUDA_TRY(launch(true, escalate_count_kernel, (G.rows + 255) / 256, 256, 0, s, jobs, Gd));
     count_launch();
-    escalate_decide_kernel<<<(G.njobs + 127) / 128, 128, 0, s>>>(jobs, Gd);
-    HM_CUDA_TRY(cudaGetLastError());
+    HM_CUDA_TRY(launch(true, escalate_decide_kernel, (G.njobs + 127) / 128, 128, 0, s, jobs, Gd));
     count_launch();
     return HM_OK;
 }
@@ -823,12 +831,8 @@ int launch_screen_threshold(const JobDev *jobs, const GroupDev &G, const GroupDe
     if (G.rows == 0) return HM_OK;
     ScopedKernelTimer timer(HM_KCLASS_SELECT, s);
     const int blocks = (int)((G.rows + 7) / 8);
-    switch (kpl) {
-    case 1: threshold_kernel<1><<<blocks, 256, 0, s>>>(jobs, Gd); break;
-    case 2: threshold_kernel<2><<<blocks, 256, 0, s>>>(jobs, Gd); break;
-    default: return set_error(HM_ERR_UNSUPPORTED, "threshold width %u", kpl);
-    }
-    HM_CUDA_TRY(cudaGetLastError());
+    if (kpl != 1 && kpl != 2) return set_error(HM_ERR_UNSUPPORTED, "threshold width %u", kpl);
+    HM_CUDA_TRY(launch(true, kpl == 1 ? threshold_kernel<1> : threshold_kernel<2>, blocks, 256, 0, s, jobs, Gd));
     count_launch();
     return HM_OK;
 }
@@ -842,14 +846,9 @@ int launch_rerank(const JobDev *jobs, const GroupDev &G, const GroupDev *Gd, uin
     ScopedKernelTimer timer(HM_KCLASS_SELECT, s);
     const int rs_blocks = (int)((G.rows + RS_WARPS - 1) / RS_WARPS);
     const size_t rs_smem = (size_t)RS_WARPS * sizeof(RsWarpSmem);
-    if (kpl == 1) {
-        HM_TRY(ensure_dynamic_smem((const void *)rr_select_kernel<1>, (int)rs_smem));
-        rr_select_kernel<1><<<rs_blocks, RS_WARPS * 32, rs_smem, s>>>(jobs, Gd);
-    } else {
-        HM_TRY(ensure_dynamic_smem((const void *)rr_select_kernel<2>, (int)rs_smem));
-        rr_select_kernel<2><<<rs_blocks, RS_WARPS * 32, rs_smem, s>>>(jobs, Gd);
-    }
-    HM_CUDA_TRY(cudaGetLastError());
+    auto *select = kpl == 1 ? rr_select_kernel<1> : rr_select_kernel<2>;
+    HM_TRY(ensure_dynamic_smem((const void *)select, (int)rs_smem));
+    HM_CUDA_TRY(launch(true, select, rs_blocks, RS_WARPS * 32, rs_smem, s, jobs, Gd));
     const size_t ex_smem = (size_t)RR_WARPS * sizeof(RrWarpSmem);
     // Rows per warp: more fill the 32-pair slices better, fewer give more warps
     // (16 fit an SM).  Measured (this phase, us; 8 / 4 / 2 rows): 3,000 x 64 14 / 9
@@ -857,18 +856,10 @@ int launch_rerank(const JobDev *jobs, const GroupDev &G, const GroupDev *Gd, uin
     // 22 / 25, 20,000 x 128 56 / 45 / 50, 50,000 x 384 492 / 453 / 465; a batch of
     // 540,000 rows with 19 survivors each 789 / 864 / -.
     const uint32_t rpw = G.rows < 8000 ? 2u : (G.rows < 200000 ? 4u : 8u);
-    const void *exact = rpw == 2   ? (const void *)rr_exact_kernel<2>
-                        : rpw == 4 ? (const void *)rr_exact_kernel<4>
-                                   : (const void *)rr_exact_kernel<8>;
-    HM_TRY(ensure_dynamic_smem(exact, (int)ex_smem));
-    void *args[] = {(void *)&jobs, (void *)&Gd};
-    HM_CUDA_TRY(cudaLaunchKernel(exact, dim3((G.rows + rpw * RR_WARPS - 1) / (rpw * RR_WARPS)), dim3(RR_WARPS * 32), args,
-                                 ex_smem, s));
-    if (kpl == 1)
-        rr_topk_kernel<1><<<rs_blocks, RS_WARPS * 32, 0, s>>>(jobs, Gd);
-    else
-        rr_topk_kernel<2><<<rs_blocks, RS_WARPS * 32, 0, s>>>(jobs, Gd);
-    HM_CUDA_TRY(cudaGetLastError());
+    auto *exact = rpw == 2 ? rr_exact_kernel<2> : (rpw == 4 ? rr_exact_kernel<4> : rr_exact_kernel<8>);
+    HM_TRY(ensure_dynamic_smem((const void *)exact, (int)ex_smem));
+    HM_CUDA_TRY(launch(true, exact, (G.rows + rpw * RR_WARPS - 1) / (rpw * RR_WARPS), RR_WARPS * 32, ex_smem, s, jobs, Gd));
+    HM_CUDA_TRY(launch(true, kpl == 1 ? rr_topk_kernel<1> : rr_topk_kernel<2>, rs_blocks, RS_WARPS * 32, 0, s, jobs, Gd));
     count_launch(3);
     return HM_OK;
 }

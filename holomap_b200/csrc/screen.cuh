@@ -93,7 +93,10 @@ struct GroupDev {
     uint32_t *row_cnt;            // rerank: survivors per group row (0: none or exact fallback)
     // emission pass: its work units (x = group job slot | sym << 31, y = row
     // block, z = first column tile, w = end column tile | column part << 24),
-    // largest first
+    // largest first; null for one job without symmetric units, whose units are its
+    // row blocks times its column parts (the table would be most of a single
+    // call's: 50,000 points 28 KB, 41 us of launches that write it; in a batch a
+    // search for a unit's job costs more, 6.8 ms against 6.4 for 256 datasets)
     const uint4 *eunits;
     uint32_t neunits;
     // emission pass in the 2-SM form (a cluster of two CTAs per unit, one
@@ -101,7 +104,7 @@ struct GroupDev {
     uint32_t pair;
     // the group has jobs whose padded row length K1 is at most / above the
     // packed operand kernel's limit (which operand kernels run)
-    uint32_t any_short_rows, any_long_rows;
+    uint32_t any_short_rows, any_long_rows, any_euclidean;
     // symmetric emission: per group row (padded like colterm) the emission
     // limit tau1 + 2 band and its cosine raw-product form; the column-side
     // candidates each CTA staged (group row of the column, raw product bits
@@ -119,6 +122,12 @@ __device__ __forceinline__ uint32_t ord32(float f) {
 }
 __device__ __forceinline__ float unord32(uint32_t o) {
     return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
+}
+
+// Whether none of the group's jobs runs (only known at a glance for a group of
+// one: the split-BF16 copy of a call that did not escalate, or its original).
+__device__ __forceinline__ bool group_idle(const JobDev *jobs, const GroupDev &G) {
+    return G.njobs == 1 && !job_active(jobs[G.job_ids[0]]);
 }
 
 // Row i's threshold-pass list s (s < tlists * parts) of job J (its k-array).

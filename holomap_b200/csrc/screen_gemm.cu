@@ -236,10 +236,20 @@ struct UnitTiles {
 
 // Pass 0 (the threshold pass) walks only the first seed_tiles tiles of each
 // part: a sample of the row's columns whose k-th smallest screened value
-// already bounds the row's k-th from above.  Pass 1 (the emission pass) takes
-// its units from the group's table.
+// already bounds the row's k-th from above.  The emission passes take their units
+// from the group's table; a group of one job without symmetric units needs none.
 __device__ __forceinline__ UnitTiles unit_tiles(const JobDev *jobs, const GroupDev &G, uint32_t u, int pass) {
     UnitTiles t;
+    if (pass == 1 && !G.eunits) {
+        t.sym = 0;
+        t.job = G.job_ids[0];
+        const JobDev &J = jobs[t.job];
+        t.rb = J.erb0 + u / J.eparts;
+        t.part = u % J.eparts;
+        t.ct_begin = t.part * J.ept;
+        t.ct_end = min(J.col_tiles, t.ct_begin + J.ept);
+        return t;
+    }
     if (pass >= 1) {
         const uint4 e = G.eunits[u];
         t.job = G.job_ids[e.x & 0x7fffffffu];
@@ -287,6 +297,8 @@ __global__ void __launch_bounds__(sc_threads(PASS, KP), 1)
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(aempty + 1);
     volatile uint32_t *abort_flag = tmem_slot + 1;
 
+    grid_ready();
+    if (group_idle(jobs, G)) return;  // every CTA alike
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t nunits = PASS >= 1 ? G.neunits : G.units;
     // 2-SM form: a cluster of two CTAs works on a unit of 256 rows (rank r
@@ -986,13 +998,15 @@ static int launch_pair(const JobDev *jobs, const GroupDev &G, const CUtensorMap 
     cfg.blockDim = dim3(sc_threads(PASS), 1, 1);
     cfg.dynamicSmemBytes = SC_SMEM_BYTES;
     cfg.stream = s;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
     const uint32_t pidesc = (idesc & ~(0x1fu << 24)) | (((uint32_t)(2 * SC_BM) >> 4) << 24);  // M = 256
     HM_CUDA_TRY(cudaLaunchKernelEx(&cfg, screen_gemm_kernel<KIND, 32, PASS, true>, ta, tb, jobs, G,
                                    (float *)nullptr, pidesc, 1u));
@@ -1012,9 +1026,8 @@ static int launch_kind(const JobDev *jobs, const GroupDev &G, const CUtensorMap 
     if (grid == 0) return HM_OK;
     // every job's K slices fit the resident A block
     const uint32_t a_res = (G.kpmax / G.kslice) <= SC_ARES_STAGES ? 1u : 0u;
-    screen_gemm_kernel<KIND, KP, PASS, false><<<grid, sc_threads(PASS, KP), SC_SMEM_BYTES, s>>>(ta, tb, jobs, G, dump,
-                                                                                      idesc, a_res);
-    HM_CUDA_TRY(cudaGetLastError());
+    HM_CUDA_TRY(launch(true, screen_gemm_kernel<KIND, KP, PASS, false>, grid, sc_threads(PASS, KP), SC_SMEM_BYTES, s, ta,
+                       tb, jobs, G, dump, idesc, a_res));
     count_launch();
     return HM_OK;
 }

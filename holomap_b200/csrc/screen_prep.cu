@@ -33,27 +33,60 @@ __device__ __forceinline__ void atomic_max_pos(unsigned long long *p, double v) 
 }
 
 constexpr uint32_t CSUM_BLOCKS = 64;  // column-sum partial blocks per euclidean job
+constexpr uint32_t CSUM_THREADS = 512;
 
-// Column sums of one slice of a job's rows, binary64 (block = job x slice).
-__global__ void colsum_partial_kernel(const JobDev *__restrict__ jobs, const GroupDev *__restrict__ G) {
+// Column means, binary64 (block = job x slice of its rows): the block's threads
+// stand side by side over the columns, in as many row strands as fit, eight loads
+// in flight each; the job's last block sums the slices' partials.  20,000 x 128:
+// 43 us with one strand and a launch of its own for the sum, 19 now (the points
+// come from HBM).
+__global__ void __launch_bounds__(CSUM_THREADS) column_mean_kernel(const JobDev *__restrict__ jobs,
+                                                                   const GroupDev *__restrict__ G) {
+    __shared__ double strand_sum[CSUM_THREADS];
+    __shared__ uint32_t s_last;
+    grid_ready();
     const uint32_t g = blockIdx.x / CSUM_BLOCKS, b = blockIdx.x % CSUM_BLOCKS;
     const JobDev &J = jobs[G->job_ids[g]];
     if (J.metric != HM_METRIC_EUCLIDEAN || !job_active(J)) return;
-    const uint32_t per = (J.n + CSUM_BLOCKS - 1) / CSUM_BLOCKS;
-    const uint32_t r0 = b * per, r1 = min(J.n, r0 + per);
-    for (uint32_t c = threadIdx.x; c < J.d; c += blockDim.x) {
+    // two rounds of loads a slice at least: small jobs of a batch take few slices
+    const uint32_t d = J.d, slices = (uint32_t)min((uint64_t)CSUM_BLOCKS, (uint64_t)J.n * d / (16 * CSUM_THREADS) + 1);
+    if (b >= slices) return;
+    const uint32_t per = (J.n + slices - 1) / slices;
+    const uint32_t r0 = min(J.n, b * per), r1 = min(J.n, r0 + per);
+    const uint32_t strands = max(1u, CSUM_THREADS / d), strand = d <= CSUM_THREADS ? threadIdx.x / d : 0u;
+    for (uint32_t c0 = 0; c0 < d; c0 += CSUM_THREADS) {  // one round up to 512 columns
+        const uint32_t c = d <= CSUM_THREADS ? threadIdx.x % d : c0 + threadIdx.x;
         double s = 0.0;
-        for (uint32_t r = r0; r < r1; ++r) s += (double)J.x[(size_t)r * J.d + c];
-        J.csum[(size_t)b * J.d + c] = s;
+        if (c < d && strand < strands) {
+            const float *x = J.x + c;
+            uint32_t r = r0 + strand;
+            for (; r + 7 * strands < r1; r += 8 * strands) {
+                float v[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) v[q] = x[(size_t)(r + q * strands) * d];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) s += (double)v[q];
+            }
+            for (; r < r1; r += strands) s += (double)x[(size_t)r * d];
+        }
+        if (strands > 1) {
+            strand_sum[threadIdx.x] = s;
+            __syncthreads();
+            if (threadIdx.x < d)
+                for (uint32_t q = 1; q < strands; ++q) s += strand_sum[q * d + threadIdx.x];
+        }
+        if (c < d && strand == 0) J.csum[(size_t)b * d + c] = s;
     }
-}
-
-__global__ void colmean_kernel(const JobDev *__restrict__ jobs, const GroupDev *__restrict__ G) {
-    const JobDev &J = jobs[G->job_ids[blockIdx.x]];
-    if (J.metric != HM_METRIC_EUCLIDEAN || !job_active(J)) return;
-    for (uint32_t c = threadIdx.x; c < J.d; c += blockDim.x) {
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&J.cnt->csum_done, 1u) == slices - 1 ? 1u : 0u;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (uint32_t c = threadIdx.x; c < d; c += CSUM_THREADS) {
         double s = 0.0;
-        for (uint32_t b = 0; b < CSUM_BLOCKS; ++b) s += J.csum[(size_t)b * J.d + c];
+#pragma unroll 16
+        for (uint32_t q = 0; q < slices; ++q) s += __ldcg(&J.csum[(size_t)q * d + c]);
         J.mu[c] = s / (double)J.n;
     }
 }
@@ -64,6 +97,7 @@ __global__ void colmean_kernel(const JobDev *__restrict__ jobs, const GroupDev *
 __global__ void __launch_bounds__(256) centred_norm_max_kernel(const JobDev *__restrict__ jobs,
                                                               const GroupDev *__restrict__ G) {
     __shared__ double s_max[8];
+    grid_ready();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t gr0 = blockIdx.x * 32;
     const JobDev &J = jobs[G->job_ids[find_job(G->row_starts, G->njobs, gr0)]];
@@ -129,6 +163,14 @@ constexpr int OP_TF32 = 0, OP_BF16 = 1, OP_SPLIT = 2;
 // the registers of half of them)
 __host__ __device__ constexpr uint32_t op_per_lane(int mode) { return mode == OP_SPLIT ? 8u : 16u; }
 
+// The column terms past the group's last row (a column tile may reach them).
+__device__ __forceinline__ void clear_column_tail(const GroupDev &G) {
+    if (blockIdx.x == 0) {
+        const uint32_t end = (G.rows + SC_BN - 1) / SC_BN * SC_BN + SC_BN;
+        for (uint32_t t = G.rows + threadIdx.x; t < end; t += blockDim.x) G.colterm[t] = 0.0f;
+    }
+}
+
 // Operand row(s), binary64 error statistics, additive terms of the screen
 // epilogue, and the row's shared threshold.  Every lane accumulates its
 // elements t = lane, lane + 32, ... in ascending order.
@@ -139,6 +181,9 @@ __global__ void __launch_bounds__(OP_WARPS * 32, OP_BLOCKS_PER_SM) operand_kerne
     __shared__ double s_wmax[OP_WARPS][6];
     __shared__ unsigned long long s_wzero[OP_WARPS];
     const GroupDev &G = *Gp;
+    grid_ready();
+    if (group_idle(jobs, G)) return;
+    clear_column_tail(G);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double *wmax = s_wmax[warp];
     const JobDev *cur = nullptr;  // the job whose maxima the warp holds
@@ -164,6 +209,7 @@ __global__ void __launch_bounds__(OP_WARPS * 32, OP_BLOCKS_PER_SM) operand_kerne
         if (!job_active(J) || J.kp1 <= OP_SHORT_K1) continue;  // inactive, or operand_packed_kernel's
         const uint32_t row = gr - J.row0;
         if (row >= J.n) {  // padding between jobs: zero operands (read only as masked rows/columns)
+            if (lane == 0) G.colterm[gr] = 0.0f;
             for (uint32_t t = lane; t < G.kpmax; t += 32) {
                 if (G.elem_bytes == 4) {
                     reinterpret_cast<uint32_t *>(G.opa)[(size_t)gr * G.kpmax + t] = 0u;
@@ -297,6 +343,9 @@ __global__ void __launch_bounds__(OP_WARPS * 32, OP_BLOCKS_PER_SM)
     __shared__ double s_wmax[OP_WARPS][OP_TILE][6];
     __shared__ unsigned long long s_wzero[OP_WARPS][OP_TILE];
     const GroupDev &G = *Gp;
+    grid_ready();
+    if (group_idle(jobs, G)) return;
+    clear_column_tail(G);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const JobDev *cur = nullptr;  // the job whose maxima the warp holds
     auto reset = [&]() {
@@ -342,6 +391,7 @@ __global__ void __launch_bounds__(OP_WARPS * 32, OP_BLOCKS_PER_SM)
         for (uint32_t p = 0; p < OP_TILE; ++p) {
             const uint32_t gr = gr0 + p;
             if (gr < G.rows && gr - J.row0 >= J.n) {
+                if (lane == 0) G.colterm[gr] = 0.0f;
                 for (uint32_t t = lane; t < G.kpmax; t += 32) {
                     if (G.elem_bytes == 4) {
                         reinterpret_cast<uint32_t *>(G.opa)[(size_t)gr * G.kpmax + t] = 0u;
@@ -501,6 +551,8 @@ __device__ __forceinline__ uint32_t band_of_row(const JobDev &J, const GroupDev 
 // Keep band 2E_i per row (see screen.cuh for the terms).
 __global__ void band_kernel(const JobDev *__restrict__ jobs, const GroupDev *__restrict__ Gp) {
     const GroupDev &G = *Gp;
+    grid_ready();
+    if (group_idle(jobs, G)) return;
     // a warp's 32 group rows belong to one job (each job's rows start
     // 32-aligned; G.rows is a multiple of 32)
     const uint32_t gr = blockIdx.x * blockDim.x + threadIdx.x;
@@ -517,35 +569,38 @@ __global__ void band_kernel(const JobDev *__restrict__ jobs, const GroupDev *__r
 
 int launch_screen_prep(const JobDev *jobs, const GroupDev &G, const GroupDev *Gd, cudaStream_t s) {
     ScopedKernelTimer timer(HM_KCLASS_PREP, s);
-    HM_CUDA_TRY(cudaMemsetAsync(G.colterm, 0, round_up(G.rows, SC_BN) * sizeof(float) + SC_BN * sizeof(float), s));
-    colsum_partial_kernel<<<G.njobs * CSUM_BLOCKS, 128, 0, s>>>(jobs, Gd);
-    colmean_kernel<<<G.njobs, 128, 0, s>>>(jobs, Gd);
-    // G.rows is a multiple of 32: 32 group rows per block
-    centred_norm_max_kernel<<<G.rows / 32, 256, 0, s>>>(jobs, Gd);
+    if (G.any_euclidean) {
+        HM_CUDA_TRY(launch(true, column_mean_kernel, G.njobs * CSUM_BLOCKS, CSUM_THREADS, 0, s, jobs, Gd));
+        // G.rows is a multiple of 32: 32 group rows per block
+        HM_CUDA_TRY(launch(true, centred_norm_max_kernel, G.rows / 32, 256, 0, s, jobs, Gd));
+        count_launch(2);
+    }
     const uint32_t op_cap = (uint32_t)device_sm_count() * OP_BLOCKS_PER_SM;
     const uint32_t row_blocks = (G.rows + OP_WARPS - 1) / OP_WARPS;
     const uint32_t row_grid = row_blocks < op_cap ? row_blocks : op_cap;
     const uint32_t tile_blocks = (G.rows + OP_WARPS * OP_TILE - 1) / (OP_WARPS * OP_TILE);
     const uint32_t tile_grid = tile_blocks < op_cap ? tile_blocks : op_cap;
     auto both = [&](auto rows_kernel, auto packed_kernel) {
-        if (G.any_long_rows) rows_kernel<<<row_grid, OP_WARPS * 32, 0, s>>>(jobs, Gd);
-        if (G.any_short_rows) packed_kernel<<<tile_grid, OP_WARPS * 32, 0, s>>>(jobs, Gd);
+        cudaError_t e = cudaSuccess;
+        if (G.any_long_rows) e = launch(true, rows_kernel, row_grid, OP_WARPS * 32, 0, s, jobs, Gd);
+        if (e == cudaSuccess && G.any_short_rows) e = launch(true, packed_kernel, tile_grid, OP_WARPS * 32, 0, s, jobs, Gd);
+        return e;
     };
+    cudaError_t err;
     if (G.kind == SCREEN_KIND_TF32)
-        both(operand_kernel<OP_TF32>, operand_packed_kernel<OP_TF32>);
+        err = both(operand_kernel<OP_TF32>, operand_packed_kernel<OP_TF32>);
     else if (!G.split)
-        both(operand_kernel<OP_BF16>, operand_packed_kernel<OP_BF16>);
+        err = both(operand_kernel<OP_BF16>, operand_packed_kernel<OP_BF16>);
     else
-        both(operand_kernel<OP_SPLIT>, operand_packed_kernel<OP_SPLIT>);
-    HM_CUDA_TRY(cudaGetLastError());
-    count_launch(3 + (G.any_long_rows ? 1 : 0) + (G.any_short_rows ? 1 : 0));
+        err = both(operand_kernel<OP_SPLIT>, operand_packed_kernel<OP_SPLIT>);
+    HM_CUDA_TRY(err);
+    count_launch((G.any_long_rows ? 1 : 0) + (G.any_short_rows ? 1 : 0));
     return HM_OK;
 }
 
 int launch_screen_band(const JobDev *jobs, const GroupDev &G, const GroupDev *Gd, cudaStream_t s) {
     ScopedKernelTimer timer(HM_KCLASS_PREP, s);
-    band_kernel<<<(G.rows + 255) / 256, 256, 0, s>>>(jobs, Gd);
-    HM_CUDA_TRY(cudaGetLastError());
+    HM_CUDA_TRY(launch(true, band_kernel, (G.rows + 255) / 256, 256, 0, s, jobs, Gd));
     count_launch();
     return HM_OK;
 }

@@ -27,6 +27,7 @@ constexpr uint32_t SK_MAX_K = 256;  // widest row of smooth_rows_kernel
 __global__ void __launch_bounds__(256) smooth_knn_kernel(const JobDev *__restrict__ jobs, uint32_t njobs,
                                                          const uint32_t *__restrict__ row_starts,
                                                          uint32_t rows) {
+    grid_ready();
     const int lane = threadIdx.x & 31;
     const uint32_t ar = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (ar >= rows) return;
@@ -153,6 +154,7 @@ __global__ void __launch_bounds__(128, G == 1 ? 4 : 6) smooth_rows_kernel(const 
                                                           uint32_t k_lo) {
     constexpr unsigned FULL = 0xffffffffu;
     constexpr float PAD = 1e30f;  // gap of the positions that are not summed: exp(-PAD c) = 0
+    grid_ready();
     const int lane = threadIdx.x & 31;
     const uint32_t q = threadIdx.x & (G - 1);
     const uint32_t at = (blockIdx.x * blockDim.x + threadIdx.x) / G;
@@ -324,16 +326,16 @@ __global__ void __launch_bounds__(128, G == 1 ? 4 : 6) smooth_rows_kernel(const 
 
 template <int G, int NV>
 static int launch_rows(const JobDev *jobs, uint32_t njobs, const uint32_t *row_starts, uint32_t rows, uint32_t k_lo,
-                       cudaStream_t s) {
+                       cudaStream_t s, bool overlap) {
     constexpr uint32_t per_block = 128 / G;
-    smooth_rows_kernel<G, NV><<<(rows + per_block - 1) / per_block, 128, 0, s>>>(jobs, njobs, row_starts, rows, k_lo);
-    HM_CUDA_TRY(cudaGetLastError());
+    HM_CUDA_TRY(launch(overlap, smooth_rows_kernel<G, NV>, (rows + per_block - 1) / per_block, 128, 0, s, jobs, njobs,
+                       row_starts, rows, k_lo));
     count_launch();
     return HM_OK;
 }
 
 int launch_smooth(const JobDev *jobs, uint32_t njobs, const uint32_t *row_starts, uint32_t rows,
-                  uint32_t kmax, cudaStream_t s) {
+                  uint32_t kmax, cudaStream_t s, bool overlap) {
     ScopedKernelTimer timer(HM_KCLASS_SMOOTH, s);
     // Lanes per row: more shorten a row's chain, fewer waste less on shuffles
     // and on waiting for the warp's slowest row.  Measured (whole calibration):
@@ -341,21 +343,20 @@ int launch_smooth(const JobDev *jobs, uint32_t njobs, const uint32_t *row_starts
     // 20.5 / 18.5 / 20.6; 50,000 rows 34.7 / 28.7 / 24.6.  k = 30: 50,000 rows
     // 45.1 / 41.0 / 66.2.  k = 100, 10,000 rows: 16 lanes 45.0, 32 lanes 49.4.
     if (kmax <= 16) {
-        if (rows < 16384) HM_TRY((launch_rows<8, 2>(jobs, njobs, row_starts, rows, 0, s)));
-        else if (rows < 32768) HM_TRY((launch_rows<4, 4>(jobs, njobs, row_starts, rows, 0, s)));
-        else HM_TRY((launch_rows<1, 16>(jobs, njobs, row_starts, rows, 0, s)));
+        if (rows < 16384) HM_TRY((launch_rows<8, 2>(jobs, njobs, row_starts, rows, 0, s, overlap)));
+        else if (rows < 32768) HM_TRY((launch_rows<4, 4>(jobs, njobs, row_starts, rows, 0, s, overlap)));
+        else HM_TRY((launch_rows<1, 16>(jobs, njobs, row_starts, rows, 0, s, overlap)));
     } else if (kmax <= 32 || njobs > 1) {
-        if (rows < 16384) HM_TRY((launch_rows<8, 4>(jobs, njobs, row_starts, rows, 0, s)));
-        else HM_TRY((launch_rows<4, 8>(jobs, njobs, row_starts, rows, 0, s)));
+        if (rows < 16384) HM_TRY((launch_rows<8, 4>(jobs, njobs, row_starts, rows, 0, s, overlap)));
+        else HM_TRY((launch_rows<4, 8>(jobs, njobs, row_starts, rows, 0, s, overlap)));
     }
     if (kmax > 32 && !(njobs == 1 && kmax > SK_MAX_K)) {
-        if (kmax <= 64) HM_TRY((launch_rows<16, 4>(jobs, njobs, row_starts, rows, 32, s)));
-        else if (kmax <= 128) HM_TRY((launch_rows<16, 8>(jobs, njobs, row_starts, rows, 32, s)));
-        else HM_TRY((launch_rows<16, 16>(jobs, njobs, row_starts, rows, 32, s)));
+        if (kmax <= 64) HM_TRY((launch_rows<16, 4>(jobs, njobs, row_starts, rows, 32, s, overlap)));
+        else if (kmax <= 128) HM_TRY((launch_rows<16, 8>(jobs, njobs, row_starts, rows, 32, s, overlap)));
+        else HM_TRY((launch_rows<16, 16>(jobs, njobs, row_starts, rows, 32, s, overlap)));
     }
     if (kmax > SK_MAX_K) {
-        smooth_knn_kernel<<<(int)((rows + 7) / 8), 256, 0, s>>>(jobs, njobs, row_starts, rows);
-        HM_CUDA_TRY(cudaGetLastError());
+        HM_CUDA_TRY(launch(overlap, smooth_knn_kernel, (rows + 7) / 8, 256, 0, s, jobs, njobs, row_starts, rows));
         count_launch();
     }
     return HM_OK;
@@ -367,6 +368,7 @@ int launch_smooth(const JobDev *jobs, uint32_t njobs, const uint32_t *row_starts
 // stage the next values through shared memory.  Idle when no row of the job
 // had rho == 0.
 __global__ void __launch_bounds__(256) mean_all_floor_kernel(const JobDev *__restrict__ jobs) {
+    grid_ready();
     const JobDev &J = jobs[blockIdx.x];
     if (!J.sigma || !J.rho) return;
     const uint32_t cnt = J.cnt->zero_count;
@@ -400,8 +402,7 @@ __global__ void __launch_bounds__(256) mean_all_floor_kernel(const JobDev *__res
 
 int launch_mean_all_floor(const JobDev *jobs, uint32_t njobs, cudaStream_t s) {
     ScopedKernelTimer timer(HM_KCLASS_SMOOTH, s);
-    mean_all_floor_kernel<<<njobs, 256, 0, s>>>(jobs);
-    HM_CUDA_TRY(cudaGetLastError());
+    HM_CUDA_TRY(launch(true, mean_all_floor_kernel, njobs, 256, 0, s, jobs));
     count_launch();
     return HM_OK;
 }
