@@ -173,36 +173,6 @@ __global__ void __launch_bounds__(256) fuzzy_scatter_kernel(const FuzzyDev D) {
         if (w[q] != 0.0f) D.stage[at[q]] = make_uint2((e0 + 256 * q) / D.k, __float_as_uint(w[q]));
 }
 
-// Bitonic sort, ascending, of 32 * NQ keys, element lane * NQ + q in v[q]: strides
-// below NQ stay in the lane.
-template <typename K, int NQ>
-__device__ __forceinline__ void warp_sort(K (&v)[NQ], uint32_t lane) {
-#pragma unroll
-    for (uint32_t size = 2; size <= 32 * NQ; size <<= 1) {
-#pragma unroll
-        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-            if (stride >= NQ) {
-                const uint32_t ls = stride / NQ;
-                const bool keep_min = ((lane & ls) == 0) == ((lane & (size / NQ)) == 0);
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) {
-                    const K o = __shfl_xor_sync(FZ_FULL, v[q], ls);
-                    v[q] = keep_min ? min(v[q], o) : max(v[q], o);
-                }
-            } else {
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) {
-                    if (q & stride) continue;
-                    const K a = min(v[q], v[q | stride]), b = max(v[q], v[q | stride]);
-                    const bool up = size < NQ ? (q & size) == 0 : (lane & (size / NQ)) == 0;
-                    v[q] = up ? a : b;
-                    v[q | stride] = up ? b : a;
-                }
-            }
-        }
-    }
-}
-
 // A row of at most 32 * NQ slots: keys column << 9 | slot (F slots below k, so an
 // F entry precedes its R partner), strengths in shared memory by slot.
 template <typename K, int NQ>

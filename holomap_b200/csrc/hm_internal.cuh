@@ -129,6 +129,36 @@ __device__ __forceinline__ uint64_t shfl_up_u64(uint64_t v, int delta) {
     return ((uint64_t)hi << 32) | lo;
 }
 
+// Bitonic sort, ascending, of 32 * NQ keys, element lane * NQ + q in v[q]: strides
+// below NQ stay in the lane.
+template <typename K, int NQ>
+__device__ __forceinline__ void warp_sort(K (&v)[NQ], uint32_t lane) {
+#pragma unroll
+    for (uint32_t size = 2; size <= 32 * NQ; size <<= 1) {
+#pragma unroll
+        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+            if (stride >= NQ) {
+                const uint32_t ls = stride / NQ;
+                const bool keep_min = ((lane & ls) == 0) == ((lane & (size / NQ)) == 0);
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) {
+                    const K o = __shfl_xor_sync(0xffffffffu, v[q], ls);
+                    v[q] = keep_min ? min(v[q], o) : max(v[q], o);
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) {
+                    if (q & stride) continue;
+                    const K a = min(v[q], v[q | stride]), b = max(v[q], v[q | stride]);
+                    const bool up = size < NQ ? (q & size) == 0 : (lane & (size / NQ)) == 0;
+                    v[q] = up ? a : b;
+                    v[q | stride] = up ? b : a;
+                }
+            }
+        }
+    }
+}
+
 // A sorted list of the KPL*32 smallest keys seen, spread over a warp: element
 // e lives in lane (e % 32) of slot (e / 32).  `tau` is element k-1, the
 // admission threshold (warp-uniform).  Insert is warp-collective and requires
@@ -176,12 +206,7 @@ struct WarpTopK {
     // smallest as one bitonic sequence.
     template <bool SORTED = false>
     __device__ __forceinline__ void merge32(uint64_t b, uint32_t k, int lane) {
-        if (!SORTED) {
-#pragma unroll
-            for (int size = 2; size <= 32; size <<= 1)
-#pragma unroll
-                for (int stride = size >> 1; stride > 0; stride >>= 1) b = exchange(b, stride, (lane & size) == 0, lane);
-        }
+        if (!SORTED) b = sort32(b, lane);
         const uint64_t rb = shfl_u64(b, 31 - lane);
         v[KPL - 1] = v[KPL - 1] < rb ? v[KPL - 1] : rb;
 #pragma unroll
@@ -198,6 +223,14 @@ struct WarpTopK {
 #pragma unroll
             for (int stride = 16; stride > 0; stride >>= 1) v[q] = exchange(v[q], stride, true, lane);
         refresh_tau(k, lane);
+    }
+    // 32 keys, one per lane, ascending
+    static __device__ __forceinline__ uint64_t sort32(uint64_t b, int lane) {
+#pragma unroll
+        for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll
+            for (int stride = size >> 1; stride > 0; stride >>= 1) b = exchange(b, stride, (lane & size) == 0, lane);
+        return b;
     }
     // compare-exchange with lane ^ stride, ascending where `up`
     static __device__ __forceinline__ uint64_t exchange(uint64_t x, int stride, bool up, int lane) {

@@ -93,6 +93,19 @@ __device__ __forceinline__ uint32_t kth_key(const uint32_t (&ov)[NQ], uint32_t t
     return min(r | ((1u << lo) - 1u), mx);
 }
 
+// The k-th smallest of a warp's 32 * NQ keys (absent ones ~0) by sorting them: up
+// to 128 keys this takes fewer instructions than a search by bits or bytes
+// (256 datasets, sorts here, in the select and in the top-k: 6,186 -> 5,753 us;
+// 5,000 x 128 cosine, k = 20: 331 -> 322).
+template <int NQ>
+__device__ __forceinline__ uint32_t kth_sorted(uint32_t (&v)[NQ], uint32_t k, int lane) {
+    warp_sort<uint32_t, NQ>(v, (uint32_t)lane);
+    uint32_t x = v[0];
+#pragma unroll
+    for (int q = 1; q < NQ; ++q) x = (k - 1) % NQ == (uint32_t)q ? v[q] : x;
+    return __shfl_sync(0xffffffffu, x, (int)((k - 1) / NQ));
+}
+
 // kth_key over keys key(e), e < total <= 512, with the register count chosen by
 // the total; `below(kth)` names a key, the count of keys at or below it is
 // returned in `under` (skipped when it returns 0)
@@ -105,7 +118,12 @@ __device__ __forceinline__ uint32_t kth_load(KeyFn key, uint32_t total, uint32_t
         const uint32_t e = q * 32 + lane;
         ov[q] = e < total ? key(e) : 0xffffffffu;
     }
-    const uint32_t kth = kth_key<NQ>(ov, total, k, lo, lane);
+    uint32_t kth;
+    if (NQ <= 4) {
+        kth = kth_sorted<NQ>(ov, k, lane);
+    } else {
+        kth = kth_key<NQ>(ov, total, k, lo, lane);
+    }
     const uint32_t limit = below(kth);
     under = 0;
     if (limit) {
@@ -258,6 +276,7 @@ __device__ __forceinline__ uint32_t kth_staged(const unsigned long long *cbuf, u
         const uint32_t e = q * 32 + lane;
         key[q] = e < total ? ord32(__uint_as_float((uint32_t)(cbuf[e] >> 32))) : 0xffffffffu;
     }
+    if (NQ <= 4) return kth_sorted<NQ>(key, k, lane);
     return radix_kth<NQ>(key, total, k, hist, lane);
 }
 
@@ -323,7 +342,9 @@ __device__ __forceinline__ uint32_t select_row(const JobDev &J, const GroupDev &
         __syncwarp();
         if (total >= k) {
             uint32_t r;
-            if (total <= 128) r = kth_staged<4>(sm.cbuf, total, k, sm.hist, lane);
+            if (total <= 32) r = kth_staged<1>(sm.cbuf, total, k, sm.hist, lane);
+            else if (total <= 64) r = kth_staged<2>(sm.cbuf, total, k, sm.hist, lane);
+            else if (total <= 128) r = kth_staged<4>(sm.cbuf, total, k, sm.hist, lane);
             else if (total <= 256) r = kth_staged<8>(sm.cbuf, total, k, sm.hist, lane);
             else r = kth_staged<16>(sm.cbuf, total, k, sm.hist, lane);
             tau = unord32(r);
@@ -597,7 +618,8 @@ __device__ __forceinline__ void bitonic64(uint64_t &a, uint64_t &b, int lane) {
 }
 
 // Top-k phase: one warp per group row; the k smallest exact keys of the
-// row's survivors are its output.
+// row's survivors are its output (sorted in registers up to 64, in merges of 32
+// beyond).
 template <int KPL>
 __global__ void __launch_bounds__(RS_WARPS * 32) rr_topk_kernel(const JobDev *__restrict__ jobs,
                                                                 const GroupDev *__restrict__ Gp) {
@@ -614,6 +636,14 @@ __global__ void __launch_bounds__(RS_WARPS * 32) rr_topk_kernel(const JobDev *__
     const unsigned long long *keys = row_region(J, G, row);
     uint32_t *idx = J.idx + (size_t)row * k;
     float *dist = J.dist + (size_t)row * k;
+    if (c <= 32) {
+        const uint64_t key = WarpTopK<1>::sort32((uint32_t)lane < c ? (uint64_t)keys[lane] : KEY_NONE, lane);
+        if ((uint32_t)lane < k) {
+            idx[lane] = key_idx(key);
+            dist[lane] = key_dist(key);
+        }
+        return;
+    }
     if (c <= 64) {
         uint64_t a = (uint32_t)lane < c ? (uint64_t)keys[lane] : KEY_NONE;
         uint64_t b = 32u + lane < c ? (uint64_t)keys[32 + lane] : KEY_NONE;
@@ -630,7 +660,10 @@ __global__ void __launch_bounds__(RS_WARPS * 32) rr_topk_kernel(const JobDev *__
     }
     WarpTopK<KPL> top;
     top.reset();
-    for (uint32_t e0 = 0; e0 < c; e0 += 32) top.offer(e0 + lane < c ? (uint64_t)keys[e0 + lane] : KEY_NONE, k, lane);
+    for (uint32_t e0 = 0; e0 < c; e0 += 32) {
+        const uint64_t key = e0 + lane < c ? (uint64_t)keys[e0 + lane] : KEY_NONE;
+        if (__any_sync(0xffffffffu, key < top.tau)) top.merge32(key, k, lane);
+    }
 #pragma unroll
     for (int q = 0; q < KPL; ++q) {
         const uint32_t e = q * 32 + lane;
