@@ -125,7 +125,7 @@ struct GroupPlan {
     size_t off_opa = 0, off_opb = 0, off_rowstat = 0, off_rowterm = 0, off_colterm = 0;
     size_t off_band = 0, off_force = 0, off_rowthr = 0, off_cand = 0, off_cnt = 0, off_topk = 0;
     size_t off_ethr = 0, off_evstar = 0, off_stage_row = 0, off_stage_key = 0, off_stage_cnt = 0;
-    size_t off_rowcnt = 0;
+    size_t off_rowcnt = 0, off_job_of = 0;
     // tables
     size_t off_gdev = 0, off_job_ids = 0, off_row_starts = 0, off_unit_starts = 0, off_eunits = 0;
     GroupDev host{};
@@ -144,7 +144,10 @@ struct hm_batch {
     uint32_t nitems[3] = {0, 0, 0};    // and their items
     std::vector<uint32_t> fb_jobs[3];  // screened jobs per metric (fallback rows)
     uint32_t fb_per_job[3] = {1, 1, 1};
-    bool any_plain = false, any_screen = false, any_smooth = false, any_split = false;
+    std::vector<uint2> merges;  // exact-path jobs with column splits: (job, first of its rows in the merge)
+    uint32_t merge_rows = 0;
+    size_t off_merge = 0;
+    bool any_plain = false, any_screen = false, any_smooth = false;
     size_t off_tables = 0, off_jobs = 0, off_counters = 0, off_row_starts = 0;
     size_t off_items[3] = {}, off_fb[3] = {};
     size_t tables_bytes = 0, tables_used = 0, total = 0;
@@ -294,7 +297,6 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
         }
         P.split_cols = (uint32_t)round_up((n + splits - 1) / splits, PL_BN);
         P.splits = (uint32_t)((n + P.split_cols - 1) / P.split_cols);
-        if (P.splits > 1) B.any_split = true;
     }
 
     // screen groups
@@ -479,6 +481,10 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
             const uint32_t groups = (P.q1 + PL_BM - 1) / PL_BM - P.q0 / PL_BM;
             B.items[m].push_back(make_uint2(j, B.nitems[m]));
             B.nitems[m] += groups * P.splits;
+            if (P.splits > 1) {
+                B.merges.push_back(make_uint2(j, B.merge_rows));
+                B.merge_rows += (uint32_t)P.spec.n;
+            }
             B.kpl_plain[m] = std::max<uint32_t>(B.kpl_plain[m], (uint32_t)kpl_for_k(P.spec.k));
         } else if (P.clone_of < 0) {
             // (an escalation copy's fallback rows are the original's: same
@@ -508,6 +514,7 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
     };
     B.off_jobs = pack(sizeof(JobDev) * njobs);
     B.off_row_starts = pack(sizeof(uint32_t) * (njobs + 1));
+    B.off_merge = pack(sizeof(uint2) * B.merges.size());
     for (int m = 0; m < 3; ++m) {
         B.off_items[m] = pack(sizeof(uint2) * B.items[m].size());
         B.off_fb[m] = pack(sizeof(uint32_t) * B.fb_jobs[m].size());
@@ -570,6 +577,7 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
         Gp.off_cnt = take(Gp.elists * sizeof(uint32_t));
         Gp.off_topk = take(Gp.topk * sizeof(float));
         Gp.off_rowcnt = take(rows * sizeof(uint32_t));
+        if (Gp.jobs.size() > 1) Gp.off_job_of = take((rows + 31) / 32 * sizeof(uint32_t));
         if (Gp.any_sym) {
             const size_t padded = round_up(rows, SC_BN) + SC_BN;
             Gp.off_ethr = take(padded * sizeof(float));
@@ -694,6 +702,7 @@ static int bind_batch(hm_batch &B, void *d_ws, size_t bytes, cudaStream_t s) {
         row_starts[j + 1] = row_starts[j] + J.n;
     }
     memcpy(host + B.off_row_starts, row_starts.data(), sizeof(uint32_t) * (njobs + 1));
+    if (!B.merges.empty()) memcpy(host + B.off_merge, B.merges.data(), sizeof(uint2) * B.merges.size());
     for (int m = 0; m < 3; ++m) {
         if (!B.items[m].empty())
             memcpy(host + B.off_items[m], B.items[m].data(), sizeof(uint2) * B.items[m].size());
@@ -741,6 +750,7 @@ static int bind_batch(hm_batch &B, void *d_ws, size_t bytes, cudaStream_t s) {
         D.cand_cnt = at<uint32_t>(ws, Gp.off_cnt);
         D.topk = at<float>(ws, Gp.off_topk);
         D.row_cnt = at<uint32_t>(ws, Gp.off_rowcnt);
+        D.job_of = Gp.jobs.size() > 1 ? at<uint32_t>(ws, Gp.off_job_of) : nullptr;
         D.eunits = Gp.eunits.empty() ? nullptr : at<uint4>(ws, Gp.off_eunits);
         D.neunits = Gp.neunits;
         D.any_euclidean = (Gp.metric_mask >> HM_METRIC_EUCLIDEAN) & 1;
@@ -778,6 +788,8 @@ static int bind_batch(hm_batch &B, void *d_ws, size_t bytes, cudaStream_t s) {
         HM_CUDA_TRY(cudaGetLastError());
         count_launch();
     }
+    for (int g = 0; g < 3; ++g)
+        if (B.groups[g].jobs.size() > 1) HM_TRY(launch_job_of(B.groups[g].host, s));
     return HM_OK;
 }
 
@@ -837,8 +849,8 @@ static int run_batch(hm_batch &B, cudaStream_t s) {
             HM_TRY(launch_plain(w, m, s));
         }
     }
-    if (B.any_split)
-        HM_TRY(launch_merge(jobs, njobs, njobs > 1 ? row_starts : nullptr, B.all_rows, B.kpl_all, s));
+    if (!B.merges.empty())
+        HM_TRY(launch_merge(jobs, at<uint2>(ws, B.off_merge), (uint32_t)B.merges.size(), B.merge_rows, B.kpl_all, s));
     if (B.any_smooth) {
         HM_TRY(launch_smooth(jobs, njobs, njobs > 1 ? row_starts : nullptr, B.all_rows, B.kmax, s));
         HM_TRY(launch_mean_all_floor(jobs, njobs, s));

@@ -384,9 +384,10 @@ struct PlainWork {
 int launch_check(const JobDev *jobs, uint32_t njobs, const uint32_t *row_starts, uint32_t all_rows, cudaStream_t s);
 
 int launch_plain(const PlainWork &w, int metric, cudaStream_t s);
-// merges split lists of every exact-path job with splits > 1
-int launch_merge(const JobDev *jobs, uint32_t njobs, const uint32_t *row_starts, uint32_t rows,
-                 uint32_t kpl, cudaStream_t s);
+// merges the split lists of the exact-path jobs with splits > 1: `merges` holds
+// (job, first of its rows among the `rows` of the merge)
+int launch_merge(const JobDev *jobs, const uint2 *merges, uint32_t nmerges, uint32_t rows, uint32_t kpl,
+                 cudaStream_t s);
 
 // ------------------------------------------------------------- smooth kNN
 // Per row of every job with smooth-kNN outputs (row_starts: all-rows space);

@@ -461,17 +461,20 @@ int launch_plain(const PlainWork &w, int metric, cudaStream_t s) {
 // ------------------------------------------------------------ split merge
 // One warp per row of an exact-path job with splits > 1 folds its split lists.
 template <int KPL>
-__global__ void __launch_bounds__(256) merge_splits_kernel(const JobDev *__restrict__ jobs, uint32_t njobs,
-                                                           const uint32_t *__restrict__ row_starts,
+__global__ void __launch_bounds__(256) merge_splits_kernel(const JobDev *__restrict__ jobs,
+                                                           const uint2 *__restrict__ merges, uint32_t nmerges,
                                                            uint32_t rows) {
     grid_ready();
     const int lane = threadIdx.x & 31;
-    const uint32_t ar = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (ar >= rows) return;
-    const uint32_t jb = row_starts ? find_job(row_starts, njobs, ar) : 0;
-    const JobDev &J = jobs[jb];
-    if (J.path != HM_PATH_PLAIN || J.splits <= 1) return;
-    const uint32_t row = ar - J.arow0, k = J.k;
+    const uint32_t mr = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (mr >= rows) return;
+    uint32_t lo = 0, hi = nmerges;  // the job whose rows hold this one
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (merges[mid].y <= mr) lo = mid; else hi = mid;
+    }
+    const JobDev &J = jobs[merges[lo].x];
+    const uint32_t row = mr - merges[lo].y, k = J.k;
     if (row < J.q0 || row >= J.q1) return;
     WarpTopK<KPL> top;
 #pragma unroll
@@ -498,8 +501,8 @@ __global__ void __launch_bounds__(256) merge_splits_kernel(const JobDev *__restr
     }
 }
 
-int launch_merge(const JobDev *jobs, uint32_t njobs, const uint32_t *row_starts, uint32_t rows,
-                 uint32_t kpl, cudaStream_t s) {
+int launch_merge(const JobDev *jobs, const uint2 *merges, uint32_t nmerges, uint32_t rows, uint32_t kpl,
+                 cudaStream_t s) {
     const int blocks = (int)((rows + 7) / 8);
     ScopedKernelTimer timer(HM_KCLASS_SELECT, s);
     auto *merge = kpl == 1   ? merge_splits_kernel<1>
@@ -508,7 +511,7 @@ int launch_merge(const JobDev *jobs, uint32_t njobs, const uint32_t *row_starts,
                   : kpl == 8 ? merge_splits_kernel<8>
                              : nullptr;
     if (!merge) return set_error(HM_ERR_UNSUPPORTED, "select width %u", kpl);
-    HM_CUDA_TRY(launch(true, merge, blocks, 256, 0, s, jobs, njobs, row_starts, rows));
+    HM_CUDA_TRY(launch(true, merge, blocks, 256, 0, s, jobs, merges, nmerges, rows));
     count_launch();
     return HM_OK;
 }

@@ -280,6 +280,16 @@ __device__ __forceinline__ uint32_t kth_staged(const unsigned long long *cbuf, u
     return radix_kth<NQ>(key, total, k, hist, lane);
 }
 
+// ... of a row's first min(total, 32 * NQ) candidates
+template <int NQ>
+__device__ __forceinline__ uint32_t kth_first(const unsigned long long (&v)[4], uint32_t total, uint32_t k, int lane) {
+    uint32_t key[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
+        key[q] = q * 32u + lane < total ? ord32(__uint_as_float((uint32_t)(v[q] >> 32))) : 0xffffffffu;
+    return kth_sorted<NQ>(key, k, lane);
+}
+
 // Select phase for one row: returns the survivor count (0 for rows sent to
 // the exact fallback).
 template <int KPL>
@@ -307,18 +317,24 @@ __device__ __forceinline__ uint32_t select_row(const JobDev &J, const GroupDev &
     const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
     unsigned long long *region = row_region(J, G, row);
     // Threshold: the k-th smallest screened value of the row over the emitted
-    // candidates (they include the row's k smallest).  Up to RR_CBUF
-    // candidates are staged in shared memory (every list's chunk c loaded
-    // before any is stored) and the k-th bounded from above by a radix select
-    // (to its lowest key byte); longer rows use a warp top-k (exact).
+    // candidates (they include the row's k smallest); kept are those within the
+    // band of it.  Up to RR_CBUF candidates: the k-th of the first 128 bounds it,
+    // so only candidates within the band of that are staged in shared memory (all
+    // of the others are out) and searched for the k-th itself; up to 128
+    // candidates it is the k-th itself and nothing is staged.  (20,000 x 96, k = 15:
+    // 46.5 -> 40.6 us; 50,000 x 384: 172 -> 159.)  Longer rows use a warp top-k.
     const bool staged = total <= RR_CBUF;
+    const float band = G.band[gr];
+    const unsigned lt_mask = (1u << lane) - 1u;
     float tau = __int_as_float(0x7f800000);
+    uint32_t nstaged = 0;
     if (staged) {
-        // flat copy: staged position e lies in the last list whose first
-        // position is <= e (an empty list shares its successor's first
-        // position, so the search lands on the list that holds e)
+        // flat position e lies in the last list whose first position is <= e (an
+        // empty list shares its successor's first position, so the search lands
+        // on the list that holds e)
         if ((uint32_t)lane < lists) sm.loff[lane] = incl - myc;
         __syncwarp();
+        float thr = __int_as_float(0x7f800000);
         for (uint32_t e0 = 0; e0 < total; e0 += 128) {
             unsigned long long v[4];
 #pragma unroll
@@ -333,20 +349,32 @@ __device__ __forceinline__ uint32_t select_row(const JobDev &J, const GroupDev &
                     v[u] = region[(size_t)lo * J.cap + (e - sm.loff[lo])];
                 }
             }
+            if (e0 == 0 && k <= total) {  // (k <= 64)
+                const uint32_t kth = total <= 32 ? kth_first<1>(v, total, k, lane)
+                                   : total <= 64 ? kth_first<2>(v, total, k, lane)
+                                                 : kth_first<4>(v, total, k, lane);
+                thr = __fadd_ru(unord32(kth), band);
+            }
+            // (a short row's candidates are all in registers before the first is overwritten)
+            unsigned long long *dst = total <= 128 ? region : sm.cbuf;
+            __syncwarp();
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                const uint32_t e = e0 + 32 * u + lane;
-                if (e < total) sm.cbuf[e] = v[u];
+                const bool pass = e0 + 32 * u + lane < total && !(__uint_as_float((uint32_t)(v[u] >> 32)) > thr);
+                const unsigned m = __ballot_sync(0xffffffffu, pass);
+                if (pass) dst[nstaged + __popc(m & lt_mask)] = v[u];
+                nstaged += __popc(m);
             }
         }
         __syncwarp();
-        if (total >= k) {
+        if (total <= 128) return nstaged;
+        if (nstaged >= k) {
             uint32_t r;
-            if (total <= 32) r = kth_staged<1>(sm.cbuf, total, k, sm.hist, lane);
-            else if (total <= 64) r = kth_staged<2>(sm.cbuf, total, k, sm.hist, lane);
-            else if (total <= 128) r = kth_staged<4>(sm.cbuf, total, k, sm.hist, lane);
-            else if (total <= 256) r = kth_staged<8>(sm.cbuf, total, k, sm.hist, lane);
-            else r = kth_staged<16>(sm.cbuf, total, k, sm.hist, lane);
+            if (nstaged <= 32) r = kth_staged<1>(sm.cbuf, nstaged, k, sm.hist, lane);
+            else if (nstaged <= 64) r = kth_staged<2>(sm.cbuf, nstaged, k, sm.hist, lane);
+            else if (nstaged <= 128) r = kth_staged<4>(sm.cbuf, nstaged, k, sm.hist, lane);
+            else if (nstaged <= 256) r = kth_staged<8>(sm.cbuf, nstaged, k, sm.hist, lane);
+            else r = kth_staged<16>(sm.cbuf, nstaged, k, sm.hist, lane);
             tau = unord32(r);
         }
     } else {
@@ -366,13 +394,12 @@ __device__ __forceinline__ uint32_t select_row(const JobDev &J, const GroupDev &
         }
         if (sel.tau != KEY_NONE) tau = unord32((uint32_t)(sel.tau >> 32));
     }
-    const float thr = __fadd_ru(tau, G.band[gr]);
+    const float thr = __fadd_ru(tau, band);
 
     // Compaction of the candidates within tau^ + band to the front of the
     // region.  From the lists themselves this is in place and safe: a write
     // lands at most at (entries kept so far) + 31 <= (position of the chunk
     // being read) + 31, every entry of which is already in registers.
-    const unsigned lt_mask = (1u << lane) - 1u;
     uint32_t fill = 0;
     auto compact = [&](const unsigned long long *src, uint32_t cnt) {
         for (uint32_t e0 = 0; e0 < cnt; e0 += 32) {
@@ -388,7 +415,7 @@ __device__ __forceinline__ uint32_t select_row(const JobDev &J, const GroupDev &
         }
     };
     if (staged) {
-        compact(sm.cbuf, total);
+        compact(sm.cbuf, nstaged);
     } else {
         for (uint32_t p = 0; p < lists; ++p) compact(region + (size_t)p * J.cap, G.cand_cnt[l0 + p]);
     }
@@ -410,7 +437,7 @@ __global__ void __launch_bounds__(RS_WARPS * 32, 4) rr_select_kernel(const JobDe
     RsWarpSmem &sm = reinterpret_cast<RsWarpSmem *>(rs_smem_raw)[warp];
     const uint32_t gr = blockIdx.x * RS_WARPS + warp;
     const uint32_t g0 = blockIdx.x * RS_WARPS;
-    const JobDev &J = jobs[G.job_ids[find_job(G.row_starts, G.njobs, g0 < G.rows ? g0 : 0u)]];
+    const JobDev &J = group_job(jobs, G, g0 < G.rows ? g0 : 0u);
     uint32_t c = 0;
     if (gr < G.rows) {
         const uint32_t row = gr - J.row0;
@@ -586,7 +613,7 @@ __global__ void __launch_bounds__(RR_WARPS * 32) rr_exact_kernel(const JobDev *_
     RrWarpSmem &sm = reinterpret_cast<RrWarpSmem *>(rr_smem_raw)[warp];
     const uint32_t gr0 = (blockIdx.x * RR_WARPS + warp) * ROWS;
     if (gr0 >= G.rows) return;
-    const JobDev &J = jobs[G.job_ids[find_job(G.row_starts, G.njobs, gr0)]];
+    const JobDev &J = group_job(jobs, G, gr0);
     const uint32_t cnt_l = lane < ROWS && gr0 + lane < G.rows ? G.row_cnt[gr0 + lane] : 0u;
     if (!__any_sync(0xffffffffu, cnt_l != 0)) return;
     if (J.metric == HM_METRIC_EUCLIDEAN)
@@ -631,7 +658,7 @@ __global__ void __launch_bounds__(RS_WARPS * 32) rr_topk_kernel(const JobDev *__
     if (gr >= G.rows) return;
     const uint32_t c = G.row_cnt[gr];
     if (c == 0) return;
-    const JobDev &J = jobs[G.job_ids[find_job(G.row_starts, G.njobs, gr)]];
+    const JobDev &J = group_job(jobs, G, gr);
     const uint32_t row = gr - J.row0, k = J.k;
     const unsigned long long *keys = row_region(J, G, row);
     uint32_t *idx = J.idx + (size_t)row * k;
@@ -687,7 +714,7 @@ __global__ void __launch_bounds__(256) emit_limits_kernel(const JobDev *__restri
     const float INF = __int_as_float(0x7f800000);
     float lim = -INF, vs = INF;
     if (gr < G.rows) {
-        const JobDev &J = jobs[G.job_ids[find_job(G.row_starts, G.njobs, gr)]];
+        const JobDev &J = group_job(jobs, G, gr);
         const uint32_t row = gr - J.row0;
         if (J.sym && row < J.n && !G.force[gr]) {
             const float b = G.band[gr];
@@ -722,7 +749,7 @@ __global__ void __launch_bounds__(256) column_scatter_kernel(const JobDev *__res
         const size_t at = (size_t)c * G.stage_cap + e;
         const uint32_t gr = G.stage_row[at];
         const unsigned long long key = G.stage_key[at];
-        const JobDev &J = jobs[G.job_ids[find_job(G.row_starts, G.njobs, gr)]];
+        const JobDev &J = group_job(jobs, G, gr);
         const uint32_t j = gr - J.row0, i = (uint32_t)key;
         const float v = __uint_as_float((uint32_t)(key >> 32));
         const float rt = J.metric == HM_METRIC_EUCLIDEAN ? G.colterm[gr] : 0.0f;
@@ -755,7 +782,7 @@ __global__ void __launch_bounds__(256) threshold_kernel(const JobDev *__restrict
     const int lane = threadIdx.x & 31;
     const uint32_t gr = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (gr >= G.rows) return;
-    const JobDev &J = jobs[G.job_ids[find_job(G.row_starts, G.njobs, gr)]];
+    const JobDev &J = group_job(jobs, G, gr);
     const uint32_t row = gr - J.row0;
     if (row < J.q0 || row >= J.q1 || !job_active(J)) return;
     const uint32_t k = J.k, lists = J.tlists * J.parts;
@@ -821,7 +848,7 @@ __global__ void __launch_bounds__(256) escalate_count_kernel(const JobDev *__res
     grid_ready();
     const uint32_t gr = blockIdx.x * blockDim.x + threadIdx.x;
     if (gr - (threadIdx.x & 31) >= G.rows) return;  // whole warps: 32 rows of one job
-    const JobDev &J = jobs[G.job_ids[find_job(G.row_starts, G.njobs, gr - (threadIdx.x & 31))]];
+    const JobDev &J = group_job(jobs, G, gr - (threadIdx.x & 31));
     if (!J.escalation) return;
     const uint32_t row = gr - J.row0;
     bool wide = false, swamped = false;

@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(256) centred_norm_max_kernel(const JobDev *__r
     grid_ready();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t gr0 = blockIdx.x * 32;
-    const JobDev &J = jobs[G->job_ids[find_job(G->row_starts, G->njobs, gr0)]];
+    const JobDev &J = group_job(jobs, *G, gr0);
     if (J.metric != HM_METRIC_EUCLIDEAN || !job_active(J)) return;  // uniform over the block
     double m = 0.0;
     for (uint32_t r = 0; r < 4; ++r) {
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(OP_WARPS * 32, OP_BLOCKS_PER_SM) operand_kerne
     reset();
     const uint32_t stride = gridDim.x * OP_WARPS;
     for (uint32_t gr = blockIdx.x * OP_WARPS + warp; gr < G.rows; gr += stride) {
-        const JobDev &J = jobs[G.job_ids[find_job(G.row_starts, G.njobs, gr)]];
+        const JobDev &J = group_job(jobs, G, gr);
         if (!job_active(J) || J.kp1 <= OP_SHORT_K1) continue;  // inactive, or operand_packed_kernel's
         const uint32_t row = gr - J.row0;
         if (row >= J.n) {  // padding between jobs: zero operands (read only as masked rows/columns)
@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(OP_WARPS * 32, OP_BLOCKS_PER_SM)
     const uint32_t stride = gridDim.x * OP_WARPS;
     for (uint32_t ti = blockIdx.x * OP_WARPS + warp; ti < tiles; ti += stride) {
         const uint32_t gr0 = ti * OP_TILE;
-        const JobDev &J = jobs[G.job_ids[find_job(G.row_starts, G.njobs, gr0)]];
+        const JobDev &J = group_job(jobs, G, gr0);
         // uniform over the warp (a tile is of one job); longer rows are operand_kernel's
         if (!job_active(J) || J.kp1 > OP_SHORT_K1) continue;
         if (&J != cur) {
@@ -557,7 +557,7 @@ __global__ void band_kernel(const JobDev *__restrict__ jobs, const GroupDev *__r
     // 32-aligned; G.rows is a multiple of 32)
     const uint32_t gr = blockIdx.x * blockDim.x + threadIdx.x;
     if (gr - (threadIdx.x & 31) >= G.rows) return;  // whole warps
-    const JobDev &J = jobs[G.job_ids[find_job(G.row_starts, G.njobs, gr)]];
+    const JobDev &J = group_job(jobs, G, gr);
     if (!job_active(J)) return;  // uniform over the warp (32 rows of one job)
     const bool real = gr < G.rows && gr - J.row0 < J.n;  // not padding between jobs
     uint32_t bits = 0;
@@ -566,6 +566,18 @@ __global__ void band_kernel(const JobDev *__restrict__ jobs, const GroupDev *__r
     if ((threadIdx.x & 31) == 0 && bits) atomicMax(&J.out->band_max_bits, bits);
 }
 
+
+__global__ void job_of_kernel(const GroupDev G) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t * 32 < G.rows) G.job_of[t] = G.job_ids[find_job(G.row_starts, G.njobs, t * 32)];
+}
+
+int launch_job_of(const GroupDev &G, cudaStream_t s) {
+    job_of_kernel<<<(G.rows / 32 + 255) / 256, 256, 0, s>>>(G);
+    HM_CUDA_TRY(cudaGetLastError());
+    count_launch();
+    return HM_OK;
+}
 
 int launch_screen_prep(const JobDev *jobs, const GroupDev &G, const GroupDev *Gd, cudaStream_t s) {
     ScopedKernelTimer timer(HM_KCLASS_PREP, s);

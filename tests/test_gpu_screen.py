@@ -308,3 +308,40 @@ def test_auto_escalates_where_the_band_spans_the_nearest_neighbours(sizes):
         if hm.autotune_path(x.shape[0], d, k, "cosine", batched=len(sizes) > 1) == hm.KnnPath.SCREEN_BF16:
             assert st.path_used == int(hm.KnnPath.SCREEN_BF16X3)
         assert st.overflow_rows == 0
+
+
+@pytest.mark.parametrize("n", [150, 1500, 5000])
+@pytest.mark.parametrize("path", ["screen_bf16", "screen_bf16x3"])
+def test_selection_at_the_edges_of_its_register_widths(path, n):
+    """k around the select's sort widths (32 and 64 keys; 64 is the screened paths'
+    limit); a row's candidates number from k up to all of the rows."""
+    g = np.random.default_rng(n)
+    x = g.normal(size=(n, 20)).astype(np.float32)
+    x[n // 2:n // 2 + 40] = x[0]  # ties at distance zero
+    for k in (1, 2, 31, 32, 33, 63, 64):
+        plain = hm.exact_knn(x, 20, k, "euclidean", "plain")
+        knn = hm.exact_knn(x, 20, k, "euclidean", path)
+        assert_same_bytes(knn.indices, plain.indices, f"k {k} indices")
+        assert_same_bytes(knn.dists, plain.dists, f"k {k} dists")
+
+
+def test_batch_merges_only_its_split_jobs():
+    """Exact jobs with and without column splits between screened jobs of both
+    short and long rows: every job's bytes are those of the job alone."""
+    import torch
+    from holomap_b200.device import DeviceBatch
+    g = np.random.default_rng(5)
+    shapes = [(90, 8, 5, "manhattan"), (3000, 12, 15, "euclidean"), (700, 40, 20, "manhattan"),
+              (33, 3, 4, "euclidean"), (2500, 100, 10, "cosine"), (1025, 70, 15, "euclidean"),
+              (2000, 5, 7, "manhattan")]
+    data = [g.normal(size=(n, d)).astype(np.float32) for n, d, _, _ in shapes]
+    batch = DeviceBatch([(torch.from_numpy(x).cuda(), k, m) for x, (_, _, k, m) in zip(data, shapes)])
+    batch.run()
+    torch.cuda.synchronize()
+    for j, (x, (n, d, k, m)) in enumerate(zip(data, shapes)):
+        plain, psm = hm.knn_smooth(x, d, k, m, "plain")
+        idx, dist, sig, rho = batch.result(j)
+        assert_same_bytes(idx.reshape(-1), plain.indices, f"job {j} indices")
+        assert_same_bytes(dist.reshape(-1), plain.dists, f"job {j} dists")
+        assert_same_bytes(sig, psm.sigmas, f"job {j} sigma")
+        assert_same_bytes(rho, psm.rhos, f"job {j} rho")
