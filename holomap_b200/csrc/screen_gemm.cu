@@ -192,6 +192,14 @@ __device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, uint32_t (&v)[32
         : "r"(taddr));
 }
 
+// (w0, w1) += (c0, c1) * h, each rounded once
+__device__ __forceinline__ void fma2(float &w0, float &w1, float c0, float c1, float h) {
+    asm("{\n\t.reg .b64 w, c, h;\n\t"
+        "mov.b64 w, {%0, %1};\n\tmov.b64 c, {%2, %3};\n\tmov.b64 h, {%4, %4};\n\t"
+        "fma.rn.f32x2 w, c, h, w;\n\tmov.b64 {%0, %1}, w;\n\t}"
+        : "+f"(w0), "+f"(w1)
+        : "f"(c0), "f"(c1), "f"(h));
+}
 __device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&v)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32"
@@ -548,6 +556,7 @@ __global__ void __launch_bounds__(sc_threads(PASS, KP), 1)
             // v >= 1 - thr - ulp(thr)/2 >= vstar (2^-20 relative margin)
             const float vstar = !(thr < INF) ? -INF
                                              : __fsub_rd(__fsub_rd(1.0f, thr), fmaxf(fabsf(thr), 1.0f) * 0x1p-20f);
+            const float hscale = -1.0f / scale;  // (scale is 1 or 2)
             uint32_t cnt = 0;
             unsigned long long *cand = PASS >= 1 ? cand_slots(J, G, list) : nullptr;
             // symmetric: this row's own term in its pairs' column-side values
@@ -778,109 +787,105 @@ __global__ void __launch_bounds__(sc_threads(PASS, KP), 1)
                             }
                         }
                     };
-                    auto emit16 = [&](uint32_t (&v)[16], uint32_t j0) {
-                        float (&c)[16] = reinterpret_cast<float (&)[16]>(v);
-                        if constexpr (SYMK) {
-                            if (colside) colside16(c, j0);
-                        }
-                        const bool full = j0 + 16 <= n;
-                        const bool self_here = diag && (row - j0 < 16u);
-                        auto put = [&](uint32_t pm, int g, bool raw) {
-                            while (pm) {
-                                const int e = __ffs(pm) - 1;
-                                pm &= pm - 1;
-                                const float a0 = (e & 1) ? c[8 * g + 1] : c[8 * g];
-                                const float a1 = (e & 1) ? c[8 * g + 3] : c[8 * g + 2];
-                                const float a2 = (e & 1) ? c[8 * g + 5] : c[8 * g + 4];
-                                const float a3 = (e & 1) ? c[8 * g + 7] : c[8 * g + 6];
-                                const float b0 = (e & 2) ? a1 : a0, b1 = (e & 2) ? a3 : a2;
-                                float x = (e & 4) ? b1 : b0;
-                                if (raw) x = __fsub_rn(1.0f, x);
-                                if (cnt < cap)
-                                    cand[cnt] = ((unsigned long long)__float_as_uint(x) << 32) | (j0 + 8 * g + e);
-                                ++cnt;
-                            }
-                        };
-                        if (fast_cos && full && !self_here) {
-                            // c = 1 - v <= thr  <=>  v >= vstar (a superset)
-                            float gm[2];
+                    // one column: its exact screened value x is a candidate if `hit`
+                    auto put = [&](bool hit, float x, uint32_t col) {
+                        if (hit && cnt < cap) cand[cnt] = ((unsigned long long)__float_as_uint(x) << 32) | col;
+                        cnt += hit ? 1u : 0u;
+                    };
+                    // 16 columns, GRP at a time: one comparison of their largest with
+                    // the row's limit skips half of the groups (one candidate in 150
+                    // columns, 32 rows a warp); the others run without branches.
+                    // c = rowterm - scale (v - cs / scale), two roundings: within the
+                    // band's 2^-21 of the squared norms, as the threshold pass's form
+                    // is.  Against 8-column groups with a loop over their candidates
+                    // and each column's value in three operations: 20,000 x 96
+                    // emission 366 -> 327 us, 50,000 x 384 cosine 1,532 -> 1,518;
+                    // groups of 8 cost 10 and 60 us more, a second register buffer of
+                    // products 18 and 80 (the loop leaves the instruction cache).
+                    constexpr int GRP = 4;
+                    auto emit16 = [&](const float (&v)[16], const float (&cs)[16], uint32_t j0, auto cosine) {
+                        constexpr bool COS = decltype(cosine)::value;
 #pragma unroll
-                            for (int g = 0; g < 2; ++g) {
-                                float x = c[8 * g];
+                        for (int q = 0; q < 16; q += GRP) {
+                            if constexpr (COS) {
+                                // fl(1 - v) is monotone in v
+                                float mx = v[q];
 #pragma unroll
-                                for (int e = 1; e < 8; ++e) x = fmaxf(x, c[8 * g + e]);
-                                gm[g] = x;
-                            }
-                            if (valid && fmaxf(gm[0], gm[1]) >= vstar) {
+                                for (int e = 1; e < GRP; ++e) mx = fmaxf(mx, v[q + e]);
+                                if (valid && mx >= vstar) {
 #pragma unroll
-                                for (int g = 0; g < 2; ++g) {
-                                    if (gm[g] >= vstar) {
-                                        uint32_t pm = 0;
-#pragma unroll
-                                        for (int e = 0; e < 8; ++e) pm |= (c[8 * g + e] >= vstar) ? (1u << e) : 0u;
-                                        put(pm, g, true);
+                                    for (int e = 0; e < GRP; ++e) {
+                                        put(v[q + e] >= vstar, __fsub_rn(1.0f, v[q + e]), j0 + q + e);
                                     }
                                 }
-                            }
-                            return;
-                        }
-                        // exact screened values (columns past n: +inf; the row itself: 0)
-                        if (fast_cos) {
+                            } else {
+                                float c[GRP];
 #pragma unroll
-                            for (int t = 0; t < 16; ++t) c[t] = __fsub_rn(1.0f, c[t]);
-                        } else {
-                            const float4 *ctp = reinterpret_cast<const float4 *>(colterm + j0);
+                                for (int e = 0; e < GRP; e += 2) {
+                                    c[e] = v[q + e], c[e + 1] = v[q + e + 1];
+                                    fma2(c[e], c[e + 1], cs[q + e], cs[q + e + 1], hscale);
+                                    float r0 = rowterm, r1 = rowterm;
+                                    fma2(r0, r1, c[e], c[e + 1], -scale);
+                                    c[e] = r0, c[e + 1] = r1;
+                                }
+                                float mn = c[0];
 #pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                                const float4 cq = __ldg(ctp + q);
-                                const float cs[4] = {cq.x, cq.y, cq.z, cq.w};
+                                for (int e = 1; e < GRP; ++e) mn = fminf(mn, c[e]);
+                                if (valid && !(mn > thr)) {
 #pragma unroll
-                                for (int e = 0; e < 4; ++e)
-                                    c[4 * q + e] = __fsub_rn(__fadd_rn(rowterm, cs[e]), __fmul_rn(scale, c[4 * q + e]));
-                            }
-                        }
-                        if (!full) {
-#pragma unroll
-                            for (int t = 0; t < 16; ++t)
-                                if (j0 + t >= n) c[t] = INF;
-                        }
-                        if (self_here) {
-#pragma unroll
-                            for (int t = 0; t < 16; ++t)
-                                if (j0 + t == row) c[t] = 0.0f;
-                        }
-                        float gm[2];
-#pragma unroll
-                        for (int g = 0; g < 2; ++g) {
-                            float x = c[8 * g];
-#pragma unroll
-                            for (int e = 1; e < 8; ++e) x = fminf(x, c[8 * g + e]);
-                            gm[g] = x;
-                        }
-                        if (valid && !(fminf(gm[0], gm[1]) > thr)) {
-#pragma unroll
-                            for (int g = 0; g < 2; ++g) {
-                                if (!(gm[g] > thr)) {
-                                    uint32_t pm = 0;
-#pragma unroll
-                                    for (int e = 0; e < 8; ++e)
-                                        pm |= (!(c[8 * g + e] > thr) && j0 + 8 * g + e < n) ? (1u << e) : 0u;
-                                    put(pm, g, false);
+                                    for (int e = 0; e < GRP; ++e) {
+                                        put(!(c[e] > thr), c[e], j0 + q + e);
+                                    }
                                 }
                             }
                         }
                     };
-                    uint32_t va[16], vb[16];
-                    tmem_ld16_issue(t_base, va);
-                    tmem_ld_wait16(va);
+                    // the row itself (value 0) or columns past n among them
+                    auto emit16_edge = [&](const float (&v)[16], uint32_t j0) {
+#pragma unroll
+                        for (int t = 0; t < 16; ++t) {
+                            const uint32_t col = j0 + t;
+                            if (valid && col < n) {
+                                float x = fast_cos ? __fsub_rn(1.0f, v[t])
+                                                   : __fsub_rn(__fadd_rn(rowterm, __ldg(colterm + col)), __fmul_rn(scale, v[t]));
+                                if (col == row) x = 0.0f;
+                                put(!(x > thr), x, col);
+                            }
+                        }
+                    };
+                    auto chunk = [&](uint32_t (&vr)[16], const float (&cs)[16], uint32_t j0) {
+                        const float (&v)[16] = reinterpret_cast<const float (&)[16]>(vr);
+                        if constexpr (SYMK) {
+                            if (colside) colside16(v, j0);
+                        }
+                        // (warp-uniform: the warp's rows are 32 columns of the diagonal tile)
+                        const bool edge = j0 + 16 > n || (diag && j0 + 16 > row - lane && j0 < row - lane + 32);
+                        if (edge)
+                            emit16_edge(v, j0);
+                        else if (fast_cos)
+                            emit16(v, cs, j0, std::true_type());
+                        else
+                            emit16(v, cs, j0, std::false_type());
+                    };
+                    auto terms = [&](float (&cs)[16], uint32_t j0) {
+                        if (fast_cos) return;
+                        const float4 *ctp = reinterpret_cast<const float4 *>(colterm + j0);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const float4 c4 = __ldg(ctp + q);
+                            cs[4 * q] = c4.x, cs[4 * q + 1] = c4.y, cs[4 * q + 2] = c4.z, cs[4 * q + 3] = c4.w;
+                        }
+                    };
 #pragma unroll 1
-                    for (uint32_t ch = 0; ch < SEGW / 16; ch += 2) {
-                        tmem_ld16_issue(t_base + (ch + 1) * 16, vb);
-                        emit16(va, c_base + ch * 16);
-                        tmem_ld_wait16(vb);
-                        if (ch + 2 < SEGW / 16) tmem_ld16_issue(t_base + (ch + 2) * 16, va);
-                        emit16(vb, c_base + (ch + 1) * 16);
-                        if (ch + 2 < SEGW / 16) tmem_ld_wait16(va);
+                    for (uint32_t ch = 0; ch < SEGW / 16; ++ch) {
+                        const uint32_t j0 = c_base + ch * 16;
+                        if (j0 >= n) break;
+                        uint32_t vr[16];
+                        float cs[16];
+                        tmem_ld16_issue(t_base + ch * 16, vr);
+                        terms(cs, j0);
+                        tmem_ld_wait16(vr);
+                        chunk(vr, cs, j0);
                     }
                 } else {
                     // two warps per scheduler: the next chunk loads while
