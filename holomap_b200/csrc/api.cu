@@ -94,7 +94,7 @@ struct JobPlan {
     size_t off_rnorm = 0, off_partial = 0, off_zero_rows = 0, off_ovf = 0;
     size_t off_mu = 0, off_csum = 0;
     int group = -1;
-    uint32_t row0 = 0, unit0 = 0, kp1 = 0, k_stages = 0, row_blocks = 0, col_tiles = 0;
+    uint32_t row0 = 0, unit0 = 0, kp1 = 0, k_steps = 0, k_stages = 0, row_blocks = 0, col_tiles = 0;
     uint32_t parts = 1, part_tiles = 0, cap = 0, seed_tiles = 0, tlists = 2;
     uint64_t slot0 = 0, cand0 = 0, topk0 = 0;
     // emission pass: symmetric (tiles on and above the diagonal), its column
@@ -308,10 +308,15 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
         P.group = g;
         Gp.jobs.push_back(j);
         B.any_screen = true;
-        P.kp1 = (uint32_t)round_up(P.spec.d, Gp.kslice);
-        const uint32_t kp = Gp.split ? 3 * P.kp1 : P.kp1;
-        P.k_stages = kp / Gp.kslice;
-        Gp.kpmax = std::max(Gp.kpmax, kp);
+        // operand columns: the split form's three segments lie side by side at the
+        // length of the data (8: a 16-byte piece), the whole rounded up to a K step;
+        // the passes load 128-byte slices and multiply the steps (20,000 x 96: K =
+        // 288, not 384)
+        const uint32_t kstep = Gp.kslice / SC_SLICE_STEPS;
+        P.kp1 = (uint32_t)round_up(P.spec.d, Gp.split ? 8u : kstep);
+        P.k_steps = ((Gp.split ? 3 * P.kp1 : P.kp1) + kstep - 1) / kstep;
+        P.k_stages = (P.k_steps + SC_SLICE_STEPS - 1) / SC_SLICE_STEPS;
+        Gp.kpmax = std::max(Gp.kpmax, P.k_stages * Gp.kslice);
         Gp.dmax = std::max(Gp.dmax, P.spec.d);
         if (P.spec.k > 32) {
             Gp.kp = 64;
@@ -666,6 +671,7 @@ static int bind_batch(hm_batch &B, void *d_ws, size_t bytes, cudaStream_t s) {
         J.row0 = P.row0;
         J.unit0 = P.unit0;
         J.kp1 = P.kp1;
+        J.k_steps = P.k_steps;
         J.k_stages = P.k_stages;
         J.row_blocks = P.row_blocks;
         J.col_tiles = P.col_tiles;

@@ -294,7 +294,7 @@ struct JobDev {
     double target;               // log2(k), host platform log2
     uint32_t *zero_rows;         // n
     // screened path
-    uint32_t group, row0, unit0, kp1, k_stages, row_blocks, col_tiles, parts, part_tiles, cap;
+    uint32_t group, row0, unit0, kp1, k_steps, k_stages, row_blocks, col_tiles, parts, part_tiles, cap;
     uint32_t seed_tiles;         // leading column tiles of each part in the threshold pass
     unsigned long long slot0;    // first threshold-pass list (tlists * parts lists per row)
     uint32_t tlists;             // threshold-pass lists per column part (its epilogue segments)

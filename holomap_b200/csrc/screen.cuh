@@ -36,6 +36,7 @@ namespace hm {
 constexpr int SC_BM = 128;
 constexpr int SC_BN = 256;
 constexpr int SC_SLICE_BYTES = 128;
+constexpr uint32_t SC_SLICE_STEPS = SC_SLICE_BYTES / 32;  // K steps (one MMA each) of a slice
 constexpr int SC_STAGES = 4;
 // K slices of the A block kept resident in shared memory for a whole unit
 // (96 KB: 6 slices of 128 B x 128 rows); deeper operands stream A with B

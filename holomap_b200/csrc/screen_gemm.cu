@@ -462,6 +462,8 @@ __global__ void __launch_bounds__(sc_threads(PASS, KP), 1)
                     }
                     fence_after_sync();
                 }
+                const uint32_t full_slices = J.k_steps / SC_SLICE_STEPS, last_steps = J.k_steps % SC_SLICE_STEPS;
+                const uint32_t k_stages = J.k_stages;
                 for (uint32_t ct = ut.ct_begin; ok && ct < ut.ct_end; ++ct, ++tile) {
                     const uint32_t buf = tile & 1, use = tile >> 1;
                     if (!mbar_wait(smem_u32(&acce[buf]), (use & 1) ^ 1, abort_flag)) {
@@ -471,7 +473,7 @@ __global__ void __launch_bounds__(sc_threads(PASS, KP), 1)
                     }
                     fence_after_sync();
                     const uint32_t d_tmem = tmem_base + buf * SC_BN;
-                    for (uint32_t ks = 0; ks < J.k_stages; ++ks, ++it) {
+                    for (uint32_t ks = 0; ks < k_stages; ++ks, ++it) {
                         const uint32_t s = it % NST, r = it / NST;
                         if (!mbar_wait(smem_u32(&full[s]), r & 1, abort_flag)) {
                             raise_error(abort_flag, &J.out->error_code, SC_ERR_MMA_FULL, peer_abort);
@@ -481,10 +483,17 @@ __global__ void __launch_bounds__(sc_threads(PASS, KP), 1)
                         fence_after_sync();
                         const uint32_t a0 = smem_u32(sA + ((PAIR || a_res) ? ks : s) * SC_A_BYTES);
                         const uint32_t b0 = smem_u32(sB + s * BST);
+                        if (ks < full_slices) {
 #pragma unroll
-                        for (uint32_t kk = 0; kk < SC_SLICE_BYTES / 32; ++kk)
-                            mma_issue<KIND, PAIR>(d_tmem, smem_desc(a0 + kk * 32), smem_desc(b0 + kk * 32),
-                                                  idesc, (ks | kk) != 0);
+                            for (uint32_t kk = 0; kk < SC_SLICE_STEPS; ++kk)
+                                mma_issue<KIND, PAIR>(d_tmem, smem_desc(a0 + kk * 32), smem_desc(b0 + kk * 32),
+                                                      idesc, (ks | kk) != 0);
+                        } else {
+#pragma unroll 1
+                            for (uint32_t kk = 0; kk < last_steps; ++kk)
+                                mma_issue<KIND, PAIR>(d_tmem, smem_desc(a0 + kk * 32), smem_desc(b0 + kk * 32),
+                                                      idesc, (ks | kk) != 0);
+                        }
                         mma_commit<PAIR>(smem_u32(&empty[s]));
                     }
                     if (!ok) break;

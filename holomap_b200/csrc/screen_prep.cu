@@ -144,24 +144,25 @@ __device__ __forceinline__ uint32_t to_tf32_bits(double v, double *rounded) {
     return b;
 }
 
-// Operand rows come in two kernels by the padded row length K1 of their job:
-// operand_kernel (K1 > OP_SHORT_K1) gives every row a warp, the warps striding
-// over the rows; operand_packed_kernel (K1 <= OP_SHORT_K1) gives a row 8 or 16
-// lanes, so a warp works on two or four short rows at once.  Both run a
-// persistent grid of OP_BLOCKS_PER_SM blocks per SM; each skips the other's
-// jobs.  A row's loads (up to 512 elements with 32 lanes; 256 in the split
-// form) are all issued before its first store, so a row costs one memory
-// round trip; a job's maxima are kept per warp (per row group) and written,
-// one atomic each, when the warp's next rows belong to another job, or at
-// its end.
+// Operand rows: the row's elements in the group's format, its binary64 error
+// statistics, the additive terms of the screen epilogue and the row's shared
+// threshold.  A row of K1 elements takes 4, 8 or 16 lanes when K1 is at most
+// OP_SHORT_K1 (a warp then holds OP_TILE consecutive rows, all loaded before the
+// first is worked on), else the warp; each kernel skips the other's jobs.  A lane
+// takes 4 consecutive elements at a time, so an operand piece is one 8 or 16 byte
+// store.  What it costs besides the traffic is the row's end: its four sums are
+// reduced transposed (6 shuffles for the four, each lane left with one of them),
+// and the four square roots are one, taken side by side.  A block takes
+// consecutive rows, mostly of one job, and combines its warps' maxima before the
+// job's counters see them.  256 datasets of d = 8..64: 659 us (both kernels) with a
+// warp's every lane summing all four, lane 0 taking the roots and 2-byte stores,
+// 448 now; 20,000 x 96: 40 -> 25; 50,000 x 384 (BF16): 104 -> 89.
 constexpr uint32_t OP_WARPS = 8;
 constexpr int OP_BLOCKS_PER_SM = 3;
 constexpr uint32_t OP_SHORT_K1 = 64;
+constexpr uint32_t OP_TILE = 8;  // short rows a warp holds (in one job, whose rows start 32-aligned)
 uint32_t operand_short_k1() { return OP_SHORT_K1; }
 constexpr int OP_TF32 = 0, OP_BF16 = 1, OP_SPLIT = 2;
-// elements per lane in flight (the split form's six stores per element need
-// the registers of half of them)
-__host__ __device__ constexpr uint32_t op_per_lane(int mode) { return mode == OP_SPLIT ? 8u : 16u; }
 
 // The column terms past the group's last row (a column tile may reach them).
 __device__ __forceinline__ void clear_column_tail(const GroupDev &G) {
@@ -171,246 +172,84 @@ __device__ __forceinline__ void clear_column_tail(const GroupDev &G) {
     }
 }
 
-// Operand row(s), binary64 error statistics, additive terms of the screen
-// epilogue, and the row's shared threshold.  Every lane accumulates its
-// elements t = lane, lane + 32, ... in ascending order.
-template <int MODE>  // OP_TF32, OP_BF16 or OP_SPLIT: the group's operand format
+template <int MODE, bool SHORT>
 __global__ void __launch_bounds__(OP_WARPS * 32, OP_BLOCKS_PER_SM) operand_kernel(const JobDev *__restrict__ jobs,
-                                                               const GroupDev *__restrict__ Gp) {
-    // the warp's maxima live in shared memory (lane 0 alone updates them)
-    __shared__ double s_wmax[OP_WARPS][6];
-    __shared__ unsigned long long s_wzero[OP_WARPS];
+                                                                                  const GroupDev *__restrict__ Gp) {
+    __shared__ double s_max[OP_WARPS][6];
+    __shared__ uint32_t s_zero[OP_WARPS];
+    __shared__ const JobDev *s_job[OP_WARPS];
     const GroupDev &G = *Gp;
     grid_ready();
     if (group_idle(jobs, G)) return;
     clear_column_tail(G);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double *wmax = s_wmax[warp];
-    const JobDev *cur = nullptr;  // the job whose maxima the warp holds
-    auto reset = [&]() {
-        if (lane == 0) {
-            for (int q = 0; q < 6; ++q) wmax[q] = 0.0;
-            s_wzero[warp] = 0;
-        }
-    };
-    auto flush = [&]() {
-        if (cur != nullptr && lane == 0) {
-            unsigned long long *maxb = cur->cnt->maxb;
-            for (int q = 0; q < 6; ++q) atomic_max_pos(&maxb[q], wmax[q]);
-            if (s_wzero[warp]) atomicAdd(&maxb[7], s_wzero[warp]);
-        }
-        reset();
-        cur = nullptr;
-    };
-    reset();
-    const uint32_t stride = gridDim.x * OP_WARPS;
-    for (uint32_t gr = blockIdx.x * OP_WARPS + warp; gr < G.rows; gr += stride) {
-        const JobDev &J = group_job(jobs, G, gr);
-        if (!job_active(J) || J.kp1 <= OP_SHORT_K1) continue;  // inactive, or operand_packed_kernel's
-        const uint32_t row = gr - J.row0;
-        if (row >= J.n) {  // padding between jobs: zero operands (read only as masked rows/columns)
-            if (lane == 0) G.colterm[gr] = 0.0f;
-            for (uint32_t t = lane; t < G.kpmax; t += 32) {
-                if (G.elem_bytes == 4) {
-                    reinterpret_cast<uint32_t *>(G.opa)[(size_t)gr * G.kpmax + t] = 0u;
-                } else {
-                    reinterpret_cast<uint16_t *>(G.opa)[(size_t)gr * G.kpmax + t] = 0;
-                    reinterpret_cast<uint16_t *>(G.opb)[(size_t)gr * G.kpmax + t] = 0;
-                }
-            }
-            continue;
-        }
-        if (&J != cur) {
-            flush();
-            cur = &J;
-        }
 
-        const bool euc = J.metric == HM_METRIC_EUCLIDEAN;
-        double scale = 1.0;
-        bool zero_row = false;
-        if (euc) {
-            const double m = sqrt(__longlong_as_double((long long)J.cnt->maxb[6]));
-            if (m > 0.0) {
-                int e;
-                frexp(m, &e);  // m = f * 2^e, f in [0.5, 1)
-                scale = ldexp(1.0, -e);
-            }
-        } else {
-            const double rn = J.rnorm[row];
-            zero_row = !(rn > 0.0);
-            scale = zero_row ? 0.0 : 1.0 / rn;
+    // the job the warp works on: lanes per row, the lane's place in its row, and
+    // the sum it is left with (o1, o2: the lane bits that name it): its largest
+    // square root so far and, of the first, the sum itself
+    const JobDev *cur = nullptr;
+    uint32_t lpr = 32, o1 = 16, o2 = 8, zeros = 0;
+    double scale = 1.0, top = 0.0, top_sq = 0.0;
+    // the maxima over the warp's rows, per sum; lane (value index) writes
+    auto maxima = [&](double *out) {
+        for (uint32_t o = 16; o > 0; o >>= 1) {
+            if (o == o1 || o == o2) continue;
+            top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+            top_sq = fmax(top_sq, __shfl_xor_sync(0xffffffffu, top_sq, o));
         }
-
-        const size_t kp = G.kpmax;
-        const uint32_t d = J.d, kp1 = J.kp1;
-        double uu = 0.0, ee = 0.0, rr = 0.0, aa = 0.0;
-        const float *xr = J.x + (size_t)row * d;
-        // cosine rows are scaled by 1 / ||x|| (the operand u is whatever this
-        // arithmetic forms: the band is measured from it)
-        const double mul = scale;
-        constexpr uint32_t PER_LANE = op_per_lane(MODE);
-        for (uint32_t t0 = 0; t0 < kp1; t0 += 32 * PER_LANE) {
-            float xs[PER_LANE];
-#pragma unroll
-            for (uint32_t q = 0; q < PER_LANE; ++q) {
-                const uint32_t t = t0 + 32 * q + lane;
-                xs[q] = t < d ? __ldg(xr + t) : 0.0f;
-            }
-#pragma unroll
-            for (uint32_t q = 0; q < PER_LANE; ++q) {
-                const uint32_t t = t0 + 32 * q + lane;
-                if (t >= kp1) break;
-                double u = 0.0;
-                if (t < d) u = euc ? ((double)xs[q] - __ldg(J.mu + t)) * mul : (double)xs[q] * mul;
-                uu += u * u;
-                if (MODE == OP_TF32) {
-                    double r;
-                    const uint32_t b = to_tf32_bits(u, &r);
-                    reinterpret_cast<uint32_t *>(G.opa)[(size_t)gr * kp + t] = b;
-                    ee += (r - u) * (r - u);
-                    aa += r * r;
-                } else if (MODE == OP_BF16) {
-                    double r;
-                    const uint16_t b = to_bf16_bits(u, &r);
-                    reinterpret_cast<uint16_t *>(G.opa)[(size_t)gr * kp + t] = b;
-                    ee += (r - u) * (r - u);
-                    aa += r * r;
-                } else {
-                    double hi, lo;
-                    const uint16_t bh = to_bf16_bits(u, &hi);
-                    const uint16_t bl = to_bf16_bits(u - hi, &lo);
-                    const double res = (u - hi) - lo;
-                    uint16_t *A = reinterpret_cast<uint16_t *>(G.opa) + (size_t)gr * kp;
-                    uint16_t *B = reinterpret_cast<uint16_t *>(G.opb) + (size_t)gr * kp;
-                    A[t] = bh;
-                    A[kp1 + t] = bh;
-                    A[2 * kp1 + t] = bl;
-                    B[t] = bh;
-                    B[kp1 + t] = bl;
-                    B[2 * kp1 + t] = bh;
-                    ee += lo * lo;
-                    rr += res * res;
-                    aa += 2.0 * hi * hi + lo * lo;
-                }
-            }
+        const uint32_t v = (lane & o1 ? 2u : 0u) + (lane & o2 ? 1u : 0u);
+        if ((lane & ~(int)(o1 | o2)) == 0) {
+            out[v] = top;
+            if (v == 3) out[4] = top;  // both operand layouts have the same row norm
+            if (v == 0) out[5] = top_sq;
         }
-        uu = warp_sum(uu);
-        ee = warp_sum(ee);
-        rr = warp_sum(rr);
-        aa = warp_sum(aa);
-        if (lane == 0) {
-            RowStat st;
-            st.unorm = sqrt(uu);
-            st.enorm = sqrt(ee);
-            st.rnorm = sqrt(rr);
-            st.anorm = sqrt(aa);
-            st.bnorm = st.anorm;  // both operand layouts have the same row norm
-            st.sqnorm = uu;
-            G.rowstat[gr] = st;
-            wmax[0] = fmax(wmax[0], st.unorm);
-            wmax[1] = fmax(wmax[1], st.enorm);
-            wmax[2] = fmax(wmax[2], st.rnorm);
-            wmax[3] = fmax(wmax[3], st.anorm);
-            wmax[4] = fmax(wmax[4], st.bnorm);
-            wmax[5] = fmax(wmax[5], st.sqnorm);
-            if (euc) {
-                const float nsq = __double2float_rn(uu);
-                G.rowterm[gr] = nsq;
-                G.colterm[gr] = nsq;
-            } else {
-                G.rowterm[gr] = 0.0f;
-                G.colterm[gr] = zero_row ? 0.0f : 1.0f;
-            }
-            G.force[gr] = zero_row ? 1 : 0;
-            if (zero_row) ++s_wzero[warp];
-            G.rowthr[gr] = 0xff800000u;  // the row's shared threshold starts at +inf
-        }
-    }
-    flush();
-}
-
-// The same for the jobs with K1 <= OP_SHORT_K1: the warps stride over tiles
-// of OP_TILE consecutive group rows (a tile lies in one job, whose rows start
-// 32-aligned), a row taking 16 lanes when K1 > 32, else 8.  Every lane
-// accumulates its elements t = s, s + L, ... (s its place among the row's L
-// lanes) in ascending order.
-constexpr uint32_t OP_TILE = 4;  // rows per tile: the most a warp holds at once
-template <int MODE>
-__global__ void __launch_bounds__(OP_WARPS * 32, OP_BLOCKS_PER_SM)
-    operand_packed_kernel(const JobDev *__restrict__ jobs, const GroupDev *__restrict__ Gp) {
-    // the maxima of each of the warp's row groups (a group's first lane alone
-    // updates them)
-    __shared__ double s_wmax[OP_WARPS][OP_TILE][6];
-    __shared__ unsigned long long s_wzero[OP_WARPS][OP_TILE];
-    const GroupDev &G = *Gp;
-    grid_ready();
-    if (group_idle(jobs, G)) return;
-    clear_column_tail(G);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const JobDev *cur = nullptr;  // the job whose maxima the warp holds
-    auto reset = [&]() {
-        if (lane < (int)OP_TILE) {
-            for (int q = 0; q < 6; ++q) s_wmax[warp][lane][q] = 0.0;
-            s_wzero[warp][lane] = 0;
-        }
+        zeros = __reduce_add_sync(0xffffffffu, zeros);
         __syncwarp();
     };
-    auto flush = [&]() {
-        __syncwarp();
-        if (cur != nullptr && lane == 0) {
-            unsigned long long *maxb = cur->cnt->maxb;
-            for (int q = 0; q < 6; ++q) {
-                double m = s_wmax[warp][0][q];
-                for (uint32_t g = 1; g < OP_TILE; ++g) m = fmax(m, s_wmax[warp][g][q]);
-                atomic_max_pos(&maxb[q], m);
-            }
-            unsigned long long z = 0;
-            for (uint32_t g = 0; g < OP_TILE; ++g) z += s_wzero[warp][g];
-            if (z) atomicAdd(&maxb[7], z);
+    auto report = [&](const JobDev *J, int from, int to) {  // lane < 6
+        double m = 0.0;
+        uint32_t z = 0;
+        for (int w = from; w < to; ++w) {
+            m = fmax(m, s_max[w][lane]);
+            z += s_zero[w];
         }
-        __syncwarp();
-        reset();
-        cur = nullptr;
+        atomic_max_pos(&J->cnt->maxb[lane], m);
+        if (lane == 0 && z) atomicAdd(&J->cnt->maxb[7], (unsigned long long)z);
     };
-    reset();
-    constexpr uint32_t PER_LANE = OP_SHORT_K1 / 16;  // a row's elements per lane: one chunk
+
     const size_t kp = G.kpmax;
-    const uint32_t tiles = (G.rows + OP_TILE - 1) / OP_TILE;
-    const uint32_t stride = gridDim.x * OP_WARPS;
-    for (uint32_t ti = blockIdx.x * OP_WARPS + warp; ti < tiles; ti += stride) {
-        const uint32_t gr0 = ti * OP_TILE;
+    constexpr int STEPS = SHORT ? OP_TILE / 2 : (MODE == OP_SPLIT ? 2 : 4);  // pieces of 4 loaded ahead
+    const uint32_t tiles = SHORT ? (G.rows + OP_TILE - 1) / OP_TILE : G.rows;
+    // the blocks take chunks of rows in turn (a group's short and long rows lie in
+    // runs, of which each kernel works on one kind).  Chunks of one tile a warp
+    // against four: short rows of 256 datasets 167 us / 257; of one row against two
+    // and eight: their long rows 312 / 281 / 268, 5,000 x 128 26 / 26 / 41
+    constexpr uint32_t CHUNK = SHORT ? 1 : 2;  // tiles a warp takes of one
+    for (uint32_t i = 0;; ++i) {
+        const uint32_t ti = ((i / CHUNK * gridDim.x + blockIdx.x) * CHUNK + i % CHUNK) * OP_WARPS + warp;
+        if (i % CHUNK == 0 && ti - warp >= tiles) break;
+        if (ti >= tiles) continue;
+        const uint32_t gr0 = SHORT ? ti * OP_TILE : ti;
         const JobDev &J = group_job(jobs, G, gr0);
-        // uniform over the warp (a tile is of one job); longer rows are operand_kernel's
-        if (!job_active(J) || J.kp1 > OP_SHORT_K1) continue;
-        if (&J != cur) {
-            flush();
-            cur = &J;
-        }
-        const uint32_t d = J.d, kp1 = J.kp1;
-        // padding rows between jobs: zero operands (read only as masked rows/columns)
-        for (uint32_t p = 0; p < OP_TILE; ++p) {
-            const uint32_t gr = gr0 + p;
-            if (gr < G.rows && gr - J.row0 >= J.n) {
-                if (lane == 0) G.colterm[gr] = 0.0f;
-                for (uint32_t t = lane; t < G.kpmax; t += 32) {
-                    if (G.elem_bytes == 4) {
-                        reinterpret_cast<uint32_t *>(G.opa)[(size_t)gr * G.kpmax + t] = 0u;
-                    } else {
-                        reinterpret_cast<uint16_t *>(G.opa)[(size_t)gr * G.kpmax + t] = 0;
-                        reinterpret_cast<uint16_t *>(G.opb)[(size_t)gr * G.kpmax + t] = 0;
-                    }
-                }
-            }
-        }
+        if (!job_active(J) || (J.kp1 <= OP_SHORT_K1) != SHORT) continue;
         const bool euc = J.metric == HM_METRIC_EUCLIDEAN;
-        const uint32_t lpr = kp1 > 32 ? 16u : 8u;  // lanes per row
-        const uint32_t g = (uint32_t)lane / lpr, sl = (uint32_t)lane % lpr;
-        for (uint32_t p0 = 0; p0 < OP_TILE; p0 += 32 / lpr) {
-            const uint32_t gr = gr0 + p0 + g;
-            const uint32_t row = gr - J.row0;
-            const bool real = gr < G.rows && row < J.n;  // padding rows compute zeros, write nothing
-            double scale = 1.0;
-            bool zero_row = false;
+        if (&J != cur) {
+            if (cur != nullptr) {
+                maxima(s_max[warp]);
+                if (lane == 0) s_zero[warp] = zeros;
+                __syncwarp();
+                if (lane < 6) report(cur, warp, warp + 1);
+                __syncwarp();
+            }
+            cur = &J;
+            zeros = 0;
+            top = top_sq = 0.0;
+            if (SHORT) {
+                lpr = J.kp1 > 32 ? 16u : J.kp1 > 16 ? 8u : 4u;
+                o1 = lpr >> 1;
+                o2 = lpr >> 2;
+            }
+            scale = 1.0;
             if (euc) {
                 const double m = sqrt(__longlong_as_double((long long)J.cnt->maxb[6]));
                 if (m > 0.0) {
@@ -418,104 +257,155 @@ __global__ void __launch_bounds__(OP_WARPS * 32, OP_BLOCKS_PER_SM)
                     frexp(m, &e);  // m = f * 2^e, f in [0.5, 1)
                     scale = ldexp(1.0, -e);
                 }
-            } else if (real) {
-                const double rn = J.rnorm[row];
-                zero_row = !(rn > 0.0);
-                scale = zero_row ? 0.0 : 1.0 / rn;
-            }
-            double uu = 0.0, ee = 0.0, rr = 0.0, aa = 0.0;
-            const float *xr = J.x + (size_t)(real ? row : 0u) * d;
-            // cosine rows are scaled by 1 / ||x|| (the operand u is whatever this
-            // arithmetic forms: the band is measured from it)
-            const double mul = scale;
-            for (uint32_t t0 = 0; t0 < kp1; t0 += lpr * PER_LANE) {
-                float xs[PER_LANE];
-#pragma unroll
-                for (uint32_t q = 0; q < PER_LANE; ++q) {
-                    const uint32_t t = t0 + lpr * q + sl;
-                    xs[q] = (real && t < d) ? __ldg(xr + t) : 0.0f;
-                }
-#pragma unroll
-                for (uint32_t q = 0; q < PER_LANE; ++q) {
-                    const uint32_t t = t0 + lpr * q + sl;
-                    if (t >= kp1) break;
-                    double u = 0.0;
-                    if (t < d) u = euc ? ((double)xs[q] - __ldg(J.mu + t)) * mul : (double)xs[q] * mul;
-                    uu += u * u;
-                    if (MODE == OP_TF32) {
-                        double r;
-                        const uint32_t b = to_tf32_bits(u, &r);
-                        if (real) reinterpret_cast<uint32_t *>(G.opa)[(size_t)gr * kp + t] = b;
-                        ee += (r - u) * (r - u);
-                        aa += r * r;
-                    } else if (MODE == OP_BF16) {
-                        double r;
-                        const uint16_t b = to_bf16_bits(u, &r);
-                        if (real) reinterpret_cast<uint16_t *>(G.opa)[(size_t)gr * kp + t] = b;
-                        ee += (r - u) * (r - u);
-                        aa += r * r;
-                    } else {
-                        double hi, lo;
-                        const uint16_t bh = to_bf16_bits(u, &hi);
-                        const uint16_t bl = to_bf16_bits(u - hi, &lo);
-                        const double res = (u - hi) - lo;
-                        if (real) {
-                            uint16_t *A = reinterpret_cast<uint16_t *>(G.opa) + (size_t)gr * kp;
-                            uint16_t *B = reinterpret_cast<uint16_t *>(G.opb) + (size_t)gr * kp;
-                            A[t] = bh;
-                            A[kp1 + t] = bh;
-                            A[2 * kp1 + t] = bl;
-                            B[t] = bh;
-                            B[kp1 + t] = bl;
-                            B[2 * kp1 + t] = bh;
-                        }
-                        ee += lo * lo;
-                        rr += res * res;
-                        aa += 2.0 * hi * hi + lo * lo;
-                    }
-                }
-            }
-            // the row's sums over its lpr lanes (xor partners stay in the group)
-#pragma unroll
-            for (uint32_t o = 8; o > 0; o >>= 1) {
-                if (o < lpr) {
-                    uu += __shfl_xor_sync(0xffffffffu, uu, o);
-                    ee += __shfl_xor_sync(0xffffffffu, ee, o);
-                    rr += __shfl_xor_sync(0xffffffffu, rr, o);
-                    aa += __shfl_xor_sync(0xffffffffu, aa, o);
-                }
-            }
-            if (sl == 0 && real) {
-                double *wmax = s_wmax[warp][p0 + g];
-                RowStat st;
-                st.unorm = sqrt(uu);
-                st.enorm = sqrt(ee);
-                st.rnorm = sqrt(rr);
-                st.anorm = sqrt(aa);
-                st.bnorm = st.anorm;  // both operand layouts have the same row norm
-                st.sqnorm = uu;
-                G.rowstat[gr] = st;
-                wmax[0] = fmax(wmax[0], st.unorm);
-                wmax[1] = fmax(wmax[1], st.enorm);
-                wmax[2] = fmax(wmax[2], st.rnorm);
-                wmax[3] = fmax(wmax[3], st.anorm);
-                wmax[4] = fmax(wmax[4], st.bnorm);
-                wmax[5] = fmax(wmax[5], st.sqnorm);
-                if (euc) {
-                    const float nsq = __double2float_rn(uu);
-                    G.rowterm[gr] = nsq;
-                    G.colterm[gr] = nsq;
-                } else {
-                    G.rowterm[gr] = 0.0f;
-                    G.colterm[gr] = zero_row ? 0.0f : 1.0f;
-                }
-                G.force[gr] = zero_row ? 1 : 0;
-                if (zero_row) ++s_wzero[warp][p0 + g];
-                G.rowthr[gr] = 0xff800000u;  // the row's shared threshold starts at +inf
             }
         }
+        const uint32_t d = J.d, kp1 = J.kp1, sl = (uint32_t)lane & (lpr - 1);
+        const bool wide = (d & 3) == 0 && (reinterpret_cast<uintptr_t>(J.x) & 15) == 0;
+        // four elements from t (0 past the row's end)
+        auto load4 = [&](float (&v)[4], const float *xr, uint32_t t, bool real) {
+            v[0] = v[1] = v[2] = v[3] = 0.0f;
+            if (!real || t >= d) return;
+            if (wide) {
+                const float4 q = __ldg(reinterpret_cast<const float4 *>(xr + t));
+                v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (t + e < d) v[e] = __ldg(xr + t + e);
+            }
+        };
+        double uu, ee, rr, aa;  // the lane's part of the row's sums
+        auto piece = [&](const float (&v)[4], uint32_t t, uint32_t gr, bool real, double mul) {
+            uint32_t hi4[4], lo4[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                double u = 0.0;
+                // cosine rows are scaled by 1 / ||x|| (the operand u is whatever
+                // this arithmetic forms: the band is measured from it)
+                if (real && t + e < d) u = euc ? ((double)v[e] - __ldg(J.mu + t + e)) * mul : (double)v[e] * mul;
+                uu += u * u;
+                if (MODE == OP_SPLIT) {
+                    double hi, lo;
+                    hi4[e] = to_bf16_bits(u, &hi);
+                    lo4[e] = to_bf16_bits(u - hi, &lo);
+                    const double res = (u - hi) - lo;
+                    ee += lo * lo;
+                    rr += res * res;
+                    aa += 2.0 * hi * hi + lo * lo;
+                } else {
+                    double r;
+                    hi4[e] = MODE == OP_TF32 ? to_tf32_bits(u, &r) : (uint32_t)to_bf16_bits(u, &r);
+                    ee += (r - u) * (r - u);
+                    aa += r * r;
+                }
+            }
+            if (MODE == OP_TF32) {
+                *reinterpret_cast<uint4 *>(static_cast<uint32_t *>(G.opa) + gr * kp + t) =
+                    make_uint4(hi4[0], hi4[1], hi4[2], hi4[3]);
+                return;
+            }
+            const uint2 h = make_uint2(hi4[0] | hi4[1] << 16, hi4[2] | hi4[3] << 16);
+            uint16_t *A = static_cast<uint16_t *>(G.opa) + gr * kp + t;
+            *reinterpret_cast<uint2 *>(A) = h;
+            if (MODE == OP_SPLIT) {
+                const uint2 l = make_uint2(lo4[0] | lo4[1] << 16, lo4[2] | lo4[3] << 16);
+                uint16_t *B = static_cast<uint16_t *>(G.opb) + gr * kp + t;
+                *reinterpret_cast<uint2 *>(A + kp1) = h;
+                *reinterpret_cast<uint2 *>(A + 2 * kp1) = l;
+                *reinterpret_cast<uint2 *>(B) = h;
+                *reinterpret_cast<uint2 *>(B + kp1) = l;
+                *reinterpret_cast<uint2 *>(B + 2 * kp1) = h;
+            }
+        };
+        auto row_end = [&](uint32_t gr, bool real, bool zero_row) {
+            if (MODE == OP_SPLIT && sl == 0) {
+                // the last K step's columns past the three segments
+                for (uint32_t t = 3 * kp1; t < J.k_steps * 16; t += 8) {
+                    *reinterpret_cast<uint4 *>(static_cast<uint16_t *>(G.opa) + gr * kp + t) = make_uint4(0, 0, 0, 0);
+                    *reinterpret_cast<uint4 *>(static_cast<uint16_t *>(G.opb) + gr * kp + t) = make_uint4(0, 0, 0, 0);
+                }
+            }
+            const bool h1 = lane & o1, h2 = lane & o2;
+            double k0 = (h1 ? rr : uu) + __shfl_xor_sync(0xffffffffu, h1 ? uu : rr, o1);
+            double k1 = (h1 ? aa : ee) + __shfl_xor_sync(0xffffffffu, h1 ? ee : aa, o1);
+            double v = (h2 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, h2 ? k0 : k1, o2);
+            for (uint32_t o = o2 >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            const double root = sqrt(v);
+            if (!real) {  // padding between jobs: operands of zeros, read only as masked rows and columns
+                if (sl == 0) G.colterm[gr] = 0.0f;
+                return;
+            }
+            top = fmax(top, root);
+            RowStat &st = G.rowstat[gr];
+            if (sl == 0) {
+                top_sq = fmax(top_sq, v);
+                st.unorm = root;
+                st.sqnorm = v;
+                const float term = euc ? __double2float_rn(v) : 0.0f;
+                G.rowterm[gr] = term;
+                G.colterm[gr] = euc ? term : zero_row ? 0.0f : 1.0f;
+                G.force[gr] = zero_row ? 1 : 0;
+                zeros += zero_row ? 1u : 0u;
+                G.rowthr[gr] = 0xff800000u;  // the row's shared threshold starts at +inf
+            } else if (sl == o2) {
+                st.enorm = root;
+            } else if (sl == o1) {
+                st.rnorm = root;
+            } else if (sl == o1 + o2) {
+                st.anorm = st.bnorm = root;
+            }
+        };
+        uu = ee = rr = aa = 0.0;
+        float xs[STEPS][4];
+        if (SHORT) {
+            const uint32_t step = 32 / lpr, first = (uint32_t)lane / lpr;
+            double rn[STEPS];
+#pragma unroll
+            for (int q = 0; q < STEPS; ++q) {
+                const uint32_t p = q * step + first, row = gr0 + p - J.row0;
+                const bool real = p < OP_TILE && row < J.n;
+                load4(xs[q], J.x + (size_t)(real ? row : 0u) * d, 4 * sl, real);
+                rn[q] = real && !euc ? J.rnorm[row] : 0.0;
+            }
+#pragma unroll
+            for (int q = 0; q < STEPS; ++q) {
+                if (q * step >= OP_TILE) break;
+                const uint32_t gr = gr0 + q * step + first;
+                const bool real = gr - J.row0 < J.n;
+                const bool zero_row = !euc && !(rn[q] > 0.0);
+                uu = ee = rr = aa = 0.0;
+                if (4 * sl < kp1) piece(xs[q], 4 * sl, gr, real, euc ? scale : zero_row ? 0.0 : 1.0 / rn[q]);
+                row_end(gr, real, zero_row);
+            }
+        } else {
+            const uint32_t row = gr0 - J.row0;
+            const bool real = row < J.n;
+            const float *xr = J.x + (size_t)(real ? row : 0u) * d;
+            const double rn = real && !euc ? J.rnorm[row] : 0.0;
+            const bool zero_row = !euc && !(rn > 0.0);
+            const double mul = euc ? scale : zero_row ? 0.0 : 1.0 / rn;
+            for (uint32_t t0 = 4 * sl; t0 < kp1; t0 += 128 * STEPS) {
+#pragma unroll
+                for (int q = 0; q < STEPS; ++q) load4(xs[q], xr, t0 + 128 * q, real);
+#pragma unroll
+                for (int q = 0; q < STEPS; ++q)
+                    if (t0 + 128 * q < kp1) piece(xs[q], t0 + 128 * q, gr0, real, mul);
+            }
+            __syncwarp();
+            row_end(gr0, real, zero_row);
+        }
     }
-    flush();
+    // the block's maxima: one report per run of warps on the same job
+    if (cur != nullptr) maxima(s_max[warp]);
+    if (lane == 0) {
+        s_zero[warp] = zeros;
+        s_job[warp] = cur;
+    }
+    __syncthreads();
+    if (cur == nullptr || lane >= 6 || (warp > 0 && s_job[warp - 1] == cur)) return;
+    int end = warp + 1;
+    while (end < (int)OP_WARPS && s_job[end] == cur) ++end;
+    report(cur, warp, end);
 }
 
 // Keep band of one row (binary32 bits, rounded up), written to G.band.
@@ -588,23 +478,23 @@ int launch_screen_prep(const JobDev *jobs, const GroupDev &G, const GroupDev *Gd
         count_launch(2);
     }
     const uint32_t op_cap = (uint32_t)device_sm_count() * OP_BLOCKS_PER_SM;
-    const uint32_t row_blocks = (G.rows + OP_WARPS - 1) / OP_WARPS;
-    const uint32_t row_grid = row_blocks < op_cap ? row_blocks : op_cap;
-    const uint32_t tile_blocks = (G.rows + OP_WARPS * OP_TILE - 1) / (OP_WARPS * OP_TILE);
-    const uint32_t tile_grid = tile_blocks < op_cap ? tile_blocks : op_cap;
-    auto both = [&](auto rows_kernel, auto packed_kernel) {
+    auto both = [&](auto rows_kernel, auto short_rows_kernel) {
+        const uint32_t row_blocks = (G.rows + OP_WARPS - 1) / OP_WARPS;
+        const uint32_t tile_blocks = (G.rows + OP_WARPS * OP_TILE - 1) / (OP_WARPS * OP_TILE);
         cudaError_t e = cudaSuccess;
-        if (G.any_long_rows) e = launch(true, rows_kernel, row_grid, OP_WARPS * 32, 0, s, jobs, Gd);
-        if (e == cudaSuccess && G.any_short_rows) e = launch(true, packed_kernel, tile_grid, OP_WARPS * 32, 0, s, jobs, Gd);
+        if (G.any_long_rows)
+            e = launch(true, rows_kernel, row_blocks < op_cap ? row_blocks : op_cap, OP_WARPS * 32, 0, s, jobs, Gd);
+        if (e == cudaSuccess && G.any_short_rows)
+            e = launch(true, short_rows_kernel, tile_blocks < op_cap ? tile_blocks : op_cap, OP_WARPS * 32, 0, s, jobs, Gd);
         return e;
     };
     cudaError_t err;
     if (G.kind == SCREEN_KIND_TF32)
-        err = both(operand_kernel<OP_TF32>, operand_packed_kernel<OP_TF32>);
+        err = both(operand_kernel<OP_TF32, false>, operand_kernel<OP_TF32, true>);
     else if (!G.split)
-        err = both(operand_kernel<OP_BF16>, operand_packed_kernel<OP_BF16>);
+        err = both(operand_kernel<OP_BF16, false>, operand_kernel<OP_BF16, true>);
     else
-        err = both(operand_kernel<OP_SPLIT>, operand_packed_kernel<OP_SPLIT>);
+        err = both(operand_kernel<OP_SPLIT, false>, operand_kernel<OP_SPLIT, true>);
     HM_CUDA_TRY(err);
     count_launch((G.any_long_rows ? 1 : 0) + (G.any_short_rows ? 1 : 0));
     return HM_OK;

@@ -345,3 +345,19 @@ def test_batch_merges_only_its_split_jobs():
         assert_same_bytes(dist.reshape(-1), plain.dists, f"job {j} dists")
         assert_same_bytes(sig, psm.sigmas, f"job {j} sigma")
         assert_same_bytes(rho, psm.rhos, f"job {j} rho")
+
+
+@pytest.mark.parametrize("path", PATHS)
+@pytest.mark.parametrize("metric", ["euclidean", "cosine"])
+@pytest.mark.parametrize("d", [1, 3, 8, 9, 16, 17, 32, 33, 63, 64, 65, 88, 127, 128, 129])
+def test_operand_rows_of_every_length_class(path, metric, d):
+    """Row lengths around the operand kernels' lanes per row (16, 32, 64), their
+    4-element pieces, the split segments' 8 and the K steps of 16 and 8; the bytes
+    are the plain path's and no row falls back for want of a bound."""
+    g = np.random.default_rng(d)
+    n, k = 333, 7
+    x = (g.normal(size=(n, d)) + 3.0).astype(np.float32)
+    plain = hm.exact_knn(x, d, k, metric, "plain")
+    knn = hm.exact_knn(x, d, k, metric, path)
+    assert_same_bytes(knn.indices, plain.indices, "indices")
+    assert_same_bytes(knn.dists, plain.dists, "dists")
