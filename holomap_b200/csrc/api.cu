@@ -95,8 +95,8 @@ struct JobPlan {
     size_t off_mu = 0, off_csum = 0;
     int group = -1;
     uint32_t row0 = 0, unit0 = 0, kp1 = 0, k_steps = 0, k_stages = 0, row_blocks = 0, col_tiles = 0;
-    uint32_t parts = 1, part_tiles = 0, cap = 0, seed_tiles = 0, tlists = 2;
-    uint64_t slot0 = 0, cand0 = 0, topk0 = 0;
+    uint32_t parts = 1, part_tiles = 0, cap = 0, seed_tiles = 0, mins = 0, min_shift = 0;
+    uint64_t min0 = 0, cand0 = 0;
     // emission pass: symmetric (tiles on and above the diagonal), its column
     // parts per row block of ept tiles, candidate lists per row
     bool sym = false;
@@ -111,10 +111,10 @@ struct GroupPlan {
     int kind = SCREEN_KIND_BF16;
     bool split = false;
     uint32_t elem_bytes = 2, kslice = 64, kpmax = 0, rows = 0, units = 0;
-    uint32_t kp = 32, kpl = 1, dmax = 0;
+    uint32_t kpl = 1, dmax = 0;
     int metric_mask = 0;
     std::vector<uint32_t> jobs;
-    uint64_t lists = 0, cand = 0, topk = 0, elists = 0;
+    uint64_t minima = 0, cand = 0, elists = 0;
     uint32_t neunits = 0;       // emission units
     std::vector<uint4> eunits;  // their table, largest first (none for one job without symmetric units)
     bool any_sym = false;
@@ -123,7 +123,7 @@ struct GroupPlan {
     bool any_escalation = false;  // a job of the group has a split-BF16 escalation copy
     uint32_t egrid = 0, stage_cap = 0;
     size_t off_opa = 0, off_opb = 0, off_rowstat = 0, off_rowterm = 0, off_colterm = 0;
-    size_t off_band = 0, off_force = 0, off_rowthr = 0, off_cand = 0, off_cnt = 0, off_topk = 0;
+    size_t off_band = 0, off_force = 0, off_rowthr = 0, off_cand = 0, off_cnt = 0, off_minima = 0;
     size_t off_ethr = 0, off_evstar = 0, off_stage_row = 0, off_stage_key = 0, off_stage_cnt = 0;
     size_t off_rowcnt = 0, off_job_of = 0;
     // tables
@@ -310,7 +310,7 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
         B.any_screen = true;
         // operand columns: the split form's three segments lie side by side at the
         // length of the data (8: a 16-byte piece), the whole rounded up to a K step;
-        // the passes load 128-byte slices and multiply the steps (20,000 x 96: K =
+        // the passes load 128-byte slices and multiply the steps (d = 96: K =
         // 288, not 384)
         const uint32_t kstep = Gp.kslice / SC_SLICE_STEPS;
         P.kp1 = (uint32_t)round_up(P.spec.d, Gp.split ? 8u : kstep);
@@ -318,10 +318,7 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
         P.k_stages = (P.k_steps + SC_SLICE_STEPS - 1) / SC_SLICE_STEPS;
         Gp.kpmax = std::max(Gp.kpmax, P.k_stages * Gp.kslice);
         Gp.dmax = std::max(Gp.dmax, P.spec.d);
-        if (P.spec.k > 32) {
-            Gp.kp = 64;
-            Gp.kpl = 2;
-        }
+        if (P.spec.k > 32) Gp.kpl = 2;
         Gp.metric_mask |= 1 << P.spec.metric;
         P.rb0 = P.q0 / SC_BM;
         P.row_blocks = (P.q1 + SC_BM - 1) / SC_BM - P.rb0;
@@ -379,13 +376,20 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
             Gp.rows += (uint32_t)round_up(P.spec.n, 32);  // rows of each job start 32-aligned
             P.unit0 = Gp.units;
             Gp.units += P.row_blocks * P.parts;
-            P.slot0 = Gp.lists;
-            // threshold-pass lists: one per epilogue segment and column part
-            P.tlists = (uint32_t)sc_epi_warps(0, (int)Gp.kp) / 4;
-            const uint64_t lists = P.spec.n * (uint64_t)P.tlists * P.parts;
-            Gp.lists += lists;
-            P.topk0 = Gp.topk;
-            Gp.topk += lists * P.spec.k;
+            // the threshold pass's chunks: as few columns each as leave at most
+            // 128, 256 or 512 minima a row (by k: the k smallest values of a row
+            // then rarely share a chunk, which loosens the bound); chunks of
+            // more than 64 columns take several tiles of a part
+            const uint32_t limit = P.spec.k <= 20 ? 128 : P.spec.k <= 40 ? 256 : TH_MAX_MINIMA;
+            const uint32_t last = std::min(P.seed_tiles, P.col_tiles - (P.parts - 1) * P.part_tiles);
+            for (P.min_shift = 0;; ++P.min_shift) {
+                const uint32_t ti = P.min_shift > 4 ? P.min_shift - 4 : 0, per = P.min_shift > 4 ? 4 : 64u >> P.min_shift;
+                auto chunks = [&](uint32_t tiles) { return ((tiles + (1u << ti) - 1) >> ti) * per; };
+                P.mins = (P.parts - 1) * chunks(P.seed_tiles) + chunks(last);
+                if (P.mins <= limit) break;
+            }
+            P.min0 = Gp.minima;
+            Gp.minima += round_up(P.spec.n, 32) * P.mins;
             // Emission pass.  A whole dataset (not a row shard) with at least
             // two column tiles takes the symmetric form: row block rb walks
             // the column tiles from the one holding its own diagonal block
@@ -580,7 +584,7 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
         Gp.off_rowthr = take(rows * sizeof(uint32_t));
         Gp.off_cand = take(Gp.cand * sizeof(unsigned long long));
         Gp.off_cnt = take(Gp.elists * sizeof(uint32_t));
-        Gp.off_topk = take(Gp.topk * sizeof(float));
+        Gp.off_minima = take(Gp.minima * sizeof(float));
         Gp.off_rowcnt = take(rows * sizeof(uint32_t));
         if (Gp.jobs.size() > 1) Gp.off_job_of = take((rows + 31) / 32 * sizeof(uint32_t));
         if (Gp.any_sym) {
@@ -679,10 +683,11 @@ static int bind_batch(hm_batch &B, void *d_ws, size_t bytes, cudaStream_t s) {
         J.part_tiles = P.part_tiles;
         J.seed_tiles = P.seed_tiles;
         J.cap = P.cap;
-        J.slot0 = P.slot0;
-        J.tlists = P.tlists;
+        J.min0 = P.min0;
+        J.mins = P.mins;
+        J.min_shift = P.min_shift;
+        J.min_rows = (uint32_t)round_up(s.n, 32);
         J.cand0 = P.cand0;
-        J.topk0 = P.topk0;
         J.elists = P.elists;
         J.sym = P.sym ? 1u : 0u;
         J.erb0 = P.erb0;
@@ -754,7 +759,7 @@ static int bind_batch(hm_batch &B, void *d_ws, size_t bytes, cudaStream_t s) {
         D.rowthr = at<uint32_t>(ws, Gp.off_rowthr);
         D.cand = at<unsigned long long>(ws, Gp.off_cand);
         D.cand_cnt = at<uint32_t>(ws, Gp.off_cnt);
-        D.topk = at<float>(ws, Gp.off_topk);
+        D.minima = at<float>(ws, Gp.off_minima);
         D.row_cnt = at<uint32_t>(ws, Gp.off_rowcnt);
         D.job_of = Gp.jobs.size() > 1 ? at<uint32_t>(ws, Gp.off_job_of) : nullptr;
         D.eunits = Gp.eunits.empty() ? nullptr : at<uint4>(ws, Gp.off_eunits);
@@ -825,8 +830,8 @@ static int run_batch(hm_batch &B, cudaStream_t s) {
         const GroupDev *Gd = at<GroupDev>(ws, Gp.off_gdev);
         HM_TRY(launch_screen_prep(jobs, Gp.host, Gd, s));
         HM_TRY(launch_screen_band(jobs, Gp.host, Gd, s));
-        HM_TRY(launch_screen_gemm(jobs, Gp.host, Gd, Gp.kp, Gp.ta, Gp.tb, debug_dump_pointer(), 0, s));
-        HM_TRY(launch_screen_threshold(jobs, Gp.host, Gd, Gp.kpl, s));
+        HM_TRY(launch_screen_gemm(jobs, Gp.host, Gd, Gp.ta, Gp.tb, debug_dump_pointer(), 0, s));
+        HM_TRY(launch_screen_threshold(jobs, Gp.host, Gd, s));
         if (Gp.any_escalation) HM_TRY(launch_escalation(jobs, Gp.host, Gd, s));
         // lists no unit writes (parts a row block does not have) and the
         // column lists the scatter fills start empty
@@ -835,7 +840,7 @@ static int run_batch(hm_batch &B, cudaStream_t s) {
         if (Gp.any_sym)
             HM_CUDA_TRY(cudaMemsetAsync(Gp.host.stage_cnt, 0, (size_t)Gp.egrid * SC_STAGE_SLOTS * sizeof(uint32_t), s));
         if (Gp.any_sym) HM_TRY(launch_emit_limits(jobs, Gp.host, Gd, s));
-        HM_TRY(launch_screen_gemm(jobs, Gp.host, Gd, Gp.kp, Gp.ta, Gp.pair ? Gp.tb_half : Gp.tb, nullptr,
+        HM_TRY(launch_screen_gemm(jobs, Gp.host, Gd, Gp.ta, Gp.pair ? Gp.tb_half : Gp.tb, nullptr,
                                   Gp.any_sym ? 2 : 1, s));
         if (Gp.any_sym) HM_TRY(launch_column_scatter(jobs, Gp.host, Gd, Gp.egrid * SC_STAGE_SLOTS, s));
         HM_TRY(launch_rerank(jobs, Gp.host, Gd, Gp.kpl, Gp.dmax, Gp.metric_mask, s));

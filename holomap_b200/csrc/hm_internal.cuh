@@ -296,9 +296,10 @@ struct JobDev {
     // screened path
     uint32_t group, row0, unit0, kp1, k_steps, k_stages, row_blocks, col_tiles, parts, part_tiles, cap;
     uint32_t seed_tiles;         // leading column tiles of each part in the threshold pass
-    unsigned long long slot0;    // first threshold-pass list (tlists * parts lists per row)
-    uint32_t tlists;             // threshold-pass lists per column part (its epilogue segments)
-    unsigned long long topk0;    // first k-array entry: list l's is [topk0 + (l - slot0) * k, +k)
+    // threshold pass: row i's chunk minimum c (c < mins, of 4 << min_shift columns)
+    // is minima[min0 + c * min_rows + i]
+    unsigned long long min0;
+    uint32_t mins, min_shift, min_rows;
     // candidate lists of the emission pass: elists per row (two per column
     // part; with the symmetric emission one more, the row's column list, last)
     uint32_t elists, sym;        // sym: the emission pass covers the tiles on and above the diagonal

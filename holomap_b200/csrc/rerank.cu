@@ -96,7 +96,7 @@ __device__ __forceinline__ uint32_t kth_key(const uint32_t (&ov)[NQ], uint32_t t
 // The k-th smallest of a warp's 32 * NQ keys (absent ones ~0) by sorting them: up
 // to 128 keys this takes fewer instructions than a search by bits or bytes
 // (256 datasets, sorts here, in the select and in the top-k: 6,186 -> 5,753 us;
-// 5,000 x 128 cosine, k = 20: 331 -> 322).
+// 5,003 x 300 cosine: 331 -> 322).
 template <int NQ>
 __device__ __forceinline__ uint32_t kth_sorted(uint32_t (&v)[NQ], uint32_t k, int lane) {
     warp_sort<uint32_t, NQ>(v, (uint32_t)lane);
@@ -119,7 +119,13 @@ __device__ __forceinline__ uint32_t kth_load(KeyFn key, uint32_t total, uint32_t
         ov[q] = e < total ? key(e) : 0xffffffffu;
     }
     uint32_t kth;
-    if (NQ <= 4) {
+    if (NQ == 4) {
+        // of each lane's four keys the two smallest: a bound of the k-th, and the
+        // k-th itself unless a lane holds three of the k smallest
+        const uint32_t a = min(ov[0], ov[1]), b = max(ov[0], ov[1]), c = min(ov[2], ov[3]), d = max(ov[2], ov[3]);
+        uint32_t two[2] = {min(a, c), min(max(a, c), min(b, d))};
+        kth = kth_sorted<2>(two, k, lane);
+    } else if (NQ < 4) {
         kth = kth_sorted<NQ>(ov, k, lane);
     } else {
         kth = kth_key<NQ>(ov, total, k, lo, lane);
@@ -321,7 +327,7 @@ __device__ __forceinline__ uint32_t select_row(const JobDev &J, const GroupDev &
     // band of it.  Up to RR_CBUF candidates: the k-th of the first 128 bounds it,
     // so only candidates within the band of that are staged in shared memory (all
     // of the others are out) and searched for the k-th itself; up to 128
-    // candidates it is the k-th itself and nothing is staged.  (20,000 x 96, k = 15:
+    // candidates it is the k-th itself and nothing is staged.  (20,000 x 128, k = 15:
     // 46.5 -> 40.6 us; 50,000 x 384: 172 -> 159.)  Longer rows use a warp top-k.
     const bool staged = total <= RR_CBUF;
     const float band = G.band[gr];
@@ -770,59 +776,41 @@ int launch_column_scatter(const JobDev *jobs, const GroupDev &G, const GroupDev 
     return HM_OK;
 }
 
-// tau1 of every row: the k-th smallest of the union of its lists' k smallest
-// mini-chunk minima (an upper bound of the row's k-th screened value).
+// tau1 of every row: the k-th smallest of its chunk minima (an upper bound of the
+// row's k-th screened value).  A block's 8 rows (one job, 32-byte pieces of the
+// chunk-major minima) are transposed through shared memory, then a warp each finds
+// its row's k-th.  (32 rows a block of 1,024 threads read whole lines and cost
+// more: 50,000 rows of 98 minima 69 us / 109.)
 constexpr int TAU1_LOW_BITS = 10;
-template <int KPL>
+constexpr uint32_t TH_STRIDE = TH_MAX_MINIMA + 4;  // floats: 8 rows x 4 chunks on 32 banks
 __global__ void __launch_bounds__(256) threshold_kernel(const JobDev *__restrict__ jobs,
                                                        const GroupDev *__restrict__ Gp) {
+    __shared__ float s_min[8 * TH_STRIDE];
     const GroupDev &G = *Gp;
     grid_ready();
     if (group_idle(jobs, G)) return;
     const int lane = threadIdx.x & 31;
-    const uint32_t gr = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (gr >= G.rows) return;
-    const JobDev &J = group_job(jobs, G, gr);
+    const uint32_t gr0 = blockIdx.x * 8, gr = gr0 + (threadIdx.x >> 5);
+    const JobDev &J = group_job(jobs, G, gr0);
+    if (!job_active(J)) return;  // uniform over the block (G.rows is a multiple of 32)
+    const uint32_t total = J.mins, k = J.k;
+    const float *base = G.minima + J.min0 + (gr0 - J.row0);
+    for (uint32_t e = threadIdx.x; e < 8 * total; e += 256)
+        s_min[(e & 7) * TH_STRIDE + (e >> 3)] = base[(size_t)(e >> 3) * J.min_rows + (e & 7)];
+    __syncthreads();
     const uint32_t row = gr - J.row0;
-    if (row < J.q0 || row >= J.q1 || !job_active(J)) return;
-    const uint32_t k = J.k, lists = J.tlists * J.parts;
-    const size_t l0 = list_index(J, row, 0);
-    // the row's lists' arrays are contiguous: lists x k values
-    const float *base = G.topk + J.topk0 + (l0 - J.slot0) * k;
-    const uint32_t total = lists * k;
+    if (row < J.q0 || row >= J.q1) return;
+    const float *mins = s_min + (threadIdx.x >> 5) * TH_STRIDE;
     // a job with an escalation copy: the minima at or below tau1 - band
     auto below = [&](uint32_t kth) { return J.escalation ? ord32(__fsub_rd(unord32(kth), G.band[gr])) : 0u; };
-    if (total <= 256) {
-        // tau1 is an upper bound in any case: resolving it to 2^-13 of its
-        // binade (ten low key bits left as ones) emits no measurable extra
-        // candidates and halves the bit loop
-        uint32_t under;
-        const uint32_t r = kth_of([&](uint32_t e) { return ord32(base[e]); }, total, k, TAU1_LOW_BITS, lane, below, under);
-        if (lane == 0) {
-            G.rowthr[gr] = r;
-            if (J.escalation) G.row_cnt[gr] = 2 * under <= k ? 1u : 0u;  // for escalate_count_kernel
-        }
-        return;
-    }
-    WarpTopK<KPL> sel;
-    sel.reset();
-    for (uint32_t p = 0; p < lists; ++p) {
-        const float *kk = base + p * k;
-        for (uint32_t e0 = 0; e0 < k; e0 += 32) {
-            const uint64_t key = (e0 + lane < k) ? (((uint64_t)ord32(kk[e0 + lane]) << 32) | (p * k + e0 + lane))
-                                                 : KEY_NONE;
-            if (!__any_sync(0xffffffffu, key < sel.tau)) break;  // arrays are ascending
-            sel.offer(key, k, lane);
-        }
-    }
-    const uint32_t kth = sel.tau == KEY_NONE ? ord32(__int_as_float(0x7f800000)) : (uint32_t)(sel.tau >> 32);
-    uint32_t under = 0;
-#pragma unroll
-    for (int q = 0; q < KPL; ++q)
-        under += __popc(__ballot_sync(0xffffffffu, (uint32_t)(sel.v[q] >> 32) <= below(kth)));
+    // tau1 is an upper bound in any case: resolving it to 2^-13 of its binade
+    // (ten low key bits left as ones) emits no measurable extra candidates and
+    // halves the bit loop of the longer rows
+    uint32_t under = 0, r = ord32(__int_as_float(0x7f800000));
+    if (total >= k) r = kth_of([&](uint32_t e) { return ord32(mins[e]); }, total, k, TAU1_LOW_BITS, lane, below, under);
     if (lane == 0) {
-        G.rowthr[gr] = kth;
-        if (J.escalation) G.row_cnt[gr] = 2 * under <= k ? 1u : 0u;
+        G.rowthr[gr] = r;
+        if (J.escalation) G.row_cnt[gr] = total >= k && 2 * under <= k ? 1u : 0u;  // for escalate_count_kernel
     }
 }
 
@@ -886,13 +874,10 @@ int launch_escalation(const JobDev *jobs, const GroupDev &G, const GroupDev *Gd,
     return HM_OK;
 }
 
-int launch_screen_threshold(const JobDev *jobs, const GroupDev &G, const GroupDev *Gd, uint32_t kpl,
-                            cudaStream_t s) {
+int launch_screen_threshold(const JobDev *jobs, const GroupDev &G, const GroupDev *Gd, cudaStream_t s) {
     if (G.rows == 0) return HM_OK;
     ScopedKernelTimer timer(HM_KCLASS_SELECT, s);
-    const int blocks = (int)((G.rows + 7) / 8);
-    if (kpl != 1 && kpl != 2) return set_error(HM_ERR_UNSUPPORTED, "threshold width %u", kpl);
-    HM_CUDA_TRY(launch(true, kpl == 1 ? threshold_kernel<1> : threshold_kernel<2>, blocks, 256, 0, s, jobs, Gd));
+    HM_CUDA_TRY(launch(true, threshold_kernel, (G.rows + 7) / 8, 256, 0, s, jobs, Gd));
     count_launch();
     return HM_OK;
 }

@@ -43,17 +43,11 @@ constexpr int SC_STAGES = 4;
 constexpr uint32_t SC_ARES_STAGES = 6;
 // Epilogue warps per CTA: warp 0 issues the TMA loads, warp 1 the MMAs, the
 // rest read the accumulator, (warp & 3) naming their TMEM lane quadrant (32
-// query rows) and (warp - 2) / 4 their segment of the tile's 256 columns.
-// Both emission passes take 16 (four segments of 64 columns: twice the
-// warps to hide the latency of the per-row tests; each warp writes its own
-// list, so a row has four lists per column part); the threshold pass (its
-// sorted arrays need the registers) takes 8 (two segments of 128 columns).
-// A 16-warp threshold pass for k <= 32 (96 registers, some spilled, four
-// k-arrays per part) measured slower.
-__host__ __device__ constexpr int sc_epi_warps(int pass, int kp = 32) {
-    return (pass >= 1 && kp > 0) ? 16 : 8;
-}
-__host__ __device__ constexpr int sc_threads(int pass, int kp = 32) { return 64 + 32 * sc_epi_warps(pass, kp); }
+// query rows) and (warp - 2) / 4 their segment of the tile's 256 columns: four
+// segments of 64 columns, enough warps to hide the latency of the per-row tests.
+constexpr int SC_EPI_WARPS = 16;
+constexpr int SC_THREADS = 64 + 32 * SC_EPI_WARPS;
+constexpr uint32_t TH_MAX_MINIMA = 512;  // chunk minima per row the threshold kernel takes
 constexpr int SC_FULL_LISTS = 4;  // candidate lists per row and column part of the emission passes
 // column-side candidate stages per CTA of the symmetric emission pass (one
 // per epilogue warp)
@@ -89,11 +83,10 @@ struct GroupDev {
     RowStat *rowstat;
     float *rowterm, *colterm, *band;  // colterm padded by SC_BN zeros
     uint8_t *force;               // rows the screen cannot bound (cosine zero vectors)
-    uint32_t *rowthr;             // per row, ordered key: pass 0 the smallest list k-th so
-                                  // far; pass 1 tau1, the k-th smallest mini-chunk minimum
+    uint32_t *rowthr;             // per row, ordered key: tau1, the k-th smallest chunk minimum
     unsigned long long *cand;     // candidate lists, (c^ bits << 32) | job-local column
     uint32_t *cand_cnt;
-    float *topk;                  // each list's k smallest mini-chunk minima, ascending
+    float *minima;                // threshold pass: chunk minima, chunk-major per job
     uint32_t *row_cnt;            // rerank: survivors per group row (0: none or exact fallback)
     // emission pass: its work units (x = group job slot | sym << 31, y = row
     // block, z = first column tile, w = end column tile | column part << 24),
@@ -140,11 +133,6 @@ __device__ __forceinline__ bool group_idle(const JobDev *jobs, const GroupDev &G
     return G.njobs == 1 && !job_active(jobs[G.job_ids[0]]);
 }
 
-// Row i's threshold-pass list s (s < tlists * parts) of job J (its k-array).
-__device__ __forceinline__ size_t list_index(const JobDev &J, uint32_t i, uint32_t s) {
-    return (size_t)J.slot0 + (size_t)i * J.tlists * J.parts + s;
-}
-
 // Row i's candidate list s (s < elists) of job J: its count is
 // G.cand_cnt[cand_list(J, i, s)], its slots follow cand_slots.
 __device__ __forceinline__ size_t cand_list(const JobDev &J, uint32_t i, uint32_t s) {
@@ -156,11 +144,10 @@ __device__ __forceinline__ unsigned long long *cand_slots(const JobDev &J, const
 
 int launch_screen_prep(const JobDev *jobs, const GroupDev &G, const GroupDev *Gd, cudaStream_t s);
 int launch_screen_band(const JobDev *jobs, const GroupDev &G, const GroupDev *Gd, cudaStream_t s);
-int launch_screen_gemm(const JobDev *jobs, const GroupDev &G, const GroupDev *Gd, uint32_t kp,
+int launch_screen_gemm(const JobDev *jobs, const GroupDev &G, const GroupDev *Gd,
                        const CUtensorMap &ta, const CUtensorMap &tb, float *dump, int pass,
                        cudaStream_t s);
-int launch_screen_threshold(const JobDev *jobs, const GroupDev &G, const GroupDev *Gd, uint32_t kpl,
-                            cudaStream_t s);
+int launch_screen_threshold(const JobDev *jobs, const GroupDev &G, const GroupDev *Gd, cudaStream_t s);
 int launch_rerank(const JobDev *jobs, const GroupDev &G, const GroupDev *Gd, uint32_t kpl,
                   uint32_t dmax, int metric_mask, cudaStream_t s);
 // symmetric emission: the per-row limits before the emission pass, and the

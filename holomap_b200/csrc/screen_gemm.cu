@@ -2,29 +2,30 @@
 // accumulators, fused with the per-row thresholds and the candidate emission,
 // so the N x N similarity matrix never leaves the SM.
 //
-// One CTA per SM (persistent), 10 warps (18 in the emission passes):
+// One CTA per SM (persistent), 18 warps:
 //   warp 0     TMA producer: the unit's 128-row A block stays resident in
 //              shared memory when its K slices fit 96 KB (else it streams
 //              with B), 256-row B slices per stage (128-byte K slices, 128B
 //              swizzle, 4-stage mbarrier ring; every CTA loads its own tiles),
 //   warp 1     allocates 512 TMEM columns (two 128 x 256 fp32 accumulators)
 //              and issues tcgen05.mma (one thread) + tcgen05.commit,
-//   warps 2-   epilogue: each thread owns one query row (its TMEM lane) and
-//              one segment of every tile's 256 columns (half, read 32 columns
-//              at a time, in the threshold pass; a quarter, read 16 columns
-//              at a time, in the emission passes).
+//   warps 2-17 epilogue: each thread owns one query row (its TMEM lane) and a
+//              quarter of every tile's 256 columns, read 16 at a time.
 // The emission passes can also run in the 2-SM form: a cluster of two
 // CTAs shares each 256 x 256 tile (one tcgen05.mma.cta_group::2 of M = 256
 // issued by the leader CTA), each CTA holding its own 128 rows of A and
 // loading half of the column tile into an 8-stage ring.
 // Two launches per group (template PASS):
-//   0  threshold pass over a sample of each part's columns: per list, the k
-//      smallest minima of column chunks, sorted in registers and shared
-//      between the row's lists (atomicMin); threshold_kernel then takes the
-//      k-th of the union, tau1, an upper bound of the row's k-th screened value;
-//   1  emission pass over all columns with the fixed limit tau1 + band: 8-column
-//      group minima gate the per-column test, which writes every column within
-//      the limit into the row's list;
+//   0  threshold pass over a sample of each part's columns: the smallest
+//      screened value of each chunk of columns, written chunk-major;
+//      threshold_kernel then takes the k-th smallest of a row's, tau1, an upper
+//      bound of the row's k-th screened value.  (Sorted arrays of the k smallest
+//      in registers, one insertion network per chunk in 8 warps: 256 datasets
+//      1,090 us for the pass and 141 for the threshold, now 571 and 297; 20,000 x
+//      128 84 + 20, now 49 + 12; 50,000 x 384 272 + 55, now 221 + 69);
+//   1  emission pass over all columns with the fixed limit tau1 + band: groups of
+//      four columns are decided by one comparison, and every column within the
+//      limit is written into the row's list;
 //   2  the emission pass of a group whose whole datasets take the symmetric
 //      form: a row block walks only the tiles from its diagonal on, with the
 //      limit tau1 + 2 band, and each value above the diagonal is also tested
@@ -176,22 +177,8 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
 }
 
 // tcgen05.ld of 32 consecutive accumulator columns of this warp's 32 lanes;
-// the registers are valid only after tmem_ld_wait on the same array (the
+// the registers are valid only after tmem_ld_wait16 on the same array (the
 // wait names them as in/out operands so no use can be scheduled before it).
-__device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32"
-        " {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15,"
-        " %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31},"
-        " [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-          "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-          "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]),
-          "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]),
-          "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr));
-}
-
 // (w0, w1) += (c0, c1) * h, each rounded once
 __device__ __forceinline__ void fma2(float &w0, float &w1, float c0, float c1, float h) {
     asm("{\n\t.reg .b64 w, c, h;\n\t"
@@ -214,17 +201,6 @@ __device__ __forceinline__ void tmem_ld_wait16(uint32_t (&v)[16]) {
                  : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]),
                    "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]),
                    "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])
-                 :
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_ld_wait(uint32_t (&v)[32]) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]),
-                   "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]),
-                   "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]), "+r"(v[16]), "+r"(v[17]),
-                   "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]),
-                   "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]),
-                   "+r"(v[30]), "+r"(v[31])
                  :
                  : "memory");
 }
@@ -280,8 +256,8 @@ __device__ __forceinline__ UnitTiles unit_tiles(const JobDev *jobs, const GroupD
     return t;
 }
 
-template <int KIND, int KP, int PASS, bool PAIR>
-__global__ void __launch_bounds__(sc_threads(PASS, KP), 1)
+template <int KIND, int PASS, bool PAIR>
+__global__ void __launch_bounds__(SC_THREADS, 1)
     screen_gemm_kernel(const __grid_constant__ CUtensorMap tma, const __grid_constant__ CUtensorMap tmb,
                        const JobDev *__restrict__ jobs, const GroupDev G, float *dump, uint32_t idesc,
                        uint32_t a_res) {
@@ -318,7 +294,7 @@ __global__ void __launch_bounds__(sc_threads(PASS, KP), 1)
     // PASS 2 is the emission pass of a group with symmetric units (the
     // column-side tests exist only in that instantiation)
     constexpr bool SYMK = PASS == 2;
-    constexpr uint32_t EW = sc_epi_warps(PASS, KP);  // epilogue warps
+    constexpr uint32_t EW = SC_EPI_WARPS;
     static_assert(!SYMK || EW == SC_STAGE_SLOTS, "one column-side stage per epilogue warp");
     constexpr uint32_t NSEG = EW / 4;             // column segments per tile (= lists per part)
     constexpr uint32_t SEGW = SC_BN / NSEG;       // columns per segment
@@ -543,19 +519,16 @@ __global__ void __launch_bounds__(sc_threads(PASS, KP), 1)
             const float band = valid ? G.band[gr] : 0.0f;
             const float rowterm = valid ? G.rowterm[gr] : 0.0f;
             const float scale = J.scale;
-            // pass 0: the row's threshold-pass list (its k-array); pass 1: its
-            // candidate list for this column part and segment
-            const size_t list = PASS == 0 ? list_index(J, valid ? row : 0, ut.part * NSEG + seg)
-                                          : cand_list(J, valid ? row : 0, ut.part * NSEG + seg);
+            // pass 1: the row's candidate list for this column part and segment
+            const size_t list = cand_list(J, valid ? row : 0, ut.part * NSEG + seg);
             const float *colterm = G.colterm + J.row0;
-            // pass 0: the k smallest mini-chunk minima seen (ascending;
-            // arr[KP-1] is the list's k-th) and the row's shared k-th
-            float arr[PASS == 0 ? KP : 1];
-#pragma unroll
-            for (int q = 0; q < (PASS == 0 ? KP : 1); ++q) arr[q] = (q < KP - (int)J.k) ? -INF : INF;
-            float tglob = INF, published = INF;
-            uint32_t tnext = 0xff800000u;  // ordered key of +inf
-            const bool chunk_min = J.seed_tiles < J.part_tiles;
+            // pass 0: the row's minima of column chunks (chunk-major, so a warp's 32
+            // rows are one line) and the running one of a chunk over several
+            // 16-column pieces, or over several tiles
+            float *mins = nullptr;
+            const size_t min_rows = J.min_rows;
+            float acc = -INF;
+            if (PASS == 0) mins = G.minima + J.min0 + row;
             // pass 1: the row's fixed limit, tau1 + band (symmetric: tau1 +
             // 2 band, precomputed; a pair's value may come from the tile of the
             // other orientation, within 2E of the threshold pass's value)
@@ -628,110 +601,90 @@ __global__ void __launch_bounds__(sc_threads(PASS, KP), 1)
                     }
                     continue;
                 }
-                if (PASS == 0 && valid) {
-                    // the row's other lists may have tightened its k-th: use the
-                    // value loaded during the previous tile, load the next one
-                    tglob = fminf(tglob, unord32(tnext));
-                    tnext = *(volatile const uint32_t *)(G.rowthr + gr);
-                }
                 const bool diag = (ct * SC_BN < myrb * SC_BM + SC_BM) && (myrb * SC_BM < ct * SC_BN + SC_BN);
                 const uint32_t t_base = tmem_base + ((quad * 32) << 16) + buf * SC_BN + seg * SEGW;
-                // the threshold pass's chunk = 32 columns; the accumulator
-                // registers are overwritten in place by the screened values
-                auto process = [&](uint32_t (&v)[32], uint32_t ch) {
-                    float (&c)[32] = reinterpret_cast<float (&)[32]>(v);
-                    const uint32_t j0 = c_base + ch * 32;  // job-local column
-                    const bool full = j0 + 32 <= n;
-                    const bool self_here = diag && (row - j0 < 32u);
-                    // exact screened values of every column of the chunk
-                    // (columns past n: +inf; the row itself: 0)
-                    auto values = [&]() {
-                        if (fast_cos) {
+                // the screened value of a product and its column's term, c = rowterm
+                // - scale (v - cs / scale), two roundings (within the band's 2^-21 of
+                // the squared norms), falls as the difference w grows: minima of c
+                // are maxima of w (cosine without zero rows: w = v, c = 1 - v)
+                auto value = [&](float w) { return fast_cos ? __fsub_rn(1.0f, w) : __fmaf_rn(-scale, w, rowterm); };
+                auto terms = [&](float (&cs)[16], uint32_t j0) {
+                    if (fast_cos) return;
+                    const float4 *ctp = reinterpret_cast<const float4 *>(colterm + j0);
 #pragma unroll
-                            for (int t = 0; t < 32; ++t) c[t] = __fsub_rn(1.0f, c[t]);
-                        } else {
-                            const float4 *ctp = reinterpret_cast<const float4 *>(colterm + j0);
-#pragma unroll
-                            for (int q = 0; q < 8; ++q) {
-                                const float4 cq = __ldg(ctp + q);
-                                const float cs[4] = {cq.x, cq.y, cq.z, cq.w};
-#pragma unroll
-                                for (int e = 0; e < 4; ++e)
-                                    c[4 * q + e] =
-                                        __fsub_rn(__fadd_rn(rowterm, cs[e]), __fmul_rn(scale, c[4 * q + e]));
-                            }
-                        }
-                        if (!full) {
-#pragma unroll
-                            for (int t = 0; t < 32; ++t)
-                                if (j0 + t >= n) c[t] = INF;
-                        }
-                        if (self_here) {
-#pragma unroll
-                            for (int t = 0; t < 32; ++t)
-                                if (j0 + t == row) c[t] = 0.0f;
-                        }
-                    };
-                    // cosine fast path: c = 1 - v is monotone in v, so a
-                    // minimum of c is 1 - (the maximum of v), bit for bit
-                    const bool quick = fast_cos && full && !self_here && !dump;
-                    if (PASS == 0) {
-                        // mini-chunk minima: columns {t, t+8, t+16, t+24}
-                        float m[8];
-                        if (quick) {
-#pragma unroll
-                            for (int t = 0; t < 8; ++t)
-                                m[t] = __fsub_rn(1.0f, fmaxf(fmaxf(c[t], c[t + 8]), fmaxf(c[t + 16], c[t + 24])));
-                        } else {
-                            values();
-                            if (dump && valid) {
-                                for (int t = 0; t < 32; ++t)
-                                    if (j0 + t < n) dump[(size_t)row * n + j0 + t] = c[t];
-                            }
-#pragma unroll
-                            for (int t = 0; t < 8; ++t)
-                                m[t] = fminf(fminf(c[t], c[t + 8]), fminf(c[t + 16], c[t + 24]));
-                        }
-                        // a sampled threshold pass keeps one minimum per 32-column
-                        // chunk (an eighth of the insertions; the sample's k smallest
-                        // rarely share a chunk), a full one the eight mini-chunk minima
-                        if (chunk_min) {
-#pragma unroll
-                            for (int t = 1; t < 8; ++t) m[0] = fminf(m[0], m[t]);
-                        }
-                        // minima that can be among the row's k smallest
-                        uint32_t pm = 0;
-#pragma unroll
-                        for (int t = 0; t < 8; ++t)
-                            pm |= (m[t] < arr[KP - 1] && !(m[t] > tglob) && (t == 0 || !chunk_min)) ? (1u << t) : 0u;
-                        if (!valid) pm = 0;
-                        if (pm) {
-                            while (pm) {
-                                const int t = __ffs(pm) - 1;
-                                pm &= pm - 1;
-                                float x = m[0];
-#pragma unroll
-                                for (int q = 1; q < 8; ++q) x = (t == q) ? m[q] : x;
-                                if (x < arr[KP - 1]) {
-#pragma unroll
-                                    for (int q = KP - 1; q > 0; --q) arr[q] = fminf(arr[q], fmaxf(arr[q - 1], x));
-                                    arr[0] = fminf(arr[0], x);
-                                }
-                            }
-                            const float tl = arr[KP - 1];
-                            if (tl < published) {
-                                // share with the row's other lists: a reduction
-                                // whose result is not waited for (the other
-                                // lists' values arrive through tnext, loaded a
-                                // tile ahead)
-                                atomicMin(G.rowthr + gr, ord32(tl));
-                                tglob = fminf(tglob, tl);
-                                published = tl;
-                            }
-                        }
+                    for (int q = 0; q < 4; ++q) {
+                        const float4 c4 = __ldg(ctp + q);
+                        cs[4 * q] = c4.x, cs[4 * q + 1] = c4.y, cs[4 * q + 2] = c4.z, cs[4 * q + 3] = c4.w;
                     }
                 };
-                if constexpr (EW >= 16) {
+                // whether a warp's 16-column piece holds columns past n or one of its
+                // rows (warp-uniform: the warp's rows are 32 columns of the diagonal tile)
+                auto edge_piece = [&](uint32_t j0) {
+                    return j0 + 16 > n || (diag && j0 + 16 > row - lane && j0 < row - lane + 32);
+                };
+                if constexpr (PASS == 0) {
+                    // chunk minima: 4 << min_shift columns, from four columns to the
+                    // warp's 64 of 2^i tiles.  The minima themselves are the output
+                    // (threshold_kernel finds the k-th), nothing is kept sorted here
+                    const uint32_t tl = ct - ut.ct_begin, shift = J.min_shift;
+                    const uint32_t ti = shift > 4 ? shift - 4 : 0;  // tiles per chunk: 1 << ti
+                    const uint32_t per = shift > 4 ? 4u : 64u >> shift;  // chunks per tile
+                    // first chunk of the tile and segment, counted over the row's parts
+                    const uint32_t at0 = (ut.part * ((J.seed_tiles + (1u << ti) - 1) >> ti) + (tl >> ti)) * per +
+                                         seg * (shift > 4 ? 1u : 16u >> shift);
+                    auto put = [&](uint32_t at, float w) {
+                        if (valid) mins[(size_t)(at0 + at) * min_rows] = value(w);
+                    };
+#pragma unroll 1
+                    for (uint32_t ch = 0; ch < SEGW / 16; ++ch) {
+                        const uint32_t j0 = c_base + ch * 16;
+                        uint32_t vr[16];
+                        float cs[16];
+                        tmem_ld16_issue(t_base + ch * 16, vr);
+                        terms(cs, j0);
+                        tmem_ld_wait16(vr);
+                        float (&w)[16] = reinterpret_cast<float (&)[16]>(vr);
+                        if (!fast_cos) {
+#pragma unroll
+                            for (int e = 0; e < 16; e += 2) fma2(w[e], w[e + 1], cs[e], cs[e + 1], hscale);
+                        }
+                        if (edge_piece(j0)) {
+                            // the row itself: value 0; columns past n: +inf
+                            const float self = fast_cos ? 1.0f : -rowterm * hscale;
+#pragma unroll
+                            for (int e = 0; e < 16; ++e) {
+                                if (j0 + e == row) w[e] = self;
+                                if (j0 + e >= n) w[e] = -INF;
+                            }
+                        }
+                        if (dump && valid) {
+                            for (uint32_t e = 0; e < 16; ++e)
+                                if (j0 + e < n) dump[(size_t)row * n + j0 + e] = value(w[e]);
+                        }
+                        float m[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            m[q] = fmaxf(fmaxf(w[4 * q], w[4 * q + 1]), fmaxf(w[4 * q + 2], w[4 * q + 3]));
+                        if (shift == 0) {
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) put(4 * ch + q, m[q]);
+                            continue;
+                        }
+                        const float m0 = fmaxf(m[0], m[1]), m1 = fmaxf(m[2], m[3]);
+                        if (shift == 1) {
+                            put(2 * ch, m0);
+                            put(2 * ch + 1, m1);
+                            continue;
+                        }
+                        acc = fmaxf(acc, fmaxf(m0, m1));
+                        const bool last = shift <= 4 ? ((ch + 1) & ((1u << (shift - 2)) - 1)) == 0
+                                                     : ch == 3 && (((tl + 1) & ((1u << ti) - 1)) == 0 || ct + 1 == ut.ct_end);
+                        if (last) {
+                            put(shift <= 4 ? ch >> (shift - 2) : 0u, acc);
+                            acc = -INF;
+                        }
+                    }
+                } else {
                     // the full emission pass (96 registers a thread): 16-column
                     // loads, the next in flight while this one is tested
                     const uint32_t cap = J.cap;
@@ -807,7 +760,7 @@ __global__ void __launch_bounds__(sc_threads(PASS, KP), 1)
                     // c = rowterm - scale (v - cs / scale), two roundings: within the
                     // band's 2^-21 of the squared norms, as the threshold pass's form
                     // is.  Against 8-column groups with a loop over their candidates
-                    // and each column's value in three operations: 20,000 x 96
+                    // and each column's value in three operations: 20,000 x 128
                     // emission 366 -> 327 us, 50,000 x 384 cosine 1,532 -> 1,518;
                     // groups of 8 cost 10 and 60 us more, a second register buffer of
                     // products 18 and 80 (the loop leaves the instruction cache).
@@ -867,23 +820,12 @@ __global__ void __launch_bounds__(sc_threads(PASS, KP), 1)
                         if constexpr (SYMK) {
                             if (colside) colside16(v, j0);
                         }
-                        // (warp-uniform: the warp's rows are 32 columns of the diagonal tile)
-                        const bool edge = j0 + 16 > n || (diag && j0 + 16 > row - lane && j0 < row - lane + 32);
-                        if (edge)
+                        if (edge_piece(j0))
                             emit16_edge(v, j0);
                         else if (fast_cos)
                             emit16(v, cs, j0, std::true_type());
                         else
                             emit16(v, cs, j0, std::false_type());
-                    };
-                    auto terms = [&](float (&cs)[16], uint32_t j0) {
-                        if (fast_cos) return;
-                        const float4 *ctp = reinterpret_cast<const float4 *>(colterm + j0);
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            const float4 c4 = __ldg(ctp + q);
-                            cs[4 * q] = c4.x, cs[4 * q + 1] = c4.y, cs[4 * q + 2] = c4.z, cs[4 * q + 3] = c4.w;
-                        }
                     };
 #pragma unroll 1
                     for (uint32_t ch = 0; ch < SEGW / 16; ++ch) {
@@ -896,21 +838,6 @@ __global__ void __launch_bounds__(sc_threads(PASS, KP), 1)
                         tmem_ld_wait16(vr);
                         chunk(vr, cs, j0);
                     }
-                } else {
-                    // two warps per scheduler: the next chunk loads while
-                    // this one is processed
-                    uint32_t va[32], vb[32];
-                    tmem_ld32_issue(t_base, va);
-                    tmem_ld_wait(va);
-#pragma unroll 1
-                    for (uint32_t ch = 0; ch < SEGW / 32; ch += 2) {
-                        tmem_ld32_issue(t_base + (ch + 1) * 32, vb);
-                        process(va, ch);
-                        tmem_ld_wait(vb);
-                        if (ch + 2 < SEGW / 32) tmem_ld32_issue(t_base + (ch + 2) * 32, va);
-                        process(vb, ch + 1);
-                        if (ch + 2 < SEGW / 32) tmem_ld_wait(va);
-                    }
                 }
                 fence_before_sync();
                 __syncwarp();
@@ -922,15 +849,7 @@ __global__ void __launch_bounds__(sc_threads(PASS, KP), 1)
                 }
             }
             if (!ok) break;
-            if (PASS == 0) {
-                if (valid) {
-                    // the list's k smallest mini-chunk minima (ascending)
-                    float *kk = G.topk + J.topk0 + (list - J.slot0) * J.k;
-#pragma unroll
-                    for (int q = 0; q < KP; ++q)
-                        if (q >= KP - (int)J.k) kk[q - (KP - (int)J.k)] = arr[q];
-                }
-            } else {
+            if (PASS >= 1) {
                 if (valid) G.cand_cnt[list] = cnt;
                 const uint32_t e = __reduce_add_sync(0xffffffffu, (valid ? cnt : 0u) + colsum);
                 if (lane == 0 && e) atomicAdd(&J.out->emitted, (unsigned long long)e);
@@ -1001,15 +920,15 @@ static uint32_t pair_slots(const void *func, uint32_t threads) {
 template <int KIND, int PASS>
 static int launch_pair(const JobDev *jobs, const GroupDev &G, const CUtensorMap &ta, const CUtensorMap &tb,
                        uint32_t idesc, cudaStream_t s) {
-    const void *func = (const void *)screen_gemm_kernel<KIND, 32, PASS, true>;
+    const void *func = (const void *)screen_gemm_kernel<KIND, PASS, true>;
     HM_TRY(ensure_dynamic_smem(func, (int)SC_SMEM_BYTES));
-    const uint32_t slots = pair_slots(func, (uint32_t)sc_threads(PASS));
+    const uint32_t slots = pair_slots(func, (uint32_t)SC_THREADS);
     if (slots == 0) return set_error(HM_ERR_CUDA, "no room for a cluster of two screen CTAs");
     const uint32_t clusters = G.neunits < slots ? G.neunits : slots;
     if (clusters == 0) return HM_OK;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * clusters, 1, 1);
-    cfg.blockDim = dim3(sc_threads(PASS), 1, 1);
+    cfg.blockDim = dim3(SC_THREADS, 1, 1);
     cfg.dynamicSmemBytes = SC_SMEM_BYTES;
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
@@ -1022,25 +941,25 @@ static int launch_pair(const JobDev *jobs, const GroupDev &G, const CUtensorMap 
     cfg.attrs = attr;
     cfg.numAttrs = 2;
     const uint32_t pidesc = (idesc & ~(0x1fu << 24)) | (((uint32_t)(2 * SC_BM) >> 4) << 24);  // M = 256
-    HM_CUDA_TRY(cudaLaunchKernelEx(&cfg, screen_gemm_kernel<KIND, 32, PASS, true>, ta, tb, jobs, G,
+    HM_CUDA_TRY(cudaLaunchKernelEx(&cfg, screen_gemm_kernel<KIND, PASS, true>, ta, tb, jobs, G,
                                    (float *)nullptr, pidesc, 1u));
     count_launch();
     return HM_OK;
 }
 
-template <int KIND, int KP, int PASS>
+template <int KIND, int PASS>
 static int launch_kind(const JobDev *jobs, const GroupDev &G, const CUtensorMap &ta,
                        const CUtensorMap &tb, float *dump, uint32_t idesc, cudaStream_t s) {
-    if constexpr (PASS >= 1 && KP == 32) {
+    if constexpr (PASS >= 1) {
         if (G.pair) return launch_pair<KIND, PASS>(jobs, G, ta, tb, idesc, s);
     }
-    HM_TRY(ensure_dynamic_smem((const void *)screen_gemm_kernel<KIND, KP, PASS, false>, (int)SC_SMEM_BYTES));
+    HM_TRY(ensure_dynamic_smem((const void *)screen_gemm_kernel<KIND, PASS, false>, (int)SC_SMEM_BYTES));
     const uint32_t sms = (uint32_t)device_sm_count();
     const uint32_t grid = PASS >= 1 ? emission_grid(G) : (G.units < sms ? G.units : sms);
     if (grid == 0) return HM_OK;
     // every job's K slices fit the resident A block
     const uint32_t a_res = (G.kpmax / G.kslice) <= SC_ARES_STAGES ? 1u : 0u;
-    HM_CUDA_TRY(launch(true, screen_gemm_kernel<KIND, KP, PASS, false>, grid, sc_threads(PASS, KP), SC_SMEM_BYTES, s, ta,
+    HM_CUDA_TRY(launch(true, screen_gemm_kernel<KIND, PASS, false>, grid, SC_THREADS, SC_SMEM_BYTES, s, ta,
                        tb, jobs, G, dump, idesc, a_res));
     count_launch();
     return HM_OK;
@@ -1060,27 +979,25 @@ static uint32_t make_idesc(int kind) {
 }
 
 template <int KIND>
-static int launch_pass(const JobDev *jobs, const GroupDev &G, uint32_t kp, const CUtensorMap &ta,
+static int launch_pass(const JobDev *jobs, const GroupDev &G, const CUtensorMap &ta,
                        const CUtensorMap &tb, float *dump, uint32_t idesc, int pass, cudaStream_t s) {
-    if (pass == 1) return launch_kind<KIND, 32, 1>(jobs, G, ta, tb, nullptr, idesc, s);
-    if (pass == 2) return launch_kind<KIND, 32, 2>(jobs, G, ta, tb, nullptr, idesc, s);
-    if (kp == 32) return launch_kind<KIND, 32, 0>(jobs, G, ta, tb, dump, idesc, s);
-    if (kp == 64) return launch_kind<KIND, 64, 0>(jobs, G, ta, tb, dump, idesc, s);
-    return set_error(HM_ERR_UNSUPPORTED, "screen top-k width %u", kp);
+    if (pass == 1) return launch_kind<KIND, 1>(jobs, G, ta, tb, nullptr, idesc, s);
+    if (pass == 2) return launch_kind<KIND, 2>(jobs, G, ta, tb, nullptr, idesc, s);
+    return launch_kind<KIND, 0>(jobs, G, ta, tb, dump, idesc, s);
 }
 
-// pass 0: each list's k smallest chunk minima over the column sample (-> tau1);
+// pass 0: each row's chunk minima over the column sample (-> tau1);
 // pass 1: emission of every column within tau1 + band; pass 2: the same for a
 // group with symmetric units (tiles on and above the diagonal, column side too)
-int launch_screen_gemm(const JobDev *jobs, const GroupDev &G, const GroupDev *, uint32_t kp,
+int launch_screen_gemm(const JobDev *jobs, const GroupDev &G, const GroupDev *,
                        const CUtensorMap &ta, const CUtensorMap &tb, float *dump, int pass,
                        cudaStream_t s) {
     if (G.units == 0) return HM_OK;
     ScopedKernelTimer timer(HM_KCLASS_BULK, s);
     const uint32_t idesc = make_idesc((int)G.kind);
     if (G.kind == SCREEN_KIND_BF16)
-        return launch_pass<SCREEN_KIND_BF16>(jobs, G, kp, ta, tb, dump, idesc, pass, s);
-    return launch_pass<SCREEN_KIND_TF32>(jobs, G, kp, ta, tb, dump, idesc, pass, s);
+        return launch_pass<SCREEN_KIND_BF16>(jobs, G, ta, tb, dump, idesc, pass, s);
+    return launch_pass<SCREEN_KIND_TF32>(jobs, G, ta, tb, dump, idesc, pass, s);
 }
 
 }  // namespace hm

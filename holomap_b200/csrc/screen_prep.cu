@@ -145,8 +145,7 @@ __device__ __forceinline__ uint32_t to_tf32_bits(double v, double *rounded) {
 }
 
 // Operand rows: the row's elements in the group's format, its binary64 error
-// statistics, the additive terms of the screen epilogue and the row's shared
-// threshold.  A row of K1 elements takes 4, 8 or 16 lanes when K1 is at most
+// statistics and the additive terms of the screen epilogue.  A row of K1 elements takes 4, 8 or 16 lanes when K1 is at most
 // OP_SHORT_K1 (a warp then holds OP_TILE consecutive rows, all loaded before the
 // first is worked on), else the warp; each kernel skips the other's jobs.  A lane
 // takes 4 consecutive elements at a time, so an operand piece is one 8 or 16 byte
@@ -154,9 +153,9 @@ __device__ __forceinline__ uint32_t to_tf32_bits(double v, double *rounded) {
 // reduced transposed (6 shuffles for the four, each lane left with one of them),
 // and the four square roots are one, taken side by side.  A block takes
 // consecutive rows, mostly of one job, and combines its warps' maxima before the
-// job's counters see them.  256 datasets of d = 8..64: 659 us (both kernels) with a
+// job's counters see them.  256 datasets: 659 us (both kernels) with a
 // warp's every lane summing all four, lane 0 taking the roots and 2-byte stores,
-// 448 now; 20,000 x 96: 40 -> 25; 50,000 x 384 (BF16): 104 -> 89.
+// 448 now; 20,000 x 128: 40 -> 25; 50,000 x 384 (BF16): 104 -> 89.
 constexpr uint32_t OP_WARPS = 8;
 constexpr int OP_BLOCKS_PER_SM = 3;
 constexpr uint32_t OP_SHORT_K1 = 64;
@@ -223,7 +222,7 @@ __global__ void __launch_bounds__(OP_WARPS * 32, OP_BLOCKS_PER_SM) operand_kerne
     // the blocks take chunks of rows in turn (a group's short and long rows lie in
     // runs, of which each kernel works on one kind).  Chunks of one tile a warp
     // against four: short rows of 256 datasets 167 us / 257; of one row against two
-    // and eight: their long rows 312 / 281 / 268, 5,000 x 128 26 / 26 / 41
+    // and eight: their long rows 312 / 281 / 268, 5,003 x 300 26 / 26 / 41
     constexpr uint32_t CHUNK = SHORT ? 1 : 2;  // tiles a warp takes of one
     for (uint32_t i = 0;; ++i) {
         const uint32_t ti = ((i / CHUNK * gridDim.x + blockIdx.x) * CHUNK + i % CHUNK) * OP_WARPS + warp;
@@ -346,7 +345,6 @@ __global__ void __launch_bounds__(OP_WARPS * 32, OP_BLOCKS_PER_SM) operand_kerne
                 G.colterm[gr] = euc ? term : zero_row ? 0.0f : 1.0f;
                 G.force[gr] = zero_row ? 1 : 0;
                 zeros += zero_row ? 1u : 0u;
-                G.rowthr[gr] = 0xff800000u;  // the row's shared threshold starts at +inf
             } else if (sl == o2) {
                 st.enorm = root;
             } else if (sl == o1) {

@@ -361,3 +361,24 @@ def test_operand_rows_of_every_length_class(path, metric, d):
     knn = hm.exact_knn(x, d, k, metric, path)
     assert_same_bytes(knn.indices, plain.indices, "indices")
     assert_same_bytes(knn.dists, plain.dists, "dists")
+
+
+@pytest.mark.parametrize("seed_div", [1, 3, 8])
+@pytest.mark.parametrize("metric", ["euclidean", "cosine"])
+def test_threshold_chunks_of_every_width(seed_div, metric):
+    """Sizes and k for which a row's chunk minima cover 4 columns up to 64 of several
+    tiles, with a last part and a last chunk that are not full; fewer minima than k."""
+    from holomap_b200 import _lib
+    g = np.random.default_rng(seed_div)
+    lib = _lib.lib()
+    assert lib.hm_tuning_override(seed_div) == 0
+    try:
+        for n, k in ((40, 20), (130, 3), (257, 5), (700, 64), (1500, 21), (2049, 15), (4100, 41), (9001, 5), (20011, 12)):
+            x = g.normal(size=(n, 10)).astype(np.float32)
+            x[n // 3] = x[n // 2]
+            plain = hm.exact_knn(x, 10, k, metric, "plain")
+            knn = hm.exact_knn(x, 10, k, metric, "screen_bf16x3")
+            assert_same_bytes(knn.indices, plain.indices, f"{n} {k} indices")
+            assert_same_bytes(knn.dists, plain.dists, f"{n} {k} dists")
+    finally:
+        lib.hm_tuning_override(0)
