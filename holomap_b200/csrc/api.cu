@@ -100,7 +100,7 @@ struct JobPlan {
     // emission pass: symmetric (tiles on and above the diagonal), its column
     // parts per row block of ept tiles, candidate lists per row
     bool sym = false;
-    uint32_t ept = 0, elists = 0, erb0 = 0, eparts = 1;
+    uint32_t ept = 0, elists = 0, erb0 = 0, erbs = 0, eparts = 1, ework = 0;
     uint64_t eslot0 = 0;
     // escalation: the job's split-BF16 copy (clone), or the job a copy is of
     int clone = -1, clone_of = -1;
@@ -198,6 +198,16 @@ static uint32_t plain_splits(const JobPlan &P, uint64_t groups, uint32_t sms) {
         }
     }
     return splits;
+}
+
+// Most workers that share a row block of a job's emission pass (their parts of its
+// columns), its tiles cut into ework equal ranges.
+static uint32_t emission_parts(const JobPlan &P) {
+    const uint64_t ct = P.col_tiles, tiles = P.erbs * ct, w = P.ework;
+    uint64_t parts = 1;
+    for (uint64_t s = 0; s < tiles; s += ct)
+        parts = std::max(parts, ((s + ct) * w - 1) / tiles - ((s + 1) * w - 1) / tiles + 1);
+    return (uint32_t)parts;
 }
 
 // `ranges` (optional): 2 per job, the job's query rows [begin, end); every
@@ -406,16 +416,31 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
                 P.ept = P.part_tiles;
             }
         }
+        // The emission pass takes the 2-SM form (a cluster of two CTAs per
+        // block of 256 rows, each loading half of every column tile) when
+        // every job's K slices fit the resident A block and the autotuner
+        // table prefers it for every job.
+        Gp.pair = !Gp.pair_vetoed && Gp.kpmax / Gp.kslice <= SC_ARES_STAGES;
         // Candidate lists per row: SC_FULL_LISTS per column part (one per
         // epilogue segment of the emission pass), and for a symmetric job the
         // column list, which takes two lists' room.  The cap of a list grows
         // with the columns it covers.
         for (uint32_t j : Gp.jobs) {
             JobPlan &P = B.jobs[j];
-            const uint32_t eparts = (P.col_tiles + P.ept - 1) / P.ept;
+            const uint32_t ubm = Gp.pair ? 2 * SC_BM : SC_BM;  // rows of an emission unit
+            P.erb0 = P.q0 / ubm;
+            P.erbs = (P.q1 + ubm - 1) / ubm - P.erb0;
+            uint32_t longest = P.ept;  // tiles of the longest unit
+            P.eparts = (P.col_tiles + P.ept - 1) / P.ept;
+            if (Gp.jobs.size() == 1 && !P.sym) {
+                const uint64_t tiles = (uint64_t)P.erbs * P.col_tiles;
+                P.ework = (uint32_t)std::min<uint64_t>(Gp.pair ? G / 2 : G, tiles);
+                while ((P.eparts = emission_parts(P)) > 8) --P.ework;
+                longest = (uint32_t)std::min<uint64_t>(P.col_tiles, (tiles + P.ework - 1) / P.ework);
+            }
             const uint32_t per_part = (uint32_t)SC_FULL_LISTS;
-            P.elists = per_part * eparts + (P.sym ? 2u : 0u);
-            const double per_list = (double)P.spec.n / ((double)per_part * eparts);
+            P.elists = per_part * P.eparts + (P.sym ? 2u : 0u);
+            const double per_list = std::min((double)P.spec.n, (double)longest * SC_BN) / per_part;
             const double expect = 1.5 * P.spec.k * (2.0 + std::log(std::fmax(1.0, per_list / P.spec.k)));
             P.cap = std::min<uint32_t>(std::max<uint32_t>(pow2ceil((uint32_t)expect), 128), 4096);
             P.eslot0 = Gp.elists;
@@ -434,11 +459,6 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
             P.cand0 = Gp.cand;
             Gp.cand += P.spec.n * (uint64_t)P.elists * P.cap;
         }
-        // The emission pass takes the 2-SM form (a cluster of two CTAs per
-        // block of 256 rows, each loading half of every column tile) when
-        // every job's K slices fit the resident A block and the autotuner
-        // table prefers it for every job.
-        Gp.pair = !Gp.pair_vetoed && Gp.kpmax / Gp.kslice <= SC_ARES_STAGES;
         // emission units of the group: (job slot | sym, row block (2-SM form:
         // block of 256 rows), first tile, end tile | part); a symmetric unit
         // starts at the tile holding its diagonal block.  One job without symmetric
@@ -446,12 +466,14 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
         const uint32_t ubm = Gp.pair ? 2 * SC_BM : SC_BM;
         for (uint32_t gj = 0; gj < Gp.jobs.size(); ++gj) {
             JobPlan &P = B.jobs[Gp.jobs[gj]];
-            const uint32_t ub0 = P.q0 / ubm, ub1 = (P.q1 + ubm - 1) / ubm;
-            P.erb0 = ub0;
-            P.eparts = (P.col_tiles + P.ept - 1) / P.ept;
-            Gp.neunits = (ub1 - ub0) * P.eparts;
-            if (Gp.jobs.size() == 1 && !P.sym) break;
-            for (uint32_t rb = ub0; rb < ub1; ++rb) {
+            if (P.ework) {
+                // pieces of a worker's range: one per row block that it can touch
+                const uint64_t tiles = (uint64_t)P.erbs * P.col_tiles;
+                const uint64_t range = (tiles + P.ework - 1) / P.ework;
+                Gp.neunits = P.ework * (uint32_t)((range + P.col_tiles - 2) / P.col_tiles + 1);
+                break;
+            }
+            for (uint32_t rb = P.erb0; rb < P.erb0 + P.erbs; ++rb) {
                 const uint32_t first = P.sym ? rb * ubm / SC_BN : 0u;
                 for (uint32_t part = 0, t0 = first; t0 < P.col_tiles; ++part, t0 += P.ept) {
                     const uint32_t t1 = std::min<uint32_t>(P.col_tiles, t0 + P.ept);
@@ -691,8 +713,8 @@ static int bind_batch(hm_batch &B, void *d_ws, size_t bytes, cudaStream_t s) {
         J.elists = P.elists;
         J.sym = P.sym ? 1u : 0u;
         J.erb0 = P.erb0;
-        J.eparts = P.eparts;
-        J.ept = P.ept;
+        J.erbs = P.erbs;
+        J.ework = P.ework;
         J.eslot0 = P.eslot0;
         J.scale = s.metric == HM_METRIC_EUCLIDEAN ? 2.0f : 1.0f;
         J.mu = P.group >= 0 ? at<double>(ws, P.off_mu) : nullptr;

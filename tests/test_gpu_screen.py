@@ -382,3 +382,18 @@ def test_threshold_chunks_of_every_width(seed_div, metric):
             assert_same_bytes(knn.dists, plain.dists, f"{n} {k} dists")
     finally:
         lib.hm_tuning_override(0)
+
+
+@pytest.mark.parametrize("path", ["screen_bf16", "screen_bf16x3"])
+@pytest.mark.parametrize("d", [10, 200])
+def test_emission_ranges_of_one_job(path, d):
+    """Sizes at which a worker's range of tiles is one tile, part of a row block, a whole
+    one and more, and where eight workers share a row block at most, in the 2-SM form
+    (d = 10) and one CTA a unit (d = 200: the split form's rows do not stay resident)."""
+    g = np.random.default_rng(d)
+    for n in (100, 256, 257, 1025, 1100, 2049, 2300, 3400, 4500, 9100):
+        x = g.normal(size=(n, d)).astype(np.float32)
+        plain = hm.exact_knn(x, d, 9, "euclidean", "plain")
+        knn = hm.exact_knn(x, d, 9, "euclidean", path)
+        assert_same_bytes(knn.indices, plain.indices, f"{n} indices")
+        assert_same_bytes(knn.dists, plain.dists, f"{n} dists")
