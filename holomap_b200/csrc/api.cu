@@ -995,6 +995,25 @@ struct Allocs {
     }
 };
 
+int CallMemory::open(size_t bytes) {
+    ThreadCtx *ctx;
+    HM_TRY(thread_ctx(ctx));
+    s = ctx->stream;
+    pooled = bytes <= CALL_POOL_BYTES;
+    void *block = nullptr;
+    HM_CUDA_TRY(pooled ? cudaMallocAsync(&block, bytes, s) : cudaMalloc(&block, bytes));
+    p = static_cast<char *>(block);
+    return HM_OK;
+}
+CallMemory::~CallMemory() {
+    if (!p) return;
+    cudaStreamSynchronize(s);
+    if (pooled)
+        cudaFreeAsync(p, s);
+    else
+        cudaFree(p);
+}
+
 static hm_job one_job(const float *data, uint64_t n, uint32_t d, uint32_t k, int metric, int path,
                       uint32_t *idx, float *dist, float *sigma, float *rho) {
     hm_job j{};

@@ -592,15 +592,17 @@ int hm_fuzzy_graph(const uint32_t *idx, const float *dist, const float *sigma, c
     const size_t o_rho = round_up(o_sig + n * 4, 256), o_rows = round_up(o_rho + n * 4, 256);
     const size_t o_cols = round_up(o_rows + cap * 4, 256), o_vals = round_up(o_cols + cap * 4, 256);
     const size_t o_nnz = round_up(o_vals + cap * 4, 256), o_ws = round_up(o_nnz + 8, 256);
-    char *d = nullptr;
-    HM_CUDA_TRY(cudaMalloc(&d, o_ws + ws));
+    CallMemory mem;
+    HM_TRY(mem.open(o_ws + ws));
+    char *const d = mem.p;
+    const cudaStream_t s = mem.s;
     int rc = HM_OK;
     uint64_t nnz = 0;
     do {
-        cudaError_t err = cudaMemcpy(d + o_idx, idx, e * 4, cudaMemcpyHostToDevice);
-        if (err == cudaSuccess) err = cudaMemcpy(d + o_dist, dist, e * 4, cudaMemcpyHostToDevice);
-        if (err == cudaSuccess) err = cudaMemcpy(d + o_sig, sigma, n * 4, cudaMemcpyHostToDevice);
-        if (err == cudaSuccess) err = cudaMemcpy(d + o_rho, rho, n * 4, cudaMemcpyHostToDevice);
+        cudaError_t err = cudaMemcpyAsync(d + o_idx, idx, e * 4, cudaMemcpyHostToDevice, s);
+        if (err == cudaSuccess) err = cudaMemcpyAsync(d + o_dist, dist, e * 4, cudaMemcpyHostToDevice, s);
+        if (err == cudaSuccess) err = cudaMemcpyAsync(d + o_sig, sigma, n * 4, cudaMemcpyHostToDevice, s);
+        if (err == cudaSuccess) err = cudaMemcpyAsync(d + o_rho, rho, n * 4, cudaMemcpyHostToDevice, s);
         if (err != cudaSuccess) {
             rc = set_error(HM_ERR_CUDA, "copy in: %s", cudaGetErrorString(err));
             break;
@@ -609,17 +611,18 @@ int hm_fuzzy_graph(const uint32_t *idx, const float *dist, const float *sigma, c
                                    reinterpret_cast<float *>(d + o_sig), reinterpret_cast<float *>(d + o_rho), n, k,
                                    reinterpret_cast<uint32_t *>(d + o_rows), reinterpret_cast<uint32_t *>(d + o_cols),
                                    reinterpret_cast<float *>(d + o_vals), reinterpret_cast<uint64_t *>(d + o_nnz),
-                                   d + o_ws, ws, nullptr);
+                                   d + o_ws, ws, s);
         if (rc != HM_OK) break;
-        rc = hm_fuzzy_graph_status(d + o_ws, n, k, nullptr);
+        rc = hm_fuzzy_graph_status(d + o_ws, n, k, s);
         if (rc != HM_OK) break;
-        err = cudaMemcpy(&nnz, d + o_nnz, 8, cudaMemcpyDeviceToHost);
-        if (err == cudaSuccess) err = cudaMemcpy(rows_out, d + o_rows, nnz * 4, cudaMemcpyDeviceToHost);
-        if (err == cudaSuccess) err = cudaMemcpy(cols_out, d + o_cols, nnz * 4, cudaMemcpyDeviceToHost);
-        if (err == cudaSuccess) err = cudaMemcpy(vals_out, d + o_vals, nnz * 4, cudaMemcpyDeviceToHost);
+        err = cudaMemcpyAsync(&nnz, d + o_nnz, 8, cudaMemcpyDeviceToHost, s);
+        if (err == cudaSuccess) err = cudaStreamSynchronize(s);
+        if (err == cudaSuccess) err = cudaMemcpyAsync(rows_out, d + o_rows, nnz * 4, cudaMemcpyDeviceToHost, s);
+        if (err == cudaSuccess) err = cudaMemcpyAsync(cols_out, d + o_cols, nnz * 4, cudaMemcpyDeviceToHost, s);
+        if (err == cudaSuccess) err = cudaMemcpyAsync(vals_out, d + o_vals, nnz * 4, cudaMemcpyDeviceToHost, s);
+        if (err == cudaSuccess) err = cudaStreamSynchronize(s);
         if (err != cudaSuccess) rc = set_error(HM_ERR_CUDA, "copy out: %s", cudaGetErrorString(err));
     } while (false);
-    cudaFree(d);
     *nnz_out = nnz;
     return rc;
 }

@@ -1007,13 +1007,15 @@ int hm_spectral_eigenpairs(const uint32_t *rows, const uint32_t *cols, const flo
     const size_t o_rows = 0, o_cols = round_up(nnz * 4 + 1, 256), o_vals = o_cols + round_up(nnz * 4 + 1, 256);
     const size_t o_ind = o_vals + round_up(nnz * 4 + 1, 256), o_sv = o_ind + round_up((n + 1) * 8, 256);
     const size_t o_deg = o_sv + round_up(nnz * 8 + 1, 256), o_ws = o_deg + round_up(n * 8, 256);
-    char *d = nullptr;
-    HM_CUDA_TRY(cudaMalloc(&d, o_ws + ws));
+    CallMemory mem;
+    HM_TRY(mem.open(o_ws + ws));
+    char *const d = mem.p;
+    const cudaStream_t s = mem.s;
     int rc = HM_OK;
     do {
-        cudaError_t err = cudaMemcpy(d + o_rows, rows, nnz * 4, cudaMemcpyHostToDevice);
-        if (err == cudaSuccess) err = cudaMemcpy(d + o_cols, cols, nnz * 4, cudaMemcpyHostToDevice);
-        if (err == cudaSuccess) err = cudaMemcpy(d + o_vals, vals, nnz * 4, cudaMemcpyHostToDevice);
+        cudaError_t err = cudaMemcpyAsync(d + o_rows, rows, nnz * 4, cudaMemcpyHostToDevice, s);
+        if (err == cudaSuccess) err = cudaMemcpyAsync(d + o_cols, cols, nnz * 4, cudaMemcpyHostToDevice, s);
+        if (err == cudaSuccess) err = cudaMemcpyAsync(d + o_vals, vals, nnz * 4, cudaMemcpyHostToDevice, s);
         if (err != cudaSuccess) {
             rc = set_error(HM_ERR_CUDA, "copy in: %s", cudaGetErrorString(err));
             break;
@@ -1022,12 +1024,11 @@ int hm_spectral_eigenpairs(const uint32_t *rows, const uint32_t *cols, const flo
         auto *sv = reinterpret_cast<double *>(d + o_sv);
         rc = laplacian_launch(reinterpret_cast<uint32_t *>(d + o_rows), reinterpret_cast<uint32_t *>(d + o_cols),
                               reinterpret_cast<float *>(d + o_vals), n, nnz, ind, sv,
-                              reinterpret_cast<double *>(d + o_deg), nullptr);
+                              reinterpret_cast<double *>(d + o_deg), s);
         if (rc != HM_OK) break;
-        rc = hm_eigenpairs_device(ind, reinterpret_cast<uint32_t *>(d + o_cols), sv, n, k, d + o_ws, ws, nullptr,
+        rc = hm_eigenpairs_device(ind, reinterpret_cast<uint32_t *>(d + o_cols), sv, n, k, d + o_ws, ws, s,
                                   values_out, vectors_out, found_out, cycles_out);
     } while (false);
-    cudaFree(d);
     return rc;
 }
 

@@ -261,3 +261,36 @@ def test_wide_columns(oracle, n, k, hubs):
     for j in range(1, hubs + 1):  # a hub's own entry for itself would repeat its first
         idx[n - j, j] = j
     check(oracle, idx.reshape(-1), dist.reshape(-1), f32(np.ones(n)), dist[:, 1].copy(), k)
+
+
+def ring(n, k):
+    idx = ((np.arange(n, dtype=np.int64)[:, None] + np.arange(1, k + 1)) % n).astype(np.uint32)
+    dist = np.tile(np.linspace(0.1, 1.0, k, dtype=np.float32), (n, 1))
+    return idx.reshape(-1), dist.reshape(-1), np.full(n, 0.5, np.float32), np.full(n, 0.1, np.float32)
+
+
+def test_host_calls_from_pooled_and_own_memory():
+    """A call whose device memory is above the pooled size, between calls below it, and
+    calls of several threads at once (each on its own stream): one ring of neighbours
+    at several sizes, whose entries are known from a small one."""
+    from concurrent.futures import ThreadPoolExecutor
+    k = 15
+
+    def run(n):
+        idx, dist, sig, rho = ring(n, k)
+        g = hm.fuzzy_simplicial_set(hm.Knn(k, idx, dist), hm.SmoothKnn(sig, rho))
+        assert g.rows.size == 2 * n * k
+        return g
+
+    small = run(1000)
+    middle = small.vals.reshape(1000, 2 * k)[500]  # columns in order: 15 before, 15 after
+    for n in (260_000, 3000):
+        g = run(n)
+        assert np.array_equal(g.rows, np.repeat(np.arange(n, dtype=np.uint32), 2 * k))
+        v = g.vals.reshape(n, 2 * k)[k:n - k]
+        assert np.array_equal(v, np.broadcast_to(middle, v.shape))
+    with ThreadPoolExecutor(4) as pool:
+        for n, g in zip([2000, 5000, 2000, 9000] * 3, pool.map(run, [2000, 5000, 2000, 9000] * 3)):
+            assert np.array_equal(g.vals.reshape(n, 2 * k)[k:n - k], np.broadcast_to(middle, (n - 2 * k, 2 * k)))
+            pairs = hm.smallest_eigenpairs(g, 2)
+            assert abs(float(pairs.values[0])) < 1e-9
