@@ -173,12 +173,31 @@ static int group_of_path(int path) {
     }
 }
 
+// Bytes of the split lists of an exact-path job cut c ways (whole column tiles).
+static size_t split_lists_bytes(const hm_job &s, uint64_t c) {
+    const uint64_t tiles = (s.n + PL_BN - 1) / PL_BN, per = (tiles + c - 1) / c, splits = (tiles + per - 1) / per;
+    return splits > 1 ? align256((size_t)splits * s.n * s.k * sizeof(uint64_t)) : 0;
+}
+static size_t plain_copy_bytes(const hm_job &s) {
+    return align256((round_up(s.n, 128) + 128) * round_up(s.d, 16) * sizeof(double));
+}
+// Scratch of an exact-path job for its split lists: the size of a binary64 copy of
+// the points and of the lists of a cut into eight items per SM.  What fits the
+// static scratch, or an arena, is a contract with the caller, so the room stays
+// what it was when the path still held such a copy.
+static size_t plain_room_bytes(const hm_job &s, uint64_t groups) {
+    const uint64_t tiles = (s.n + PL_BN - 1) / PL_BN;
+    const uint64_t c = std::min<uint64_t>(std::min<uint64_t>(std::max<uint64_t>((1184 + groups - 1) / groups, 1), 32), tiles);
+    return plain_copy_bytes(s) + split_lists_bytes(s, c);
+}
+
 // Column splits of one exact-path job: the waves of resident CTAs times a split's
 // instructions per warp (8 rows: the tiles' arithmetic and the filling of the
 // rows' lists, k (1 + ln(columns / k)) keys in merges of 32), least over the
 // splits.  More splits even out the last wave, fewer fill fewer lists: 12,007 x 64
 // manhattan, k = 15 (376 row groups, 444 CTAs resident) 1,565 us with the 7 it
 // chooses, 1,602 with 4; 1,000 points take one per 128-column tile.
+// (Lists take the room of a problem's scratch and no more: plain_room_bytes.)
 static uint32_t plain_splits(const JobPlan &P, uint64_t groups, uint32_t sms) {
     const hm_job &s = P.spec;
     const uint32_t tiles = (uint32_t)((s.n + PL_BN - 1) / PL_BN);
@@ -190,8 +209,9 @@ static uint32_t plain_splits(const JobPlan &P, uint64_t groups, uint32_t sms) {
     uint32_t splits = 1;
     for (uint32_t c = 1; c <= std::min<uint32_t>(32, tiles); ++c) {
         const double per = std::ceil((double)tiles / c), cols = per * PL_BN;
-        const double fill = 8 * merge * (1 + s.k / 32.0 * (1 + std::log(std::max(1.0, cols / s.k))));
-        const double cost = std::ceil(groups * (double)c / resident) * (per * tile + fill) + 40.0 * c;
+        const double lists = 8 * merge * (1 + s.k / 32.0 * (1 + std::log(std::max(1.0, cols / s.k))));
+        if (split_lists_bytes(s, c) > plain_room_bytes(s, groups)) continue;
+        const double cost = std::ceil(groups * (double)c / resident) * (per * tile + lists) + 40.0 * c;
         if (cost < best * 0.999) {
             best = cost;
             splits = c;
@@ -390,7 +410,10 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
             // 128, 256 or 512 minima a row (by k: the k smallest values of a row
             // then rarely share a chunk, which loosens the bound); chunks of
             // more than 64 columns take several tiles of a part
-            const uint32_t limit = P.spec.k <= 20 ? 128 : P.spec.k <= 40 ? 256 : TH_MAX_MINIMA;
+            // (and no more scratch than sorted lists of each part's two halves and a
+            // row's binary64 copy took)
+            const uint32_t limit = std::min<uint32_t>(P.spec.k <= 20 ? 128 : P.spec.k <= 40 ? 256 : TH_MAX_MINIMA,
+                                                      2 * P.parts * P.spec.k + 2 * (uint32_t)round_up(P.spec.d, 16));
             const uint32_t last = std::min(P.seed_tiles, P.col_tiles - (P.parts - 1) * P.part_tiles);
             for (P.min_shift = 0;; ++P.min_shift) {
                 const uint32_t ti = P.min_shift > 4 ? P.min_shift - 4 : 0, per = P.min_shift > 4 ? 4 : 64u >> P.min_shift;
@@ -430,19 +453,39 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
             const uint32_t ubm = Gp.pair ? 2 * SC_BM : SC_BM;  // rows of an emission unit
             P.erb0 = P.q0 / ubm;
             P.erbs = (P.q1 + ubm - 1) / ubm - P.erb0;
-            uint32_t longest = P.ept;  // tiles of the longest unit
-            P.eparts = (P.col_tiles + P.ept - 1) / P.ept;
-            if (Gp.jobs.size() == 1 && !P.sym) {
-                const uint64_t tiles = (uint64_t)P.erbs * P.col_tiles;
-                P.ework = (uint32_t)std::min<uint64_t>(Gp.pair ? G / 2 : G, tiles);
-                while ((P.eparts = emission_parts(P)) > 8) --P.ework;
-                longest = (uint32_t)std::min<uint64_t>(P.col_tiles, (tiles + P.ework - 1) / P.ework);
-            }
             const uint32_t per_part = (uint32_t)SC_FULL_LISTS;
+            auto expect = [&](double per_list) {  // candidates of a row in one list
+                return (uint32_t)(1.5 * P.spec.k * (2.0 + std::log(std::fmax(1.0, per_list / P.spec.k))));
+            };
+            auto cap_for = [&](uint32_t e) { return std::min<uint32_t>(std::max<uint32_t>(pow2ceil(e), 128), 4096); };
+            P.eparts = (P.col_tiles + P.ept - 1) / P.ept;
+            P.cap = cap_for(expect((double)P.spec.n / ((double)per_part * P.eparts)));
+            if (Gp.jobs.size() == 1 && !P.sym) {
+                // one job: its tiles dealt out evenly, by as many workers as leave
+                // its rows' lists within the slots of whole column parts (a caller's
+                // arena may be sized to them; a row's copy in binary64 is no longer
+                // kept), which a few idle workers may buy; else those parts
+                const uint64_t tiles = (uint64_t)P.erbs * P.col_tiles;
+                const uint32_t most = (uint32_t)std::min<uint64_t>(Gp.pair ? G / 2 : G, tiles);
+                const uint32_t more = 2 * P.parts * P.spec.k;  // minima per row of the parts' sorted lists
+                const uint32_t slots = P.clone_of >= 0
+                                           ? B.jobs[P.clone_of].elists * B.jobs[P.clone_of].cap
+                                           : per_part * P.eparts * P.cap + (uint32_t)round_up(P.spec.d, 16) -
+                                                 (P.mins > more ? (P.mins - more + 1) / 2 : 0);
+                for (P.ework = most; P.ework > 0; --P.ework) {
+                    const uint32_t parts = emission_parts(P);
+                    const uint64_t longest = std::min<uint64_t>(P.col_tiles, (tiles + P.ework - 1) / P.ework);
+                    const uint32_t e = expect(std::min((double)P.spec.n, (double)longest * SC_BN) / per_part);
+                    const uint32_t need = std::min<uint32_t>(std::max<uint32_t>((uint32_t)round_up(e, 32), 128), 4096);
+                    if (parts <= 8 && per_part * parts * need <= slots) {
+                        P.eparts = parts;
+                        P.cap = std::min(cap_for(e), slots / (per_part * parts) / 32 * 32);
+                        break;
+                    }
+                    if (10ull * P.ework < 9ull * most) P.ework = 1;  // (no such number: the table's parts)
+                }
+            }
             P.elists = per_part * P.eparts + (P.sym ? 2u : 0u);
-            const double per_list = std::min((double)P.spec.n, (double)longest * SC_BN) / per_part;
-            const double expect = 1.5 * P.spec.k * (2.0 + std::log(std::fmax(1.0, per_list / P.spec.k)));
-            P.cap = std::min<uint32_t>(std::max<uint32_t>(pow2ceil((uint32_t)expect), 128), 4096);
             P.eslot0 = Gp.elists;
             Gp.elists += P.spec.n * (uint64_t)P.elists;
             if (P.clone_of >= 0) {
@@ -578,14 +621,12 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
             P.off_csum = take((size_t)64 * P.spec.d * sizeof(double));
             continue;
         }
-        // The plain path's scratch keeps the room of the binary64 copy it once held
-        // (rows padded to 128 and one block more, dimensions to 16): which problems
-        // fit a caller's fixed scratch, the allocation-free entry point's above all,
-        // is part of its contract.
-        if (P.path == HM_PATH_PLAIN) take((round_up(n, 128) + 128) * round_up(P.spec.d, 16) * sizeof(double));
+        // (a batch's splits are eight items per SM, so its jobs' room is the same)
+        if (P.path == HM_PATH_PLAIN)
+            P.off_partial = take(njobs == 1 ? plain_room_bytes(P.spec, (P.q1 + PL_BM - 1) / PL_BM - P.q0 / PL_BM)
+                                            : plain_copy_bytes(P.spec) + split_lists_bytes(P.spec, P.splits));
         P.off_rnorm = take(n * sizeof(double));
         P.off_zero_rows = take(n * sizeof(uint32_t));
-        if (P.splits > 1) P.off_partial = take((size_t)P.splits * n * P.spec.k * sizeof(uint64_t));
         if (P.group >= 0) {
             P.off_ovf = take(n * sizeof(uint32_t));
             P.off_mu = take((size_t)P.spec.d * sizeof(double));
@@ -786,6 +827,7 @@ static int bind_batch(hm_batch &B, void *d_ws, size_t bytes, cudaStream_t s) {
         D.job_of = Gp.jobs.size() > 1 ? at<uint32_t>(ws, Gp.off_job_of) : nullptr;
         D.eunits = Gp.eunits.empty() ? nullptr : at<uint4>(ws, Gp.off_eunits);
         D.neunits = Gp.neunits;
+        D.eworkers = Gp.jobs.size() == 1 && B.jobs[Gp.jobs[0]].ework ? B.jobs[Gp.jobs[0]].ework : Gp.neunits;
         D.any_euclidean = (Gp.metric_mask >> HM_METRIC_EUCLIDEAN) & 1;
         D.pair = Gp.pair ? 1u : 0u;
         for (uint32_t j : Gp.jobs) {

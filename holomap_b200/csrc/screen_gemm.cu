@@ -935,7 +935,7 @@ static int launch_pair(const JobDev *jobs, const GroupDev &G, const CUtensorMap 
     HM_TRY(ensure_dynamic_smem(func, (int)SC_SMEM_BYTES));
     const uint32_t slots = pair_slots(func, (uint32_t)SC_THREADS);
     if (slots == 0) return set_error(HM_ERR_CUDA, "no room for a cluster of two screen CTAs");
-    const uint32_t clusters = G.neunits < slots ? G.neunits : slots;
+    const uint32_t clusters = G.eworkers < slots ? G.eworkers : slots;
     if (clusters == 0) return HM_OK;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * clusters, 1, 1);
@@ -978,7 +978,7 @@ static int launch_kind(const JobDev *jobs, const GroupDev &G, const CUtensorMap 
 
 uint32_t emission_grid(const GroupDev &G) {
     const uint32_t sms = (uint32_t)device_sm_count();
-    return G.neunits < sms ? G.neunits : sms;
+    return G.eworkers < sms ? G.eworkers : sms;
 }
 
 static uint32_t make_idesc(int kind) {

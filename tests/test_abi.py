@@ -247,3 +247,15 @@ def test_tridiagonal_eigensolver(m, seed):
     assert np.abs(t @ z - z * vals).max() < 1e-13
     assert np.abs(z.T @ z - np.eye(m)).max() < 1e-13
     assert np.abs(np.sort(vals) - np.linalg.eigvalsh(t)).max() < 1e-13
+
+
+@pytest.mark.parametrize("n,d,k,metric,path,most", [
+    (217868, 5, 15, 1, 1, 30_590_208), (117698, 53, 100, 0, 1, 61_803_008), (12007, 64, 15, 2, 1, 12_147_712),
+    (1000, 50, 15, 0, 1, 1_565_952), (20000, 128, 15, 0, 0, 886_008_064), (5003, 300, 15, 1, 0, 332_789_248),
+    (50000, 384, 30, 1, 0, 3_579_964_416), (2402, 1, 64, 0, 2, 105_578_240), (127828, 6, 1, 1, 2, 570_281_728)])
+def test_workspace_stays_within_what_callers_sized_for(n, d, k, metric, path, most):
+    """A problem that fits a fixed scratch or an arena has to go on fitting: split lists
+    take the room of the plain path's scratch and no more, the emission pass's lists
+    the slots of whole column parts."""
+    got = hm.lib().hm_workspace_bytes(n, d, k, metric, path)
+    assert 0 < got <= most
