@@ -100,7 +100,7 @@ struct JobPlan {
     // emission pass: symmetric (tiles on and above the diagonal), its column
     // parts per row block of ept tiles, candidate lists per row
     bool sym = false;
-    uint32_t ept = 0, elists = 0, erb0 = 0, erbs = 0, eparts = 1, ework = 0;
+    uint32_t ept = 0, elists = 0, erb0 = 0, erbs = 0, eparts = 1;
     uint64_t eslot0 = 0;
     // escalation: the job's split-BF16 copy (clone), or the job a copy is of
     int clone = -1, clone_of = -1;
@@ -218,16 +218,6 @@ static uint32_t plain_splits(const JobPlan &P, uint64_t groups, uint32_t sms) {
         }
     }
     return splits;
-}
-
-// Most workers that share a row block of a job's emission pass (their parts of its
-// columns), its tiles cut into ework equal ranges.
-static uint32_t emission_parts(const JobPlan &P) {
-    const uint64_t ct = P.col_tiles, tiles = P.erbs * ct, w = P.ework;
-    uint64_t parts = 1;
-    for (uint64_t s = 0; s < tiles; s += ct)
-        parts = std::max(parts, ((s + ct) * w - 1) / tiles - ((s + 1) * w - 1) / tiles + 1);
-    return (uint32_t)parts;
 }
 
 // `ranges` (optional): 2 per job, the job's query rows [begin, end); every
@@ -454,37 +444,10 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
             P.erb0 = P.q0 / ubm;
             P.erbs = (P.q1 + ubm - 1) / ubm - P.erb0;
             const uint32_t per_part = (uint32_t)SC_FULL_LISTS;
-            auto expect = [&](double per_list) {  // candidates of a row in one list
-                return (uint32_t)(1.5 * P.spec.k * (2.0 + std::log(std::fmax(1.0, per_list / P.spec.k))));
-            };
-            auto cap_for = [&](uint32_t e) { return std::min<uint32_t>(std::max<uint32_t>(pow2ceil(e), 128), 4096); };
             P.eparts = (P.col_tiles + P.ept - 1) / P.ept;
-            P.cap = cap_for(expect((double)P.spec.n / ((double)per_part * P.eparts)));
-            if (Gp.jobs.size() == 1 && !P.sym) {
-                // one job: its tiles dealt out evenly, by as many workers as leave
-                // its rows' lists within the slots of whole column parts (a caller's
-                // arena may be sized to them; a row's copy in binary64 is no longer
-                // kept), which a few idle workers may buy; else those parts
-                const uint64_t tiles = (uint64_t)P.erbs * P.col_tiles;
-                const uint32_t most = (uint32_t)std::min<uint64_t>(Gp.pair ? G / 2 : G, tiles);
-                const uint32_t more = 2 * P.parts * P.spec.k;  // minima per row of the parts' sorted lists
-                const uint32_t slots = P.clone_of >= 0
-                                           ? B.jobs[P.clone_of].elists * B.jobs[P.clone_of].cap
-                                           : per_part * P.eparts * P.cap + (uint32_t)round_up(P.spec.d, 16) -
-                                                 (P.mins > more ? (P.mins - more + 1) / 2 : 0);
-                for (P.ework = most; P.ework > 0; --P.ework) {
-                    const uint32_t parts = emission_parts(P);
-                    const uint64_t longest = std::min<uint64_t>(P.col_tiles, (tiles + P.ework - 1) / P.ework);
-                    const uint32_t e = expect(std::min((double)P.spec.n, (double)longest * SC_BN) / per_part);
-                    const uint32_t need = std::min<uint32_t>(std::max<uint32_t>((uint32_t)round_up(e, 32), 128), 4096);
-                    if (parts <= 8 && per_part * parts * need <= slots) {
-                        P.eparts = parts;
-                        P.cap = std::min(cap_for(e), slots / (per_part * parts) / 32 * 32);
-                        break;
-                    }
-                    if (10ull * P.ework < 9ull * most) P.ework = 1;  // (no such number: the table's parts)
-                }
-            }
+            const double per_list = (double)P.spec.n / ((double)per_part * P.eparts);
+            const double expect = 1.5 * P.spec.k * (2.0 + std::log(std::fmax(1.0, per_list / P.spec.k)));
+            P.cap = std::min<uint32_t>(std::max<uint32_t>(pow2ceil((uint32_t)expect), 128), 4096);
             P.elists = per_part * P.eparts + (P.sym ? 2u : 0u);
             P.eslot0 = Gp.elists;
             Gp.elists += P.spec.n * (uint64_t)P.elists;
@@ -509,13 +472,8 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
         const uint32_t ubm = Gp.pair ? 2 * SC_BM : SC_BM;
         for (uint32_t gj = 0; gj < Gp.jobs.size(); ++gj) {
             JobPlan &P = B.jobs[Gp.jobs[gj]];
-            if (P.ework) {
-                // pieces of a worker's range: one per row block that it can touch
-                const uint64_t tiles = (uint64_t)P.erbs * P.col_tiles;
-                const uint64_t range = (tiles + P.ework - 1) / P.ework;
-                Gp.neunits = P.ework * (uint32_t)((range + P.col_tiles - 2) / P.col_tiles + 1);
-                break;
-            }
+            Gp.neunits = P.erbs * P.eparts;
+            if (Gp.jobs.size() == 1 && !P.sym) break;
             for (uint32_t rb = P.erb0; rb < P.erb0 + P.erbs; ++rb) {
                 const uint32_t first = P.sym ? rb * ubm / SC_BN : 0u;
                 for (uint32_t part = 0, t0 = first; t0 < P.col_tiles; ++part, t0 += P.ept) {
@@ -754,8 +712,8 @@ static int bind_batch(hm_batch &B, void *d_ws, size_t bytes, cudaStream_t s) {
         J.elists = P.elists;
         J.sym = P.sym ? 1u : 0u;
         J.erb0 = P.erb0;
-        J.erbs = P.erbs;
-        J.ework = P.ework;
+        J.eparts = P.eparts;
+        J.ept = P.ept;
         J.eslot0 = P.eslot0;
         J.scale = s.metric == HM_METRIC_EUCLIDEAN ? 2.0f : 1.0f;
         J.mu = P.group >= 0 ? at<double>(ws, P.off_mu) : nullptr;
@@ -827,7 +785,6 @@ static int bind_batch(hm_batch &B, void *d_ws, size_t bytes, cudaStream_t s) {
         D.job_of = Gp.jobs.size() > 1 ? at<uint32_t>(ws, Gp.off_job_of) : nullptr;
         D.eunits = Gp.eunits.empty() ? nullptr : at<uint4>(ws, Gp.off_eunits);
         D.neunits = Gp.neunits;
-        D.eworkers = Gp.jobs.size() == 1 && B.jobs[Gp.jobs[0]].ework ? B.jobs[Gp.jobs[0]].ework : Gp.neunits;
         D.any_euclidean = (Gp.metric_mask >> HM_METRIC_EUCLIDEAN) & 1;
         D.pair = Gp.pair ? 1u : 0u;
         for (uint32_t j : Gp.jobs) {

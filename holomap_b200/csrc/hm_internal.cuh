@@ -303,7 +303,7 @@ struct JobDev {
     // candidate lists of the emission pass: elists per row (two per column
     // part; with the symmetric emission one more, the row's column list, last)
     uint32_t elists, sym;        // sym: the emission pass covers the tiles on and above the diagonal
-    uint32_t erb0, erbs, ework;  // emission units: first row block, row blocks, workers that share them
+    uint32_t erb0, eparts, ept;  // emission units: first row block, column parts per row block, tiles per part
     unsigned long long eslot0;   // first candidate list of the job
     unsigned long long cand0;    // first candidate slot: list l holds [cand0 + (l - eslot0) * cap, +cap)
     float scale;                 // 1 (cosine) or 2 (euclidean)

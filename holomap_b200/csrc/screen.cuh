@@ -96,7 +96,6 @@ struct GroupDev {
     // search for a unit's job costs more, 6.8 ms against 6.4 for 256 datasets)
     const uint4 *eunits;
     uint32_t neunits;
-    uint32_t eworkers;  // CTAs or clusters the units are laid out for (at most one per unit)
     // emission pass in the 2-SM form (a cluster of two CTAs per unit, one
     // MMA of 256 rows; eunits' y is then a block of 256 rows)
     uint32_t pair;

@@ -221,28 +221,20 @@ struct UnitTiles {
 // Pass 0 (the threshold pass) walks only the first seed_tiles tiles of each
 // part: a sample of the row's columns whose k-th smallest screened value
 // already bounds the row's k-th from above.  The emission passes take their units
-// from the group's table; one job without symmetric units needs none: its row blocks'
-// tiles are dealt out evenly, so that the workers finish together (whole column
-// parts of row blocks left 15% of them idle at 20,000 x 128: 326 us, now 301).
+// from the group's table; a group of one job without symmetric units needs none.
+// (Its tiles cut into equal ranges, one per worker, take 20,000 x 128 from 326 to 301
+// us, but a row's columns then lie mostly in one worker's four lists: of 45,000 x 300
+// clustered points 1,551 rows overflowed them, 4.7 ms against 42.)
 __device__ __forceinline__ UnitTiles unit_tiles(const JobDev *jobs, const GroupDev &G, uint32_t u, int pass) {
     UnitTiles t;
     if (pass == 1 && !G.eunits) {
         t.sym = 0;
         t.job = G.job_ids[0];
         const JobDev &J = jobs[t.job];
-        // worker w's range of the row blocks' tiles, laid end to end; piece i of it
-        // is what lies in the range's i-th row block (none: an empty unit), and
-        // the workers of a row block number its column parts
-        const uint64_t W = J.ework, w = u % J.ework, ct = J.col_tiles, tiles = J.erbs * ct;
-        const uint64_t lo = w * tiles / W, hi = (w + 1) * tiles / W, rb = lo / ct + u / J.ework;
-        const uint64_t b = max(lo, rb * ct), e = min(hi, (rb + 1) * ct);
-        t.rb = J.erb0 + (uint32_t)rb;
-        t.part = t.ct_begin = t.ct_end = 0;
-        if (b < e) {
-            t.part = (uint32_t)(w - ((rb * ct + 1) * W - 1) / tiles);
-            t.ct_begin = (uint32_t)(b - rb * ct);
-            t.ct_end = (uint32_t)(e - rb * ct);
-        }
+        t.rb = J.erb0 + u / J.eparts;
+        t.part = u % J.eparts;
+        t.ct_begin = t.part * J.ept;
+        t.ct_end = min(J.col_tiles, t.ct_begin + J.ept);
         return t;
     }
     if (pass >= 1) {
@@ -354,7 +346,7 @@ __global__ void __launch_bounds__(SC_THREADS, 1)
             for (uint32_t u = wid; ok && u < nunits; u += nworkers) {
                 const UnitTiles ut = unit_tiles(jobs, G, u, PASS);
                 const JobDev &J = jobs[ut.job];
-                if (!job_active(J) || ut.ct_begin >= ut.ct_end) continue;  // every role skips the same units
+                if (!job_active(J)) continue;  // every role skips the same units
                 const uint32_t myrb = PAIR ? 2 * ut.rb + rank : ut.rb;  // this CTA's 128-row block
                 if (PAIR || a_res) {
                     // the previous unit's MMAs must be done with the A block
@@ -440,7 +432,7 @@ __global__ void __launch_bounds__(SC_THREADS, 1)
             for (uint32_t u = wid; ok && u < nunits; u += nworkers) {
                 const UnitTiles ut = unit_tiles(jobs, G, u, PASS);
                 const JobDev &J = jobs[ut.job];
-                if (!job_active(J) || ut.ct_begin >= ut.ct_end) continue;
+                if (!job_active(J)) continue;
                 if (PAIR || a_res) {
                     if (!mbar_wait(smem_u32(afull), un & 1, abort_flag)) {
                         raise_error(abort_flag, &J.out->error_code, SC_ERR_MMA_FULL, peer_abort);
@@ -518,7 +510,7 @@ __global__ void __launch_bounds__(SC_THREADS, 1)
         for (uint32_t u = wid; ok && u < nunits; u += nworkers) {
             const UnitTiles ut = unit_tiles(jobs, G, u, PASS);
             const JobDev &J = jobs[ut.job];
-            if (!job_active(J) || ut.ct_begin >= ut.ct_end) continue;
+            if (!job_active(J)) continue;
             const uint32_t n = J.n;
             const uint32_t myrb = PAIR ? 2 * ut.rb + rank : ut.rb;  // this CTA's 128-row block
             const uint32_t row = myrb * SC_BM + row_in_tile;  // job-local
@@ -935,7 +927,7 @@ static int launch_pair(const JobDev *jobs, const GroupDev &G, const CUtensorMap 
     HM_TRY(ensure_dynamic_smem(func, (int)SC_SMEM_BYTES));
     const uint32_t slots = pair_slots(func, (uint32_t)SC_THREADS);
     if (slots == 0) return set_error(HM_ERR_CUDA, "no room for a cluster of two screen CTAs");
-    const uint32_t clusters = G.eworkers < slots ? G.eworkers : slots;
+    const uint32_t clusters = G.neunits < slots ? G.neunits : slots;
     if (clusters == 0) return HM_OK;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * clusters, 1, 1);
@@ -978,7 +970,7 @@ static int launch_kind(const JobDev *jobs, const GroupDev &G, const CUtensorMap 
 
 uint32_t emission_grid(const GroupDev &G) {
     const uint32_t sms = (uint32_t)device_sm_count();
-    return G.eworkers < sms ? G.eworkers : sms;
+    return G.neunits < sms ? G.neunits : sms;
 }
 
 static uint32_t make_idesc(int kind) {

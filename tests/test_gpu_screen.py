@@ -387,9 +387,9 @@ def test_threshold_chunks_of_every_width(seed_div, metric):
 @pytest.mark.parametrize("path", ["screen_bf16", "screen_bf16x3"])
 @pytest.mark.parametrize("d", [10, 200])
 def test_emission_ranges_of_one_job(path, d):
-    """Sizes at which a worker's range of tiles is one tile, part of a row block, a whole
-    one and more, and where eight workers share a row block at most, in the 2-SM form
-    (d = 10) and one CTA a unit (d = 200: the split form's rows do not stay resident)."""
+    """One job's emission units from one tile to several row blocks with a part each, in
+    the 2-SM form (d = 10) and one CTA a unit (d = 200: the split form's rows do not
+    stay resident)."""
     g = np.random.default_rng(d)
     for n in (100, 256, 257, 1025, 1100, 2049, 2300, 3400, 4500, 9100):
         x = g.normal(size=(n, d)).astype(np.float32)
@@ -397,3 +397,18 @@ def test_emission_ranges_of_one_job(path, d):
         knn = hm.exact_knn(x, d, 9, "euclidean", path)
         assert_same_bytes(knn.indices, plain.indices, f"{n} indices")
         assert_same_bytes(knn.dists, plain.dists, f"{n} dists")
+
+
+@pytest.mark.parametrize("d,n,k,metric", [(64, 20000, 15, "cosine"), (300, 45000, 15, "euclidean")])
+def test_clustered_rows_do_not_overflow_their_lists(d, n, k, metric):
+    """Gaussian clusters whose rows have several hundred candidates, few of them far
+    apart: the candidate lists of a single job hold them (a row that overflows costs an
+    exact search of all of the points)."""
+    import torch
+    from holomap_b200.device import DeviceKnnProblem
+    from holomap_b200.synth import serve_pool
+    x = torch.from_numpy(np.ascontiguousarray(serve_pool(d, 0)[:n])).cuda()
+    p = DeviceKnnProblem(n, d, k, metric, "auto")
+    p.run(x)
+    torch.cuda.synchronize()
+    assert p.stats().overflow_rows == 0
