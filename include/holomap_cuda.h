@@ -168,10 +168,11 @@ HM_API int hm_smooth_knn_rows_device(const float *d_dists, uint64_t n, uint32_t 
  * bound).  Capacity of rows / cols / vals: 2 n k entries; *nnz receives the
  * count.  n k must stay below 2^31.
  *
- * hm_fuzzy_graph: host buffers in and out (one allocation, synchronous).
+ * hm_fuzzy_graph: host buffers in and out (device memory from the stream-ordered
+ * pool, the calling thread's own stream, synchronous).
  * hm_fuzzy_graph_device: device pointers; d_nnz is a device uint64; the
- * workspace (hm_fuzzy_workspace_bytes, 256-byte aligned) holds the sort's
- * buffers; ordered on `stream`, nothing synchronised. */
+ * workspace (hm_fuzzy_workspace_bytes, 256-byte aligned) holds the rows'
+ * segments; ordered on `stream`, nothing synchronised. */
 HM_API size_t hm_fuzzy_workspace_bytes(uint64_t n, uint32_t k);
 HM_API int hm_fuzzy_graph_device(const uint32_t *d_idx, const float *d_dist, const float *d_sigma,
                                  const float *d_rho, uint64_t n, uint32_t k, uint32_t *d_rows,
@@ -415,7 +416,8 @@ HM_API int hm_tuning_pair(int mode);
  * after the threshold pass the device compares each row's keep band with its
  * threshold, and when the coarse screen would keep a large share of the
  * dataset for more than a tenth of the rows (points in clusters far tighter
- * than its rounding), the copy screens the job instead.  Same results either
+ * than its rounding), or the band spans half of a row's nearest sampled values
+ * for more than half of the rows, the copy screens the job instead.  Same results either
  * way; hm_stats.path_used then reports HM_PATH_SCREEN_BF16X3. */
 HM_API int hm_tuning_escalation(int on);
 
@@ -427,7 +429,7 @@ HM_API int hm_tuning_escalation(int on);
 #define HM_KCLASS_BULK 0   /* tensor-core screen (the screened paths' N x N bulk) */
 #define HM_KCLASS_SELECT 1 /* split merge / exact rerank + select */
 #define HM_KCLASS_SMOOTH 2 /* smooth-kNN calibration */
-#define HM_KCLASS_PREP 3   /* input checks, binary64 copy, operand prep */
+#define HM_KCLASS_PREP 3   /* input checks, norms, operand prep */
 #define HM_KCLASS_EXACT 4  /* exact binary64 kernel (plain path and fallback rows) */
 #define HM_KCLASS_COUNT 5
 
