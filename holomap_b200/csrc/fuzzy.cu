@@ -246,7 +246,12 @@ __global__ void __launch_bounds__(FZ_WARPS * 32, sizeof(K) == 4 ? 16 : 8) fuzzy_
     else if (slots <= FZ_SHORT_SLOTS) count = union_row<K, 4>(D, r, slots, w_all[warp], lane);
     else {
         if (lane == 0) {
-            if (slots <= FZ_WARP_SLOTS) D.mids[atomicAdd(&D.words[FZ_MIDS], 1u)] = r;
+            if (D.n + D.k <= FZ_SHORT_SLOTS) {
+                // (no long-row kernel follows: distinct indices give a row k slots and
+                // at most n - 1 arrivals, so an index is repeated)
+                atomicOr(&D.words[FZ_BAD], FZ_BAD_DUPLICATE);
+                D.count[r] = 0;
+            } else if (slots <= FZ_WARP_SLOTS) D.mids[atomicAdd(&D.words[FZ_MIDS], 1u)] = r;
             else D.hubs[atomicAdd(&D.words[FZ_HUBS], 1u)] = r;
         }
         return;
@@ -539,7 +544,9 @@ int hm_fuzzy_graph_device(const uint32_t *d_idx, const float *d_dist, const floa
     const unsigned union_blocks = (D.n + FZ_WARPS - 1) / FZ_WARPS;
     HM_CUDA_TRY(launch(true, narrow ? fuzzy_union_kernel<uint32_t> : fuzzy_union_kernel<unsigned long long>, union_blocks,
                        FZ_WARPS * 32, 0, s, D));
-    if (n + k > FZ_SHORT_SLOTS) {  // a row's slots: k and at most n - 1 sources
+    // a row's slots: k and, indices not repeating, at most n - 1 sources (the union
+    // kernel refuses a longer row where this one does not run)
+    if (n + k > FZ_SHORT_SLOTS) {
         auto *kernel = narrow ? fuzzy_long_kernel<uint32_t> : fuzzy_long_kernel<unsigned long long>;
         const size_t bitmaps = (size_t)3 * ((std::min(D.n, FZ_WINDOW) + 31) / 32) * 4, rows_w = 32 * FZ_WARP_SLOTS * 4;
         HM_TRY(ensure_dynamic_smem((const void *)kernel, (int)(3 * FZ_WINDOW / 8)));
@@ -550,7 +557,7 @@ int hm_fuzzy_graph_device(const uint32_t *d_idx, const float *d_dist, const floa
     HM_CUDA_TRY(launch(true, fuzzy_write_kernel, L.tiles, 256, 0, s, D, L.tiles, d_rows, d_cols, d_vals,
                        reinterpret_cast<unsigned long long *>(d_nnz)));
     count_launch(5);
-    if (n + k > FZ_WARP_SLOTS) {
+    if (n + k > FZ_WARP_SLOTS) {  // (a row's entries are distinct columns, repeated indices or not)
         HM_CUDA_TRY(launch(true, fuzzy_hub_write_kernel, 4 * device_sm_count(), 256, 0, s, D, d_rows, d_cols, d_vals));
         count_launch();
     }

@@ -1,6 +1,7 @@
 """GPU parity of the fuzzy simplicial set (src/fuzzy.rs:25-91) against the
 oracle's restatement, entry for entry and bit for bit, and against the
 reference's own unit cases and golden fixtures."""
+import ctypes
 import json
 from pathlib import Path
 
@@ -294,3 +295,59 @@ def test_host_calls_from_pooled_and_own_memory():
             assert np.array_equal(g.vals.reshape(n, 2 * k)[k:n - k], np.broadcast_to(middle, (n - 2 * k, 2 * k)))
             pairs = hm.smallest_eigenpairs(g, 2)
             assert abs(float(pairs.values[0])) < 1e-9
+
+
+class DeviceGraph:
+    """hm_fuzzy_graph_device on torch memory: outputs with guard words behind
+    them and a workspace full of ones (what an earlier call may have left)."""
+    GUARD = 4096
+
+    def __init__(self, n, k):
+        import torch
+        self.n, self.k, self.cap = n, k, 2 * n * k
+        self.out = [torch.full((self.cap + self.GUARD,), -7, dtype=torch.int32, device="cuda") for _ in range(3)]
+        self.nnz = torch.full((1,), -1, dtype=torch.int64, device="cuda")
+        self.ws_bytes = hm.lib().hm_fuzzy_workspace_bytes(n, k)
+        self.ws = torch.full((self.ws_bytes + self.GUARD,), 255, dtype=torch.uint8, device="cuda")
+
+    def run(self, idx, dist, sig, rho):
+        """Status of the graph; (nnz, rows, cols, vals) of the device arrays."""
+        import torch
+        dev = lambda a: torch.from_numpy(np.ascontiguousarray(a).view(np.int32)).cuda()
+        keep = [dev(a) for a in (idx, dist, sig, rho)]
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        check_rc(hm.lib().hm_fuzzy_graph_device(*[t.data_ptr() for t in keep], self.n, self.k,
+                                                *[t.data_ptr() for t in self.out], self.nnz.data_ptr(),
+                                                self.ws.data_ptr(), self.ws_bytes, stream))
+        rc = hm.lib().hm_fuzzy_graph_status(self.ws.data_ptr(), self.n, self.k, stream)
+        nnz = int(self.nnz.item())
+        assert 0 <= nnz <= self.cap
+        for t in self.out:
+            assert bool((t[self.cap:] == -7).all()), "written past the outputs"
+        assert bool((self.ws[self.ws_bytes:] == 255).all()), "written past the workspace"
+        return rc, [nnz] + [t[:nnz].cpu().numpy() for t in self.out]
+
+
+@pytest.mark.parametrize("n", [100, 113, 114, 1000])  # n + k up to 128: no row of a valid graph is long
+@pytest.mark.parametrize("repeaters", [3, 20, 99])     # slots of the repeated column: k + 15 each
+def test_repeated_indices_are_refused_in_bounds(oracle, n, repeaters):
+    """Rows that list one column k times over: its k + in-degree reaches the
+    widths of all three row kernels (75, 315 and 1,500 slots), also where n + k
+    would rule long rows out.  Both entry points answer HM_ERR_INVALID and write
+    nothing outside their arrays; a valid graph on the same workspace follows."""
+    k = 15
+    idx, dist = random_knn(n, k, seed=n)
+    sig, rho = f32(np.full(n, 0.7)), dist.reshape(n, k)[:, 1].copy()
+    bad = idx.copy().reshape(n, k)
+    bad[1:1 + repeaters] = 0
+    g = DeviceGraph(n, k)
+    rc, _ = g.run(bad.reshape(-1), dist, sig, rho)
+    assert rc == hm.HM_ERR_INVALID and b"repeats" in hm.lib().hm_last_error()
+    with pytest.raises(Exception, match="repeats"):
+        hm.fuzzy_simplicial_set(hm.Knn(k, bad.reshape(-1), dist), hm.SmoothKnn(sig, rho))
+    rc, (nnz, rows, cols, vals) = g.run(idx, dist, sig, rho)
+    r, c, v = oracle.fuzzy_graph(idx, dist, sig, rho, k)
+    assert rc == hm.HM_OK and nnz == r.size
+    assert_same_bytes(rows.view(np.uint32), r, "rows")
+    assert_same_bytes(cols.view(np.uint32), c, "cols")
+    assert_same_bytes(vals.view(np.float32), v, "vals")
