@@ -216,6 +216,7 @@ SIGNATURES = {
     "hm_noalloc_stats": (_i32, [_vp, _vp]),
     "hm_debug_set_screen_dump": (_i32, [_vp]),
     "hm_debug_tridiag_eigen": (_i32, [_vp, _vp, _u32, _vp, _vp]),
+    "hm_debug_smooth_row": (_u32, [_u32, _u32, _u32]),
     "hm_batch_create": (_i32, [_vp, _u32, _vp]),
     "hm_batch_destroy": (None, [_vp]),
     "hm_batch_workspace_bytes": (_sz, [_vp]),

@@ -21,6 +21,13 @@
 namespace hm {
 
 constexpr uint32_t SK_MAX_K = 256;  // widest row of smooth_rows_kernel
+constexpr uint32_t SK_THREADS = 128;  // threads of its blocks
+
+// Row of a thread of smooth_rows_kernel with `lanes` lanes a row.  (The flat thread
+// index passes 2^32 from 2^28 rows of 16 lanes on; the rows of a call stay below 2^31.)
+__host__ __device__ __forceinline__ uint32_t smooth_row(uint32_t block, uint32_t thread, uint32_t lanes) {
+    return block * (SK_THREADS / lanes) + thread / lanes;
+}
 
 // One warp per row of the all-rows space; the row's values are read per
 // 32-element chunk from global memory (L1 resident after the first pass).
@@ -149,7 +156,7 @@ __device__ __forceinline__ float row_max(float v) {
 // 1,000 x 15 43 -> 14 us, 50,000 x 30 162 -> 41 us, 150,001 x 15 149 -> 45 us,
 // 10,000 x 100 285 -> 45 us.
 template <int G, int NV>
-__global__ void __launch_bounds__(128, G == 1 ? 4 : 6) smooth_rows_kernel(const JobDev *__restrict__ jobs, uint32_t njobs,
+__global__ void __launch_bounds__(SK_THREADS, G == 1 ? 4 : 6) smooth_rows_kernel(const JobDev *__restrict__ jobs, uint32_t njobs,
                                                           const uint32_t *__restrict__ row_starts, uint32_t rows,
                                                           uint32_t k_lo) {
     constexpr unsigned FULL = 0xffffffffu;
@@ -157,7 +164,7 @@ __global__ void __launch_bounds__(128, G == 1 ? 4 : 6) smooth_rows_kernel(const 
     grid_ready();
     const int lane = threadIdx.x & 31;
     const uint32_t q = threadIdx.x & (G - 1);
-    const uint32_t at = (blockIdx.x * blockDim.x + threadIdx.x) / G;
+    const uint32_t at = smooth_row(blockIdx.x, threadIdx.x, G);
     const uint32_t ar = min(at, rows - 1);  // lanes past the last row idle along
     const JobDev &J = jobs[row_starts ? find_job(row_starts, njobs, ar) : 0];
     const uint32_t k = J.k;
@@ -327,9 +334,9 @@ __global__ void __launch_bounds__(128, G == 1 ? 4 : 6) smooth_rows_kernel(const 
 template <int G, int NV>
 static int launch_rows(const JobDev *jobs, uint32_t njobs, const uint32_t *row_starts, uint32_t rows, uint32_t k_lo,
                        cudaStream_t s, bool overlap) {
-    constexpr uint32_t per_block = 128 / G;
-    HM_CUDA_TRY(launch(overlap, smooth_rows_kernel<G, NV>, (rows + per_block - 1) / per_block, 128, 0, s, jobs, njobs,
-                       row_starts, rows, k_lo));
+    constexpr uint32_t per_block = SK_THREADS / G;
+    HM_CUDA_TRY(launch(overlap, smooth_rows_kernel<G, NV>, (rows + per_block - 1) / per_block, SK_THREADS, 0, s, jobs,
+                       njobs, row_starts, rows, k_lo));
     count_launch();
     return HM_OK;
 }
@@ -408,3 +415,7 @@ int launch_mean_all_floor(const JobDev *jobs, uint32_t njobs, cudaStream_t s) {
 }
 
 }  // namespace hm
+
+extern "C" uint32_t hm_debug_smooth_row(uint32_t block, uint32_t thread, uint32_t lanes) {
+    return hm::smooth_row(block, thread, lanes);
+}

@@ -455,6 +455,10 @@ HM_API int hm_debug_set_screen_dump(float *d_out);
 HM_API int hm_debug_tridiag_eigen(const double *d, const double *e, uint32_t m, double *vals_out,
                                   double *vecs_out);
 
+/* Test hook (host only, no device): the row that thread `thread` of block
+ * `block` of the smooth-kNN calibration works on, at `lanes` lanes a row. */
+HM_API uint32_t hm_debug_smooth_row(uint32_t block, uint32_t thread, uint32_t lanes);
+
 #ifdef __cplusplus
 }
 #endif

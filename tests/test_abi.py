@@ -259,3 +259,15 @@ def test_workspace_stays_within_what_callers_sized_for(n, d, k, metric, path, mo
     the slots of whole column parts."""
     got = hm.lib().hm_workspace_bytes(n, d, k, metric, path)
     assert 0 < got <= most
+
+
+@pytest.mark.parametrize("lanes", [1, 4, 8, 16])
+def test_smooth_row_index_up_to_the_largest_call(lanes):
+    """The calibration's row index over 2^31 - 1 rows, the largest call: 16 lanes a
+    row (k above 32) make the flat thread index pass 2^32 from 2^28 rows on, 4 lanes
+    (k above 16) from 2^30."""
+    per_block = 128 // lanes
+    for row in (0, 1, per_block - 1, per_block, 2**28 - 1, 2**28, 2**28 + 3, 2**30, 2**30 + 5, 2**31 - 2):
+        for lane in (0, lanes - 1):
+            block, thread = row // per_block, row % per_block * lanes + lane
+            assert hm.lib().hm_debug_smooth_row(block, thread, lanes) == row
