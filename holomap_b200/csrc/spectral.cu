@@ -571,7 +571,9 @@ __global__ void __launch_bounds__(LZ_THREADS, 1) lanczos_cycle_kernel(const LzDe
                 double s = 0.0;
                 for (uint32_t u = tid; u < nu; u += 32) s = __fma_rn(c[u], c[u], s);
                 s = warp_sum_fixed(s);
-                if (tid == 0) s_beta = __dsqrt_rn(fmax(__dsub_rn(c[nu], s), 0.0));
+                // (a NaN stays one, so that the tridiagonal solver refuses the graph)
+                const double sq = __dsub_rn(c[nu], s);
+                if (tid == 0) s_beta = __dsqrt_rn(sq < 0.0 ? 0.0 : sq);
             }
             chunk_project(U, nu, c, v, ne, split, red);  // ends with the block's barrier
         }

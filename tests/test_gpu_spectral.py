@@ -239,3 +239,20 @@ def test_eigenpairs_of_expanders(oracle, n, degree, hub, k):
     ip, sv, _ = oracle.laplacian(r, c, v, n)
     eigen_close(oracle, ip, c, sv, pairs, 1e-9)
     assert np.abs(pairs.vectors @ pairs.vectors.T - np.eye(k)).max() < 1e-9
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -9.0])  # (the last one's row sum is negative)
+@pytest.mark.parametrize("n", [2, 40, 3000])
+def test_graph_without_a_laplacian_is_refused(n, value):
+    """A weight whose normalized Laplacian is not a number is an error, not an
+    empty success."""
+    i = np.arange(n - 1)
+    rows = np.stack([i, i + 1], 1).reshape(-1)
+    cols = np.stack([i + 1, i], 1).reshape(-1)
+    order = np.lexsort((cols, rows))
+    vals = np.ones(rows.size, dtype=np.float32)
+    vals[rows.size // 2] = value
+    g = hm.FuzzyGraph(n, rows[order].astype(np.uint32), cols[order].astype(np.uint32), vals)
+    with pytest.raises(hm.HolomapCudaError) as e:
+        hm.smallest_eigenpairs(g, 1)
+    assert e.value.code == hm.HM_ERR_UNSUPPORTED
