@@ -70,9 +70,11 @@ struct FuzzyDev {
     uint32_t *count;    // entries of output row r
     uint32_t *tile_sum;
     uint32_t *hub_off;  // output offset of a hub row
-    uint32_t *hubs, *mids;  // rows of more than 512 and of 129 to 512 slots
+    uint32_t *longs;    // rows of more than 512 slots from the front, of 129 to 512 from the back (mid_row)
     uint32_t *words;    // FZ_*
 };
+
+__device__ __forceinline__ uint32_t &mid_row(const FuzzyDev &D, uint32_t i) { return D.longs[D.n - 1 - i]; }
 
 __device__ __forceinline__ float tconorm(float v, float vt) {
     return __fsub_rn(__fadd_rn(v, vt), __fmul_rn(v, vt));
@@ -251,8 +253,11 @@ __global__ void __launch_bounds__(FZ_WARPS * 32, sizeof(K) == 4 ? 16 : 8) fuzzy_
                 // at most n - 1 arrivals, so an index is repeated)
                 atomicOr(&D.words[FZ_BAD], FZ_BAD_DUPLICATE);
                 D.count[r] = 0;
-            } else if (slots <= FZ_WARP_SLOTS) D.mids[atomicAdd(&D.words[FZ_MIDS], 1u)] = r;
-            else D.hubs[atomicAdd(&D.words[FZ_HUBS], 1u)] = r;
+            } else if (slots <= FZ_WARP_SLOTS) {
+                mid_row(D, atomicAdd(&D.words[FZ_MIDS], 1u)) = r;
+            } else {
+                D.longs[atomicAdd(&D.words[FZ_HUBS], 1u)] = r;
+            }
         }
         return;
     }
@@ -278,7 +283,7 @@ __global__ void __launch_bounds__(1024) fuzzy_long_kernel(const FuzzyDev D, uint
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t hubs = D.words[FZ_HUBS], k = D.k;
     for (uint32_t h = blockIdx.x; h < hubs; h += gridDim.x) {
-        const uint32_t r = D.hubs[h], rc = D.indeg[r];
+        const uint32_t r = D.longs[h], rc = D.indeg[r];
         const uint64_t base = (uint64_t)r * k;
         uint2 *seg = D.stage + D.seg[r], *out = out_all + D.seg[r];
         uint32_t total = 0;
@@ -364,7 +369,7 @@ __global__ void __launch_bounds__(1024) fuzzy_long_kernel(const FuzzyDev D, uint
         uint32_t i = lane == 0 ? atomicAdd(&D.words[FZ_NEXT], 1u) : 0u;
         i = __shfl_sync(FZ_FULL, i, 0);
         if (i >= mids) break;
-        const uint32_t r = D.mids[i], slots = k + D.indeg[r];
+        const uint32_t r = mid_row(D, i), slots = k + D.indeg[r];
         const uint32_t count = slots <= 256 ? union_row<K, 8>(D, r, slots, w, lane) : union_row<K, 16>(D, r, slots, w, lane);
         __syncwarp();
         if (lane == 0) {
@@ -434,7 +439,7 @@ __global__ void __launch_bounds__(256) fuzzy_hub_write_kernel(const FuzzyDev D, 
     const uint32_t parts = max(1u, gridDim.x / max(hubs, 1u)), at_once = gridDim.x / parts;  // blocks a row, rows
     if (blockIdx.x >= parts * at_once) return;
     for (uint32_t h = blockIdx.x / parts; h < hubs; h += at_once) {
-        const uint32_t r = D.hubs[h], c = D.count[r];
+        const uint32_t r = D.longs[h], c = D.count[r];
         if (c <= FZ_WARP_SLOTS) continue;  // many partners: written with the others
         const uint2 *seg = D.stage + D.seg[r];
         const uint32_t o = D.hub_off[r];
@@ -447,10 +452,12 @@ __global__ void __launch_bounds__(256) fuzzy_hub_write_kernel(const FuzzyDev D, 
     }
 }
 
-// Workspace.  The hub kernel's output buffer doubles the segments; it is only
-// touched when there are rows of more than 512 slots.
+// Workspace: 36 bytes an entry and about 20 a row, no more than callers sized for when
+// the arrivals were sorted.  The hub kernel's output buffer, as large as the segments
+// and touched only when there are rows of more than 512 slots, lies over the entries'
+// slots, which are used up by then.
 struct FuzzyLayout {
-    size_t w, slot, stage, hub_out, seg, count, hubs, mids, zeroed, zeroed_bytes, bad, total;
+    size_t w, slot, stage, hub_out, seg, count, longs, zeroed, zeroed_bytes, bad, total;
     uint32_t tiles, tile_rows;
 };
 
@@ -467,17 +474,15 @@ static int fuzzy_layout(uint64_t n, uint32_t k, FuzzyLayout *L) {
     L->tile_rows = (uint32_t)std::max<uint64_t>(FZ_TILE_ROWS, (n + FZ_TILES - 1) / FZ_TILES);
     L->tiles = (uint32_t)((n + L->tile_rows - 1) / L->tile_rows);
     L->w = take(entries * 4);
-    L->slot = take(entries * 4);
     L->stage = take(2 * entries * sizeof(uint2));
-    L->hub_out = take(2 * entries * sizeof(uint2));
+    L->hub_out = L->slot = take(2 * entries * sizeof(uint2));
     L->seg = take(n * 4);
     L->count = take(n * 4);
-    L->hubs = take(n * 4);
-    L->mids = take(n * 4);
+    L->longs = take(n * 4);
     // cleared at the start of every run: in-degrees, tile sums, words
-    L->zeroed_bytes = (n + FZ_TILES + FZ_WORDS) * 4;
+    L->zeroed_bytes = (n + L->tiles + FZ_WORDS) * 4;
     L->zeroed = take(L->zeroed_bytes);
-    L->bad = L->zeroed + (n + FZ_TILES + FZ_BAD) * 4;
+    L->bad = L->zeroed + (n + L->tiles + FZ_BAD) * 4;
     L->total = at;
     return HM_OK;
 }
@@ -528,12 +533,11 @@ int hm_fuzzy_graph_device(const uint32_t *d_idx, const float *d_dist, const floa
     D.stage = reinterpret_cast<uint2 *>(ws + L.stage);
     D.seg = reinterpret_cast<uint32_t *>(ws + L.seg);
     D.count = reinterpret_cast<uint32_t *>(ws + L.count);
-    D.hubs = reinterpret_cast<uint32_t *>(ws + L.hubs);
-    D.mids = reinterpret_cast<uint32_t *>(ws + L.mids);
+    D.longs = reinterpret_cast<uint32_t *>(ws + L.longs);
     D.indeg = reinterpret_cast<uint32_t *>(ws + L.zeroed);
-    D.hub_off = D.slot;  // the entries' slots are used up by then
+    D.hub_off = reinterpret_cast<uint32_t *>(D.w);  // the strengths are used up by then
     D.tile_sum = D.indeg + n;
-    D.words = D.tile_sum + FZ_TILES;
+    D.words = D.tile_sum + L.tiles;
     const unsigned entry_blocks = (D.entries + 256 * FZ_PER_THREAD - 1) / (256 * FZ_PER_THREAD);
     HM_CUDA_TRY(cudaMemsetAsync(ws + L.zeroed, 0, L.zeroed_bytes, s));
     HM_CUDA_TRY(launch(false, fuzzy_entries_kernel, entry_blocks, 256, 0, s, D));

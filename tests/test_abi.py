@@ -271,3 +271,12 @@ def test_smooth_row_index_up_to_the_largest_call(lanes):
         for lane in (0, lanes - 1):
             block, thread = row // per_block, row % per_block * lanes + lane
             assert hm.lib().hm_debug_smooth_row(block, thread, lanes) == row
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 63, 64, 100, 1000, 2402, 32768, 50000, 1_000_003])
+@pytest.mark.parametrize("k", [1, 2, 15, 30, 256, 600])
+def test_fuzzy_workspace_stays_within_what_callers_sized_for(n, k):
+    """Nine 4-byte arrays over the entries, five over the rows and two small blocks of
+    256 bytes are the least that callers have ever been told to bring."""
+    up = lambda b: (b + 255) // 256 * 256
+    assert 0 < hm.lib().hm_fuzzy_workspace_bytes(n, k) <= 9 * up(4 * n * k) + 5 * up(4 * n) + 512
