@@ -745,7 +745,6 @@ struct Lanczos {
     uint32_t k = 0, m = 0, blocks = 0;
     double *stat = nullptr;  // alpha, beta, resid and the sync words, read back in one copy
     uint32_t stat_rows = 0;
-    double *y = nullptr;
     double *ritz = nullptr;  // block partials of the Ritz stage
     cudaStream_t s = nullptr;
 
@@ -815,6 +814,9 @@ struct Lanczos {
                     for (uint32_t q = 0; q < nsteps; ++q)
                         ybuf[(size_t)c * (nsteps + 1) + 1 + q] = z[(size_t)col * nsteps + q];
                 }
+                // (into the rows of U past the cycle's basis: see lanczos_layout)
+                double *const y = D.U + ((uint64_t)L + nsteps) * n;
+                D.y = y;
                 HM_CUDA_TRY(cudaMemcpyAsync(y, ybuf.data(), ybuf.size() * sizeof(double), cudaMemcpyHostToDevice, s));
                 D.X = X0 + (uint64_t)c0 * n;
                 D.part1 = ritz;
@@ -879,10 +881,13 @@ static int laplacian_launch(const uint32_t *d_rows, const uint32_t *d_cols, cons
 }
 
 // Workspace of an eigenpair run (beyond the Laplacian itself), in bytes from its
-// start.  The block partials of a cycle lie in the candidates' room (the two are
-// never live together).
+// start; no larger than callers sized for when every step was its own launches.  The
+// block partials of a cycle lie in the candidates' room (the two are never live
+// together).  The candidates' coefficients lie in the rows of U past the cycle's
+// basis: a cycle with L locked vectors has at most k + 1 - L candidates of nsteps + 1
+// <= n + 1 coefficients each, and at least k + 1 - L rows are free.
 struct LzLayout {
-    size_t U, X, w, r, ritz, y, stat, total;
+    size_t U, X, w, r, ritz, stat, total;
     uint32_t m, rows, blocks;
 };
 static LzLayout lanczos_layout(uint64_t n, uint32_t k) {
@@ -896,12 +901,11 @@ static LzLayout lanczos_layout(uint64_t n, uint32_t k) {
         at += round_up(doubles * sizeof(double), 256);
         return here;
     };
-    l.U = take((size_t)l.rows * n);
+    l.U = take((size_t)l.rows * n + LZ_RITZ);
     l.X = take(std::max<size_t>((size_t)(k + 1) * n, (size_t)2 * (l.rows + 1) * l.blocks));
     l.w = take(n);
     l.r = take(n);
     l.ritz = take((size_t)2 * LZ_RITZ * l.blocks);
-    l.y = take((size_t)LZ_RITZ * (l.m + 1));
     l.stat = take((size_t)2 * l.rows + LZ_RITZ + LZ_WORDS / 2);
     l.total = at;
     return l;
@@ -969,7 +973,6 @@ int hm_eigenpairs_device(const uint64_t *d_indptr, const uint32_t *d_cols, const
     lz.s = static_cast<cudaStream_t>(stream);
     lz.stat = at(l.stat);
     lz.stat_rows = l.rows;
-    lz.y = at(l.y);
     LzDev &D = lz.D;
     D.indptr = d_indptr;
     D.cols = d_cols;
@@ -986,7 +989,6 @@ int hm_eigenpairs_device(const uint64_t *d_indptr, const uint32_t *d_cols, const
     D.beta = lz.stat + l.rows;
     D.resid = lz.stat + 2 * (size_t)l.rows;
     D.sync = reinterpret_cast<uint32_t *>(D.resid + LZ_RITZ);
-    D.y = lz.y;
     lz.ritz = at(l.ritz);
     return lz.run(values_out, vectors_out, found_out, cycles_out);
 }

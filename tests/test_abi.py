@@ -280,3 +280,14 @@ def test_fuzzy_workspace_stays_within_what_callers_sized_for(n, k):
     256 bytes are the least that callers have ever been told to bring."""
     up = lambda b: (b + 255) // 256 * 256
     assert 0 < hm.lib().hm_fuzzy_workspace_bytes(n, k) <= 9 * up(4 * n * k) + 5 * up(4 * n) + 512
+
+
+@pytest.mark.parametrize("n", [1, 2, 30, 61, 386, 609, 1024, 1986, 2048, 2049, 50000])
+def test_eigenpairs_workspace_stays_within_what_callers_sized_for(n):
+    """The Krylov basis, the candidates and three vectors, the partial sums of 2,048
+    elements each, three scalars a row and 4 KB."""
+    for k in {1, 3, 47, 48, 162, 246, 255, 1024}:
+        if k <= n:
+            rows = k + min(n, max(8 * k, 60)) + 1
+            most = (rows + k + 1 + 3) * n * 8 + rows * ((n + 2047) // 2048) * 8 + rows * 8 * 3 + 4096
+            assert 0 < hm.lib().hm_eigenpairs_workspace_bytes(n, k) <= most
