@@ -20,8 +20,8 @@
 //      (src/fuzzy.rs:67-75) and leaves the sorted row at the front of its
 //      segment; fuzzy_long_kernel does the rows above 128 slots: a warp each up
 //      to 512, a block each beyond.
-//   5. fuzzy_write_kernel (one block per tile of rows) sums the tiles before
-//      it, scans its rows' counts and writes the COO.
+//   5. fuzzy_write_kernel (one block per tile of rows, several per very long row)
+//      sums the tiles before it, scans its rows' counts and writes the COO.
 //
 // Strengths lie in [0, 1] (or are NaN) when every sigma is non-negative, and
 // then no fused value of a union coordinate is zero: fl(v * vt) <= min(v,
@@ -34,9 +34,7 @@
 // What bounds it: latency of the L2-resident arrays and the sorts' issue.  With a
 // radix sort of the reverse copies and binary-search merges -> now: kNN graph of
 // 50,000 x 384 embeddings, k = 30 (2.7 M entries) 180 -> 117 us; random graphs of
-// 50,000 x 15 140 -> 76, 2,000 x 15 62 -> 42, 1,000,000 x 15 2133 -> 1274.  A graph
-// whose rows all share the same 29 neighbours (29 rows of 50,000 entries, one
-// block each) is slower, 151 -> 194 us.
+// 50,000 x 15 140 -> 76, 2,000 x 15 62 -> 42, 1,000,000 x 15 2133 -> 1274.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -56,6 +54,10 @@ constexpr uint32_t FZ_SHORT_SLOTS = 128;                 // and of the short-row
 constexpr uint32_t FZ_TILES = 1024;                      // write tiles at most
 constexpr uint32_t FZ_TILE_ROWS = 32;                    // and rows per tile at least
 constexpr uint32_t FZ_WINDOW = 1u << 19;                 // columns per pass of the hub kernel
+constexpr uint32_t FZ_PART_WINDOW = 1u << 14;            // and where several blocks share a hub
+constexpr uint32_t FZ_SHARED_HUB = 8192;                 // of this many arrivals
+constexpr uint32_t FZ_HOT = 8;                           // matches that make a block of entries count jointly
+constexpr uint32_t FZ_JOINT_ROWS = 2048;                 // in graphs of this many rows
 enum { FZ_ALLOCATED = 0, FZ_HUBS = 1, FZ_BAD = 2, FZ_MIDS = 3, FZ_NEXT = 4, FZ_WORDS = 8 };
 
 struct FuzzyDev {
@@ -67,9 +69,9 @@ struct FuzzyDev {
     uint32_t *indeg;    // |R_r|
     uint32_t *seg;      // first slot of row r's segment
     uint2 *stage;       // segments: (source or column, strength bits)
+    uint2 *hub_out;     // rows of more than 512 slots, at their segments' places
     uint32_t *count;    // entries of output row r
     uint32_t *tile_sum;
-    uint32_t *hub_off;  // output offset of a hub row
     uint32_t *longs;    // rows of more than 512 slots from the front, of 129 to 512 from the back (mid_row)
     uint32_t *words;    // FZ_*
 };
@@ -81,7 +83,30 @@ __device__ __forceinline__ float tconorm(float v, float vt) {
 }
 
 constexpr uint32_t FZ_PER_THREAD = 4;  // entries in flight per thread of the entry kernels
+
+// Arrival slots of a block's 256 * FZ_PER_THREAD entries whose rows list the same
+// columns at the same places (points at distance 0 from all, such as zero vectors
+// under cosine): a column's counter would take an atomic from every row.  The warps
+// go down the places instead, 32 rows at a time, and equal columns share one.
+// col[e]: the column of the block's entry e, or ~0u; receives its slot.
+__device__ __noinline__ void joint_slots(const FuzzyDev &D, uint32_t *col) {
+    constexpr uint32_t N = 256 * FZ_PER_THREAD;
+    const uint32_t lane = threadIdx.x & 31, k = min(D.k, N), rows = (N + k - 1) / k;
+    for (uint32_t t0 = 0; t0 < k * rows; t0 += 256) {  // whole warps
+        const uint32_t t = t0 + threadIdx.x, e = (t % rows) * k + t / rows;
+        const bool in = t < k * rows && e < N;
+        const uint32_t c = in ? col[e] : ~0u;
+        const unsigned m = __match_any_sync(FZ_FULL, c);
+        const int leader = __ffs(m) - 1;
+        uint32_t base = 0;
+        if (c != ~0u && (int)lane == leader) base = atomicAdd(&D.indeg[c], (uint32_t)__popc(m));
+        base = __shfl_sync(FZ_FULL, base, leader);
+        if (in) col[e] = base + __popc(m & ((1u << lane) - 1u));
+    }
+}
+
 __global__ void __launch_bounds__(256) fuzzy_entries_kernel(const FuzzyDev D) {
+    __shared__ uint32_t s_col[256 * FZ_PER_THREAD];
     grid_ready();
     const uint32_t e0 = blockIdx.x * 256 * FZ_PER_THREAD + threadIdx.x;
     uint32_t col[FZ_PER_THREAD], row[FZ_PER_THREAD], slot[FZ_PER_THREAD];
@@ -93,6 +118,15 @@ __global__ void __launch_bounds__(256) fuzzy_entries_kernel(const FuzzyDev D) {
         col[q] = D.idx[e];
         d[q] = __fsub_rn(D.dist[e], D.rho[row[q]]);
         sg[q] = D.sigma[row[q]];
+    }
+    // whether rows list the same columns at the same places: a quarter of the block's
+    // entries against the row below (FZ_HOT of 256: one shared column in 30).  A counter
+    // takes an atomic in 2.5 ns, so small graphs gain nothing (100 x 50: 25 us, 27 if
+    // counted jointly).
+    bool joint = false;
+    if (D.n >= FZ_JOINT_ROWS) {
+        const bool same = e0 + D.k < D.entries && D.idx[e0 + D.k] == col[0];
+        joint = __syncthreads_count(same) >= FZ_HOT;
     }
 #pragma unroll
     for (uint32_t q = 0; q < FZ_PER_THREAD; ++q) {
@@ -110,8 +144,17 @@ __global__ void __launch_bounds__(256) fuzzy_entries_kernel(const FuzzyDev D) {
             } else {
                 w[q] = 1.0f;
             }
-            if (w[q] != 0.0f) slot[q] = atomicAdd(&D.indeg[col[q]], 1u);
+            if (w[q] != 0.0f && !joint) slot[q] = atomicAdd(&D.indeg[col[q]], 1u);
         }
+    }
+    if (joint) {
+#pragma unroll
+        for (uint32_t q = 0; q < FZ_PER_THREAD; ++q) s_col[256 * q + threadIdx.x] = w[q] != 0.0f ? col[q] : ~0u;
+        __syncthreads();
+        joint_slots(D, s_col);
+        __syncthreads();
+#pragma unroll
+        for (uint32_t q = 0; q < FZ_PER_THREAD; ++q) slot[q] = s_col[256 * q + threadIdx.x];
     }
 #pragma unroll
     for (uint32_t q = 0; q < FZ_PER_THREAD; ++q) {
@@ -172,7 +215,7 @@ __global__ void __launch_bounds__(256) fuzzy_scatter_kernel(const FuzzyDev D) {
     }
 #pragma unroll
     for (uint32_t q = 0; q < FZ_PER_THREAD; ++q)
-        if (w[q] != 0.0f) D.stage[at[q]] = make_uint2((e0 + 256 * q) / D.k, __float_as_uint(w[q]));
+        if (w[q] != 0.0f && at[q] < 2 * D.entries) D.stage[at[q]] = make_uint2((e0 + 256 * q) / D.k, __float_as_uint(w[q]));
 }
 
 // A row of at most 32 * NQ slots: keys column << 9 | slot (F slots below k, so an
@@ -267,25 +310,118 @@ __global__ void __launch_bounds__(FZ_WARPS * 32, sizeof(K) == 4 ? 16 : 8) fuzzy_
     }
 }
 
-// Rows of more than 512 slots, one block each (taken in turn): R_r and F_r as
-// bitmaps over the columns (windows of 2^19), whose prefix counts give every
-// entry's place with no sort.  Zero vectors under cosine are at distance 0 from
-// every point, so rows with n entries do occur.  The row is built beside the
-// segments (`out_all`) and copied back, since every window reads the segment.
+// The block's columns [c0, c0 + width) of a hub row, for one of several blocks that
+// share it.  One pass over the arrivals counts those below the window and leaves the
+// others' strengths by column; with the F entries below the window less those that
+// arrived too (found in the lists of their own rows), that is where the window starts
+// in the row.  smem: width strengths, then three words per 32 columns.
+__device__ __forceinline__ void hub_part(const FuzzyDev &D, uint32_t r, uint32_t c0, uint32_t width, uint32_t *smem,
+                                         uint32_t *warp_sums) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, k = D.k;
+    const uint32_t c1 = min(D.n - c0, width), nw = (c1 + 31) / 32;  // the window's columns, words (at most 1,024)
+    uint32_t *strength = smem, *rbits = strength + width, *fbits = rbits + (width + 31) / 32, *pre = fbits + (width + 31) / 32;
+    const uint32_t rc = D.indeg[r];
+    const uint64_t base = (uint64_t)r * k;
+    const uint2 *seg = D.stage + D.seg[r];
+    uint2 *out = D.hub_out + D.seg[r];
+    __shared__ uint32_t s_below;
+    __syncthreads();
+    if (tid < nw) rbits[tid] = fbits[tid] = 0u;
+    if (tid == 0) s_below = 0;
+    __syncthreads();
+    uint32_t below = 0;
+    for (uint32_t e = tid; e < rc; e += 8 * 1024) {
+        uint2 s[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) s[q] = e + 1024 * q < rc ? seg[k + e + 1024 * q] : make_uint2(~0u, 0u);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const uint32_t c = s[q].x - c0;
+            below += s[q].x < c0 ? 1u : 0u;
+            if (s[q].x >= c0 && c < c1) {
+                atomicOr(&rbits[c >> 5], 1u << (c & 31));
+                strength[c] = s[q].y;
+            }
+        }
+    }
+    for (uint32_t e = warp; e < k; e += 32) {  // a warp per F entry
+        const uint32_t col = D.idx[base + e];
+        if (D.w[base + e] == 0.0f) continue;
+        if (col < c0) {
+            const uint64_t other = (uint64_t)col * k;
+            bool partner = false;
+            for (uint32_t j = lane; j < k; j += 32) partner |= D.idx[other + j] == r && D.w[other + j] != 0.0f;
+            if (!__any_sync(FZ_FULL, partner) && lane == 0) ++below;
+        } else if (col - c0 < c1 && lane == 0) {
+            const uint32_t c = col - c0, bit = 1u << (c & 31);
+            if (atomicOr(&fbits[c >> 5], bit) & bit) atomicOr(&D.words[FZ_BAD], FZ_BAD_DUPLICATE);
+        }
+    }
+    below = __reduce_add_sync(FZ_FULL, below);
+    if (lane == 0 && below) atomicAdd(&s_below, below);
+    __syncthreads();
+    const uint32_t v = tid < nw ? __popc(rbits[tid] | fbits[tid]) : 0u, incl = warp_scan(v, lane);
+    if (lane == 31) warp_sums[warp] = incl;
+    __syncthreads();
+    const uint32_t ws = warp_scan(warp_sums[lane], lane);
+    const uint32_t before = __shfl_sync(FZ_FULL, ws, warp ? warp - 1 : 0), sum = __shfl_sync(FZ_FULL, ws, 31);
+    const uint32_t start = s_below;
+    if (tid < nw) pre[tid] = start + (warp ? before : 0u) + incl - v;
+    __syncthreads();
+    auto place = [&](uint32_t c) {
+        const uint32_t q = c >> 5;
+        return pre[q] + __popc((rbits[q] | fbits[q]) & ((1u << (c & 31)) - 1u));
+    };
+    for (uint32_t c = tid; c < c1; c += 1024)  // R entries without an F partner
+        if ((rbits[c >> 5] & ~fbits[c >> 5]) >> (c & 31) & 1u)
+            out[place(c)] = make_uint2(c0 + c, __float_as_uint(tconorm(0.0f, __uint_as_float(strength[c]))));
+    for (uint32_t e = tid; e < k; e += 1024) {
+        const uint32_t col = D.idx[base + e], c = col - c0;
+        const float f = D.w[base + e];
+        if (f == 0.0f || col < c0 || c >= c1) continue;
+        const float vt = rbits[c >> 5] >> (c & 31) & 1u ? __uint_as_float(strength[c]) : 0.0f;
+        out[place(c)] = make_uint2(col, __float_as_uint(tconorm(f, vt)));
+    }
+    if (tid == 0 && c0 + c1 == D.n) {
+        D.count[r] = start + sum;
+        atomicAdd(&D.tile_sum[r / D.tile_rows], start + sum);
+    }
+}
+
+// Rows of more than 512 slots (hubs): R_r and F_r as bitmaps over the columns, whose
+// prefix counts give every entry's place with no sort.  Zero vectors under cosine are
+// at distance 0 from every point, so rows with n entries do occur, and then there are
+// few of them: where the blocks are at least twice the hubs, each long hub is shared
+// by several (hub_part); else a block takes hubs in turn, windows of 2^19 columns at a
+// time.  (Sharing hubs of 600 arrivals as well keeps all blocks from the other rows:
+// the embeddings' graph above 105 -> 112 us.)  The rows are built beside the segments,
+// which every window reads.
 // The blocks' warps then take the rows of 129 to 512 slots, one each.
+// Graphs whose rows share their neighbours, one block a hub and an atomic an entry ->
+// now (both kernels): 50,000 x 30 with 29 shared 260 -> 110 us, 200,000 x 15 with 14
+// 656 -> 270, with one 530 -> 236; sorting the arrivals took 141, 335 and 447.
 template <typename K>
-__global__ void __launch_bounds__(1024) fuzzy_long_kernel(const FuzzyDev D, uint2 *out_all) {
+__global__ void __launch_bounds__(1024) fuzzy_long_kernel(const FuzzyDev D) {
     grid_ready();
     extern __shared__ uint32_t hub_smem[];
     __shared__ uint32_t warp_sums[32];
     const uint32_t words_n = (min(D.n, FZ_WINDOW) + 31) / 32;
     uint32_t *rbits = hub_smem, *fbits = rbits + words_n, *pre = fbits + words_n;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t hubs = D.words[FZ_HUBS], k = D.k;
-    for (uint32_t h = blockIdx.x; h < hubs; h += gridDim.x) {
+    const uint32_t hubs = D.words[FZ_HUBS], k = D.k, parts = hubs ? gridDim.x / hubs : 0u;
+    const bool spread = parts > 1;  // the blocks of hub h: h parts, ..., h parts + parts - 1
+    for (uint32_t h = spread ? blockIdx.x / parts : blockIdx.x; h < hubs; h += spread ? hubs : gridDim.x) {
         const uint32_t r = D.longs[h], rc = D.indeg[r];
+        if (spread && rc >= FZ_SHARED_HUB) {
+            const uint32_t width = min(((D.n + parts - 1) / parts + 31) & ~31u, FZ_PART_WINDOW);
+            for (uint64_t c0 = (uint64_t)(blockIdx.x % parts) * width; c0 < D.n; c0 += (uint64_t)parts * width)
+                hub_part(D, r, (uint32_t)c0, width, hub_smem, warp_sums);
+            continue;
+        }
+        if (spread && blockIdx.x % parts) continue;
         const uint64_t base = (uint64_t)r * k;
-        uint2 *seg = D.stage + D.seg[r], *out = out_all + D.seg[r];
+        const uint2 *seg = D.stage + D.seg[r];
+        uint2 *out = D.hub_out + D.seg[r];
         uint32_t total = 0;
         for (uint32_t c0 = 0; c0 < D.n; c0 += FZ_WINDOW) {
             const uint32_t c1 = min(D.n - c0, FZ_WINDOW), nw = (c1 + 31) / 32;  // the window's columns, words
@@ -347,16 +483,6 @@ __global__ void __launch_bounds__(1024) fuzzy_long_kernel(const FuzzyDev D, uint
             }
             total = carry;
         }
-        __syncthreads();
-        for (uint32_t e = tid; e < total; e += 4 * 1024) {
-            uint2 s[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (e + 1024 * q < total) s[q] = out[e + 1024 * q];
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (e + 1024 * q < total) seg[e + 1024 * q] = s[q];
-        }
         if (tid == 0) {
             D.count[r] = total;
             atomicAdd(&D.tile_sum[r / D.tile_rows], total);
@@ -379,33 +505,62 @@ __global__ void __launch_bounds__(1024) fuzzy_long_kernel(const FuzzyDev D, uint
     }
 }
 
-// One block per tile of tile_rows rows.
+// Entries of the tiles before `tile` (a whole block).
+__device__ __forceinline__ uint32_t tile_offset(const FuzzyDev &D, uint32_t tile, uint32_t *warp_sums) {
+    uint32_t sum = 0, total;
+    for (uint32_t t = threadIdx.x; t < tile; t += 256) sum += D.tile_sum[t];
+    block_scan(sum, warp_sums, total);
+    return total;
+}
+
+// The COO: a block per tile of tile_rows rows, its warps taking the rows in turn.  Hub
+// rows of more than 512 entries are left to the blocks past the tiles, several to a
+// row, unless there are more such rows than blocks.  (Every offset lies below 2 n k;
+// the comparisons keep a kernel that was handed something else in its arrays.)
 __global__ void __launch_bounds__(256) fuzzy_write_kernel(const FuzzyDev D, uint32_t tiles, uint32_t *__restrict__ rows,
                                                           uint32_t *__restrict__ cols, float *__restrict__ vals,
                                                           unsigned long long *__restrict__ nnz) {
     grid_ready();
-    __shared__ uint32_t warp_sums[8], off[256], cnt[256], first[256];
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tile = blockIdx.x;
-    uint32_t sum = 0;
-    for (uint32_t t = threadIdx.x; t < tile; t += 256) sum += D.tile_sum[t];
-    uint32_t at;
-    block_scan(sum, warp_sums, at);  // at: entries of the tiles before
+    __shared__ uint32_t warp_sums[8], off[256], cnt[256];
+    __shared__ const uint2 *first[256];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tile = blockIdx.x, capacity = 2 * D.entries;
+    const uint32_t hubs = D.words[FZ_HUBS], spare = gridDim.x - tiles;
+    const bool apart = hubs <= spare;
+    if (tile >= tiles) {
+        const uint32_t parts = apart && hubs ? spare / hubs : 1u, b = tile - tiles, h = b / parts;
+        if (!apart || h >= hubs) return;
+        const uint32_t r = D.longs[h], c = D.count[r], t = r / D.tile_rows;
+        if (c <= FZ_WARP_SLOTS) return;  // many partners: written with the others
+        uint32_t sum = 0, before;
+        for (uint32_t q = t * D.tile_rows + threadIdx.x; q < r; q += 256) sum += D.count[q];
+        const uint32_t at = tile_offset(D, t, warp_sums);
+        block_scan(sum, warp_sums, before);
+        const uint2 *seg = D.hub_out + D.seg[r];
+        const uint32_t o = at + before;
+        for (uint32_t e = b % parts * 256 + threadIdx.x; e < c && o + e < capacity; e += parts * 256) {
+            const uint2 s = seg[e];
+            rows[o + e] = r;
+            cols[o + e] = s.x;
+            vals[o + e] = __uint_as_float(s.y);
+        }
+        return;
+    }
+    uint32_t at = tile_offset(D, tile, warp_sums);
     const uint32_t r0 = tile * D.tile_rows, r1 = min(D.n, r0 + D.tile_rows);
     for (uint32_t b = r0; b < r1; b += 256) {
         const uint32_t r = b + threadIdx.x, c = r < r1 ? D.count[r] : 0u;
-        first[threadIdx.x] = r < r1 ? D.seg[r] : 0u;
+        first[threadIdx.x] =
+            r < r1 ? (D.k + D.indeg[r] > FZ_WARP_SLOTS ? D.hub_out : D.stage) + D.seg[r] : D.stage;
         uint32_t chunk;
         const uint32_t before = block_scan(c, warp_sums, chunk);
-        const bool hub = c > FZ_WARP_SLOTS;  // fuzzy_hub_write_kernel's
-        if (hub) D.hub_off[r] = at + before;
         off[threadIdx.x] = at + before;
-        cnt[threadIdx.x] = hub ? 0u : c;
+        cnt[threadIdx.x] = apart && c > FZ_WARP_SLOTS ? 0u : c;
         __syncthreads();
         // two rows a warp, 64 entries of each, loaded before any is stored
         for (uint32_t q = warp; q < min(256u, r1 - b); q += 16) {
             const uint32_t q2 = q + 8;
             const uint32_t c0 = cnt[q], c1 = q2 < 256u ? cnt[q2] : 0u;
-            const uint2 *g0 = D.stage + first[q], *g1 = D.stage + first[q2 < 256u ? q2 : q];
+            const uint2 *g0 = first[q], *g1 = first[q2 < 256u ? q2 : q];
             for (uint32_t e = lane; e < max(c0, c1); e += 64) {
                 uint2 v[4];
 #pragma unroll
@@ -418,6 +573,7 @@ __global__ void __launch_bounds__(256) fuzzy_write_kernel(const FuzzyDev D, uint
                     const uint32_t x = e + 32 * (h & 1), row = h < 2 ? q : q2;
                     if (x < (h < 2 ? c0 : c1)) {
                         const uint32_t o = off[row] + x;
+                        if (o >= capacity) continue;
                         rows[o] = b + row;
                         cols[o] = v[h].x;
                         vals[o] = __uint_as_float(v[h].y);
@@ -429,27 +585,6 @@ __global__ void __launch_bounds__(256) fuzzy_write_kernel(const FuzzyDev D, uint
         __syncthreads();
     }
     if (tile == tiles - 1 && threadIdx.x == 0) *nnz = at;
-}
-
-// Rows of more than 512 entries (all of them hubs), each spread over the grid.
-__global__ void __launch_bounds__(256) fuzzy_hub_write_kernel(const FuzzyDev D, uint32_t *__restrict__ rows,
-                                                              uint32_t *__restrict__ cols, float *__restrict__ vals) {
-    grid_ready();
-    const uint32_t hubs = D.words[FZ_HUBS];
-    const uint32_t parts = max(1u, gridDim.x / max(hubs, 1u)), at_once = gridDim.x / parts;  // blocks a row, rows
-    if (blockIdx.x >= parts * at_once) return;
-    for (uint32_t h = blockIdx.x / parts; h < hubs; h += at_once) {
-        const uint32_t r = D.longs[h], c = D.count[r];
-        if (c <= FZ_WARP_SLOTS) continue;  // many partners: written with the others
-        const uint2 *seg = D.stage + D.seg[r];
-        const uint32_t o = D.hub_off[r];
-        for (uint32_t e = blockIdx.x % parts * 256 + threadIdx.x; e < c; e += parts * 256) {
-            const uint2 s = seg[e];
-            rows[o + e] = r;
-            cols[o + e] = s.x;
-            vals[o + e] = __uint_as_float(s.y);
-        }
-    }
 }
 
 // Workspace: 36 bytes an entry and about 20 a row, no more than callers sized for when
@@ -531,11 +666,11 @@ int hm_fuzzy_graph_device(const uint32_t *d_idx, const float *d_dist, const floa
     D.w = reinterpret_cast<float *>(ws + L.w);
     D.slot = reinterpret_cast<uint32_t *>(ws + L.slot);
     D.stage = reinterpret_cast<uint2 *>(ws + L.stage);
+    D.hub_out = reinterpret_cast<uint2 *>(ws + L.hub_out);
     D.seg = reinterpret_cast<uint32_t *>(ws + L.seg);
     D.count = reinterpret_cast<uint32_t *>(ws + L.count);
     D.longs = reinterpret_cast<uint32_t *>(ws + L.longs);
     D.indeg = reinterpret_cast<uint32_t *>(ws + L.zeroed);
-    D.hub_off = reinterpret_cast<uint32_t *>(D.w);  // the strengths are used up by then
     D.tile_sum = D.indeg + n;
     D.words = D.tile_sum + L.tiles;
     const unsigned entry_blocks = (D.entries + 256 * FZ_PER_THREAD - 1) / (256 * FZ_PER_THREAD);
@@ -553,18 +688,16 @@ int hm_fuzzy_graph_device(const uint32_t *d_idx, const float *d_dist, const floa
     if (n + k > FZ_SHORT_SLOTS) {
         auto *kernel = narrow ? fuzzy_long_kernel<uint32_t> : fuzzy_long_kernel<unsigned long long>;
         const size_t bitmaps = (size_t)3 * ((std::min(D.n, FZ_WINDOW) + 31) / 32) * 4, rows_w = 32 * FZ_WARP_SLOTS * 4;
+        const size_t part_words = (std::min(D.n, FZ_PART_WINDOW) + 31) / 32, part = part_words * 35 * 4;
         HM_TRY(ensure_dynamic_smem((const void *)kernel, (int)(3 * FZ_WINDOW / 8)));
-        HM_CUDA_TRY(launch(true, kernel, device_sm_count(), 1024, std::max(bitmaps, rows_w), s, D,
-                           reinterpret_cast<uint2 *>(ws + L.hub_out)));
+        HM_CUDA_TRY(launch(true, kernel, device_sm_count(), 1024, std::max({bitmaps, rows_w, part}), s, D));
         count_launch();
     }
-    HM_CUDA_TRY(launch(true, fuzzy_write_kernel, L.tiles, 256, 0, s, D, L.tiles, d_rows, d_cols, d_vals,
+    // (a row's entries are distinct columns, repeated indices or not)
+    const unsigned spare = n > FZ_WARP_SLOTS ? 4 * device_sm_count() : 0;
+    HM_CUDA_TRY(launch(true, fuzzy_write_kernel, L.tiles + spare, 256, 0, s, D, L.tiles, d_rows, d_cols, d_vals,
                        reinterpret_cast<unsigned long long *>(d_nnz)));
     count_launch(5);
-    if (n + k > FZ_WARP_SLOTS) {  // (a row's entries are distinct columns, repeated indices or not)
-        HM_CUDA_TRY(launch(true, fuzzy_hub_write_kernel, 4 * device_sm_count(), 256, 0, s, D, d_rows, d_cols, d_vals));
-        count_launch();
-    }
     return HM_OK;
 }
 

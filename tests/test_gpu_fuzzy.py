@@ -351,3 +351,52 @@ def test_repeated_indices_are_refused_in_bounds(oracle, n, repeaters):
     assert_same_bytes(rows.view(np.uint32), r, "rows")
     assert_same_bytes(cols.view(np.uint32), c, "cols")
     assert_same_bytes(vals.view(np.float32), v, "vals")
+
+
+@pytest.mark.parametrize("n,k", [(1500, 3), (3000, 15), (2000, 100), (1300, 1100)])
+def test_rows_that_list_the_same_points(oracle, n, k):
+    """Every row lists the same k - 1 other points at the same places, which the
+    entries' blocks count jointly: 1,024 entries are 342 rows, 69, 11 and part of one."""
+    idx = np.empty((n, k), dtype=np.uint32)
+    idx[:, 0] = np.arange(n)
+    idx[:, 1:] = np.arange(k - 1)
+    for r in range(k - 1):
+        idx[r, 1:] = [c for c in range(k) if c != r]
+    g = np.random.default_rng(k)
+    dist = np.sort(g.gamma(2.0, 1.0, (n, k)).astype(np.float32), axis=1)
+    dist[:, 0] = 0.0
+    dist[::3, k - 1] = np.float32(3e38)  # strength 0
+    check(oracle, idx.reshape(-1), dist.reshape(-1), f32(np.full(n, 0.7)), dist[:, 1].copy(), k)
+
+
+@pytest.mark.parametrize("hubs", [1, 40, 74, 75, 160])
+def test_hubs_shared_by_blocks(oracle, hubs):
+    """Points that 600 rows or more list, over more columns than one window: one hub
+    over all blocks, two blocks a hub with several windows each, and a block a hub (up
+    to 74 and from 75 on with 148 blocks); more hubs than blocks.  A hub's own
+    neighbours lie in every window, some listing it back, some with strength 0."""
+    n, k, per = 140_003, 13, 600
+    g = np.random.default_rng(hubs)
+    hub = (37 + np.arange(hubs) * (n // hubs)).astype(np.int64)
+    idx = (np.arange(n)[:, None] + np.arange(k)) % n  # itself and the next points
+    lists = [[] for _ in range(n)]
+    rows = g.permutation(n)
+    for h in range(hubs):
+        for r in rows[(h * per // 4 + np.arange(per)) % n]:  # about four hubs a row
+            lists[r].append(hub[h])
+    for h in hub:  # neighbours over the whole range, half of them listing the hub
+        away = g.choice(n, k - 1, replace=False)
+        lists[h] = [a for a in away if a != h]
+        for a in away[::2]:
+            lists[a].append(h)
+    for r, extra in enumerate(lists):
+        if extra:
+            extra = [c for c in dict.fromkeys(extra) if c != r][: k - 1]
+            rest = [c for c in idx[r, 1:] if c not in extra]
+            idx[r] = [r] + (extra + rest)[: k - 1]
+    dist = np.sort(g.gamma(2.0, 1.0, (n, k)).astype(np.float32), axis=1)
+    dist[:, 0] = 0.0
+    dist[::5, k // 2:] = np.float32(3e38)
+    dist[::5] = np.sort(dist[::5], axis=1)
+    out = check(oracle, idx.astype(np.uint32).reshape(-1), dist.reshape(-1), f32(np.full(n, 0.7)), dist[:, 1].copy(), k)
+    assert (np.bincount(out.rows, minlength=n)[hub] > 512 - k).all()
