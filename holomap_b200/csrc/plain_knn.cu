@@ -9,9 +9,8 @@
 // operations the reference performs: per dimension f64(x) - f64(y), square,
 // add to a running sum that starts at +0.0, in dimension order (euclidean), or
 // dot += f64(x) * f64(y) (cosine, whose per-row norm sums are precomputed in
-// the same order by prep), then sqrt / divide / cast.  Dimensions past d are
-// zero in the padded copy and add an exact +0.0, which leaves a sum that is
-// never -0.0 unchanged.
+// the same order by check_norms_kernel), then sqrt / divide / cast.  A stage's last
+// dimensions past d are loaded as zeros and left out of the loop.
 //
 // Layout: a CTA owns 32 query rows of one job (4 warps x 8 rows) and walks the
 // columns of its split 128 at a time; every lane computes an 8x4 block of pairs
@@ -167,18 +166,37 @@ __device__ __forceinline__ float pair_finish(double acc, double rn_a, double rn_
     }
 }
 
-// What a pair's accumulator has to reach for its distance to be at most the row's
-// k-th distance tau, with room for every rounding on the way: a returned distance
-// of at most tau comes from a value of at most up = tau (1 + 2^-21) + 1.5 * 2^-149.
-// Euclidean: acc <= up^2 (1 + 2^-50); manhattan: acc <= up; cosine: acc >=
-// (1 - up - 2^-44) |a| |b|, returned with |a| multiplied in (test it times |b|).
+// What a pair's accumulator has to reach for its returned distance to be at most
+// `dist`, with room for every rounding on the way: one of at most dist comes from a
+// value of at most up = dist (1 + 2^-21) + 1.5 * 2^-149.  Euclidean: acc <= up^2 (1 +
+// 2^-50); manhattan: acc <= up; cosine: acc >= (1 - up - 2^-44) |a| |b|, returned with
+// |a| multiplied in (test it times |b|).
 template <int METRIC>
-__device__ __forceinline__ double pair_limit(uint64_t tau_key, double rn_a) {
-    const float tau = tau_key == KEY_NONE ? __int_as_float(0x7f800000) : key_dist(tau_key);
-    const double up = (double)tau * (1.0 + 0x1p-21) + 1.5 * 0x1p-149;
+__device__ __forceinline__ double limit_of(double up, double rn_a) {
     if (METRIC == HM_METRIC_EUCLIDEAN) return up * up * (1.0 + 0x1p-50);
-    if (METRIC == HM_METRIC_COSINE) return fmax(1.0 - up - 0x1p-44, -1e30) * rn_a;
+    if (METRIC == HM_METRIC_COSINE) {
+        const double v = 1.0 - up - 0x1p-44;
+        return (v < -1e30 ? -1e30 : v) * rn_a;  // (a NaN stays one)
+    }
     return up;
+}
+template <int METRIC>
+__device__ __forceinline__ double pair_limit(float dist, double rn_a) {
+    return limit_of<METRIC>((double)dist * (1.0 + 0x1p-21) + 1.5 * 0x1p-149, rn_a);
+}
+// The limit of a row whose k-th key is tau_key.  The columns come in ascending order,
+// so a later pair at exactly the k-th distance stays behind it and only a smaller
+// distance counts, a value below the midpoint of tau and the next smaller binary32.
+// Ties are common where points repeat: at distance 0, as all pairs of a zero vector are
+// under cosine, every later pair would be merged for nothing (6,000 x 24, k = 15, 300
+// zero vectors: 1,755 us with ties let through, 1,310 without).  A row that nothing can
+// enter any more (tau 0) has the limit NaN, which no pair reaches; one with fewer than
+// k keys, or an infinite tau, takes every pair.
+template <int METRIC>
+__device__ __forceinline__ double next_limit(uint64_t tau_key, double rn_a) {
+    const uint32_t bits = min((uint32_t)(tau_key >> 32), 0x7f800000u);  // the distance's; KEY_NONE: infinity
+    const double below = (double)__uint_as_float(bits - 1u), tau = (double)__uint_as_float(bits);
+    return limit_of<METRIC>(0.5 * (below + tau) * (1.0 + 0x1p-50), rn_a);
 }
 
 // Shared memory of one CTA.
@@ -193,9 +211,10 @@ struct PlainSmem {
 };
 
 // Merges the first `have` (at most 32) waiting keys into the row's list; returns
-// its k-th key.
-template <int KPL>
-__device__ __noinline__ uint64_t plain_merge(uint64_t *list, const uint64_t *fresh, uint32_t have, uint32_t k) {
+// the row's new limit.
+template <int METRIC, int KPL>
+__device__ __noinline__ double plain_merge(uint64_t *list, const uint64_t *fresh, uint32_t have, uint32_t k,
+                                           double rn_a) {
     const int lane = threadIdx.x & 31;
     WarpTopK<KPL> top;
 #pragma unroll
@@ -205,7 +224,7 @@ __device__ __noinline__ uint64_t plain_merge(uint64_t *list, const uint64_t *fre
 #pragma unroll
     for (int q = 0; q < KPL; ++q) list[q * 32 + lane] = top.v[q];
     __syncwarp();
-    return top.tau;
+    return next_limit<METRIC>(top.tau, rn_a);
 }
 
 template <int METRIC, int KPL>
@@ -297,7 +316,10 @@ __global__ void __launch_bounds__(PL_THREADS, KPL <= 2 ? 3 : 2) plain_knn_kernel
         uint32_t have[8];  // waiting keys
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
-            limit[r] = pair_limit<METRIC>(KEY_NONE, sm.rn_a[warp * 8 + r]);
+            // (a place without a row takes no pairs, as if its tau were 0: its accumulators
+            // are some other row's, and under cosine a norm of 0 would let every pair
+            // through.  6,000 x 24 cosine, 16 such places: 911 us for the call, 388 now)
+            limit[r] = next_limit<METRIC>(sm.rows[warp * 8 + r] == 0xffffffffu ? 0ull : KEY_NONE, sm.rn_a[warp * 8 + r]);
             have[r] = 0;
         }
         fetch(c_begin, 0);
@@ -352,8 +374,8 @@ __global__ void __launch_bounds__(PL_THREADS, KPL <= 2 ? 3 : 2) plain_knn_kernel
                                 f = ((lane & stride) == 0) == ((lane & size) == 0) ? fminf(f, o) : fmaxf(f, o);
                             }
                         const double t = (double)__shfl_sync(0xffffffffu, f, (int)k - 1);
-                        const float dist = pair_finish<METRIC>(t, 0.0, 0.0);
-                        limit[r] = pair_limit<METRIC>(make_key(dist, 0), 0.0);
+                        if (sm.rows[warp * 8 + r] != 0xffffffffu)
+                            limit[r] = pair_limit<METRIC>(pair_finish<METRIC>(t, 0.0, 0.0), 0.0);
                     }
                 }
                 // pairs that may enter a row's list wait in `fresh`
@@ -384,8 +406,8 @@ __global__ void __launch_bounds__(PL_THREADS, KPL <= 2 ? 3 : 2) plain_knn_kernel
                         have[r] += __popc(m);
                         __syncwarp();
                         if (have[r] >= 32) {
-                            const uint64_t tau = plain_merge<KPL>(sm.list[warp * 8 + r], fresh, 32, k);
-                            limit[r] = pair_limit<METRIC>(tau, sm.rn_a[warp * 8 + r]);
+                            limit[r] = plain_merge<METRIC, KPL>(sm.list[warp * 8 + r], fresh, 32, k,
+                                                                sm.rn_a[warp * 8 + r]);
                             have[r] -= 32;
                             const uint64_t rest = fresh[32 + lane];
                             __syncwarp();
@@ -410,7 +432,7 @@ __global__ void __launch_bounds__(PL_THREADS, KPL <= 2 ? 3 : 2) plain_knn_kernel
             const uint32_t row = sm.rows[warp * 8 + r];
             if (row == 0xffffffffu) continue;
             uint64_t *list = sm.list[warp * 8 + r];
-            if (left) plain_merge<KPL>(list, sm.fresh[warp * 8 + r], left, k);
+            if (left) plain_merge<METRIC, KPL>(list, sm.fresh[warp * 8 + r], left, k, 0.0);
             for (uint32_t e = lane; e < k; e += 32) {
                 const uint64_t key = list[e];
                 if (J.splits > 1 && !w.fallback) {
