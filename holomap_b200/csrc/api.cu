@@ -525,10 +525,22 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
             B.kpl_fb[m] = std::max<uint32_t>(B.kpl_fb[m], (uint32_t)kpl_for_k(P.spec.k));
         }
     }
-    for (int m = 0; m < 3; ++m)
-        if (!B.fb_jobs[m].empty())
-            B.fb_per_job[m] = std::max<uint32_t>(
-                1, std::min<uint32_t>(64, (uint32_t)((2 * G + B.fb_jobs[m].size() - 1) / B.fb_jobs[m].size())));
+    // CTAs of the fallback launch, per job.  They share a job's row groups by columns
+    // where they outnumber them; a launch without any rows is what nearly every call
+    // has, and three CTAs an SM cost it 5 us (their shared memory has to be set up), one
+    // an SM nothing: 3,000 x 64 134 / 135 / 140 us with 64 / 148 / 444 of them.  A single
+    // large problem takes three, half a percent of its time at the line: 20,000 x 1,536
+    // with 18,391 such rows 773 ms with 64, 197 with 444; 10,000 x 768 with 7,389 66 and 25.
+    for (int m = 0; m < 3; ++m) {
+        if (B.fb_jobs[m].empty()) continue;
+        const uint64_t count = B.fb_jobs[m].size();
+        uint64_t most = 3 * G;
+        if (count == 1) {
+            const hm_job &s = B.jobs[B.fb_jobs[m][0]].spec;
+            if ((double)s.n * s.n * s.d < 0x1p36) most = G;
+        }
+        B.fb_per_job[m] = (uint32_t)std::max<uint64_t>(2, std::min<uint64_t>(most, (4 * G + count - 1) / count));
+    }
     // ---------------------------------------------------------- layout
     size_t off = 0;
     auto take = [&](size_t bytes) {
@@ -689,7 +701,9 @@ static int bind_batch(hm_batch &B, void *d_ws, size_t bytes, cudaStream_t s) {
         J.rnorm = at<double>(ws, P.off_rnorm);
         J.splits = P.splits;
         J.split_cols = P.split_cols;
-        J.partial = P.splits > 1 ? at<uint64_t>(ws, P.off_partial) : nullptr;
+        J.partial = P.splits > 1   ? at<uint64_t>(ws, P.off_partial)
+                    : P.group >= 0 ? at<uint64_t>(ws, B.groups[P.group].off_cand) + P.cand0
+                                   : nullptr;
         J.target = std::log2((double)s.k);  // src/smooth_knn.rs:25 (platform log2)
         J.zero_rows = at<uint32_t>(ws, P.off_zero_rows);
         J.group = P.group < 0 ? 0u : (uint32_t)P.group;

@@ -289,10 +289,11 @@ struct JobDev {
     // exact path (and the screened path's fallback)
     double *rnorm;               // sqrt of the sequential sum of squares (cosine)
     uint32_t splits, split_cols;
-    uint64_t *partial;           // splits x n x k keys (splits > 1)
+    uint64_t *partial;           // splits x n x k keys (splits > 1); a screened job: its candidate
+                                 // lists, elists * cap keys a row, for the fallback's parts
     // smooth-kNN
     double target;               // log2(k), host platform log2
-    uint32_t *zero_rows;         // n
+    uint32_t *zero_rows;         // n (before that: finished parts of each group of fallback rows)
     // screened path
     uint32_t group, row0, unit0, kp1, k_steps, k_stages, row_blocks, col_tiles, parts, part_tiles, cap;
     uint32_t seed_tiles;         // leading column tiles of each part in the threshold pass
@@ -362,10 +363,11 @@ constexpr int PL_BM = 32;     // rows per CTA (4 warps x 8 rows)
 constexpr int PL_BN = 128;    // columns per tile (32 lanes x 4)
 constexpr int PL_BK = 16;     // dimensions per shared-memory stage
 constexpr int PL_THREADS = 128;
+constexpr uint32_t FB_MAX_PARTS = 32;  // column parts of a group of fallback rows
 
 // Work of the exact path: items (job, group of PL_BM rows, column split); or,
-// in fallback mode, each job's overflow list strided over
-// `per_job` CTAs.
+// in fallback mode, each job's overflow list strided over `per_job` CTAs, which
+// share its groups by columns where they are few.
 struct PlainWork {
     const JobDev *jobs;
     uint32_t njobs;

@@ -208,6 +208,7 @@ struct PlainSmem {
     uint64_t fresh[PL_BM][64];       // keys waiting to be merged
     double rn_a[PL_BM];
     uint32_t rows[PL_BM];            // the query rows (0xffffffff: none)
+    uint32_t last;                   // fallback parts: this one finished last
 };
 
 // Merges the first `have` (at most 32) waiting keys into the row's list; returns
@@ -227,14 +228,53 @@ __device__ __noinline__ double plain_merge(uint64_t *list, const uint64_t *fresh
     return next_limit<METRIC>(top.tau, rn_a);
 }
 
-template <int METRIC, int KPL>
+// The part of a fallback group that finishes last merges the group's lists (its
+// counter: see select_row).
+template <int KPL>
+__device__ __noinline__ void merge_parts(const JobDev &J, PlainSmem<KPL> &sm, uint32_t grp, uint32_t parts) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t k = J.k;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) sm.last = atomicAdd(&J.zero_rows[grp], 1u) == parts - 1 ? 1u : 0u;
+    __syncthreads();
+    if (!sm.last) return;
+    __threadfence();
+#pragma unroll 1
+    for (int r = 0; r < 8; ++r) {
+        const uint32_t row = sm.rows[warp * 8 + r];
+        if (row == 0xffffffffu) continue;
+        const uint64_t *lists = J.partial + (size_t)row * J.elists * J.cap;
+        WarpTopK<KPL> top;
+        top.reset();
+        for (uint32_t p = 0; p < parts; ++p)
+            for (uint32_t e0 = 0; e0 < k; e0 += 32) {
+                uint64_t key = KEY_NONE;
+                if (e0 + lane < k) key = __ldcg(reinterpret_cast<const unsigned long long *>(lists) + p * k + e0 + lane);
+                if (!__any_sync(0xffffffffu, key < top.tau)) break;  // lists are sorted
+                top.template merge32<true>(key, k, lane);
+            }
+#pragma unroll
+        for (int q = 0; q < KPL; ++q) {
+            const uint32_t e = q * 32 + lane;
+            if (e < k) {
+                J.idx[(size_t)row * k + e] = key_idx(top.v[q]);
+                J.dist[(size_t)row * k + e] = key_dist(top.v[q]);
+            }
+        }
+    }
+}
+
+// FALLBACK: the rows are the jobs' overflow lists (a kernel of its own: with both forms
+// in one a 700 x 100 call took 68 us, 58 without the fallback's parts).
+template <int METRIC, int KPL, bool FALLBACK>
 __global__ void __launch_bounds__(PL_THREADS, KPL <= 2 ? 3 : 2) plain_knn_kernel(const PlainWork w) {
     extern __shared__ __align__(16) unsigned char pl_smem_raw[];
     PlainSmem<KPL> &sm = *reinterpret_cast<PlainSmem<KPL> *>(pl_smem_raw);
     grid_ready();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    uint32_t jb, first_grp, grp_stride, n_groups, split = 0;
-    if (!w.fallback) {
+    uint32_t jb, first_grp, grp_stride, n_groups, split = 0, parts = 1;
+    if (!FALLBACK) {
         uint32_t lo = 0, hi = w.njobs_m;  // the job whose items hold this block's
         while (hi - lo > 1) {
             const uint32_t mid = (lo + hi) >> 1;
@@ -251,9 +291,27 @@ __global__ void __launch_bounds__(PL_THREADS, KPL <= 2 ? 3 : 2) plain_knn_kernel
         first_grp = blockIdx.x % w.per_job;
         grp_stride = w.per_job;
         n_groups = (w.jobs[jb].cnt->ovf_count + PL_BM - 1) / PL_BM;
+        if (first_grp >= n_groups * FB_MAX_PARTS) return;
     }
     const JobDev &J = w.jobs[jb];
-    const uint32_t c_begin = split * J.split_cols, c_end = min(J.n, c_begin + J.split_cols);
+    uint32_t split_cols = J.split_cols;
+    if (FALLBACK && 2 * n_groups <= w.per_job) {
+        // fewer row groups than CTAs: several to a group, a part of the columns each,
+        // as many as the row's candidate lists (read for the last time by now) hold lists
+        const uint32_t tiles = (J.n + PL_BN - 1) / PL_BN;
+        parts = min(min(w.per_job / n_groups, FB_MAX_PARTS), min(tiles, J.elists * J.cap / J.k));
+        const uint32_t per = (tiles + parts - 1) / parts;
+        parts = (tiles + per - 1) / per;
+        split_cols = per * PL_BN;
+        split = first_grp % parts;
+        first_grp /= parts;
+        if (first_grp >= n_groups) return;
+        n_groups = first_grp + 1;
+    }
+    // (a loop the compiler knows to run once costs registers: addresses are hoisted out of
+    // it, and the accumulators spill)
+    asm volatile("" : "+r"(n_groups));
+    const uint32_t c_begin = split * split_cols, c_end = min(J.n, c_begin + split_cols);
     const uint32_t n = J.n, d = J.d, k = J.k;
     const float *__restrict__ x = J.x;
     const bool vec = (d & 3u) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
@@ -262,7 +320,7 @@ __global__ void __launch_bounds__(PL_THREADS, KPL <= 2 ? 3 : 2) plain_knn_kernel
     for (uint32_t grp = first_grp; grp < n_groups; grp += grp_stride) {
         if (tid < PL_BM) {
             uint32_t r;
-            if (w.fallback) {
+            if (FALLBACK) {
                 const uint32_t at = grp * PL_BM + tid;
                 r = at < J.cnt->ovf_count ? J.ovf_list[at] : 0xffffffffu;
             } else {
@@ -435,8 +493,10 @@ __global__ void __launch_bounds__(PL_THREADS, KPL <= 2 ? 3 : 2) plain_knn_kernel
             if (left) plain_merge<METRIC, KPL>(list, sm.fresh[warp * 8 + r], left, k, 0.0);
             for (uint32_t e = lane; e < k; e += 32) {
                 const uint64_t key = list[e];
-                if (J.splits > 1 && !w.fallback) {
+                if (!FALLBACK && J.splits > 1) {
                     J.partial[((size_t)split * n + row) * k + e] = key;
+                } else if (FALLBACK && parts > 1) {
+                    J.partial[(size_t)row * J.elists * J.cap + split * k + e] = key;
                 } else {
                     J.idx[(size_t)row * k + e] = key_idx(key);
                     J.dist[(size_t)row * k + e] = key_dist(key);
@@ -445,23 +505,34 @@ __global__ void __launch_bounds__(PL_THREADS, KPL <= 2 ? 3 : 2) plain_knn_kernel
         }
         __syncthreads();  // the rows and lists are rewritten by the next group
     }
+    if (FALLBACK && parts > 1) merge_parts<KPL>(J, sm, first_grp, parts);
 }
 
-template <int METRIC, int KPL>
+template <int METRIC, int KPL, bool FALLBACK>
 static int launch_plain_kernel(const PlainWork &w, uint32_t grid, cudaStream_t s) {
     const int smem = (int)sizeof(PlainSmem<KPL>);
-    HM_TRY(ensure_dynamic_smem((const void *)plain_knn_kernel<METRIC, KPL>, smem));
-    HM_CUDA_TRY(launch(true, plain_knn_kernel<METRIC, KPL>, grid, PL_THREADS, smem, s, w));
+    auto *kernel = plain_knn_kernel<METRIC, KPL, FALLBACK>;
+    HM_TRY(ensure_dynamic_smem((const void *)kernel, smem));
+    HM_CUDA_TRY(launch(true, kernel, grid, PL_THREADS, smem, s, w));
     count_launch();
     return HM_OK;
 }
 template <int METRIC>
 static int launch_plain_metric(const PlainWork &w, uint32_t grid, cudaStream_t s) {
     switch (w.kpl) {
-    case 1: return launch_plain_kernel<METRIC, 1>(w, grid, s);
-    case 2: return launch_plain_kernel<METRIC, 2>(w, grid, s);
-    case 4: return launch_plain_kernel<METRIC, 4>(w, grid, s);
-    case 8: return launch_plain_kernel<METRIC, 8>(w, grid, s);
+    case 1: return launch_plain_kernel<METRIC, 1, false>(w, grid, s);
+    case 2: return launch_plain_kernel<METRIC, 2, false>(w, grid, s);
+    case 4: return launch_plain_kernel<METRIC, 4, false>(w, grid, s);
+    case 8: return launch_plain_kernel<METRIC, 8, false>(w, grid, s);
+    default: return set_error(HM_ERR_UNSUPPORTED, "select width %u", w.kpl);
+    }
+}
+// (the screened paths take k up to 64, and not the manhattan metric)
+template <int METRIC>
+static int launch_fallback_metric(const PlainWork &w, uint32_t grid, cudaStream_t s) {
+    switch (w.kpl) {
+    case 1: return launch_plain_kernel<METRIC, 1, true>(w, grid, s);
+    case 2: return launch_plain_kernel<METRIC, 2, true>(w, grid, s);
     default: return set_error(HM_ERR_UNSUPPORTED, "select width %u", w.kpl);
     }
 }
@@ -472,6 +543,13 @@ int launch_plain(const PlainWork &w, int metric, cudaStream_t s) {
     const uint32_t grid = w.fallback ? w.fb_njobs * w.per_job : w.nitems;
     if (grid == 0) return HM_OK;
     ScopedKernelTimer timer(HM_KCLASS_EXACT, s);
+    if (w.fallback) {
+        switch (metric) {
+        case HM_METRIC_EUCLIDEAN: return launch_fallback_metric<HM_METRIC_EUCLIDEAN>(w, grid, s);
+        case HM_METRIC_COSINE: return launch_fallback_metric<HM_METRIC_COSINE>(w, grid, s);
+        default: return set_error(HM_ERR_INVALID, "no fallback for metric %d", metric);
+        }
+    }
     switch (metric) {
     case HM_METRIC_EUCLIDEAN: return launch_plain_metric<HM_METRIC_EUCLIDEAN>(w, grid, s);
     case HM_METRIC_COSINE: return launch_plain_metric<HM_METRIC_COSINE>(w, grid, s);

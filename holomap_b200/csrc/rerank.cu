@@ -311,6 +311,7 @@ __device__ __forceinline__ uint32_t select_row(const JobDev &J, const GroupDev &
         if (lane == 0) {
             const uint32_t at = atomicAdd(&J.out->ovf_count, 1u);
             J.ovf_list[at] = row;
+            if (at % PL_BM == 0) J.zero_rows[at / PL_BM] = 0;  // the fallback counts a group's parts there
         }
         return 0;
     }

@@ -412,3 +412,53 @@ def test_clustered_rows_do_not_overflow_their_lists(d, n, k, metric):
     p.run(x)
     torch.cuda.synchronize()
     assert p.stats().overflow_rows == 0
+
+
+@pytest.mark.parametrize("path", ["screen_bf16", "screen_bf16x3"])
+@pytest.mark.parametrize("n,centres,k", [(6000, 1, 15), (6000, 14, 15), (20000, 31, 64), (20000, 33, 64), (20000, 60, 64)])
+def test_fallback_rows_shared_by_columns(path, n, centres, k):
+    """A few rows whose neighbours all lie at one distance (centres of a sphere of points)
+    overflow their lists and take the exact search, several CTAs to a group of 32 rows:
+    one group and two, one row and one short of a group, k of one list and of two."""
+    import torch
+    from holomap_b200.device import DeviceKnnProblem
+    g = np.random.default_rng(n + centres)
+    d = 48
+    x = g.normal(size=(n, d))
+    x /= np.linalg.norm(x, axis=1, keepdims=True)  # (the radii differ by the points' rounding)
+    x[g.permutation(n)[:centres]] = 1e-6 * g.normal(size=(centres, d))
+    x = torch.from_numpy(x.astype(np.float32)).cuda()
+    want = DeviceKnnProblem(n, d, k, "euclidean", "plain")
+    want.run(x)
+    p = DeviceKnnProblem(n, d, k, "euclidean", path)
+    for _ in range(2):  # (the second run finds the first one's counters)
+        p.idx.fill_(-1)
+        p.run(x)
+        torch.cuda.synchronize()
+        assert p.stats().overflow_rows >= centres
+        assert torch.equal(p.idx, want.idx) and torch.equal(p.dist, want.dist)
+
+
+@pytest.mark.parametrize("tight", [4000, 8200])  # 125 row groups: 3 CTAs each; 257: one each
+def test_fallback_rows_of_a_tight_cluster(tight):
+    """Thousands of rows in a cluster tighter than the screen's rounding, all of them
+    searched exactly; as one job and in a batch of three."""
+    import torch
+    from holomap_b200.device import DeviceBatch, DeviceKnnProblem
+    g = np.random.default_rng(tight)
+    n, d, k = tight + 800, 24, 20
+    x = g.normal(size=(n, d))
+    x[g.permutation(n)[:tight]] *= 1e-4
+    x = torch.from_numpy(x.astype(np.float32)).cuda()
+    want = DeviceKnnProblem(n, d, k, "euclidean", "plain")
+    want.run(x)
+    p = DeviceKnnProblem(n, d, k, "euclidean", "screen_bf16")
+    p.run(x)
+    small = x[:500].contiguous()
+    b = DeviceBatch([(small, k, "cosine", "screen_bf16"), (x, k, "euclidean", "screen_bf16"),
+                     (small, 7, "euclidean", "screen_bf16")])
+    b.run()
+    torch.cuda.synchronize()
+    assert p.stats().overflow_rows >= tight
+    for idx, dist in ((p.idx, p.dist), b.problems[1][1:3]):
+        assert torch.equal(idx, want.idx) and torch.equal(dist, want.dist)
