@@ -191,27 +191,33 @@ static size_t plain_room_bytes(const hm_job &s, uint64_t groups) {
     return plain_copy_bytes(s) + split_lists_bytes(s, c);
 }
 
-// Column splits of one exact-path job: the waves of resident CTAs times a split's
-// instructions per warp (8 rows: the tiles' arithmetic and the filling of the
-// rows' lists, k (1 + ln(columns / k)) keys in merges of 32), least over the
-// splits.  More splits even out the last wave, fewer fill fewer lists: 12,007 x 64
-// manhattan, k = 15 (376 row groups, 444 CTAs resident) 1,565 us with the 7 it
-// chooses, 1,602 with 4; 1,000 points take one per 128-column tile.
-// (Lists take the room of a problem's scratch and no more: plain_room_bytes.)
+// Column splits of one exact-path job, least time over the splits.  A split's item costs
+// a warp (8 rows) the pairs' binary64 operations and, beside them, the tiles' other
+// instructions and the filling of the rows' lists (k (1 + ln(columns / k)) keys in merges
+// of 32).  Four fifths of the former keep the SM's binary64 pipe busy whichever CTA they
+// come from: they add up over the items an SM gets (one alone reaches 1 / 1.2 of a
+// third of its rate).  The rest is latency, one item's for each wave of resident CTAs.
+// More splits even out both, fewer fill fewer lists.  2,000 x 300, k = 15: 305 us with
+// the 16 it chooses, 384 with the 6 that fill one wave; 20,000 x 32 cosine: 2,510 with 2,
+// 2,754 with 3.  (179 shapes, metrics and k: 0.7 % over the best split on average; a
+// count of waves alone 2.4 %, 32 % at worst.)  Lists take the room of a problem's scratch
+// and no more: plain_room_bytes.
 static uint32_t plain_splits(const JobPlan &P, uint64_t groups, uint32_t sms) {
     const hm_job &s = P.spec;
     const uint32_t tiles = (uint32_t)((s.n + PL_BN - 1) / PL_BN);
     const int kpl = kpl_for_k(s.k);
-    const double resident = (double)sms * (kpl <= 2 ? 3 : kpl == 4 ? 2 : 1);
+    const double resident = kpl <= 2 ? 3 : kpl == 4 ? 2 : 1;  // CTAs an SM holds
     const double ops = s.metric == HM_METRIC_EUCLIDEAN ? 3 : s.metric == HM_METRIC_MANHATTAN ? 2 : 1;
-    const double tile = s.d * (32 * ops + 12) + 400, merge = 150 + 70 * kpl;
+    const double pairs = 32.0 * ops * s.d, other = 8.0 * s.d + 640, merge = 150 + 70 * kpl;
     double best = 1e300;
     uint32_t splits = 1;
     for (uint32_t c = 1; c <= std::min<uint32_t>(32, tiles); ++c) {
-        const double per = std::ceil((double)tiles / c), cols = per * PL_BN;
-        const double lists = 8 * merge * (1 + s.k / 32.0 * (1 + std::log(std::max(1.0, cols / s.k))));
         if (split_lists_bytes(s, c) > plain_room_bytes(s, groups)) continue;
-        const double cost = std::ceil(groups * (double)c / resident) * (per * tile + lists) + 40.0 * c;
+        const double per = std::ceil((double)tiles / c), cols = per * PL_BN, items = groups * (double)c;
+        const double lists = 8 * merge * (1 + s.k / 32.0 * (1 + std::log(std::max(1.0, cols / s.k))));
+        const double pipe = std::max(std::ceil(items / sms), 1.2) / resident * 0.8 * per * pairs;
+        const double waves = std::ceil(items / (sms * resident));
+        const double cost = pipe + waves * (per * (0.2 * pairs + other) + lists) + 25.0 * c;
         if (cost < best * 0.999) {
             best = cost;
             splits = c;
