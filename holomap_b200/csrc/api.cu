@@ -404,13 +404,19 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
             Gp.units += P.row_blocks * P.parts;
             // the threshold pass's chunks: as few columns each as leave at most
             // 128, 256 or 512 minima a row (by k: the k smallest values of a row
-            // then rarely share a chunk, which loosens the bound); chunks of
-            // more than 64 columns take several tiles of a part
+            // then rarely share a chunk, which loosens the bound), but no more than 32 in
+            // a sample: points stored cluster by cluster have their neighbours side by
+            // side, and a row needs k chunks of its own cluster (rows of 20,000 x 64 in 12
+            // clusters, k = 15: 52 candidates a row at 32 columns, 1,665 at 64, more than
+            // the lists hold); chunks of more than 64 columns take several tiles of a part
             // (and no more scratch than sorted lists of each part's two halves and a
             // row's binary64 copy took)
-            const uint32_t limit = std::min<uint32_t>(P.spec.k <= 20 ? 128 : P.spec.k <= 40 ? 256 : TH_MAX_MINIMA,
-                                                      2 * P.parts * P.spec.k + 2 * (uint32_t)round_up(P.spec.d, 16));
             const uint32_t last = std::min(P.seed_tiles, P.col_tiles - (P.parts - 1) * P.part_tiles);
+            const uint32_t sampled = P.seed_tiles < P.part_tiles ? (P.parts - 1) * P.seed_tiles + last : 0u;
+            const uint32_t limit = std::min<uint32_t>(
+                std::max(P.spec.k <= 20 ? 128u : P.spec.k <= 40 ? 256u : TH_MAX_MINIMA,
+                         std::min(sampled * (SC_BN / 32), TH_MAX_MINIMA)),
+                2 * P.parts * P.spec.k + 2 * (uint32_t)round_up(P.spec.d, 16));
             for (P.min_shift = 0;; ++P.min_shift) {
                 const uint32_t ti = P.min_shift > 4 ? P.min_shift - 4 : 0, per = P.min_shift > 4 ? 4 : 64u >> P.min_shift;
                 auto chunks = [&](uint32_t tiles) { return ((tiles + (1u << ti) - 1) >> ti) * per; };
@@ -531,21 +537,16 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
             B.kpl_fb[m] = std::max<uint32_t>(B.kpl_fb[m], (uint32_t)kpl_for_k(P.spec.k));
         }
     }
-    // CTAs of the fallback launch, per job.  They share a job's row groups by columns
-    // where they outnumber them; a launch without any rows is what nearly every call
-    // has, and three CTAs an SM cost it 5 us (their shared memory has to be set up), one
-    // an SM nothing: 3,000 x 64 134 / 135 / 140 us with 64 / 148 / 444 of them.  A single
-    // large problem takes three, half a percent of its time at the line: 20,000 x 1,536
-    // with 18,391 such rows 773 ms with 64, 197 with 444; 10,000 x 768 with 7,389 66 and 25.
+    // CTAs of the fallback launch, per job: what three an SM hold, shared by a batch's
+    // jobs.  They share a job's row groups by columns where they outnumber them.  Nearly
+    // every call has no such rows, and then each CTA leaves after one load
+    // (PlainWork::ovf; after three dependent ones, 444 CTAs cost a call 5 us more than
+    // 64).  20,000 x 1,536 with 18,391 such rows 773 ms with 64 CTAs, 197 with 444;
+    // 20,000 x 64 with 11,655 14.1 with 148, 5.2 with 444.
     for (int m = 0; m < 3; ++m) {
         if (B.fb_jobs[m].empty()) continue;
         const uint64_t count = B.fb_jobs[m].size();
-        uint64_t most = 3 * G;
-        if (count == 1) {
-            const hm_job &s = B.jobs[B.fb_jobs[m][0]].spec;
-            if ((double)s.n * s.n * s.d < 0x1p36) most = G;
-        }
-        B.fb_per_job[m] = (uint32_t)std::max<uint64_t>(2, std::min<uint64_t>(most, (4 * G + count - 1) / count));
+        B.fb_per_job[m] = (uint32_t)std::max<uint64_t>(2, std::min<uint64_t>(3 * G, (4 * G + count - 1) / count));
     }
     // ---------------------------------------------------------- layout
     size_t off = 0;
@@ -898,6 +899,7 @@ static int run_batch(hm_batch &B, cudaStream_t s) {
             w.per_job = B.fb_per_job[m];
             w.fb_jobs = at<uint32_t>(ws, B.off_fb[m]);
             w.fb_njobs = (uint32_t)B.fb_jobs[m].size();
+            if (w.fb_njobs == 1) w.ovf = &(at<JobCounters>(ws, B.off_counters) + B.fb_jobs[m][0])->ovf_count;
             HM_TRY(launch_plain(w, m, s));
         }
     }

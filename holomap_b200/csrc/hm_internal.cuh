@@ -377,6 +377,8 @@ struct PlainWork {
     uint32_t kpl;           // WarpTopK width for the largest k
     uint32_t fallback;      // 1: rows come from the jobs' overflow lists
     uint32_t per_job;       // fallback: CTAs per job
+    const uint32_t *ovf;    // fallback of one job: its count of rows, so that a CTA without any leaves
+                            // after one load (null: several jobs)
     const uint32_t *fb_jobs;  // fallback: the jobs that may have overflow rows
     uint32_t fb_njobs;
 };

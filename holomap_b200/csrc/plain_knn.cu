@@ -272,6 +272,7 @@ __global__ void __launch_bounds__(PL_THREADS, KPL <= 2 ? 3 : 2) plain_knn_kernel
     extern __shared__ __align__(16) unsigned char pl_smem_raw[];
     PlainSmem<KPL> &sm = *reinterpret_cast<PlainSmem<KPL> *>(pl_smem_raw);
     grid_ready();
+    if (FALLBACK && w.ovf && blockIdx.x >= (*w.ovf + PL_BM - 1) / PL_BM * FB_MAX_PARTS) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint32_t jb, first_grp, grp_stride, n_groups, split = 0, parts = 1;
     if (!FALLBACK) {

@@ -119,11 +119,18 @@ __device__ __forceinline__ uint32_t kth_load(KeyFn key, uint32_t total, uint32_t
         ov[q] = e < total ? key(e) : 0xffffffffu;
     }
     uint32_t kth;
-    if (NQ == 4) {
-        // of each lane's four keys the two smallest: a bound of the k-th, and the
-        // k-th itself unless a lane holds three of the k smallest
-        const uint32_t a = min(ov[0], ov[1]), b = max(ov[0], ov[1]), c = min(ov[2], ov[3]), d = max(ov[2], ov[3]);
-        uint32_t two[2] = {min(a, c), min(max(a, c), min(b, d))};
+    if (NQ == 4 || (NQ == 8 && k <= 32)) {
+        // of each lane's keys the two smallest: a bound of the k-th, and the k-th itself
+        // unless a lane holds three of the k smallest (50,000 x 64, k = 15, 200 minima a row:
+        // 1,519 us for the call, 1,526 with the search by bits)
+        uint32_t two[2] = {0xffffffffu, 0xffffffffu};
+#pragma unroll
+        for (int q = 0; q < NQ; q += 2) {
+            const uint32_t a = min(ov[q], ov[q + 1]), b = max(ov[q], ov[q + 1]);
+            const uint32_t hi = max(two[0], a);
+            two[0] = min(two[0], a);
+            two[1] = min(hi, min(two[1], b));
+        }
         kth = kth_sorted<2>(two, k, lane);
     } else if (NQ < 4) {
         kth = kth_sorted<NQ>(ov, k, lane);

@@ -462,3 +462,28 @@ def test_fallback_rows_of_a_tight_cluster(tight):
     assert p.stats().overflow_rows >= tight
     for idx, dist in ((p.idx, p.dist), b.problems[1][1:3]):
         assert torch.equal(idx, want.idx) and torch.equal(dist, want.dist)
+
+
+@pytest.mark.parametrize("path", ["screen_bf16x3", "screen_tf32"])
+@pytest.mark.parametrize("begin,end", [(1005, 1105), (7005, 7105), (11005, 11105)])
+def test_rows_of_points_stored_cluster_by_cluster(path, begin, end):
+    """A row's neighbours lie side by side, and its bound needs k chunks of the sample
+    from its own cluster: with chunks of 64 columns the rows' lists overflowed."""
+    import ctypes
+    import torch
+    from holomap_b200._lib import check as check_rc
+    g = np.random.default_rng(3)
+    n, d, k = 20000, 64, 15
+    x = 4.0 * g.normal(size=(12, d))[np.sort(g.integers(0, 12, n))] + g.normal(size=(n, d))
+    x = torch.from_numpy(x.astype(np.float32)).cuda()
+    p = int(hm.KnnPath.parse(path))
+    ws_bytes = hm.lib().hm_knn_rows_workspace_bytes(n, d, k, 0, p, begin, end)
+    ws = torch.empty(ws_bytes + 256, dtype=torch.uint8, device="cuda")
+    idx = torch.empty((end - begin) * k, dtype=torch.int32, device="cuda")
+    dist = torch.empty((end - begin) * k, dtype=torch.float32, device="cuda")
+    st = hm.HmStats()
+    ptr = (ws.data_ptr() + 255) // 256 * 256
+    check_rc(hm.lib().hm_knn_rows_device(x.data_ptr(), n, d, k, 0, p, begin, end, idx.data_ptr(), dist.data_ptr(),
+                                         ptr, ws_bytes, None, ctypes.byref(st)))
+    torch.cuda.synchronize()
+    assert st.overflow_rows == 0
