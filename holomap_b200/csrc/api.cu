@@ -173,10 +173,11 @@ static int group_of_path(int path) {
     }
 }
 
-// Bytes of the split lists of an exact-path job cut c ways (whole column tiles).
-static size_t split_lists_bytes(const hm_job &s, uint64_t c) {
+// Bytes of the split lists of `rows` rows of an exact-path job cut c ways (whole column
+// tiles).
+static size_t split_lists_bytes(const hm_job &s, uint64_t c, uint64_t rows) {
     const uint64_t tiles = (s.n + PL_BN - 1) / PL_BN, per = (tiles + c - 1) / c, splits = (tiles + per - 1) / per;
-    return splits > 1 ? align256((size_t)splits * s.n * s.k * sizeof(uint64_t)) : 0;
+    return splits > 1 ? align256((size_t)splits * rows * s.k * sizeof(uint64_t)) : 0;
 }
 static size_t plain_copy_bytes(const hm_job &s) {
     return align256((round_up(s.n, 128) + 128) * round_up(s.d, 16) * sizeof(double));
@@ -188,7 +189,7 @@ static size_t plain_copy_bytes(const hm_job &s) {
 static size_t plain_room_bytes(const hm_job &s, uint64_t groups) {
     const uint64_t tiles = (s.n + PL_BN - 1) / PL_BN;
     const uint64_t c = std::min<uint64_t>(std::min<uint64_t>(std::max<uint64_t>((1184 + groups - 1) / groups, 1), 32), tiles);
-    return plain_copy_bytes(s) + split_lists_bytes(s, c);
+    return plain_copy_bytes(s) + split_lists_bytes(s, c, s.n);
 }
 
 // Column splits of one exact-path job, least time over the splits.  A split's item costs
@@ -211,8 +212,11 @@ static uint32_t plain_splits(const JobPlan &P, uint64_t groups, uint32_t sms) {
     const double pairs = 32.0 * ops * s.d, other = 8.0 * s.d + 640, merge = 150 + 70 * kpl;
     double best = 1e300;
     uint32_t splits = 1;
-    for (uint32_t c = 1; c <= std::min<uint32_t>(32, tiles); ++c) {
-        if (split_lists_bytes(s, c) > plain_room_bytes(s, groups)) continue;
+    // (32 at most, but a shard of few rows may take what fills the SMs: 100 rows of
+    // 20,000 x 64 146 us with 32, 122 with 79)
+    const uint32_t most = std::max<uint32_t>(32, (uint32_t)(resident * sms / (double)groups));
+    for (uint32_t c = 1; c <= std::min<uint32_t>(most, tiles); ++c) {
+        if (split_lists_bytes(s, c, P.q1 - P.q0) > plain_room_bytes(s, groups)) continue;
         const double per = std::ceil((double)tiles / c), cols = per * PL_BN, items = groups * (double)c;
         const double lists = 8 * merge * (1 + s.k / 32.0 * (1 + std::log(std::max(1.0, cols / s.k))));
         const double pipe = std::max(std::ceil(items / sms), 1.2) / resident * 0.8 * per * pairs;
@@ -527,7 +531,7 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
             B.nitems[m] += groups * P.splits;
             if (P.splits > 1) {
                 B.merges.push_back(make_uint2(j, B.merge_rows));
-                B.merge_rows += (uint32_t)P.spec.n;
+                B.merge_rows += P.q1 - P.q0;
             }
             B.kpl_plain[m] = std::max<uint32_t>(B.kpl_plain[m], (uint32_t)kpl_for_k(P.spec.k));
         } else if (P.clone_of < 0) {
@@ -601,7 +605,7 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
         // (a batch's splits are eight items per SM, so its jobs' room is the same)
         if (P.path == HM_PATH_PLAIN)
             P.off_partial = take(njobs == 1 ? plain_room_bytes(P.spec, (P.q1 + PL_BM - 1) / PL_BM - P.q0 / PL_BM)
-                                            : plain_copy_bytes(P.spec) + split_lists_bytes(P.spec, P.splits));
+                                            : plain_copy_bytes(P.spec) + split_lists_bytes(P.spec, P.splits, P.spec.n));
         P.off_rnorm = take(n * sizeof(double));
         P.off_zero_rows = take(n * sizeof(uint32_t));
         if (P.group >= 0) {

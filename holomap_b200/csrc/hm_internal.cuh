@@ -289,7 +289,7 @@ struct JobDev {
     // exact path (and the screened path's fallback)
     double *rnorm;               // sqrt of the sequential sum of squares (cosine)
     uint32_t splits, split_cols;
-    uint64_t *partial;           // splits x n x k keys (splits > 1); a screened job: its candidate
+    uint64_t *partial;           // splits x (q1 - q0) x k keys (splits > 1); a screened job: its candidate
                                  // lists, elists * cap keys a row, for the fallback's parts
     // smooth-kNN
     double target;               // log2(k), host platform log2

@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(PL_THREADS, KPL <= 2 ? 3 : 2) plain_knn_kernel
             for (uint32_t e = lane; e < k; e += 32) {
                 const uint64_t key = list[e];
                 if (!FALLBACK && J.splits > 1) {
-                    J.partial[((size_t)split * n + row) * k + e] = key;
+                    J.partial[((size_t)split * (J.q1 - J.q0) + (row - J.q0)) * k + e] = key;
                 } else if (FALLBACK && parts > 1) {
                     J.partial[(size_t)row * J.elists * J.cap + split * k + e] = key;
                 } else {
@@ -575,17 +575,16 @@ __global__ void __launch_bounds__(256) merge_splits_kernel(const JobDev *__restr
         if (merges[mid].y <= mr) lo = mid; else hi = mid;
     }
     const JobDev &J = jobs[merges[lo].x];
-    const uint32_t row = mr - merges[lo].y, k = J.k;
-    if (row < J.q0 || row >= J.q1) return;
+    const uint32_t at = mr - merges[lo].y, row = J.q0 + at, rows_j = J.q1 - J.q0, k = J.k;
     WarpTopK<KPL> top;
 #pragma unroll
     for (int q = 0; q < KPL; ++q) {
         const uint32_t e = q * 32 + lane;
-        top.v[q] = (e < k) ? J.partial[(size_t)row * k + e] : KEY_NONE;
+        top.v[q] = (e < k) ? J.partial[(size_t)at * k + e] : KEY_NONE;
     }
     top.refresh_tau(k, lane);
     for (uint32_t sp = 1; sp < J.splits; ++sp) {
-        const uint64_t *list = J.partial + ((size_t)sp * J.n + row) * k;
+        const uint64_t *list = J.partial + ((size_t)sp * rows_j + at) * k;
         for (uint32_t e0 = 0; e0 < k; e0 += 32) {
             const uint64_t key = (e0 + lane < k) ? list[e0 + lane] : KEY_NONE;
             if (!__any_sync(0xffffffffu, key < top.tau)) break;  // lists are sorted

@@ -99,3 +99,21 @@ def test_row_ranges_of_an_escalating_job():
         torch.cuda.synchronize()
         assert_same_bytes(idx.cpu().numpy().view(np.uint32), pi[b:e], f"rows [{b},{e}) indices")
         assert_same_bytes(dist.cpu().numpy(), pd[b:e], f"rows [{b},{e}) dists")
+
+
+@pytest.mark.parametrize("metric", ["euclidean", "cosine", "manhattan"])
+@pytest.mark.parametrize("k", [15, 100])
+def test_shards_of_few_rows_take_many_splits(metric, k):
+    """Shards whose row groups are fewer than the SMs are cut into more than 32 column
+    splits (71 column tiles here), whose lists hold the shard's rows alone."""
+    import torch
+    from holomap_b200.device import DeviceKnnProblem
+    from holomap_b200.shard import rows_cuda
+    n, d = 9001, 12
+    x = torch.from_numpy(edge_case("gauss", n, d, seed=k)).cuda()
+    whole = DeviceKnnProblem(n, d, k, metric, "plain")
+    whole.run(x)
+    for b, e in [(100, 101), (5, 37), (4000, 4130), (n - 1, n)]:
+        idx, dist = rows_cuda(x, k, metric, "plain", b, e)
+        torch.cuda.synchronize()
+        assert torch.equal(idx, whole.idx.view(n, k)[b:e]) and torch.equal(dist, whole.dist.view(n, k)[b:e])
