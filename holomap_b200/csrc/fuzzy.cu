@@ -19,7 +19,7 @@
 //      (v + vt) - v * vt of equal columns in the reference's order
 //      (src/fuzzy.rs:67-75) and leaves the sorted row at the front of its
 //      segment; fuzzy_long_kernel does the rows above 128 slots: a warp each up
-//      to 512, a block each beyond.
+//      to 512, a block each beyond, several to one of very many arrivals.
 //   5. fuzzy_write_kernel (one block per tile of rows, several per very long row)
 //      sums the tiles before it, scans its rows' counts and writes the COO.
 //
@@ -33,8 +33,8 @@
 //
 // What bounds it: latency of the L2-resident arrays and the sorts' issue.  With a
 // radix sort of the reverse copies and binary-search merges -> now: kNN graph of
-// 50,000 x 384 embeddings, k = 30 (2.7 M entries) 180 -> 117 us; random graphs of
-// 50,000 x 15 140 -> 76, 2,000 x 15 62 -> 42, 1,000,000 x 15 2133 -> 1274.
+// 50,000 x 384 embeddings, k = 30 (2.7 M entries) 183 -> 110 us; random graphs of
+// 100,000 x 15 250 -> 104, 2,000 x 15 60 -> 28.
 #include <cuda_runtime.h>
 
 #include <algorithm>

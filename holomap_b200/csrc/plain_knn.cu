@@ -25,8 +25,8 @@
 // euclidean, 2 manhattan, 1 cosine: the product of two widened binary32 values is
 // exact, so the reference's multiply and add are one fused operation).
 // Whole calls, with every key inserted one at a time and a separate binary64 copy
-// of the points -> now: 1,000 x 50, k = 15 89 -> 65 us; 12,007 x 64 manhattan 1,744
-// -> 1,631 us (0.64 of the binary64 rate); 10,000 x 32, k = 100 4,080 -> 1,766 us.
+// of the points -> now: 1,000 x 50, k = 15 89 -> 58 us; 12,007 x 64 manhattan 1,744
+// -> 1,596 us (0.65 of the binary64 rate); 10,000 x 32, k = 100 4,080 -> 1,672 us.
 // Registers limit it to 12 warps an SM; 16 (128 registers, spills) measured 2,489
 // us on the manhattan call, an unroll of 8 or 16 dimensions 1,668 and 1,875.
 #include <cuda_runtime.h>

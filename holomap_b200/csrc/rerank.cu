@@ -1,13 +1,14 @@
 // rerank.cu -- the row threshold between the two screen passes, and the
 // exact rerank of the screen's candidates.
 //
-// threshold: one warp per row merges the k smallest mini-chunk minima of the
-// row's lists into tau1, the k-th smallest of their union rounded up to 2^-13
-// of its binade.  Every mini-chunk minimum is a screened value of the row, so
-// at least k screened values are <= tau1 and the row's k-th smallest screened
-// value tau^ <= tau1.
+// threshold: the threshold pass left the smallest screened value of each chunk of
+// the sampled columns, chunk-major; a block transposes those of 8 rows through shared
+// memory, and a warp each takes the k-th smallest of a row's, or a value slightly above
+// it (kth_load), as tau1.  Every chunk minimum is a screened value of the row, so at
+// least k screened values are <= tau1 and the row's k-th smallest screened value tau^
+// <= tau1.
 //
-// rerank: one warp per 2 or 4 consecutive group rows (always of one job: each
+// rerank: one warp per 2, 4 or 8 consecutive group rows (always of one job: each
 // job's rows start 32-aligned in the group) in the second of three phases.
 //   1. select, per row: tau^ is recomputed as the k-th smallest screened
 //      value among the emitted candidates (the emission pass wrote every

@@ -176,9 +176,6 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
                      : "memory");
 }
 
-// tcgen05.ld of 32 consecutive accumulator columns of this warp's 32 lanes;
-// the registers are valid only after tmem_ld_wait16 on the same array (the
-// wait names them as in/out operands so no use can be scheduled before it).
 // (w0, w1) += (c0, c1) * h, each rounded once
 __device__ __forceinline__ void fma2(float &w0, float &w1, float c0, float c1, float h) {
     asm("{\n\t.reg .b64 w, c, h;\n\t"
@@ -187,6 +184,9 @@ __device__ __forceinline__ void fma2(float &w0, float &w1, float c0, float c1, f
         : "+f"(w0), "+f"(w1)
         : "f"(c0), "f"(c1), "f"(h));
 }
+// tcgen05.ld of 16 consecutive accumulator columns of this warp's 32 lanes;
+// the registers are valid only after tmem_ld_wait16 on the same array (the
+// wait names them as in/out operands so no use can be scheduled before it).
 __device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&v)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32"
@@ -688,8 +688,8 @@ __global__ void __launch_bounds__(SC_THREADS, 1)
                         }
                     }
                 } else {
-                    // the full emission pass (96 registers a thread): 16-column
-                    // loads, the next in flight while this one is tested
+                    // the emission passes (at most 96 registers a thread, so that 16
+                    // epilogue warps fit): 16 columns loaded and tested at a time
                     const uint32_t cap = J.cap;
                     // symmetric emission, column side, on the raw products:
                     // column j of the chunk takes this row as a candidate when

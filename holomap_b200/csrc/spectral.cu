@@ -23,10 +23,12 @@
 // largest first, explicit residual ||B x - theta x|| < 1e-10 to lock, restart
 // from the best unconverged Ritz vector, 200 cycles at most, and the
 // canonical sign of each vector.  Where the device differs in operation order
-// (dot products as fixed two-stage tree reductions; classical Gram-Schmidt,
-// applied twice, in place of the modified form; the implicit QL method for
-// the tridiagonal in place of nalgebra's SymmetricEigen) the eigenpairs agree
-// with the reference to its own tolerances rather than bit for bit.  Every
+// (dot products as fixed two-stage tree reductions; the products L x inside a
+// cycle as two chains a lane and a tree per row instead of column order; beta from
+// the second orthogonalisation pass's sums; classical Gram-Schmidt, applied twice,
+// in place of the modified form; the implicit QL method for the tridiagonal in
+// place of nalgebra's SymmetricEigen) the eigenpairs agree with the reference to
+// its own tolerances rather than bit for bit.  Every
 // reduction has a fixed order, so a graph gives the same bits on every run
 // (src/eigen.rs:337-344 asks that of the reference).  The reference uses a
 // dense eigensolver when n <= 2000 (src/eigen.rs:31-37); this build runs the

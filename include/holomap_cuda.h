@@ -168,10 +168,12 @@ HM_API int hm_smooth_knn_rows_device(const float *d_dists, uint64_t n, uint32_t 
  * bound).  Capacity of rows / cols / vals: 2 n k entries; *nnz receives the
  * count.  n k must stay below 2^31.
  *
- * hm_fuzzy_graph: host buffers in and out (device memory from the stream-ordered
- * pool, the calling thread's own stream, synchronous).
+ * hm_fuzzy_graph: host buffers in and out (device memory up to 256 MiB from the
+ * stream-ordered pool, above that allocated for the call; the calling thread's own
+ * stream; synchronous).
  * hm_fuzzy_graph_device: device pointers; d_nnz is a device uint64; the
- * workspace (hm_fuzzy_workspace_bytes, 256-byte aligned) holds the rows'
+ * workspace (hm_fuzzy_workspace_bytes: 36 bytes an entry and about 20 a row,
+ * 256-byte aligned) holds the rows'
  * segments; ordered on `stream`, nothing synchronised. */
 HM_API size_t hm_fuzzy_workspace_bytes(uint64_t n, uint32_t k);
 HM_API int hm_fuzzy_graph_device(const uint32_t *d_idx, const float *d_dist, const float *d_sigma,
