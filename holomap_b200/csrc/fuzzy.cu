@@ -119,15 +119,7 @@ __global__ void __launch_bounds__(256) fuzzy_entries_kernel(const FuzzyDev D) {
         d[q] = __fsub_rn(D.dist[e], D.rho[row[q]]);
         sg[q] = D.sigma[row[q]];
     }
-    // whether rows list the same columns at the same places: a quarter of the block's
-    // entries against the row below (FZ_HOT of 256: one shared column in 30).  A counter
-    // takes an atomic in 2.5 ns, so small graphs gain nothing (100 x 50: 25 us, 27 if
-    // counted jointly).
-    bool joint = false;
-    if (D.n >= FZ_JOINT_ROWS) {
-        const bool same = e0 + D.k < D.entries && D.idx[e0 + D.k] == col[0];
-        joint = __syncthreads_count(same) >= FZ_HOT;
-    }
+    const bool same = D.n >= FZ_JOINT_ROWS && e0 + D.k < D.entries && D.idx[e0 + D.k] == col[0];
 #pragma unroll
     for (uint32_t q = 0; q < FZ_PER_THREAD; ++q) {
         w[q] = 0.0f;
@@ -144,10 +136,18 @@ __global__ void __launch_bounds__(256) fuzzy_entries_kernel(const FuzzyDev D) {
             } else {
                 w[q] = 1.0f;
             }
-            if (w[q] != 0.0f && !joint) slot[q] = atomicAdd(&D.indeg[col[q]], 1u);
         }
     }
-    if (joint) {
+    // whether rows list the same columns at the same places: a quarter of the block's
+    // entries against the row below (FZ_HOT of 256: one shared column in 30).  A counter
+    // takes an atomic in 2.5 ns, so small graphs gain nothing (100 x 50: 25 us, 27 if
+    // counted jointly).
+    const bool joint = D.n >= FZ_JOINT_ROWS && __syncthreads_count(same) >= FZ_HOT;
+    if (!joint) {
+#pragma unroll
+        for (uint32_t q = 0; q < FZ_PER_THREAD; ++q)
+            if (w[q] != 0.0f) slot[q] = atomicAdd(&D.indeg[col[q]], 1u);
+    } else {
 #pragma unroll
         for (uint32_t q = 0; q < FZ_PER_THREAD; ++q) s_col[256 * q + threadIdx.x] = w[q] != 0.0f ? col[q] : ~0u;
         __syncthreads();

@@ -185,18 +185,20 @@ __device__ __forceinline__ double pair_limit(float dist, double rn_a) {
     return limit_of<METRIC>((double)dist * (1.0 + 0x1p-21) + 1.5 * 0x1p-149, rn_a);
 }
 // The limit of a row whose k-th key is tau_key.  The columns come in ascending order,
-// so a later pair at exactly the k-th distance stays behind it and only a smaller
-// distance counts, a value below the midpoint of tau and the next smaller binary32.
-// Ties are common where points repeat: at distance 0, as all pairs of a zero vector are
-// under cosine, every later pair would be merged for nothing (6,000 x 24, k = 15, 300
-// zero vectors: 1,755 us with ties let through, 1,310 without).  A row that nothing can
-// enter any more (tau 0) has the limit NaN, which no pair reaches; one with fewer than
-// k keys, or an infinite tau, takes every pair.
+// so a later pair at exactly the k-th distance tau stays behind it and only a smaller
+// distance counts: a value of at most tau (1 - 2^-25), which no midpoint between tau and
+// the next smaller binary32 exceeds.  Ties are common where points repeat: at distance
+// 0, as all pairs of a zero vector are under cosine, every later pair would be merged for
+// nothing (6,000 x 24, k = 15, 300 zero vectors: 1,755 us with ties let through, 1,310
+// without).  A row that nothing can enter any more (tau 0) has the limit NaN, which no
+// pair reaches; one with fewer than k keys, or an infinite tau, takes every pair.
 template <int METRIC>
 __device__ __forceinline__ double next_limit(uint64_t tau_key, double rn_a) {
-    const uint32_t bits = min((uint32_t)(tau_key >> 32), 0x7f800000u);  // the distance's; KEY_NONE: infinity
-    const double below = (double)__uint_as_float(bits - 1u), tau = (double)__uint_as_float(bits);
-    return limit_of<METRIC>(0.5 * (below + tau) * (1.0 + 0x1p-50), rn_a);
+    const float f = __uint_as_float(min((uint32_t)(tau_key >> 32), 0x7f800000u));  // (KEY_NONE: infinity)
+    const double tau = (double)(f > 0.0f ? f : __uint_as_float(0x7fffffffu));
+    constexpr double below = (1.0 - 0x1p-25) * (1.0 + 0x1p-49);
+    if (METRIC == HM_METRIC_EUCLIDEAN) return tau * tau * (below * below);  // (tau * tau is exact)
+    return limit_of<METRIC>(tau * below, rn_a);
 }
 
 // Shared memory of one CTA.
