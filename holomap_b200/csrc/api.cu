@@ -114,7 +114,7 @@ struct GroupPlan {
     uint32_t kpl = 1, dmax = 0;
     int metric_mask = 0;
     std::vector<uint32_t> jobs;
-    uint64_t minima = 0, cand = 0, elists = 0;
+    uint64_t cand = 0, elists = 0;
     uint32_t neunits = 0;       // emission units
     std::vector<uint4> eunits;  // their table, largest first (none for one job without symmetric units)
     bool any_sym = false;
@@ -123,7 +123,7 @@ struct GroupPlan {
     bool any_escalation = false;  // a job of the group has a split-BF16 escalation copy
     uint32_t egrid = 0, stage_cap = 0;
     size_t off_opa = 0, off_opb = 0, off_rowstat = 0, off_rowterm = 0, off_colterm = 0;
-    size_t off_band = 0, off_force = 0, off_rowthr = 0, off_cand = 0, off_cnt = 0, off_minima = 0;
+    size_t off_band = 0, off_force = 0, off_rowthr = 0, off_cand = 0, off_cnt = 0;
     size_t off_ethr = 0, off_evstar = 0, off_stage_row = 0, off_stage_key = 0, off_stage_cnt = 0;
     size_t off_rowcnt = 0, off_job_of = 0;
     // tables
@@ -412,9 +412,14 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
             // a sample: points stored cluster by cluster have their neighbours side by
             // side, and a row needs k chunks of its own cluster (rows of 20,000 x 64 in 12
             // clusters, k = 15: 52 candidates a row at 32 columns, 1,665 at 64, more than
-            // the lists hold); chunks of more than 64 columns take several tiles of a part
-            // (and no more scratch than sorted lists of each part's two halves and a
-            // row's binary64 copy took)
+            // the lists hold); chunks of more than 64 columns take several tiles of a part.
+            // The last bound keeps the minima of few columns and small k from outgrowing
+            // what a finer bound is worth (without it 50,000 x 128, k = 10: 1,404 -> 1,468
+            // us, 100,000 x 32, k = 12: 3,900 -> 4,046).
+            // The minima (2 KB a row at most) lie in the job's candidate room (4 KB a row
+            // at least), which is written only when the threshold kernel has read them;
+            // an escalation copy that shares its original's room runs only where the
+            // original has emitted nothing.
             const uint32_t last = std::min(P.seed_tiles, P.col_tiles - (P.parts - 1) * P.part_tiles);
             const uint32_t sampled = P.seed_tiles < P.part_tiles ? (P.parts - 1) * P.seed_tiles + last : 0u;
             const uint32_t limit = std::min<uint32_t>(
@@ -427,8 +432,6 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
                 P.mins = (P.parts - 1) * chunks(P.seed_tiles) + chunks(last);
                 if (P.mins <= limit) break;
             }
-            P.min0 = Gp.minima;
-            Gp.minima += round_up(P.spec.n, 32) * P.mins;
             // Emission pass.  A whole dataset (not a row shard) with at least
             // two column tiles takes the symmetric form: row block rb walks
             // the column tiles from the one holding its own diagonal block
@@ -479,7 +482,9 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
                 if (P.shares_cand) continue;
             }
             P.cand0 = Gp.cand;
-            Gp.cand += P.spec.n * (uint64_t)P.elists * P.cap;
+            // (at least the chunk minima of a job of one or two points: its rows rounded
+            // up to 32, and 64 chunks of the one column tile)
+            Gp.cand += std::max<uint64_t>(P.spec.n * (uint64_t)P.elists * P.cap, 32 * 64 * sizeof(float) / sizeof(uint64_t));
         }
         // emission units of the group: (job slot | sym, row block (2-SM form:
         // block of 256 rows), first tile, end tile | part); a symmetric unit
@@ -628,7 +633,6 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
         Gp.off_rowthr = take(rows * sizeof(uint32_t));
         Gp.off_cand = take(Gp.cand * sizeof(unsigned long long));
         Gp.off_cnt = take(Gp.elists * sizeof(uint32_t));
-        Gp.off_minima = take(Gp.minima * sizeof(float));
         Gp.off_rowcnt = take(rows * sizeof(uint32_t));
         if (Gp.jobs.size() > 1) Gp.off_job_of = take((rows + 31) / 32 * sizeof(uint32_t));
         if (Gp.any_sym) {
@@ -647,6 +651,8 @@ static int plan_batch(const hm_job *user_specs, uint32_t user_jobs, hm_batch &B,
             const int64_t apart = (int64_t)B.groups[O.group].off_cand - (int64_t)B.groups[P.group].off_cand;
             P.cand0 = (uint64_t)((int64_t)O.cand0 + apart / (int64_t)sizeof(unsigned long long));
         }
+    for (JobPlan &P : B.jobs)
+        if (P.group >= 0) P.min0 = (B.groups[P.group].off_cand + P.cand0 * sizeof(unsigned long long)) / sizeof(float);
     B.total = off;
     return HM_OK;
 }
@@ -805,7 +811,7 @@ static int bind_batch(hm_batch &B, void *d_ws, size_t bytes, cudaStream_t s) {
         D.rowthr = at<uint32_t>(ws, Gp.off_rowthr);
         D.cand = at<unsigned long long>(ws, Gp.off_cand);
         D.cand_cnt = at<uint32_t>(ws, Gp.off_cnt);
-        D.minima = at<float>(ws, Gp.off_minima);
+        D.minima = at<float>(ws, 0);
         D.row_cnt = at<uint32_t>(ws, Gp.off_rowcnt);
         D.job_of = Gp.jobs.size() > 1 ? at<uint32_t>(ws, Gp.off_job_of) : nullptr;
         D.eunits = Gp.eunits.empty() ? nullptr : at<uint4>(ws, Gp.off_eunits);

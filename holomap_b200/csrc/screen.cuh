@@ -86,7 +86,8 @@ struct GroupDev {
     uint32_t *rowthr;             // per row, ordered key: tau1, the k-th smallest chunk minimum
     unsigned long long *cand;     // candidate lists, (c^ bits << 32) | job-local column
     uint32_t *cand_cnt;
-    float *minima;                // threshold pass: chunk minima, chunk-major per job
+    float *minima;                // threshold pass: chunk minima, chunk-major per job (the workspace; a
+                                  // job's lie at JobDev::min0, in its candidate room)
     uint32_t *row_cnt;            // rerank: survivors per group row (0: none or exact fallback)
     // emission pass: its work units (x = group job slot | sym << 31, y = row
     // block, z = first column tile, w = end column tile | column part << 24),

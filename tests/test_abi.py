@@ -261,6 +261,16 @@ def test_workspace_stays_within_what_callers_sized_for(n, d, k, metric, path, mo
     assert 0 < got <= most
 
 
+@pytest.mark.parametrize("n,d,k,metric,path,most", [
+    (256920, 262, 5, 1, 0, 2_382_996_480), (200000, 256, 5, 1, 0, 1_733_472_000),
+    (100000, 512, 8, 0, 0, 2_159_938_560), (250000, 128, 10, 0, 0, 4_637_353_984),
+    (50000, 64, 15, 0, 0, 1_295_507_456), (50000, 384, 30, 1, 0, 2_825_822_208)])
+def test_chunk_minima_take_no_room_of_their_own(n, d, k, metric, path, most):
+    """However many minima a row's sample has, they lie where the row's candidates go
+    later: sizes from before a clustered sample got chunks of at most 32 columns."""
+    assert 0 < hm.lib().hm_workspace_bytes(n, d, k, metric, path) <= most
+
+
 @pytest.mark.parametrize("lanes", [1, 4, 8, 16])
 def test_smooth_row_index_up_to_the_largest_call(lanes):
     """The calibration's row index over 2^31 - 1 rows, the largest call: 16 lanes a
